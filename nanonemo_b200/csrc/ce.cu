@@ -169,6 +169,36 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_from_stats_kernel(T* __res
   row_write_grad<T>(x, V >> 3, tgt, lse, valid ? grad_scale : 0.f);
 }
 
+// Row losses of a head product that kept no logits (nnb_gemm_ce_loss): one warp combines the row's tile statistics. It reads
+// n_tiles x 8 bytes a row (3.2 KB at a vocabulary of 50304, 1/32 of the row's logits).
+__global__ void __launch_bounds__(kCeThreads) ce_loss_from_stats_kernel(const float* __restrict__ tile_stats, int n_tiles,
+                                                                        const float* __restrict__ target_logit,
+                                                                        const long long* __restrict__ targets,
+                                                                        float* __restrict__ loss_rows, long long R, int V) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  const long long row = (long long)blockIdx.x * (kCeThreads / 32) + (threadIdx.x >> 5);
+  if (row >= R) return;
+  const int lane = threadIdx.x & 31;
+  const float2* st = reinterpret_cast<const float2*>(tile_stats) + row * n_tiles;
+  float m = -INFINITY, s = 0.f;
+  auto add = [&](float m2, float s2) {
+    const float mn = fmaxf(m, m2);
+    s = (m == -INFINITY ? 0.f : s * exp2f((m - mn) * kLog2e)) + (m2 == -INFINITY ? 0.f : s2 * exp2f((m2 - mn) * kLog2e));
+    m = mn;
+  };
+  for (int i = lane; i < n_tiles; i += 32) {
+    const float2 v = st[i];
+    add(v.x, v.y);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
+    add(m2, s2);
+  }
+  const long long tgt = targets[row];
+  if (lane == 0) loss_rows[row] = tgt >= 0 && tgt < V ? m + logf(s) - target_logit[row] : 0.f;
+}
+
 // Vocabulary-parallel variant, first half: this rank's slice of the row -> stats[row] = (max, sum-exp, target logit or 0).
 // `targets` are GLOBAL ids; this rank owns columns [v0, v0 + V).
 template <typename T>
@@ -253,6 +283,17 @@ extern "C" int nnb_ce_grad_from_stats(void* logits, const void* targets, const v
   return 0;
 }
 
+// loss_rows[r] = logsumexp - target logit from the statistics of nnb_gemm_ce_loss (0 for a target outside [0, V)).
+extern "C" int nnb_ce_loss_from_stats(const void* tile_stats, int n_tiles, const void* target_logit, const void* targets,
+                                      void* loss_rows, long long R, int V, cudaStream_t st) {
+  NNB_REQUIRE(n_tiles > 0 && V > 0 && (reinterpret_cast<uintptr_t>(tile_stats) & 7) == 0, "ce_loss_from_stats: bad statistics");
+  if (R == 0) return 0;
+  constexpr int rows = kCeThreads / 32;
+  ce_loss_from_stats_kernel<<<(unsigned)((R + rows - 1) / rows), kCeThreads, 0, st>>>(
+      (const float*)tile_stats, n_tiles, (const float*)target_logit, (const long long*)targets, (float*)loss_rows, R, V);
+  NNB_LAUNCH_OK("ce_loss_from_stats");
+  return 0;
+}
 
 // Vocabulary-parallel cross-entropy in two launches with one small all-gather of `stats` between them (done by the caller).
 // logits: this rank's [R, V] slice of the row (columns v0 .. v0+V of v_total); targets: global ids.

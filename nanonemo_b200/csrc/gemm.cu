@@ -786,6 +786,16 @@ extern "C" int nnb_gemm_ce_stats(const void* X, const void* W, void* logits, voi
   return nnb_gemm2_launch(g, st);
 }
 
+// The statistics of nnb_gemm_ce_stats without the logits, plus target_logit[m] = the (16-bit rounded) logit of column
+// targets[m] (int64; rows whose target lies outside [0, N) leave theirs unwritten): all that a loss without gradients needs.
+extern "C" int nnb_gemm_ce_loss(const void* X, const void* W, const void* targets, void* stats, void* target_logit, int M, int N, int K,
+                                long long lda, long long ldw, int dtype, void* status, cudaStream_t st) {
+  NnbGemm2Args g{};
+  if (int rc = fused_gemm_common(g, X, W, nullptr, M, N, K, lda, ldw, N, dtype, status)) return rc;
+  g.epilogue = EPI_CE_LOSS; g.stats = stats; g.targets = targets; g.target_logit = target_logit;
+  return nnb_gemm2_launch(g, st);
+}
+
 // GEMM -> reduce-scatter in one kernel (row-parallel linear under tensor + sequence parallelism):
 //   out_shard[rank r] [M / world, N]  +=  (A[M, K] @ B[N, K]^T) rows [r M / world, (r + 1) M / world)   summed over ranks.
 // Every output tile is TMA-reduce-added into the owner's buffer over NVLink as soon as it leaves TMEM, so the

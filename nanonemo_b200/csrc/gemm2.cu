@@ -24,7 +24,11 @@
 //   EPI_CE_STATS  LM head: besides the 16-bit logits, every (row, 256-column tile) gets its (max, sum of exp(x - max)), so
 //                 the cross-entropy kernel needs one sweep over the logits instead of two
 //                 (nanonemo/kernels/triton/linear_ce.py:21-41).
-// All three compute on the values ROUNDED to the 16-bit output type, so they match the unfused kernels bit for bit.
+//   EPI_CE_LOSS   LM head of a loss without gradients (validation): the statistics and the target's logit of every row, and no
+//                 logits at all. Against EPI_CE_STATS + the one-sweep kernel this drops the 16-bit logits' write, read and
+//                 rewrite; the accumulator goes straight from tensor memory to the statistics, so the staging tiles' shared
+//                 memory holds a seventh operand stage instead.
+// All of them compute on the values ROUNDED to the 16-bit output type, so they match the unfused kernels bit for bit.
 #include "gemm2.cuh"
 
 #include "common.cuh"
@@ -43,8 +47,8 @@ constexpr int kTmemCols = 512;
 // The SwiGLU epilogue fills three staging tiles per 64-feature round (gate, up, act); its backward keeps two (gate, up)
 // tile pairs in flight: both pay for the staging with one stage of the operand ring.
 template <int EPI> struct Cfg {
-  static constexpr int kStages = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD) ? 5 : 6;
-  static constexpr int kStagingTiles = EPI == EPI_SWIGLU ? 3 : (EPI == EPI_SWIGLU_BWD ? 4 : 2);
+  static constexpr int kStages = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD) ? 5 : (EPI == EPI_CE_LOSS ? 7 : 6);
+  static constexpr int kStagingTiles = EPI == EPI_SWIGLU ? 3 : (EPI == EPI_SWIGLU_BWD ? 4 : (EPI == EPI_CE_LOSS ? 0 : 2));
   static constexpr int kStagingBytes = kStagingTiles * BM * 128;
   // Epilogue groups of four warps. The SwiGLU backward does the most arithmetic per accumulator element (a sigmoid and both
   // products, operands read from shared memory): two groups take alternate 64-column chunks, each with its own staging
@@ -52,7 +56,7 @@ template <int EPI> struct Cfg {
   // The softmax statistics (an exponential per logit) get the same split, one staging tile per group.
   // (The SwiGLU forward stays with one group: a second one needs six staging tiles, which leaves four operand stages, and
   // measured slower: 0.201 vs 0.182 ms at M = 32768, N = 4096, K = 768.)
-  static constexpr int kEpiGroups = (EPI == EPI_SWIGLU_BWD || EPI == EPI_CE_STATS) ? 2 : 1;
+  static constexpr int kEpiGroups = (EPI == EPI_SWIGLU_BWD || EPI == EPI_CE_STATS || EPI == EPI_CE_LOSS) ? 2 : 1;
   static constexpr int kThreads = 64 + kEpiGroups * kEpilogueThreads;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
@@ -71,6 +75,8 @@ struct Params2 {
   const float* sin_t;
   float* stats;        // EPI_CE_STATS: [M, 2 n_blocks, 2] fp32 (max, sum of exp(x - max)): two entries per 256-column tile (64-column
                        // chunks 0, 2 and 1, 3 of the tile: one entry per epilogue warp group; (-inf, 0) when the group had no chunk)
+  const long long* targets;  // EPI_CE_LOSS: [M]
+  float* target_logit;       // EPI_CE_LOSS: [M]
 };
 
 __device__ __forceinline__ uint32_t pack16(float lo, float hi, bool bf) {
@@ -307,6 +313,10 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       tile_coords(tile, m_pair, n_blk);
       const int d_row = (m_pair * 2 + (int)rank) * BM;
       const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+      long long tgt_col = -1;  // EPI_CE_LOSS: this row's target relative to the tile's first column
+      if constexpr (EPI == EPI_CE_LOSS) {
+        if (d_row + row < p.M) tgt_col = p.targets[d_row + row] - (long long)n_blk * BN;
+      }
       float rope_c[32], rope_s[32];  // EPI_ROPE, head_dim 64: this token's table row, fetched while the tile is still being multiplied
       if constexpr (EPI == EPI_ROPE) {
         if (p.half_dim == 32 && n_blk * BN < p.epi_cols) {
@@ -518,18 +528,20 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int cols_per_chunk = p.out_f32 ? 32 : 64;
         const int chunks = BN / cols_per_chunk;
         constexpr int G = Cfg<EPI>::kEpiGroups;  // with two groups: group g takes chunks g, g + 2 through staging tile g
-        float st_m = -INFINITY, st_s = 0.f;  // EPI_CE_STATS: this row's running (max, sum of exp) over the group's chunks of the tile
+        constexpr bool kStats = EPI == EPI_CE_STATS || EPI == EPI_CE_LOSS, kStore = EPI != EPI_CE_LOSS;
+        float st_m = -INFINITY, st_s = 0.f;  // kStats: this row's running (max, sum of exp) over the group's chunks of the tile
         for (int c = (G == 2 ? grp : 0); c < chunks && rows_live; c += G) {
           const int col0 = c * cols_per_chunk;
           if (n_blk * BN + col0 >= p.N) break;
           uint8_t* buf = staging + (G == 2 ? grp : (int)(gchunk & 1)) * (BM * 128);
           ++gchunk;
-          if (G == 2) {
+          if (!kStore) {
+          } else if (G == 2) {
             if (et == 0 && pending_stores >= 1) tma_wait_group_read<0>();
           } else if (et == 0 && pending_stores >= 2) {
             tma_wait_group_read<1>();
           }
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          if (kStore) named_barrier_sync(epi_bar, kEpilogueThreads);
           uint8_t* my_row = buf + row * 128;
           if (p.out_f32) {
             uint32_t r[32];
@@ -545,7 +557,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             tmem_ld_wait();
             pack32(r0, w0, bf);
             pack32(r1, w1, bf);
-            if constexpr (EPI == EPI_CE_STATS) {
+            if constexpr (kStats) {
               constexpr float kLog2e = 1.4426950408889634f;
               float x[64];
               float cm = -INFINITY;
@@ -562,10 +574,22 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
               const float mb = st_m * kLog2e;
 #pragma unroll
               for (int i = 0; i < 64; ++i) st_s += exp2f(x[i] * kLog2e - mb);
+              if constexpr (EPI == EPI_CE_LOSS) {
+                const long long off = tgt_col - col0;  // one chunk of the whole row holds the target: the branch is rarely taken
+                if (off >= 0 && off < 64) {
+                  float xt = 0.f;
+#pragma unroll
+                  for (int i = 0; i < 64; ++i) xt = i == (int)off ? x[i] : xt;
+                  p.target_logit[d_row + row] = xt;
+                }
+              }
             }
-            stage32(my_row, sw, 0, w0);
-            stage32(my_row, sw, 4, w1);
+            if constexpr (kStore) {
+              stage32(my_row, sw, 0, w0);
+              stage32(my_row, sw, 4, w1);
+            }
           }
+          if constexpr (!kStore) continue;
           fence_proxy_async_smem();
           named_barrier_sync(epi_bar, kEpilogueThreads);
           if (et == 0) {
@@ -575,7 +599,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
           if (pending_stores < 2) ++pending_stores;
         }
-        if constexpr (EPI == EPI_CE_STATS) {
+        if constexpr (kStats) {
           if (rows_live && d_row + row < p.M)
             *reinterpret_cast<float2*>(p.stats + (((size_t)(d_row + row) * p.n_blocks + n_blk) * G + grp) * 2) = make_float2(st_m, st_s);
         }
@@ -664,6 +688,12 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
                 "gemm_rope: head_dim must be 64 or 128, columns whole heads, tables 16-byte aligned");
     p.epi_cols = a.rope_cols; p.t_len = a.t_len; p.half_dim = a.head_dim / 2;
     p.cos_t = static_cast<const float*>(a.cos_t); p.sin_t = static_cast<const float*>(a.sin_t);
+  } else if (EPI == EPI_CE_LOSS) {
+    NNB_REQUIRE(!a.out_f32 && !a.accumulate && a.N % 64 == 0 && a.stats != nullptr && a.targets != nullptr && a.target_logit != nullptr,
+                "gemm_ce_loss: N a multiple of 64, targets and both outputs expected");
+    p.stats = static_cast<float*>(a.stats);
+    p.targets = static_cast<const long long*>(a.targets);
+    p.target_logit = static_cast<float*>(a.target_logit);
   } else if (EPI == EPI_CE_STATS) {
     NNB_REQUIRE(!a.out_f32 && !a.accumulate && a.N % 64 == 0 && a.stats != nullptr, "gemm_ce_stats: 16-bit output with N a multiple of 64 expected");
     p.stats = static_cast<float*>(a.stats);
@@ -711,7 +741,8 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   const int d_bytes = a.out_f32 ? 4 : 2, d_box = a.out_f32 ? 32 : 64;
   // (EPI_SWIGLU_BWD writes d(gate) | d(up): its output, like the projection it reads through tmE, is 2 N columns wide)
   const int d_cols = EPI == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
-  if (!nnb_make_tmap_2d(&tmD, d_dt, d_bytes, a.D, a.M, d_cols, a.ldd * d_bytes, BM, d_box, "gemm2 D")) return -4;
+  if (EPI == EPI_CE_LOSS) tmD = tmA;  // nothing is stored
+  else if (!nnb_make_tmap_2d(&tmD, d_dt, d_bytes, a.D, a.M, d_cols, a.ldd * d_bytes, BM, d_box, "gemm2 D")) return -4;
   tmE = tmD;
   if (EPI == EPI_SWIGLU_BWD && !nnb_make_tmap_2d(&tmE, in_dt, 2, a.E, a.M, 2 * a.N, a.lde * 2, BM, 64, "gemm2 gate|up")) return -4;
   if (EPI == EPI_SWIGLU && !nnb_make_tmap_2d(&tmE, in_dt, 2, a.E, a.M, a.N / 2, a.lde * 2, BM, 64, "gemm2 act")) return -4;
@@ -736,6 +767,7 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st) {
     case EPI_ROPE: return NNB_LAUNCH2(EPI_ROPE);
     case EPI_CE_STATS: return NNB_LAUNCH2(EPI_CE_STATS);
     case EPI_SWIGLU_BWD: return NNB_LAUNCH2(EPI_SWIGLU_BWD);
+    case EPI_CE_LOSS: return NNB_LAUNCH2(EPI_CE_LOSS);
 #undef NNB_LAUNCH2
     default: nnb_set_error("gemm2: unknown epilogue %d", a.epilogue); return -1;
   }

@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 
 // Work fused into the epilogue while a tile leaves tensor memory (see gemm2.cu).
-enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4 };
+enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4, EPI_CE_LOSS = 5 };
 
 struct NnbGemm2Args {
   const void *A, *B;
@@ -27,6 +27,10 @@ struct NnbGemm2Args {
   // EPI_CE_STATS: fp32 [M, 2 ceil(N / 256), 2] receiving (max, sum of exp(x - max)) of every row's logits in two parts per
   // 256-column tile (the tile's even and odd 64-column chunks); a part without columns holds (-inf, 0)
   void* stats = nullptr;
+  // EPI_CE_LOSS: the same statistics without the logits (D is not written); target_logit[m] fp32 receives the logit of column
+  // targets[m] (int64) and is left alone where that column does not exist
+  const void* targets = nullptr;
+  void* target_logit = nullptr;
 };
 
 // Returns 0 on success, 1 when the shape is not served by the pair kernel (caller falls back), < 0 on error.

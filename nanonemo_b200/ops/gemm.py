@@ -136,6 +136,21 @@ def gemm_ce_stats(x2: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
     return stats if ok else None
 
 
+def gemm_ce_loss(x2: torch.Tensor, w: torch.Tensor, targets: torch.Tensor):
+    """The statistics of ``gemm_ce_stats`` without the logits, and the logit of every row's target ->
+    (stats fp32 [M, 2 ceil(N / 256), 2], target_logit fp32 [M], unwritten where the target is no column) or None."""
+    M, K = x2.shape
+    N = w.shape[0]
+    if M < 256 or N < 128 or N % 64:
+        return None
+    stats = torch.empty((M, 2 * ((N + 255) // 256), 2), dtype=torch.float32, device=x2.device)
+    target_logit = torch.empty(M, dtype=torch.float32, device=x2.device)
+    ok = _fused_call("nnb_gemm_ce_loss", _lib.ptr(x2), _lib.ptr(w), _lib.ptr(targets), _lib.ptr(stats), _lib.ptr(target_logit),
+                     _lib.i32(M), _lib.i32(N), _lib.i32(K), _lib.i64(x2.stride(0)), _lib.i64(w.stride(0)), _lib.i32(_CODE[x2.dtype]),
+                     _lib.ptr(status_tensor(x2.device)), _lib.vp(_lib.stream_ptr()))
+    return (stats, target_logit) if ok else None
+
+
 def compute_dtype() -> torch.dtype:
     if torch.is_autocast_enabled("cuda"):
         dt = torch.get_autocast_dtype("cuda")

@@ -13,7 +13,7 @@ waves; the reference uses 512-row chunks on 8 GB parts).
 import torch
 
 from nanonemo_b200.ops import _lib
-from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_stats, shadow_of
+from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_loss, gemm_ce_stats, shadow_of
 
 DEFAULT_CHUNK_ROWS = 32768
 
@@ -59,6 +59,28 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     return loss_rows.sum(), dx
 
 
+def linear_ce_loss(x16, w16, targets, chunk_rows):
+    """Sum of row losses [fp32 scalar] when nobody asks for gradients (validation): one product per chunk instead of three, and
+    its logits are reduced to softmax statistics before they leave the tensor core's accumulator."""
+    N, V = x16.shape[0], w16.shape[0]
+    loss_rows = torch.empty(N, dtype=torch.float32, device=x16.device)
+    for r0 in range(0, N, chunk_rows):
+        xc, tg = x16[r0:r0 + chunk_rows], targets[r0:r0 + chunk_rows]
+        rows = loss_rows[r0:r0 + chunk_rows]
+        got = gemm_ce_loss(xc, w16, tg) if FUSE_STATS else None
+        if got is None:  # the CTA-pair kernel does not serve the shape
+            ce_inplace(gemm(xc, w16), tg, rows, 1.0 / N)
+            continue
+        stats, target_logit = got
+        _lib.call("nnb_ce_loss_from_stats", _lib.ptr(stats), _lib.i32(stats.shape[1]), _lib.ptr(target_logit), _lib.ptr(tg),
+                  _lib.ptr(rows), _lib.i64(xc.shape[0]), _lib.i32(V), _lib.vp(_lib.stream_ptr()))
+    return loss_rows.sum()
+
+
+def needs_grad(x, weight) -> bool:
+    return torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
+
+
 class _LinearCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, targets, chunk_rows):
@@ -68,7 +90,6 @@ class _LinearCE(torch.autograd.Function):
         x16 = x16 if x16.is_contiguous() else x16.contiguous()
         tg = targets if targets.dtype == torch.int64 else targets.long()
         tg = tg if tg.is_contiguous() else tg.contiguous()
-        need_grad = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
         dW = torch.zeros(weight.shape, dtype=torch.float32, device=x.device)
         loss_sum, dx = linear_ce_fwd(x16, w16, tg, chunk_rows or DEFAULT_CHUNK_ROWS, dW)
         ctx.save_for_backward(dx, dW, weight)
@@ -91,6 +112,10 @@ class _LinearCE(torch.autograd.Function):
 
 def linear_cross_entropy(x, weight, targets, chunk_rows=None):
     """x: [N, D]; weight: [V, D] (fp32 master or 16-bit); targets: [N] int64 -> scalar mean loss (fp32)."""
+    if not needs_grad(x, weight):
+        dt = compute_dtype()
+        loss = linear_ce_loss(x.to(dt).contiguous(), shadow_of(weight, dt), targets.long().contiguous(), chunk_rows or DEFAULT_CHUNK_ROWS)
+        return loss / x.shape[0]
     return _LinearCE.apply(x, weight, targets, chunk_rows)
 
 

@@ -30,6 +30,29 @@ def test_linear_ce_loss_and_grads(N, D, V, chunk):
         assert err <= 3e-2 * want.abs().max().item() + 1e-5, err
 
 
+@pytest.mark.parametrize("N,D,V,chunk", [(256, 64, 128, None), (300, 256, 1088, None), (1000, 768, 50304, 384), (130, 64, 520, 64), (513, 128, 4160, 257)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_loss_without_gradients_equals_the_loss_with_them(N, D, V, chunk, dtype):
+    """Rows that are no multiple of a tile, a last tile of one chunk, targets in the first and last column, ignored rows.
+    The same rounded logits go into both; only the order of an fp32 sum of at most 394 terms differs (1e-5 of the loss)."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(N)
+    x = (torch.randn(N, D, device=DEV) * 2).to(dtype)
+    w = torch.randn(V, D, device=DEV) * 0.2
+    t = torch.randint(0, V, (N,), device=DEV)
+    t[0], t[1], t[2], t[3] = 0, V - 1, -100, V
+    with torch.autocast("cuda", dtype=dtype):
+        plain = ops.linear_cross_entropy(x, w, t, chunk_rows=chunk)
+        with torch.no_grad():
+            quiet = ops.linear_cross_entropy(x.requires_grad_(), w, t, chunk_rows=chunk)
+        full = ops.linear_cross_entropy(x, w, t, chunk_rows=chunk)
+    check_status()
+    assert full.requires_grad and not plain.requires_grad and torch.equal(plain, quiet)
+    torch.testing.assert_close(plain, full.detach(), rtol=1e-5, atol=0)
+
+
 @pytest.mark.parametrize("world", [1, 2, 4])
 def test_vocab_parallel_linear_ce_over_emulated_ranks(world):
     """Every 'rank' holds V/world rows of the head; the stats exchange is emulated by running the ranks' first halves,
