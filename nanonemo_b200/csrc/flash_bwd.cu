@@ -14,22 +14,29 @@
 // MN-major (dK, dV) without any transposed copy. dQ partial tiles leave through a swizzled fp32
 // staging tile and a TMA reduce-add (cp.reduce.async.bulk.tensor .add.f32) into an fp32 buffer that a
 // small kernel converts at the end. D = rowsum(dO * O) is a pre-pass kernel in this file.
-// 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 compute: two threads per query row,
+// 512 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4..7 drain dQ, warps 8..15 compute: two threads per query row,
 // one for keys 0..63 of the tile and one for keys 64..127 (same TMEM lanes, different columns).
 //
 // Software pipeline. The score tile is double buffered in tensor memory (S0 | S1 | dP | dV | dK = 512 columns; the dQ
 // partial product of a visit is accumulated into the first 64 columns of THAT visit's S buffer, which is free once P has
-// been computed from it), and the compute work of a visit is split into  A: P = exp(S scale - L)  /  B: dS = P (dP - D) scale,
-// with the dQ drain of the PREVIOUS visit between them. The tensor core then always has work that does not depend on the
-// phase the compute warps are in:
-//     compute :  A(n)          drain dQ(n-1)     B(n)                    A(n+1)   ...
-//     tensor  :        dV(n)               S(n+1)      dK(n) dQ(n) dP(n+1)
-// S(n+1) is ready long before A(n+1) starts, dP(n+1) before B(n+1), dQ(n) before its drain, so neither side waits for the
-// other in steady state; a visit costs about the compute warps' own work instead of the sum of all phases.
+// been computed from it). The compute warps only do  A: P = exp(S scale - L)  and  B: dS = P (dP - D) scale;  the dQ tile
+// leaves through four warps of its own, and a visit's L and D are fetched one visit ahead:
+//     compute :  A(n)                    B(n)                     A(n+1)   ...
+//     tensor  :        S(n+1)   dV(n)          dQ(n) dK(n) dP(n+1)
+//     drain   :  dQ(n-1)                                          dQ(n)
+// S(n+1) needs only the drained buffer, so it is issued before dV(n) and is complete long before A(n+1); dP(n+1) before
+// B(n+1). No block barrier is left in the loop: the compute warps meet the tensor core through mbarriers alone.
+// What bounded a visit, by clock counters of one thread per role (cycles, B8 H12/4 T4096): with dQ drained by the compute warps
+// and the L / D loads in their chain 4286 (wait for S and the loads 890, A 1531, drain 949, wait for dP 206, B 709), and the one-lane
+// MMA issuer needed 2760 for the 32 products of a visit, up to 115 each, because every descriptor had to be moved to a uniform
+// register. Now the visit is about 3180: A 1700 (1024 of it the exponentials on the special-function unit), B 770, and the products
+// issue in 1780 (about 1660 at the tensor core's rate). What is left is A's latency and shared memory: 368 KB a visit, 2900 cycles.
+// Whole backward at T4096: 950 -> 696 us, at B32 T1024 360 -> 299 us (of which 50 are the two elementwise kernels).
 // All waits are bounded.
 #include <cstdlib>
 #include <type_traits>
 
+#define NNB_PROF_THREAD 256  // a compute thread
 #include "sm100.cuh"
 
 namespace {
@@ -37,8 +44,12 @@ namespace {
 using namespace sm100;
 
 constexpr int BQ = 128, BKV = 128, HD = 64;
-constexpr int kThreads = 320;           // TMA warp, MMA warp, 2 x 4 compute warps
-constexpr int kComputeThreads = 256;
+// Four warpgroups: TMA + MMA issuers (and two idle warps), drain, 2 x compute. The block is launched with 512 x 128 registers; the
+// compute warps keep 64 probabilities each and need more, so the others hand registers over: 104 + 104 + 2 x 152 = 4 x 128.
+constexpr int kThreads = 512;
+constexpr int kComputeThreads = 256, kDrainThreads = 128;
+constexpr int kDrainWarp0 = 4, kComputeWarp0 = 8;
+constexpr int kRegsIssue = 104, kRegsDrain = 104, kRegsCompute = 152;
 constexpr int kTile16 = 128 * 64 * 2;     // a [128 x 64] 16-bit tile = 16 KB
 constexpr int kStagesQ = 3;             // a stage is released when dK / dQ of its visit are done and refilled two visits ahead
 // shared memory map (bytes)
@@ -75,11 +86,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBars);
-  // barriers: kv_full, q_full[3], q_empty[3], s_full[2], dp_full, p_written, ds_written, dq_full, dq_read
+  // barriers: kv_full, q_full[3], q_empty[3], s_full[2], dp_full, p_written, ds_written, dq_full, dq_read, p_free, all_done
   const uint32_t bar_kv = smem_u32(bars), bar_qf = bar_kv + 8, bar_qe = bar_qf + 8 * kStagesQ;
   const uint32_t bar_s = bar_qe + 8 * kStagesQ, bar_dp = bar_s + 16, bar_p = bar_dp + 8, bar_ds = bar_p + 8;
-  const uint32_t bar_dq = bar_ds + 8, bar_dqr = bar_dq + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kStagesQ + 7);
+  const uint32_t bar_dq = bar_ds + 8, bar_dqr = bar_dq + 8, bar_pf = bar_dqr + 8, bar_fin = bar_pf + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kStagesQ + 9);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -103,7 +114,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     mbar_init(bar_p, kComputeThreads);
     mbar_init(bar_ds, kComputeThreads);
     mbar_init(bar_dq, 1);
-    mbar_init(bar_dqr, kComputeThreads);
+    mbar_init(bar_dqr, kDrainThreads);
+    mbar_init(bar_pf, 1);
+    mbar_init(bar_fin, 1);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -118,9 +131,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   int fail_role = 0;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+  if (warp < kDrainWarp0) {
+    regs_dec<kRegsIssue>();
+    if (warp == 0 && lane == 0) {
+      // ---------------------------------------------------------------- TMA producer
       mbar_expect_tx(bar_kv, 2 * kTile16);
       tma_load_4d(s_base + kOffK, &tmK, bar_kv, 0, kvh, kt * BKV, b);
       tma_load_4d(s_base + kOffV, &tmV, bar_kv, 0, kvh, kt * BKV, b);
@@ -134,202 +148,232 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tma_load_4d(dst + kTile16, &tmdO, bar_qf + 8 * s, 0, hq, qt * BQ, b);
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (warp == 1) {
+      // ---------------------------------------------------------------- MMA issuer (warp-uniform: see umma_f16_elect)
+      const bool el = elect_one();
       bool ok = mbar_wait(bar_kv, 0, abort_flag);
       const uint32_t sK = s_base + kOffK, sV = s_base + kOffV, sP = s_base + kOffP, sdS = s_base + kOffdS;
-      auto stage_of = [&](int n) { return s_base + kOffQdO + (uint32_t)(n % kStagesQ) * 2 * kTile16; };
-      auto wait_q = [&](int n) { return mbar_wait(bar_qf + 8 * (n % kStagesQ), (n / kStagesQ) & 1, abort_flag); };
+      // ring positions of visits n (cur) and n + 1 (nxt) and the phase of nxt, counted along instead of divided out
+      uint32_t cur = 0, nxt = 0, nxt_ph = 0;
+      auto stage_at = [&](uint32_t s) { return s_base + kOffQdO + s * 2 * kTile16; };
       // S(n) = Q K^T into score buffer n & 1 (K-major operands, 4 k-steps of 16 over head_dim)
-      auto issue_s = [&](int n) {
-        const uint32_t sQ = stage_of(n);
+      auto issue_s = [&](int n, uint32_t s) {
+        const uint32_t sQ = stage_at(s);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_f16(tmem_base + kColS + (n & 1) * BKV, make_smem_desc(sQ + k * 32, 16, 1024), make_smem_desc(sK + k * 32, 16, 1024), p.idesc_s, k > 0);
-        umma_commit(bar_s + 8 * (n & 1));
+          umma_f16_elect(el, tmem_base + kColS + (n & 1) * BKV, make_smem_desc(sQ + k * 32, 16, 1024), make_smem_desc(sK + k * 32, 16, 1024), p.idesc_s, k > 0);
+        umma_commit_elect(el, bar_s + 8 * (n & 1));
       };
       // dP(n) = dO V^T
-      auto issue_dp = [&](int n) {
-        const uint32_t sdO = stage_of(n) + kTile16;
+      auto issue_dp = [&](uint32_t s) {
+        const uint32_t sdO = stage_at(s) + kTile16;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_f16(tmem_base + kColdP, make_smem_desc(sdO + k * 32, 16, 1024), make_smem_desc(sV + k * 32, 16, 1024), p.idesc_s, k > 0);
-        umma_commit(bar_dp);
+          umma_f16_elect(el, tmem_base + kColdP, make_smem_desc(sdO + k * 32, 16, 1024), make_smem_desc(sV + k * 32, 16, 1024), p.idesc_s, k > 0);
+        umma_commit_elect(el, bar_dp);
       };
       if (ok && iters > 0) {
-        ok = wait_q(0);
+        ok = mbar_wait(bar_qf, 0, abort_flag);
         if (ok) {
           tc_fence_after();
-          issue_s(0);
+          issue_s(0, 0);
           issue_dp(0);
         }
       }
       for (int n = 0; n < iters && ok; ++n) {
-        const uint32_t sQ = stage_of(n), sdO = sQ + kTile16;
+        const uint32_t sQ = stage_at(cur), sdO = sQ + kTile16;
+        if (++nxt == kStagesQ) { nxt = 0; nxt_ph ^= 1; }
+        // S(n + 1) goes into the other score buffer, whose scores were read before bar_p(n - 1) and whose first columns held
+        // dQ(n - 1): wait until that was drained. (Waited for in every visit, so that bar_dq is never two phases ahead of the drain.)
+        if (n >= 1 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }
+        if (n + 1 < iters) {
+          if (!mbar_wait(bar_qf + 8 * nxt, nxt_ph, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          issue_s(n + 1, nxt);
+        }
         if (!mbar_wait(bar_p, n & 1, abort_flag)) { ok = false; break; }     // P(n) is in shared memory, S(n) has been read
         tc_fence_after();
         // dV += P^T dO: A = [query][key] tile read MN-major (M = keys: two 64-key groups 16 KB apart), B = [query][hd]
         // tile read MN-major; 8 k-steps of 16 query rows (2048 bytes each).
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k)
-          umma_f16(tmem_base + kColdV, make_smem_desc(sP + k * 2048, kTile16, 1024), make_smem_desc(sdO + k * 2048, kTile16, 1024),
+          umma_f16_elect(el, tmem_base + kColdV, make_smem_desc(sP + k * 2048, kTile16, 1024), make_smem_desc(sdO + k * 2048, kTile16, 1024),
                    p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
-        if (n + 1 < iters) {
-          // S(n + 1) goes into the other score buffer, whose first columns held dQ(n - 1): wait until that was drained.
-          // Its commit also covers dV(n) above, so P may be overwritten as soon as S(n + 1) is seen complete.
-          if (n >= 1 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }
-          if (!wait_q(n + 1)) { ok = false; break; }
-          tc_fence_after();
-          issue_s(n + 1);
-        }
+        umma_commit_elect(el, bar_pf);   // P may be overwritten
         if (!mbar_wait(bar_ds, n & 1, abort_flag)) { ok = false; break; }    // dS(n) is in shared memory, dP(n) has been read
         tc_fence_after();
-        // dK += dS^T Q (operands as for dV)
-#pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          umma_f16(tmem_base + kColdK, make_smem_desc(sdS + k * 2048, kTile16, 1024), make_smem_desc(sQ + k * 2048, kTile16, 1024),
-                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
         // dQ(n) = dS K into the score buffer of this visit: A = dS K-major over keys (two 64-key blocks), B = K tile read
         // MN-major (16 key rows per step)
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k)
-          umma_f16(tmem_base + kColdQ + (n & 1) * BKV, make_smem_desc(sdS + (k / 4) * kTile16 + (k % 4) * 32, 16, 1024),
+          umma_f16_elect(el, tmem_base + kColdQ + (n & 1) * BKV, make_smem_desc(sdS + (k / 4) * kTile16 + (k % 4) * 32, 16, 1024),
                    make_smem_desc(sK + k * 2048, kTile16, 1024), p.idesc_dq, k > 0);
-        umma_commit(bar_dq);
-        umma_commit(bar_qe + 8 * (n % kStagesQ));
-        if (n + 1 < iters) issue_dp(n + 1);   // dP(n) was consumed (bar_ds), Q / dO of visit n + 1 were awaited above
+        umma_commit_elect(el, bar_dq);        // before dK(n): the drain runs beside dK(n) and dP(n + 1)
+        // dK += dS^T Q (operands as for dV)
+#pragma unroll
+        for (int k = 0; k < BQ / 16; ++k)
+          umma_f16_elect(el, tmem_base + kColdK, make_smem_desc(sdS + k * 2048, kTile16, 1024), make_smem_desc(sQ + k * 2048, kTile16, 1024),
+                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
+        umma_commit_elect(el, bar_qe + 8 * cur);
+        if (n + 1 < iters) issue_dp(nxt);   // dP(n) was consumed (bar_ds), Q / dO of visit n + 1 were awaited above
+        else umma_commit_elect(el, bar_fin);            // one-shot: every product has been accumulated
+        cur = nxt;
       }
-      if (!ok) fail_role = 2;
+      if (!ok && lane == 0) fail_role = 2;
     }
+  } else if (warp < kComputeWarp0) {
+    regs_dec<kRegsDrain>();
+    // ------------------------------------------------------------------ drain warps: the dQ partial tile of every visit
+    // TMEM (score buffer m & 1) -> swizzled fp32 staging (two [128 x 32] boxes) -> TMA reduce-add into the fp32 accumulator
+    const int row = (warp & 3) * 32 + lane, sw = row & 7;
+    const bool leader = warp == kDrainWarp0 && lane == 0;
+    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColdQ;
+    uint8_t* my_stage = smem + kOffStage + row * 128;
+    int hq = kvh * p.group, qt = first_qt;
+    for (int m = 0; m < iters; ++m) {
+      const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
+      tc_fence_after();
+      if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
+      if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }  // all leave together
+      uint32_t r0[32], r1[32];
+      tmem_ld_32x32b_x32(t_row + (m & 1) * BKV, r0);
+      tmem_ld_32x32b_x32(t_row + (m & 1) * BKV + 32, r1);
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(bar_dqr);
+#pragma unroll
+      for (int jj = 0; jj < 8; ++jj) {
+        *reinterpret_cast<uint4*>(my_stage + ((jj ^ sw) << 4)) = make_uint4(r0[4 * jj], r0[4 * jj + 1], r0[4 * jj + 2], r0[4 * jj + 3]);
+        *reinterpret_cast<uint4*>(my_stage + kTile16 + ((jj ^ sw) << 4)) = make_uint4(r1[4 * jj], r1[4 * jj + 1], r1[4 * jj + 2], r1[4 * jj + 3]);
+      }
+      fence_proxy_async_smem();
+      named_barrier_sync(1, kDrainThreads);
+      if (leader) {
+        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage, 0, hq, qt * BQ, b);
+        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage + kTile16, 32, hq, qt * BQ, b);
+        tma_commit_group();
+      }
+      if (++qt == p.n_q_tiles) { qt = first_qt; ++hq; }
+    }
+    if (leader) tma_wait_group<0>();
   } else {
+    regs_inc<kRegsCompute>();
     // ------------------------------------------------------------------ compute warps (two threads per query row)
-    const int half = (warp - 2) >> 2;          // 0: keys 0..63 / dQ columns 0..31 / dV; 1: keys 64..127 / dQ columns 32..63 / dK
+    const int half = (warp - kComputeWarp0) >> 2;  // 0: keys 0..63 / dV; 1: keys 64..127 / dK
     const int q = warp & 3, row = q * 32 + lane, sw = row & 7;
     const bool leader = half == 0 && row == 0;
     const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
     uint8_t* my_p = smem + kOffP + half * kTile16 + row * 128;
     uint8_t* my_ds = smem + kOffdS + half * kTile16 + row * 128;
-    uint8_t* my_stage = smem + kOffStage + half * kTile16 + row * 128;
     const int key0 = kt * BKV + half * 64;
     bool ok = true;
     NNB_PROF_DECL;
     constexpr float kLog2e = 1.4426950408889634f;
-    // dQ partial tile of visit m: TMEM (score buffer m & 1) -> swizzled fp32 staging (one [128 x 32] box per half) -> TMA
-    // reduce-add. Every compute thread runs it, good or bad, so the two block barriers inside always see all 256 threads.
-    auto drain_dq = [&](int m) {
-      const int hq = kvh * p.group + m / n_qt, qt = first_qt + m % n_qt;
-      if (ok && !mbar_wait(bar_dq, m & 1, abort_flag)) ok = false;
-      tc_fence_after();
-      if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
-      if (named_barrier_or(1, kComputeThreads, !ok)) ok = false;
-      if (ok) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(t_lane + kColdQ + (m & 1) * BKV + half * 32, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
-          *reinterpret_cast<uint4*>(my_stage + ((jj ^ sw) << 4)) = make_uint4(r[4 * jj], r[4 * jj + 1], r[4 * jj + 2], r[4 * jj + 3]);
-      }
-      tc_fence_before();
-      mbar_arrive(bar_dqr);
-      fence_proxy_async_smem();
-      named_barrier_sync(1, kComputeThreads);
-      if (leader && ok) {
-        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage, 0, hq, qt * BQ, b);
-        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage + kTile16, 32, hq, qt * BQ, b);
-        tma_commit_group();
+    // L and D of this thread's query row, fetched one visit ahead: their latency hides behind a whole visit
+    float L_next = 0.f, D_next = 0.f;
+    int qt = first_qt, qt_next = first_qt;
+    const float* stat_L = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T + row;
+    const float* stat_D = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T + row;
+    auto fetch_ld = [&]() {  // of the visit at qt_next, and steps to the one after it
+      const bool live = qt_next * BQ + row < p.T;
+      L_next = live ? __ldg(stat_L + qt_next * BQ) : 0.f;
+      D_next = live ? __ldg(stat_D + qt_next * BQ) : 0.f;
+      if (++qt_next == p.n_q_tiles) {
+        qt_next = first_qt;
+        stat_L += p.T;
+        stat_D += p.T;
       }
     };
-    for (int n = 0; n < iters; ++n) {
+    fetch_ld();
+    const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    for (int n = 0; n < iters && ok; ++n) {
       NNB_PROF_T0;
-      const int hq = kvh * p.group + n / n_qt, qt = first_qt + n % n_qt;
       const int qi = qt * BQ + row;
       const bool row_ok = qi < p.T;
-      const size_t stat = ((size_t)b * p.H + hq) * p.T + (row_ok ? qi : 0);
-      const float L = row_ok ? p.lse[stat] * kLog2e : 0.f;
-      const float D = row_ok ? p.delta[stat] : 0.f;
+      const float L = L_next * kLog2e, Ds = D_next * p.scale;
+      const uint64_t nL2 = pack_f32x2(-L, -L), nDs2 = pack_f32x2(-Ds, -Ds);
+      if (n + 1 < iters) fetch_ld();
       // Only tiles on the diagonal, past the end of the sequence, or with padded query rows need the
       // per-element mask; every other tile takes the branch-free version.
       const bool need_mask = key0 + 63 > qt * BQ || key0 + 63 >= p.T || qt * BQ + BQ > p.T;
-      const float Ds = D * p.scale;
       const uint32_t t_s = t_lane + kColS + (n & 1) * BKV + half * 64;
       float prob[64];  // P of this thread's 64 keys, kept in fp32 from phase A to phase B
       // ---- phase A: P = exp2(S scale log2e - L log2e)
-      if (ok && !mbar_wait(bar_s + 8 * (n & 1), (n >> 1) & 1, abort_flag)) ok = false;
+      if (!mbar_wait(bar_s + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (n > 0 && !mbar_wait(bar_pf, (n - 1) & 1, abort_flag)) { ok = false; break; }  // dV(n - 1) has read P
       tc_fence_after();
       NNB_PROF_ADD(0);
       auto phase_a = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
+        uint32_t rs[2][16];  // 16 columns at a time, the next load in flight while these are worked on
+        tmem_ld_32x32b_x16(t_s, rs[0]);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t rs[32], pk[16];
-          tmem_ld_32x32b_x32(t_s + c * 32, rs);
-          tmem_ld_wait();
+        for (int c = 0; c < 4; ++c) {
+          tmem_ld_wait(rs[c & 1]);
+          if (c < 3) tmem_ld_32x32b_x16(t_s + (c + 1) * 16, rs[(c + 1) & 1]);
+          uint32_t pk[8];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float pr = exp2f(__uint_as_float(rs[i]) * p.scale_log2 - L);
+          for (int i = 0; i < 16; i += 2) {
+            const uint64_t s2 = pack_f32x2(__uint_as_float(rs[c & 1][i]), __uint_as_float(rs[c & 1][i + 1]));
+            const float2 e = unpack_f32x2(fma_f32x2(s2, scale_log2_2, nL2));
+            float p0 = exp2f(e.x), p1 = exp2f(e.y);
             if (kMask) {
-              const int key = key0 + c * 32 + i;
-              pr = (row_ok && key <= qi && key < p.T) ? pr : 0.f;
+              const int key = key0 + c * 16 + i;
+              p0 = (row_ok && key <= qi && key < p.T) ? p0 : 0.f;
+              p1 = (row_ok && key + 1 <= qi && key + 1 < p.T) ? p1 : 0.f;
             }
-            prob[c * 32 + i] = pr;
+            prob[c * 16 + i] = p0;
+            prob[c * 16 + i + 1] = p1;
+            pk[i >> 1] = pack2_16<F16>(p0, p1);
           }
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            pk[i >> 1] = pack2_16<F16>(prob[c * 32 + i], prob[c * 32 + i + 1]);
-          }
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj)
-            *reinterpret_cast<uint4*>(my_p + (((c * 4 + jj) ^ sw) << 4)) = make_uint4(pk[4 * jj], pk[4 * jj + 1], pk[4 * jj + 2], pk[4 * jj + 3]);
+          for (int jj = 0; jj < 2; ++jj)
+            *reinterpret_cast<uint4*>(my_p + (((c * 2 + jj) ^ sw) << 4)) = make_uint4(pk[4 * jj], pk[4 * jj + 1], pk[4 * jj + 2], pk[4 * jj + 3]);
         }
       };
-      if (ok) {
-        if (need_mask) phase_a(std::true_type{});
-        else phase_a(std::false_type{});
-      }
+      if (need_mask) phase_a(std::true_type{});
+      else phase_a(std::false_type{});
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(bar_p);
       NNB_PROF_ADD(1);
-      // ---- the previous visit's dQ leaves while the tensor core works on dV(n) and S(n + 1)
-      if (n > 0) drain_dq(n - 1);
-      NNB_PROF_ADD(2);
       // ---- phase B: dS = P (dP scale - D scale)
-      if (ok && !mbar_wait(bar_dp, n & 1, abort_flag)) ok = false;
+      // (dP(n) was issued after dK(n - 1) and dQ(n - 1): once it is complete they have read dS)
+      if (!mbar_wait(bar_dp, n & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      NNB_PROF_ADD(3);
-      if (ok) {
+      NNB_PROF_ADD(2);
+      uint32_t rp[2][16];
+      tmem_ld_32x32b_x16(t_lane + kColdP + half * 64, rp[0]);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t rp[32], dk[16];
-          tmem_ld_32x32b_x32(t_lane + kColdP + half * 64 + c * 32, rp);
-          tmem_ld_wait();
+      for (int c = 0; c < 4; ++c) {
+        tmem_ld_wait(rp[c & 1]);
+        if (c < 3) tmem_ld_32x32b_x16(t_lane + kColdP + half * 64 + (c + 1) * 16, rp[(c + 1) & 1]);
+        uint32_t dk[8];
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float d0 = prob[c * 32 + i] * (__uint_as_float(rp[i]) * p.scale - Ds);
-            const float d1 = prob[c * 32 + i + 1] * (__uint_as_float(rp[i + 1]) * p.scale - Ds);
-            dk[i >> 1] = pack2_16<F16>(d0, d1);
-          }
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj)
-            *reinterpret_cast<uint4*>(my_ds + (((c * 4 + jj) ^ sw) << 4)) = make_uint4(dk[4 * jj], dk[4 * jj + 1], dk[4 * jj + 2], dk[4 * jj + 3]);
+        for (int i = 0; i < 16; i += 2) {
+          const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c & 1][i]), __uint_as_float(rp[c & 1][i + 1])), scale2, nDs2);
+          const float2 d = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i], prob[c * 16 + i + 1]), t));
+          dk[i >> 1] = pack2_16<F16>(d.x, d.y);
         }
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj)
+          *reinterpret_cast<uint4*>(my_ds + (((c * 2 + jj) ^ sw) << 4)) = make_uint4(dk[4 * jj], dk[4 * jj + 1], dk[4 * jj + 2], dk[4 * jj + 3]);
       }
       fence_proxy_async_smem();
       tc_fence_before();
       mbar_arrive(bar_ds);
-      NNB_PROF_ADD(4);
-      if (named_barrier_or(2, kComputeThreads, !ok)) { ok = false; fail_role = 3; break; }  // all leave together
+      if (++qt == p.n_q_tiles) qt = first_qt;
+      NNB_PROF_ADD(3);
     }
-    if (iters > 0) drain_dq(iters - 1);
-    if (!ok && fail_role == 0) fail_role = 3;
+    if (ok && iters > 0 && !mbar_wait(bar_fin, 0, abort_flag)) ok = false;
+    tc_fence_after();
+    if (named_barrier_or(2, kComputeThreads, !ok)) {  // all leave together
+      ok = false;
+      fail_role = 3;
+    }
     NNB_PROF_FLUSH_N(iters);
     // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the P / dS tiles) -> TMA store
     if (ok && iters > 0) {
-      // bar_dq of the last visit was awaited above, so every MMA (including dV / dK accumulation) has completed
-      if (leader) tma_wait_group_read<0>();
-      named_barrier_sync(1, kComputeThreads);
       uint8_t* dst = (half == 0 ? smem + kOffP : smem + kOffdS) + row * 128;
       uint32_t r0[32], r1[32];
       tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
@@ -362,7 +406,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         *reinterpret_cast<uint4*>(dst + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
       fence_proxy_async_smem();
-      named_barrier_sync(1, kComputeThreads);
+      named_barrier_sync(2, kComputeThreads);
       if (leader) {
         tma_store_4d(&tmdV, s_base + kOffP, 0, kvh, kt * BKV, b);
         tma_store_4d(&tmdK, s_base + kOffdS, 0, kvh, kt * BKV, b);
