@@ -142,8 +142,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------------ MMA issuer (warp-uniform: see umma_f16_elect)
+    {
+      const bool el = elect_one();
       bool ok = mbar_wait(bar_q, 0, abort_flag);
       auto issue_s = [&](int j) -> bool {  // S_j = Q K_j^T into score buffer j & 1
         const uint32_t s = j % C::kStages, ph = (j / C::kStages) & 1;
@@ -153,10 +154,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off_q = (k / 4) * (BQ * 128) + (k % 4) * 32, off_k = (k / 4) * (BN * 128) + (k % 4) * 32;
-          umma_f16(tmem_base + C::kColS + (j & 1) * BN, make_smem_desc(smem_u32(sQ) + off_q, 16, 1024),
+          umma_f16_elect(el, tmem_base + C::kColS + (j & 1) * BN, make_smem_desc(smem_u32(sQ) + off_q, 16, 1024),
                    make_smem_desc(sk + off_k, 16, 1024), p.idesc_qk, k > 0 ? 1u : 0u);
         }
-        umma_commit(bar_s + 8 * (j & 1));
+        umma_commit_elect(el, bar_s + 8 * (j & 1));
         return true;
       };
       if (ok && n_kv > 0) ok = issue_s(0);
@@ -171,14 +172,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t sp = smem_u32(sP) + pb * C::kPBytes;
 #pragma unroll
         for (int k = 0; k < BN / 16; ++k)  // P is K-major over keys; V is MN-major: 16 key rows (2048 B) per step
-          umma_f16(tmem_base + C::kColO, make_smem_desc(sp + k * 32, 16, 1024),
+          umma_f16_elect(el, tmem_base + C::kColO, make_smem_desc(sp + k * 32, 16, 1024),
                    make_smem_desc(sv + k * (16 * 128), BN * 128, 1024), p.idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit(bar_o);  // one completion per tile: O holds the sum over tiles 0..j
-        if (j == n_kv - 1) umma_commit(bar_o + 8);  // one-shot "all products done" for the epilogue (no phase aliasing)
-        umma_commit(bar_e + 8 * s);  // K_j and V_j are free once everything issued so far has run
+        umma_commit_elect(el, bar_o);  // one completion per tile: O holds the sum over tiles 0..j
+        if (j == n_kv - 1) umma_commit_elect(el, bar_o + 8);  // one-shot "all products done" for the epilogue (no phase aliasing)
+        umma_commit_elect(el, bar_e + 8 * s);  // K_j and V_j are free once everything issued so far has run
         if (j + 2 < n_kv) ok = issue_s(j + 2);  // score buffer j & 1 was released by bar_p above
       }
-      if (!ok) fail_role = 2;
+      if (!ok && lane == 0) fail_role = 2;
     }
   } else {
 #include "flash_fwd_softmax.inc"
