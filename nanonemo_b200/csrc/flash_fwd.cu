@@ -1,18 +1,18 @@
 // Causal grouped-query FlashAttention forward on tcgen05 / TMEM / TMA for sm_100a.
 //
 // One CTA owns one 128-row query tile of one (batch, query head) and walks the key/value tiles (64 keys
-// each) up to the diagonal; two CTAs are resident per SM at head_dim 64. 192 threads per CTA:
+// each) up to the diagonal; two CTAs are resident per SM. 192 threads per CTA:
 //   warp 0        TMA producer: Q once, then K_j / V_j into a ring of stages (4-D tensor maps over
 //                 (head_dim, head, t, batch), so any (B,T,H,hd) / (B,H,T,hd) / packed-QKV strides work and
 //                 query head h reads KV head h / group directly — nothing is repeated or copied);
 //   warp 1        MMA issuer: S_j = Q K_j^T and O_j = P_j V_j with tcgen05.mma, accumulators in TMEM;
 //   warps 2..5    softmax, one thread per query row (= TMEM lane): tcgen05.ld the scores, online max and
-//                 sum with exp2, bf16 P_j into a 128-byte swizzled shared tile (the A operand of the second
-//                 MMA). O accumulates IN TENSOR MEMORY over the key tiles; the row maximum used for the
+//                 sum with exp2, 16-bit P_j back into tensor memory over the scores it came from (the A operand of
+//                 the second MMA: no shared-memory round trip). O accumulates IN TENSOR MEMORY over the key tiles; the row maximum used for the
 //                 exponentials is only raised when a tile exceeds it by more than 2^8 (probabilities then
 //                 stay below 256, exact in fp32 / safe in bf16), so the accumulator has to be rescaled —
 //                 tcgen05.ld, multiply, tcgen05.st by the softmax threads — on a few tiles only.
-// The score tile and the P tile are DOUBLE BUFFERED and the MMA warp runs two tiles ahead: S_{j+2} is
+// The score tile (and the P tile in it) is DOUBLE BUFFERED and the MMA warp runs two tiles ahead: S_{j+2} is
 // issued as soon as the softmax threads have read S_j, and P_j V_j runs while they work on tile j+1, so
 // neither side waits for a hand-off in steady state.
 // Outputs: O (bf16) through a swizzled staging tile + TMA store, and L = m * scale + ln(l) per row (fp32)
@@ -41,14 +41,15 @@ constexpr int kSoftmaxThreads = 128;
 template <int HD>
 struct FCfg {
   static constexpr int BN = 64;                             // keys per KV tile
-  static constexpr int kStages = 3;  // 3 x 16 KB at head_dim 64: two CTAs (2 x ~100 KB) fit in one SM
-  static constexpr int kCtasPerSm = (HD == 64) ? 2 : 1;
+  // K and V have rings of their own: K_j is free once S_j has been computed, V_j only after P_j V_j. Two CTAs per SM at both head
+  // sizes (256 of the 512 tensor-memory columns each): while one's softmax runs on the special-function unit the other's
+  // products run. At head_dim 128 that takes two stages instead of three (100 KB a CTA): 228 -> 142 us at B8 H16/4 T2048.
+  static constexpr int kStages = HD == 64 ? 3 : 2;
   static constexpr int kQBytes = BQ * HD * 2;               // HD/64 swizzled K-blocks of 16 KB
   static constexpr int kKBytes = BN * HD * 2;
   static constexpr int kVBytes = BN * HD * 2;
-  static constexpr int kPBytes = BQ * BN * 2;               // one swizzled K-block of 16 KB per buffer
-  static constexpr int kSmem = kQBytes + kStages * (kKBytes + kVBytes) + 2 * kPBytes + 1024 + 256;
-  static constexpr int kColS = 0;                           // S buffers at columns 0 and 64
+  static constexpr int kSmem = kQBytes + kStages * (kKBytes + kVBytes) + 1024 + 256;
+  static constexpr int kColS = 0;                           // S buffers at columns 0 and 64; P_j takes the first 32 of S_j's
   static constexpr int kColO = 128;                         // O accumulator from column 128
   static constexpr int kTmemCols = 256;
 };
@@ -64,7 +65,7 @@ struct FParams {
 };
 
 template <int HD, bool F16>
-__global__ void __launch_bounds__(kThreads, FCfg<HD>::kCtasPerSm)
+__global__ void __launch_bounds__(kThreads, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FParams p) {
   using C = FCfg<HD>;
@@ -73,13 +74,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sKV = sQ + C::kQBytes;                              // [stages][K | V]
-  uint8_t* sP = sKV + C::kStages * (C::kKBytes + C::kVBytes);  // [2][kPBytes]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * C::kPBytes);
-  // barriers: q_full, k_full[S], v_full[S], kv_empty[S], s_full[2], p_full[2], o_tile, o_all (+ 2 unused slots)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + C::kStages * (C::kKBytes + C::kVBytes));
+  // barriers: q_full, k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_full[2], o_tile, o_all
   const uint32_t bar_q = smem_u32(bars);
-  const uint32_t bar_k = bar_q + 8, bar_v = bar_k + 8 * C::kStages, bar_e = bar_v + 8 * C::kStages;
-  const uint32_t bar_s = bar_e + 8 * C::kStages, bar_p = bar_s + 16, bar_o = bar_p + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 3 * C::kStages + 8);
+  const uint32_t bar_k = bar_q + 8, bar_v = bar_k + 8 * C::kStages;
+  const uint32_t bar_ke = bar_v + 8 * C::kStages, bar_ve = bar_ke + 8 * C::kStages;
+  const uint32_t bar_s = bar_ve + 8 * C::kStages, bar_p = bar_s + 16, bar_o = bar_p + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 4 * C::kStages + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -96,7 +97,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(bar_k + 8 * s, 1);
       mbar_init(bar_v + 8 * s, 1);
-      mbar_init(bar_e + 8 * s, 1);
+      mbar_init(bar_ke + 8 * s, 1);
+      mbar_init(bar_ve + 8 * s, 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar_s + 8 * i, 1);
@@ -131,11 +133,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int c = 0; c < HD / 64; ++c) tma_load_4d(smem_u32(sQ) + c * (BQ * 128), &tmQ, bar_q, c * 64, h, qt * BQ, b);
       for (int j = 0; j < n_kv; ++j) {
         const uint32_t s = j % C::kStages, ph = (j / C::kStages) & 1;
-        if (!mbar_wait(bar_e + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
+        if (!mbar_wait(bar_ke + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
         const uint32_t sk = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes), sv = sk + C::kKBytes;
         mbar_expect_tx(bar_k + 8 * s, C::kKBytes);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) tma_load_4d(sk + c * (BN * 128), &tmK, bar_k + 8 * s, c * 64, kvh, j * BN, b);
+        if (!mbar_wait(bar_ve + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
         mbar_expect_tx(bar_v + 8 * s, C::kVBytes);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) tma_load_4d(sv + c * (BN * 128), &tmV, bar_v + 8 * s, c * 64, kvh, j * BN, b);
@@ -158,6 +161,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                    make_smem_desc(sk + off_k, 16, 1024), p.idesc_qk, k > 0 ? 1u : 0u);
         }
         umma_commit_elect(el, bar_s + 8 * (j & 1));
+        umma_commit_elect(el, bar_ke + 8 * s);
         return true;
       };
       if (ok && n_kv > 0) ok = issue_s(0);
@@ -169,14 +173,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (!mbar_wait(bar_p + 8 * pb, (j >> 1) & 1, abort_flag)) { ok = false; break; }   // P_j written, S_j consumed, O rescaled if needed
         tc_fence_after();
         const uint32_t sv = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes) + C::kKBytes;
-        const uint32_t sp = smem_u32(sP) + pb * C::kPBytes;
+        const uint32_t tp = tmem_base + C::kColS + pb * BN;
 #pragma unroll
-        for (int k = 0; k < BN / 16; ++k)  // P is K-major over keys; V is MN-major: 16 key rows (2048 B) per step
-          umma_f16_elect(el, tmem_base + C::kColO, make_smem_desc(sp + k * 32, 16, 1024),
-                   make_smem_desc(sv + k * (16 * 128), BN * 128, 1024), p.idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < BN / 16; ++k)  // P from tensor memory: 16 keys = 8 columns per step; V is MN-major: 16 key rows (2048 B)
+          umma_f16_ts_elect(el, tmem_base + C::kColO, tp + k * 8, make_smem_desc(sv + k * (16 * 128), BN * 128, 1024), p.idesc_pv,
+                            (j > 0 || k > 0) ? 1u : 0u);
         umma_commit_elect(el, bar_o);  // one completion per tile: O holds the sum over tiles 0..j
         if (j == n_kv - 1) umma_commit_elect(el, bar_o + 8);  // one-shot "all products done" for the epilogue (no phase aliasing)
-        umma_commit_elect(el, bar_e + 8 * s);  // K_j and V_j are free once everything issued so far has run
+        umma_commit_elect(el, bar_ve + 8 * s);  // V_j is free
         if (j + 2 < n_kv) ok = issue_s(j + 2);  // score buffer j & 1 was released by bar_p above
       }
       if (!ok && lane == 0) fail_role = 2;
