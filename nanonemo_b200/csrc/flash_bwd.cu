@@ -525,8 +525,8 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   const bool f16 = dtype == NNB_F16;
   NNB_REQUIRE(H % KVH == 0 && B > 0 && T > 0, "flash_bwd: bad shape");
   // head_dim 128 runs on the transposed-tile kernel (flash_bwd_t.cu). It also serves head_dim 64
-  // (NANONEMO_FLASH_BWD=transposed), but there the 128 x 128 formulation of this file measured faster (0.43 vs 0.57 ms at
-  // B32 H12/4 T1024): with 64-wide tiles every MMA has N = 64 and is bound by shared-memory operand reads.
+  // (NANONEMO_FLASH_BWD=transposed), but there the 128 x 128 formulation of this file measured faster (299 vs 361 us at
+  // B32 H12/4 T1024; 696 vs 1058 us at B8 T4096): with 64-wide tiles every product has N = 64 and is bound by shared-memory operand reads.
   static const bool square = [] { const char* e = getenv("NANONEMO_FLASH_BWD"); return !(e && e[0] == 't'); }();
   NNB_REQUIRE((rope_cos == nullptr) == (rope_sin == nullptr), "flash_bwd: give both RoPE tables or neither");
   NNB_REQUIRE(rope_cos == nullptr || (hd == HD && square && nnb_aligned16(rope_cos) && nnb_aligned16(rope_sin)),

@@ -6,20 +6,26 @@
 //     P^T  = exp(S^T scale - L[q]) ; dS^T = P^T (dP^T - D[q]) scale     (256 threads: key row x half of the queries)
 //     dV  += P^T dO         dK  += dS^T Q                  (M = 128 keys,  N = head_dim,   K = 64 queries)
 //     dQ^T = K^T dS^T                                      (M = head_dim,  N = 64 queries, K = 128 keys)
-// Why transposed: with 64-query tiles the scores take 64 TMEM columns each, so at head_dim 64 S^T and dP^T are DOUBLE
-// BUFFERED (2 x 64 + 2 x 64 + dV 64 + dK 64 + dQ^T 64 = 448 columns) and the softmax-gradient math of visit n + 1 runs while
-// the tensor core accumulates dV / dK / dQ^T of visit n — in the 128 x 128 formulation (flash_bwd.cu) the two phases
-// alternate, because two score buffers alone would fill the 512 columns. At head_dim 128 the accumulators are twice as wide
-// (64 + 64 + 128 + 128 + 64 = 448 columns), the scores single buffered; the 128 x 128 formulation does not fit at all.
-// P^T / dS^T are written once to shared memory as bf16 [key][query] tiles (128-byte rows, swizzled) and serve as K-major A
-// operand (dV, dK) and MN-major B operand (dQ^T); K is read K-major (S^T) and MN-major (dQ^T), Q / dO K-major (scores) and
-// MN-major (dK, dV): no transposed copies. dQ^T (lanes = head_dim index; at head_dim 64 an M = 64 accumulator: row m in
-// lane m % 16 of lane quarter m / 16) leaves through an fp32 [query][head_dim] staging tile — the transpose happens in the
-// shared-memory write — and a TMA reduce-add into an fp32 buffer. dK / dV accumulate over the GQA group and are stored once.
-// With double-buffered scores the compute warps are software pipelined: math(n), then the drain of dQ^T(n - 1), so they do
-// not wait for the MMAs they have just unblocked. Same contract as the reference backward (nanonemo/kernels/cuda/flash_attn.cu:176-340; head_dim 64 only).
+// Why transposed: at head_dim 128 the 128 x 128 formulation of flash_bwd.cu does not fit tensor memory; here S^T is double buffered
+// and everything fits in 64 + 64 (S^T) + 64 (dP^T) + 128 + 128 (dV, dK) + 64 (dQ^T) = 512 columns. And P^T, dS^T have the keys as rows,
+// which is how dV and dK want their A operand: both are written back into tensor memory over the scores / products they came
+// from and multiplied from there. Only dS^T also goes to shared memory (16-bit [key][query], 128-byte rows, swizzled), as the
+// MN-major B operand of dQ^T. K is read K-major (S^T) and MN-major (dQ^T), Q / dO K-major (scores) and MN-major (dK, dV): no
+// transposed copies. dQ^T (lanes = head_dim index; at head_dim 64 an M = 64 accumulator: row m in lane m % 16 of lane quarter
+// m / 16) leaves through an fp32 [query][head_dim] staging tile — the transpose happens in the shared-memory write — and a TMA
+// reduce-add into an fp32 buffer. dK / dV accumulate over the GQA group and are stored once.
+// 512 threads: warp 0 TMA producer, warp 1 MMA issuer (warp-uniform, see umma_f16_elect), warp 2 fetches L and D of the visits'
+// queries, warps 4..7 drain dQ^T, warps 8..15 compute. No block barrier in the loop:
+//     compute :  A(n)                      B(n)                            A(n+1)  ...
+//     tensor  :        S^T(n+1)   dV(n)           dQ^T(n) dK(n) dP^T(n+1)
+//     drain   :  dQ^T(n-1)                                                 dQ^T(n)
+// What bounded it: one chain. With single-buffered scores, the drain in the compute warps and a one-lane MMA issuer a visit
+// took 5000 cycles (wait for the products 1245, P and dS 1371, wait for dQ^T 1630, drain 749) of which the tensor core needs
+// about 1660. Backward at B8 H16/4 T2048 head_dim 128: 785 us then, 469 us now.
+// Same contract as the reference backward (nanonemo/kernels/cuda/flash_attn.cu:176-340; head_dim 64 only).
 #include <type_traits>
 
+#define NNB_PROF_THREAD 256  // a compute thread
 #include "sm100.cuh"
 
 namespace {
@@ -27,7 +33,9 @@ namespace {
 using namespace sm100;
 
 constexpr int BQ = 64, BKV = 128;
-constexpr int kThreads = 320, kComputeThreads = 256;
+constexpr int kThreads = 512, kComputeThreads = 256, kDrainThreads = 128;
+constexpr int kDrainWarp0 = 4, kComputeWarp0 = 8;
+constexpr int kStagesQ = 3;            // ring of (Q | dO) blocks
 constexpr int kHalfK = BKV * 64 * 2;   // [128 keys x 64] 16-bit tile = 16 KB
 constexpr int kHalfQ = BQ * 64 * 2;    // [64 queries x 64] 16-bit tile = 8 KB
 constexpr int kTmemCols = 512;
@@ -35,17 +43,15 @@ constexpr int kTmemCols = 512;
 template <int HD>
 struct Cfg {
   static constexpr int NH = HD / 64;                 // 64-wide head_dim groups (one TMA box / swizzle span each)
-  static constexpr int NBUF = HD == 64 ? 2 : 1;      // buffers of S^T / dP^T (TMEM) and P^T / dS^T (shared memory)
-  static constexpr int kStagesQ = HD == 64 ? 4 : 2;  // ring of (Q | dO) blocks
   static constexpr int kTileK = NH * kHalfK;         // K or V tile
   static constexpr int kStageQdO = 2 * NH * kHalfQ;  // Q block + dO block
   static constexpr int kOffK = 0, kOffV = kTileK, kOffQdO = 2 * kTileK;
-  static constexpr int kOffP = kOffQdO + kStagesQ * kStageQdO, kOffdS = kOffP + NBUF * kHalfK;
-  static constexpr int kOffStage = kOffdS + NBUF * kHalfK;     // fp32 [64 queries x HD]
+  static constexpr int kOffdS = kOffQdO + kStagesQ * kStageQdO;
+  static constexpr int kOffStage = kOffdS + kHalfK;            // fp32 [64 queries x HD]
   static constexpr int kOffBars = kOffStage + BQ * HD * 4;
-  static constexpr int kOffLD = kOffBars + 256;                // float [2 parities][2 (L, D)][64]
+  static constexpr int kOffLD = kOffBars + 256;                // float [2 parities][2 (-L log2e, -D scale)][64]
   static constexpr int kSmem = kOffLD + 2 * 2 * 64 * 4 + 1024;
-  static constexpr int kColS = 0, kColdP = 64 * NBUF, kColdV = 128 * NBUF, kColdK = kColdV + HD, kColdQ = kColdK + HD;
+  static constexpr int kColS = 0 /* + 64 * (visit & 1) */, kColdP = 128, kColdV = 192, kColdK = kColdV + HD, kColdQ = kColdK + HD;
   static_assert(kColdQ + 64 <= kTmemCols, "TMEM budget");
   static_assert(kStagesQ * kStageQdO >= 2 * kTileK, "the (Q | dO) ring doubles as the dV / dK staging area");
 };
@@ -66,15 +72,16 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmdQacc, const __grid_constant__ CUtensorMap tmdK,
                    const __grid_constant__ CUtensorMap tmdV, const BParams p) {
   using C = Cfg<HD>;
-  constexpr int NH = C::NH, NBUF = C::NBUF, S = C::kStagesQ;
+  constexpr int NH = C::NH, S = kStagesQ;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBars);
-  // barriers: kv, q_full[4], q_empty[4], sdp[2], pds[2], pfree[2], dq, dq_read
-  const uint32_t bar_kv = smem_u32(bars), bar_qf = bar_kv + 8, bar_qe = bar_qf + 32;
-  const uint32_t bar_sdp = bar_qe + 32, bar_pds = bar_sdp + 16, bar_pfree = bar_pds + 16, bar_dq = bar_pfree + 16, bar_dqr = bar_dq + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  // barriers: kv, q_full[3], q_empty[3], s_full[2], p_written[2], ld_full[2], ld_empty[2], dp_full, ds_written, dq_full, dq_read, all_done
+  const uint32_t bar_kv = smem_u32(bars), bar_qf = bar_kv + 8, bar_qe = bar_qf + 8 * S, bar_s = bar_qe + 8 * S, bar_p = bar_s + 16;
+  const uint32_t bar_lf = bar_p + 16, bar_le = bar_lf + 16, bar_dp = bar_le + 16, bar_ds = bar_dp + 8, bar_dq = bar_ds + 8;
+  const uint32_t bar_dqr = bar_dq + 8, bar_fin = bar_dqr + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * S + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_ld = reinterpret_cast<float*>(smem + C::kOffLD);
 
@@ -86,17 +93,21 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(bar_kv, 1);
-    for (int s = 0; s < 4; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(bar_qf + 8 * s, 1);
       mbar_init(bar_qe + 8 * s, 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_sdp + 8 * i, 1);
-      mbar_init(bar_pds + 8 * i, kComputeThreads);
-      mbar_init(bar_pfree + 8 * i, 1);
+      mbar_init(bar_s + 8 * i, 1);
+      mbar_init(bar_p + 8 * i, kComputeThreads);
+      mbar_init(bar_lf + 8 * i, 32);
+      mbar_init(bar_le + 8 * i, kComputeThreads);
     }
+    mbar_init(bar_dp, 1);
+    mbar_init(bar_ds, kComputeThreads);
     mbar_init(bar_dq, 1);
-    mbar_init(bar_dqr, kComputeThreads);
+    mbar_init(bar_dqr, kDrainThreads);
+    mbar_init(bar_fin, 1);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -134,179 +145,242 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = mbar_wait(bar_kv, 0, abort_flag);
-      const uint32_t sK = s_base + C::kOffK, sV = s_base + C::kOffV;
-      // S^T = K Q^T and dP^T = V dO^T of visit n into score buffer n % NBUF: K-major operands, k-steps of 16 over head_dim
-      auto issue_sdp = [&](int n) -> bool {
-        const uint32_t s = n % S, ph = (n / S) & 1, buf = n % NBUF;
-        const uint32_t sQ = s_base + C::kOffQdO + s * C::kStageQdO, sdO = sQ + NH * kHalfQ;
-        if (!mbar_wait(bar_qf + 8 * s, ph, abort_flag)) return false;
+    // ------------------------------------------------------------------ MMA issuer (every lane runs the loop, one lane's instructions count)
+    const bool el = elect_one();
+    bool ok = mbar_wait(bar_kv, 0, abort_flag);
+    const uint32_t sK = s_base + C::kOffK, sV = s_base + C::kOffV, sdS = s_base + C::kOffdS;
+    uint32_t cur = 0, nxt = 0, nxt_ph = 0;  // ring positions of visits n and n + 1, and the phase of the latter
+    auto stage_at = [&](uint32_t s) { return s_base + C::kOffQdO + s * C::kStageQdO; };
+    // S^T = K Q^T of visit n into score buffer n & 1, dP^T = V dO^T: K-major operands, k-steps of 16 over head_dim
+    auto issue_s = [&](int n, uint32_t s) {
+      const uint32_t sQ = stage_at(s);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_f16_elect(el, tmem_base + C::kColS + 64 * (n & 1), make_smem_desc(sK + (k / 4) * kHalfK + (k % 4) * 32, 16, 1024),
+                       make_smem_desc(sQ + (k / 4) * kHalfQ + (k % 4) * 32, 16, 1024), p.idesc_s, k > 0);
+      umma_commit_elect(el, bar_s + 8 * (n & 1));
+    };
+    auto issue_dp = [&](uint32_t s) {
+      const uint32_t sdO = stage_at(s) + NH * kHalfQ;
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_f16_elect(el, tmem_base + C::kColdP, make_smem_desc(sV + (k / 4) * kHalfK + (k % 4) * 32, 16, 1024),
+                       make_smem_desc(sdO + (k / 4) * kHalfQ + (k % 4) * 32, 16, 1024), p.idesc_s, k > 0);
+      umma_commit_elect(el, bar_dp);
+    };
+    if (ok && iters > 0) {
+      ok = mbar_wait(bar_qf, 0, abort_flag);
+      if (ok) {
         tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          umma_f16(tmem_base + C::kColS + 64 * buf, make_smem_desc(sK + (k / 4) * kHalfK + (k % 4) * 32, 16, 1024),
-                   make_smem_desc(sQ + (k / 4) * kHalfQ + (k % 4) * 32, 16, 1024), p.idesc_s, k > 0);
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          umma_f16(tmem_base + C::kColdP + 64 * buf, make_smem_desc(sV + (k / 4) * kHalfK + (k % 4) * 32, 16, 1024),
-                   make_smem_desc(sdO + (k / 4) * kHalfQ + (k % 4) * 32, 16, 1024), p.idesc_s, k > 0);
-        umma_commit(bar_sdp + 8 * buf);
-        return true;
-      };
-      for (int i = 0; i < NBUF && i < iters && ok; ++i) ok = issue_sdp(i);
-      for (int n = 0; n < iters && ok; ++n) {
-        const uint32_t s = n % S, buf = n % NBUF;
-        const uint32_t sQ = s_base + C::kOffQdO + s * C::kStageQdO, sdO = sQ + NH * kHalfQ;
-        const uint32_t sP = s_base + C::kOffP + buf * kHalfK, sdS = s_base + C::kOffdS + buf * kHalfK;
-        if (!mbar_wait(bar_pds + 8 * buf, (n / NBUF) & 1, abort_flag)) { ok = false; break; }  // P^T, dS^T written; scores consumed
-        if (n > 0 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }       // dQ^T of the previous visit drained
-        tc_fence_after();
-        // dV += P^T dO, dK += dS^T Q: A = [key][query] tile K-major (4 k-steps of 16 queries = 32 bytes), B = [query][head_dim]
-        // block read MN-major (64-wide head_dim groups kHalfQ apart; 16 query rows = 2048 bytes per step)
-#pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          umma_f16(tmem_base + C::kColdV, make_smem_desc(sP + k * 32, 16, 1024), make_smem_desc(sdO + k * 2048, kHalfQ, 1024),
-                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < BQ / 16; ++k)
-          umma_f16(tmem_base + C::kColdK, make_smem_desc(sdS + k * 32, 16, 1024), make_smem_desc(sQ + k * 2048, kHalfQ, 1024),
-                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
-        // dQ^T = K^T dS^T: A = K tile read MN-major (M = head_dim in 64-wide groups kHalfK apart), B = dS^T tile read MN-major
-        // (N = 64 queries: one group); 8 k-steps of 16 key rows = 2048 bytes
-#pragma unroll
-        for (int k = 0; k < BKV / 16; ++k)
-          umma_f16(tmem_base + C::kColdQ, make_smem_desc(sK + k * 2048, kHalfK, 1024), make_smem_desc(sdS + k * 2048, kHalfK, 1024),
-                   p.idesc_dq, k > 0);
-        umma_commit(bar_dq);
-        umma_commit(bar_qe + 8 * s);
-        umma_commit(bar_pfree + 8 * buf);
-        if (n + NBUF < iters) ok = issue_sdp(n + NBUF);  // its score buffer was released by bar_pds above
+        issue_s(0, 0);
+        issue_dp(0);
       }
-      if (!ok) fail_role = 2;
     }
-  } else {
-    // ------------------------------------------------------------------ compute warps: (key row) x (half of the 64 queries)
-    const int half = (warp - 2) >> 2;
-    const int q4 = warp & 3, row = q4 * 32 + lane, sw = row & 7;
-    const int ct = threadIdx.x - 64;  // 0..255
-    const bool leader = ct == 0;
-    const uint32_t t_lane = tmem_base + ((uint32_t)(q4 * 32) << 16);
-    float* stage = reinterpret_cast<float*>(smem + C::kOffStage);
-    const int key = kt * BKV + row;
-    bool ok = true;
+    for (int n = 0; n < iters && ok; ++n) {
+      const uint32_t sQ = stage_at(cur), sdO = sQ + NH * kHalfQ;
+      if (++nxt == S) { nxt = 0; nxt_ph ^= 1; }
+      if (n + 1 < iters) {
+        // the other score buffer: its scores were read before bar_p of visit n - 1, and dV(n - 1), which read P^T there, is ahead in order
+        if (!mbar_wait(bar_qf + 8 * nxt, nxt_ph, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        issue_s(n + 1, nxt);
+      }
+      if (!mbar_wait(bar_p + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }  // P^T(n) is in tensor memory
+      tc_fence_after();
+      // dV += P^T dO: A = P^T in tensor memory (16 queries = 8 columns per k-step; the two halves of the queries sit 32 columns apart,
+      // each over the scores its own threads have read), B = [query][head_dim] block read MN-major (64-wide head_dim groups
+      // kHalfQ apart; 16 query rows = 2048 bytes per step)
+      const uint32_t tP = tmem_base + C::kColS + 64 * (n & 1), tdS = tmem_base + C::kColdP;
+#pragma unroll
+      for (int k = 0; k < BQ / 16; ++k)
+        umma_f16_ts_elect(el, tmem_base + C::kColdV, tP + (k / 2) * 32 + (k % 2) * 8, make_smem_desc(sdO + k * 2048, kHalfQ, 1024),
+                          p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
+      if (!mbar_wait(bar_ds, n & 1, abort_flag)) { ok = false; break; }                     // dS^T(n) written, dP^T(n) read
+      if (n > 0 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }     // dQ^T(n - 1) drained
+      tc_fence_after();
+      // dQ^T = K^T dS^T: A = K tile read MN-major (M = head_dim in 64-wide groups kHalfK apart), B = dS^T tile read MN-major
+      // (N = 64 queries: one group); 8 k-steps of 16 key rows = 2048 bytes. First, so that its drain runs beside the others.
+#pragma unroll
+      for (int k = 0; k < BKV / 16; ++k)
+        umma_f16_elect(el, tmem_base + C::kColdQ, make_smem_desc(sK + k * 2048, kHalfK, 1024), make_smem_desc(sdS + k * 2048, kHalfK, 1024),
+                       p.idesc_dq, k > 0);
+      umma_commit_elect(el, bar_dq);
+      // dK += dS^T Q, operands as for dV
+#pragma unroll
+      for (int k = 0; k < BQ / 16; ++k)
+        umma_f16_ts_elect(el, tmem_base + C::kColdK, tdS + (k / 2) * 32 + (k % 2) * 8, make_smem_desc(sQ + k * 2048, kHalfQ, 1024),
+                          p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
+      umma_commit_elect(el, bar_qe + 8 * cur);
+      if (n + 1 < iters) issue_dp(nxt);  // over dS^T(n), which dK(n), ahead in order, reads
+      else umma_commit_elect(el, bar_fin);  // one-shot: every product has been accumulated
+      cur = nxt;
+    }
+    if (!ok && lane == 0) fail_role = 2;
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ L and D of a visit's 64 queries, up to two visits ahead:
+    // -L log2(e) and -D scale, the addends of the packed multiply-adds
     constexpr float kLog2e = 1.4426950408889634f;
-    NNB_PROF_DECL;
-    // dQ^T of visit m: TMEM (lane = head_dim index, columns = queries) -> fp32 staging [query][head_dim] -> TMA reduce-add
-    auto drain_dq = [&](int m) -> bool {
-      const int hq = kvh * p.group + m / n_qb, q0 = (first_qb + m % n_qb) * BQ;
-      if (!mbar_wait(bar_dq, m & 1, abort_flag)) ok = false;
+    const float* gL = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T;
+    const float* gD = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T;
+    int qb = first_qb;
+    for (int n = 0; n < iters; ++n) {
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int qi = qb * BQ + i * 32 + lane;
+        v[i] = qi < p.T ? -gL[qi] * kLog2e : 0.f;
+        v[2 + i] = qi < p.T ? -gD[qi] * p.scale : 0.f;
+      }
+      if (++qb == p.n_q_blocks) { qb = first_qb; gL += p.T; gD += p.T; }
+      if (n >= 2 && !mbar_wait(bar_le + 8 * (n & 1), ((n >> 1) - 1) & 1, abort_flag)) { fail_role = 5; break; }
+      float* dst = s_ld + (n & 1) * 128 + lane;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[i * 32] = v[i];
+      mbar_arrive(bar_lf + 8 * (n & 1));
+    }
+  } else if (warp >= kDrainWarp0 && warp < kComputeWarp0) {
+    // ------------------------------------------------------------------ drain warps: dQ^T of every visit, TMEM (lane = head_dim index,
+    // columns = queries) -> fp32 staging [query][head_dim] -> TMA reduce-add
+    const int q4 = warp & 3;
+    const bool leader = warp == kDrainWarp0 && lane == 0;
+    const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16) + C::kColdQ;
+    float* stage = reinterpret_cast<float*>(smem + C::kOffStage);
+    int hq = kvh * p.group, qb = first_qb;
+    for (int m = 0; m < iters; ++m) {
+      const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
       tc_fence_after();
       if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
-      if (named_barrier_or(1, kComputeThreads, !ok)) return false;
-      NNB_PROF_ADD(2);
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(t_lane + C::kColdQ + half * 32, r);
+      if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }  // all leave together
+      uint32_t r0[32], r1[32];
+      tmem_ld_32x32b_x32(t_row, r0);
+      tmem_ld_32x32b_x32(t_row + 32, r1);
       tmem_ld_wait();
-      if (HD == 128) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) stage[(half * 32 + c) * HD + row] = __uint_as_float(r[c]);
-      } else if (lane < 16) {                    // M = 64 accumulator: row 16 q4 + lane lives in lane `lane` of this quarter
-#pragma unroll
-        for (int c = 0; c < 32; ++c) stage[(half * 32 + c) * HD + q4 * 16 + lane] = __uint_as_float(r[c]);
-      }
       tc_fence_before();
       mbar_arrive(bar_dqr);
+      if (HD == 128 || lane < 16) {              // HD 64: M = 64 accumulator, row 16 q4 + lane lives in lane `lane` of this quarter
+        float* col = stage + (HD == 128 ? q4 * 32 + lane : q4 * 16 + lane);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          col[c * HD] = __uint_as_float(r0[c]);
+          col[(c + 32) * HD] = __uint_as_float(r1[c]);
+        }
+      }
       fence_proxy_async_smem();
-      named_barrier_sync(1, kComputeThreads);
+      named_barrier_sync(1, kDrainThreads);
       if (leader) {
-        tma_reduce_add_4d(&tmdQacc, s_base + C::kOffStage, 0, hq, q0, b);
+        tma_reduce_add_4d(&tmdQacc, s_base + C::kOffStage, 0, hq, qb * BQ, b);
         tma_commit_group();
       }
-      NNB_PROF_ADD(3);
-      return true;
-    };
-    // L (log-sum-exp, log2 units) and D * scale of the 64 queries of a visit: threads 0..63 fetch L, 64..127 fetch D, one
-    // visit AHEAD into a register, so the global-memory latency hides behind the previous visit
-    auto fetch_ld = [&](int n) -> float {
-      if (ct >= 128 || n >= iters) return 0.f;
-      const int hq = kvh * p.group + n / n_qb, qi = (first_qb + n % n_qb) * BQ + (ct & 63);
-      if (qi >= p.T) return 0.f;
-      const size_t stat = ((size_t)b * p.H + hq) * p.T + qi;
-      return ct < 64 ? p.lse[stat] * kLog2e : p.delta[stat] * p.scale;
-    };
-    float ld_next = fetch_ld(0);
+      if (++qb == p.n_q_blocks) { qb = first_qb; ++hq; }
+    }
+    if (leader) tma_wait_group<0>();
+  } else if (warp >= kComputeWarp0) {
+    // ------------------------------------------------------------------ compute warps: (key row) x (half of the 64 queries)
+    const int half = (warp - kComputeWarp0) >> 2;
+    const int q4 = warp & 3, row = q4 * 32 + lane, sw = row & 7;
+    const bool leader = half == 0 && row == 0;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(q4 * 32) << 16);
+    const int key = kt * BKV + row;
+    uint8_t* my_ds = smem + C::kOffdS + row * 128;
+    const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    bool ok = true;
+    NNB_PROF_DECL;
+    int qb = first_qb;
     for (int n = 0; n < iters; ++n) {
       NNB_PROF_T0;
-      const int q0 = (first_qb + n % n_qb) * BQ;
-      const int buf = n % NBUF;
-      uint8_t* my_p = smem + C::kOffP + buf * kHalfK + row * 128;
-      uint8_t* my_ds = smem + C::kOffdS + buf * kHalfK + row * 128;
-      float* sL = s_ld + (n & 1) * 128;
-      float* sD = sL + 64;
-      if (ct < 128) sL[ct] = ld_next;  // sD = sL + 64: threads 64..127 land in the D half
-      ld_next = fetch_ld(n + 1);
-      if (!mbar_wait(bar_sdp + 8 * buf, (n / NBUF) & 1, abort_flag)) ok = false;
-      // the MMAs of the visit that last read this P^T / dS^T buffer have completed
-      if (n >= NBUF && !mbar_wait(bar_pfree + 8 * buf, (n / NBUF - 1) & 1, abort_flag)) ok = false;
-      if (named_barrier_or(1, kComputeThreads, !ok)) { ok = false; fail_role = 3; break; }  // L / D visible; all leave together
-      tc_fence_after();
-      NNB_PROF_ADD(0);
+      const int q0 = qb * BQ;
+      if (++qb == p.n_q_blocks) qb = first_qb;
+      const int buf = n & 1;
+      const ulonglong2* sL = reinterpret_cast<const ulonglong2*>(s_ld + buf * 128 + half * 32);
+      const ulonglong2* sD = sL + 16;
+      const uint32_t t_s = t_lane + C::kColS + 64 * buf + half * 32, t_dp = t_lane + C::kColdP + half * 32;
       // per-element mask only on the diagonal blocks, at the end of the sequence or for padded key rows
       const bool need_mask = q0 < kt * BKV + BKV - 1 || q0 + BQ > p.T || kt * BKV + BKV > p.T;
-      auto tile = [&](auto masked) {
+      float prob[32];  // P^T of this thread's 32 queries, kept in fp32 from phase A to phase B
+      // ---- phase A: P^T = exp2(S^T scale log2e - L log2e)
+      if (!mbar_wait(bar_lf + 8 * buf, (n >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait(bar_s + 8 * buf, (n >> 1) & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      NNB_PROF_ADD(0);
+      auto phase_a = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
-        uint32_t rs[32], rp[32];
-        tmem_ld_32x32b_x32(t_lane + C::kColS + 64 * buf + half * 32, rs);
-        tmem_ld_32x32b_x32(t_lane + C::kColdP + 64 * buf + half * 32, rp);
-        tmem_ld_wait();
-        uint32_t pk[16], dk[16];
+        uint32_t rs[2][16], pk[16];
+        tmem_ld_32x32b_x16(t_s, rs[0]);
+        tmem_ld_32x32b_x16(t_s + 16, rs[1]);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float pv[2], dv[2];
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld_wait(rs[c]);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int c = half * 32 + i + e;
-            float prob = exp2f(__uint_as_float(rs[i + e]) * p.scale_log2 - sL[c]);
-            if (kMask) {
-              const int qi = q0 + c;
-              prob = (key <= qi && qi < p.T && key < p.T) ? prob : 0.f;
+          for (int i = 0; i < 16; i += 4) {
+            const ulonglong2 l = sL[c * 4 + i / 4];
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const uint64_t s2 = pack_f32x2(__uint_as_float(rs[c][i + e]), __uint_as_float(rs[c][i + e + 1]));
+              const float2 x = unpack_f32x2(fma_f32x2(s2, scale_log2_2, e == 0 ? l.x : l.y));
+              float p0 = exp2f(x.x), p1 = exp2f(x.y);
+              if (kMask) {
+                const int qi = q0 + half * 32 + c * 16 + i + e;
+                p0 = (key <= qi && qi < p.T && key < p.T) ? p0 : 0.f;
+                p1 = (key <= qi + 1 && qi + 1 < p.T && key < p.T) ? p1 : 0.f;
+              }
+              prob[c * 16 + i + e] = p0;
+              prob[c * 16 + i + e + 1] = p1;
+              pk[(c * 16 + i + e) >> 1] = pack2_16<F16>(p0, p1);
             }
-            pv[e] = prob;
-            dv[e] = prob * (__uint_as_float(rp[i + e]) * p.scale - sD[c]);
           }
-          pk[i >> 1] = pack2_16<F16>(pv[0], pv[1]);
-          dk[i >> 1] = pack2_16<F16>(dv[0], dv[1]);
         }
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const int chunk = ((half * 4 + jj) ^ sw) << 4;
-          *reinterpret_cast<uint4*>(my_p + chunk) = make_uint4(pk[4 * jj], pk[4 * jj + 1], pk[4 * jj + 2], pk[4 * jj + 3]);
-          *reinterpret_cast<uint4*>(my_ds + chunk) = make_uint4(dk[4 * jj], dk[4 * jj + 1], dk[4 * jj + 2], dk[4 * jj + 3]);
-        }
+        tmem_st_32x32b_x16(t_s, pk);
       };
-      if (need_mask) tile(std::true_type{});
-      else tile(std::false_type{});
-      fence_proxy_async_smem();
+      if (need_mask) phase_a(std::true_type{});
+      else phase_a(std::false_type{});
+      tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(bar_pds + 8 * buf);
+      mbar_arrive(bar_p + 8 * buf);
       NNB_PROF_ADD(1);
-      if (NBUF == 1) {
-        // single score buffer: the next visit's math needs this visit's MMAs anyway, so drain dQ^T right away
-        if (!drain_dq(n)) { ok = false; fail_role = 3; break; }
-      } else if (n > 0 && !drain_dq(n - 1)) {
-        // double buffered: the MMAs of this visit are now unblocked; drain the PREVIOUS visit's dQ^T meanwhile
-        ok = false; fail_role = 3; break;
+      // ---- phase B: dS^T = P^T (dP^T scale - D scale)
+      // (dP^T(n) was issued after dQ^T(n - 1) and dK(n - 1): once it is complete they have read dS^T)
+      if (!mbar_wait(bar_dp, n & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      NNB_PROF_ADD(2);
+      {
+        uint32_t rp[2][16], dk[16];
+        tmem_ld_32x32b_x16(t_dp, rp[0]);
+        tmem_ld_32x32b_x16(t_dp + 16, rp[1]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          tmem_ld_wait(rp[c]);
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const ulonglong2 d = sD[c * 4 + i / 4];
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c][i + e]), __uint_as_float(rp[c][i + e + 1])), scale2, e == 0 ? d.x : d.y);
+              const float2 g = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i + e], prob[c * 16 + i + e + 1]), t));
+              dk[(c * 16 + i + e) >> 1] = pack2_16<F16>(g.x, g.y);
+            }
+          }
+        }
+        tmem_st_32x32b_x16(t_dp, dk);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+          *reinterpret_cast<uint4*>(my_ds + (((half * 4 + jj) ^ sw) << 4)) = make_uint4(dk[4 * jj], dk[4 * jj + 1], dk[4 * jj + 2], dk[4 * jj + 3]);
       }
+      mbar_arrive(bar_le + 8 * buf);
+      fence_proxy_async_smem();
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(bar_ds);
+      NNB_PROF_ADD(3);
     }
-    if (NBUF == 2 && ok && iters > 0 && !drain_dq(iters - 1)) { ok = false; fail_role = 3; }
+    if (ok && iters > 0 && !mbar_wait(bar_fin, 0, abort_flag)) ok = false;
+    tc_fence_after();
+    if (named_barrier_or(2, kComputeThreads, !ok)) {  // all leave together
+      ok = false;
+      fail_role = 3;
+    }
     NNB_PROF_FLUSH_N(iters);
     // dV then dK of this key tile: TMEM -> bf16 staging (the (Q | dO) ring: every load has been consumed) -> TMA store
     if (ok && iters > 0) {
-      // bar_dq of the last visit was awaited in drain_dq, so every MMA (including the dV / dK accumulation) has completed
-      if (leader) tma_wait_group_read<0>();
-      named_barrier_sync(1, kComputeThreads);
 #pragma unroll
       for (int u = half; u < 2 * NH; u += 2) {
         const int which = u / NH, g = u % NH;  // 0 = dV, 1 = dK; 64-wide head_dim group
@@ -328,7 +402,7 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       fence_proxy_async_smem();
-      named_barrier_sync(1, kComputeThreads);
+      named_barrier_sync(2, kComputeThreads);
       if (leader) {
 #pragma unroll
         for (int g = 0; g < NH; ++g) {
