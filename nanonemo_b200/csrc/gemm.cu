@@ -3,7 +3,7 @@
 // Structure (one persistent CTA per SM, 192 threads, warp-specialised):
 //   warp 0      TMA producer: cp.async.bulk.tensor loads of 128-byte swizzled A/B tiles into a ring of
 //               shared-memory stages, completion on mbarriers (expect-tx bytes);
-//   warp 1      MMA issuer: one elected thread issues tcgen05.mma (M=128, N=BN, K=16) from shared-memory
+//   warp 1      MMA issuer: warp-uniform code, one elected lane issues tcgen05.mma (M=128, N=BN, K=16) from shared-memory
 //               descriptors into a TMEM accumulator, tcgen05.commit releases the stage / publishes the tile;
 //   warps 2..5  epilogue: tcgen05.ld of the accumulator (each warp its lane quarter), convert, write a
 //               128-byte swizzled staging tile, TMA store (or TMA reduce-add for fp32 accumulation).
@@ -386,9 +386,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      uint32_t it = 0, tile_iter = 0;
+    // ------------------------------------------------------------------ MMA issuer (every lane runs the loop, one lane's instructions count)
+    {
+      const bool el = elect_one();
+      uint32_t s = 0, ph = 0, tile_iter = 0;  // ring position and phase, counted along
       bool ok = true;
       const uint32_t a_step = p.a_mn ? (16 * 128) >> 4 : 32 >> 4;  // descriptor start-address step per UMMA_K = 16
       const uint32_t b_step = p.b_mn ? (16 * 128) >> 4 : 32 >> 4;
@@ -397,12 +398,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const int ks = item % p.k_splits;
         const int kb0 = ks * p.kblocks_per_split, kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
         const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = item; break; }
+        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1;
-          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = item; break; }
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(stage_base + s * C::kStageBytes), sb = sa + C::kStageBytesA;
           const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
@@ -410,22 +410,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             // scales of this stage: shared memory -> tensor memory (tcgen05 operations of one thread execute in order, so the
             // copy neither overtakes the previous stage's MMAs nor is overtaken by the ones below)
             const uint32_t sf_tmem = tmem_base + C::kSfCol;
-            tmem_cp_32x128b_warpx4(sf_tmem, make_smem_desc_noswizzle(sa + C::kOperandBytes, 0, 128));
+            tmem_cp_32x128b_warpx4_elect(el, sf_tmem, make_smem_desc_noswizzle(sa + C::kOperandBytes, 0, 128));
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j)
-              tmem_cp_32x128b_warpx4(sf_tmem + 4 + 4 * j, make_smem_desc_noswizzle(sa + C::kOperandBytes + 512 + 512 * j, 0, 128));
+              tmem_cp_32x128b_warpx4_elect(el, sf_tmem + 4 + 4 * j, make_smem_desc_noswizzle(sa + C::kOperandBytes + 512 + 512 * j, 0, 128));
 #pragma unroll
             for (uint32_t k = 0; k < 4; ++k)  // 4 x K = 32 (32 bytes of every 128-byte row); scale byte k of each column
-              umma_mxf8(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), p.idesc | (k << 4) | (k << 29),
+              umma_mxf8_elect(el, d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), p.idesc | (k << 4) | (k << 29),
                         sf_tmem | (k << 30), (sf_tmem + 4) | (k << 30), (kb > kb0 || k > 0) ? 1u : 0u);
           } else {
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
-              umma_f16(d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+              umma_f16_elect(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(bar_empty + 8 * s);  // the stage is free once these MMAs have read it
+          umma_commit_elect(el, bar_empty + 8 * s);  // the stage is free once these MMAs have read it
+          if (++s == C::kStages) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(bar_tfull + 8 * acc);  // accumulator complete
+        if (ok) umma_commit_elect(el, bar_tfull + 8 * acc);  // accumulator complete
       }
     }
   } else {

@@ -152,13 +152,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(leader_bar), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+__device__ __forceinline__ void umma_f16_pair(bool elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %5, 0;\n@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"((uint32_t)elected) : "memory");
 }
 // Arrive on ONE mbarrier (a shared::cluster address, own or the peer's) once the pair MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
+__device__ __forceinline__ void umma_commit_pair(bool elected, uint32_t cluster_bar) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}"
+               ::"r"(cluster_bar), "r"((uint32_t)elected) : "memory");
 }
 
 // BF16: the 16-bit format of operands and output (false = fp16). A template parameter rather than a launch argument so that the
@@ -263,9 +265,10 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
-      uint32_t it = 0, tile_iter = 0;
+    // ------------------------------------------------------------------ MMA issuer (leader CTA only; warp-uniform, see umma_f16_elect)
+    if (rank == 0) {
+      const bool el = elect_one();
+      uint32_t s = 0, ph = 0, tile_iter = 0;  // ring position and phase, counted along
       bool ok = true;
       const uint32_t a_step = p.a_mn ? (16 * 128) >> 4 : 32 >> 4, b_step = p.b_mn ? (16 * 128) >> 4 : 32 >> 4;
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
@@ -274,24 +277,24 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int ks = item % p.k_splits;
         const int kb0 = ks * p.kblocks_per_split, kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
         const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = item; break; }
+        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % kStages, ph = (it / kStages) & 1;
-          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = item; break; }
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(stage_base + s * kStageBytes), sb = sa + kStageBytesA;
           const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16_pair(d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(bar_empty + 8 * s);    // this CTA's stage is free once the MMAs have read it
-          umma_commit_pair(peer_empty + 8 * s);   // ... and so is the peer's
+            umma_f16_pair(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(el, bar_empty + 8 * s);    // this CTA's stage is free once the MMAs have read it
+          umma_commit_pair(el, peer_empty + 8 * s);   // ... and so is the peer's
+          if (++s == kStages) { s = 0; ph ^= 1; }
         }
         if (ok) {
-          umma_commit_pair(bar_tfull + 8 * acc);
-          umma_commit_pair(peer_tfull + 8 * acc);
+          umma_commit_pair(el, bar_tfull + 8 * acc);
+          umma_commit_pair(el, peer_tfull + 8 * acc);
         }
       }
     }

@@ -234,13 +234,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc], 16-bit inputs, fp32 accumulate; one thread issues.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// A operand from tensor memory (e.g. softmax probabilities written back with tcgen05.st).
-// The same from WARP-UNIFORM code: every lane of the issuing warp runs the loop and the waits, and only the elected lane's
+// D[tmem] (+)= A[smem desc] * B[smem desc], 16-bit inputs, fp32 accumulate, from WARP-UNIFORM code: every lane of the issuing warp runs the loop and the waits, and only the elected lane's
 // instruction takes effect. tcgen05.mma reads its descriptors from uniform registers; inside a one-lane branch each of them has
 // to be moved there from a lane's registers first, and the issuing thread, not the tensor core, sets the pace (see flash_bwd.cu).
 __device__ __forceinline__ void umma_f16_elect(bool elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -255,16 +249,17 @@ __device__ __forceinline__ void umma_f16_ts_elect(bool elected, uint32_t d_tmem,
 // row; K = 32 per instruction. The scales sit in tensor memory (32-bit column c, lane l holds the 4 scale bytes of row
 // 32 c' + l of 4 consecutive K blocks, replicated over the four lane quarters); the byte used is picked by the scale ids in
 // the instruction descriptor AND by bits 30-31 of the scale addresses.
-__device__ __forceinline__ void umma_mxf8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem,
+__device__ __forceinline__ void umma_mxf8_elect(bool elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem,
                                           uint32_t sfb_tmem, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-               "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n}"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem) : "memory");
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nsetp.ne.b32 q, %7, 0;\n"
+               "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n}"
+               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem), "r"((uint32_t)elected) : "memory");
 }
 // Shared memory -> tensor memory copy of 32 rows x 16 bytes, broadcast to the four lane quarters: the scale factors of 128
 // rows x 4 K-blocks (row r at byte (r % 32) * 16 + (r / 32) * 4 of the 512-byte chunk) land in 4 columns.
-__device__ __forceinline__ void tmem_cp_32x128b_warpx4(uint32_t taddr, uint64_t smem_desc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
+__device__ __forceinline__ void tmem_cp_32x128b_warpx4_elect(bool elected, uint32_t taddr, uint64_t smem_desc) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %2, 0;\n@q tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n}"
+               ::"r"(taddr), "l"(smem_desc), "r"((uint32_t)elected) : "memory");
 }
 // Descriptor of an unswizzled K-major block whose 8-row groups of 16-byte rows are `sbo_bytes` apart (128 when contiguous).
 __device__ __forceinline__ uint64_t make_smem_desc_noswizzle(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -289,9 +284,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 __device__ __forceinline__ void umma_commit_elect(bool elected, uint32_t bar) {
   asm volatile("{\n.reg .pred q;\nsetp.ne.b32 q, %1, 0;\n@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}"
                ::"r"(bar), "r"((uint32_t)elected) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread (thread t reads lane t of the
