@@ -589,12 +589,12 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   NNB_REQUIRE(!accumulate || out_f32 || mode == 1, "gemm: accumulate needs an fp32 output");
   const CUtensorMapDataType in_dt = dtype == NNB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const int sms = max_ctas > 0 ? min(max_ctas, nnb_num_sms()) : nnb_num_sms();
-  // CTA-pair kernel (gemm2.cu): 256 x 256 tiles over two SMs. Measured faster than the single-CTA tiles at every shape of
-  // the 114M model (1-20 %: K = 768 with any N, or N = 768 with any K), slower when N and K are both large (the 1.3B
-  // shapes: 32768 x 2048 x 5632 runs at 1166 vs 1428 TFLOP/s; 8192^3 at 1233 vs 1274), where the single-CTA kernel stays.
+  // CTA-pair kernel (gemm2.cu): 256 x 256 tiles over two SMs, for every problem that has one. Measured (us, pair / 256-wide / 128-wide
+  // single-CTA tiles, alternating runs): 8192 x 2048 x 5632 169 / 183 / 232, 8192^3 736 / 814 / 1237, 32768 x 2048 x 5632
+  // 472 / 507 / 780, 4096 x 768 x 50304 255 / 292 / 416, 16384 x 768 x 4096 87 / 99 / 134; below about 512 x 4096 x 768 all
+  // three take the 13-16 us of a launch. Weight gradients likewise (11264 x 2048 x 8192: 318 / 359).
   static const bool pair_enabled = [] { const char* e = getenv("NANONEMO_GEMM_PAIR"); return !(e && e[0] == '0'); }();
-  const bool big_cube = M >= 2048 && N >= 2048 && K >= 2048;
-  if (mode == 0 && (bn_hint == 512 || (bn_hint == 0 && pair_enabled && M >= 256 && N >= 256 && !big_cube))) {
+  if (mode == 0 && (bn_hint == 512 || (bn_hint == 0 && pair_enabled && M >= 256 && N >= 256))) {
     const NnbGemm2Args g{A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, dtype, out_f32, accumulate, k_splits, max_ctas, status};
     const int rc = nnb_gemm2_launch(g, st);
     if (rc <= 0) return rc;  // 1 = shape not served: fall through to the single-CTA kernel
@@ -630,15 +630,7 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   if (out_f32 && mode == 0) {
     if (k_splits > 0) splits = k_splits;
     else {
-      // makespan of `tiles * s` equal items on `sms` persistent CTAs is ceil(tiles * s / sms) / s of the
-      // whole K loop; take the split count that minimises it (ties: fewer splits = less reduce traffic)
-      const long long tiles = (long long)p.m_blocks * p.n_blocks;
-      const int s_max = max(1, min(32, p.kblocks_total / 4));
-      double best = 1e30;
-      for (int sp = 1; sp <= s_max; ++sp) {
-        const double cost = (double)((tiles * sp + sms - 1) / sms) / sp + 0.002 * sp;
-        if (cost < best - 1e-9) { best = cost; splits = sp; }
-      }
+      splits = nnb_pick_k_splits((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total, 0.5, (double)M * N * 4, accumulate != 0);
     }
     splits = max(1, min(splits, p.kblocks_total));
   }
@@ -865,13 +857,7 @@ extern "C" int nnb_gemm_mxfp8(const void* A, const void* sfa, const void* B, con
   if (out_f32) {
     if (k_splits > 0) splits = k_splits;
     else {
-      const long long tiles = (long long)p.m_blocks * p.n_blocks;
-      const int s_max = max(1, min(32, p.kblocks_total / 4));
-      double best = 1e30;
-      for (int sp = 1; sp <= s_max; ++sp) {
-        const double cost = (double)((tiles * sp + sms - 1) / sms) / sp + 0.002 * sp;
-        if (cost < best - 1e-9) { best = cost; splits = sp; }
-      }
+      splits = nnb_pick_k_splits((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total, 0.3, (double)M * N * 4, accumulate != 0);
     }
     splits = max(1, min(splits, p.kblocks_total));
   }

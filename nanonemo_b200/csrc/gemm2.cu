@@ -709,13 +709,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   if (a.out_f32) {
     if (a.k_splits > 0) splits = a.k_splits;
     else {
-      const long long tiles = (long long)p.m_pairs * p.n_blocks;
-      const int s_max = max(1, min(32, p.kblocks_total / 4));
-      double best = 1e30;
-      for (int sp = 1; sp <= s_max; ++sp) {
-        const double cost = (double)((tiles * sp + pairs - 1) / pairs) / sp + 0.002 * sp;
-        if (cost < best - 1e-9) { best = cost; splits = sp; }
-      }
+      splits = nnb_pick_k_splits((long long)p.m_pairs * p.n_blocks, pairs, p.kblocks_total, 0.5, (double)a.M * a.N * 4, a.accumulate != 0);
     }
     splits = max(1, min(splits, p.kblocks_total));
   }

@@ -35,3 +35,20 @@ struct NnbGemm2Args {
 
 // Returns 0 on success, 1 when the shape is not served by the pair kernel (caller falls back), < 0 on error.
 int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st);
+
+// K splits of an fp32-output product of `tiles` tiles on `workers` persistent CTAs (or pairs). Splitting evens out the last wave
+// (ceil(tiles s / workers) / s of a whole tile's K loop) but adds the output's bytes once more per split, and a cleared output
+// where the product does not accumulate. Measured: a k-block of a tile takes `us_per_kblock`, a megabyte reduce-added about
+// 0.1 us. With that traffic left out of the count, 50304 x 2048 x 8192 took 8 splits and 1859 us (1 split: 1320), 11264 x 2048 x
+// 8192 486 us (318); 4096 x 768 x 32768 keeps its 3 splits (142 us, 1 split: 186), 768 x 768 x 32768 its 8 (39, 172).
+inline int nnb_pick_k_splits(long long tiles, int workers, int kblocks, double us_per_kblock, double out_bytes, bool accumulate) {
+  const double us_tile = kblocks * us_per_kblock, us_out = out_bytes * 1e-7;
+  const int s_max = kblocks / 4 < 1 ? 1 : (kblocks / 4 > 32 ? 32 : kblocks / 4);
+  int best_s = 1;
+  double best = 1e30;
+  for (int s = 1; s <= s_max; ++s) {
+    const double cost = (double)((tiles * s + workers - 1) / workers) / s * us_tile + s * us_out + (s > 1 && !accumulate ? us_out + 2.0 : 0.0);
+    if (cost < best - 1e-9) { best = cost; best_s = s; }
+  }
+  return best_s;
+}

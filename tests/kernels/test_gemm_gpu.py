@@ -91,6 +91,26 @@ def test_cta_pair_kernel(layout, M, N, K):
     _check(out, ref, K)
 
 
+@pytest.mark.parametrize("M,N,K", [(2048, 2048, 2048), (2056, 2304, 2120), (255, 4096, 768), (256, 256, 2048), (4104, 768, 8200), (768, 776, 4104)])
+def test_default_dispatch(M, N, K):
+    """The kernel and the K splits that the rules pick, on both sides of their lines: large in all three sizes, one row short of a
+    pair tile, one pair tile, few tiles with a long K (several splits when the output is fp32), K no multiple of a k-block."""
+    from nanonemo_b200.ops.gemm import check_status, gemm
+
+    torch.manual_seed(M + N + K)
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    at, bt = a.t().contiguous() if M % 8 == 0 else None, b.t().contiguous()
+    ref = _ref(a, b, False, False)
+    outs = [gemm(a, b), gemm(a, bt, b_mn=True), gemm(a, b, out_dtype=torch.float32)]
+    if at is not None:
+        acc = torch.ones(M, N, device=DEV)
+        gemm(at, bt, a_mn=True, b_mn=True, out=acc, accumulate=True)
+        outs += [gemm(at, bt, a_mn=True, b_mn=True, out_dtype=torch.float32), acc - 1]
+    check_status()
+    for out in outs:
+        _check(out, ref, K)
+
+
 def test_strided_views_and_bn128():
     from nanonemo_b200.ops.gemm import check_status, gemm
 
