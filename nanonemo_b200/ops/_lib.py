@@ -9,6 +9,7 @@ library sits in the source tree. Every launcher returns 0 on success or a negati
 """
 
 import ctypes
+import operator
 import os
 from functools import lru_cache
 from pathlib import Path
@@ -40,18 +41,77 @@ def lib():
     return handle
 
 
+# Argument types of every launcher (p pointer, i int, q long long, f float, d double), in the order of its C declaration. With
+# them a call passes plain Python numbers; wrapping each of a launcher's 10 to 45 arguments in a ctypes object first took longer
+# than the launch itself.
+_SIGNATURES = {
+    "nnb_sumsq_blocks": "",
+    "nnb_sumsq_f32": "pqppip",
+    "nnb_adamw_flat": "ppppppqfffffipfiip",
+    "nnb_sumsq_f32_noalloc": "pqpp",
+    "nnb_ce_inplace": "pppqiqfip",
+    "nnb_ce_grad_from_stats": "pppipqiqfip",
+    "nnb_ce_loss_from_stats": "pipppqip",
+    "nnb_ce_stats": "pppqiqqip",
+    "nnb_ce_grad_vp": "ppppqiqqqifip",
+    "nnb_comm_timeout_probe": "pppiip",
+    "nnb_comm_flag_words": "i",
+    "nnb_allreduce_f32": "ppppppiiqqfiidp",
+    "nnb_sumsq_combine": "pqpp",
+    "nnb_reduce_scatter_f32": "pppppppiiqqfiidp",
+    "nnb_reduce_scatter_adamw": "ppppppppppiiqqfiidfffffiip",
+    "nnb_allgather_bytes": "pppppiiqqidp",
+    "nnb_peer_fetch": "pppippiiidp",
+    "nnb_vp_embedding_fwd": "pppppqiqqippiiidp",
+    "nnb_vp_embedding_bwd": "pppppqiqqippiiidp",
+    "nnb_add_rmsnorm_fwd": "ppppppiifiiip",
+    "nnb_rmsnorm_bwd_blocks": "",
+    "nnb_add_rmsnorm_bwd": "pppppppppiiiiiip",
+    "nnb_rope_packed": "ppppqiiiiqqfip",
+    "nnb_swiglu_fwd": "pppqiqqqip",
+    "nnb_swiglu_bwd": "pppppqiqqqqqip",
+    "nnb_embedding_fwd": "pppqiiip",
+    "nnb_embedding_bwd": "pppqiiip",
+    "nnb_warmup_add": "pppqp",
+    "nnb_cast_from_f32": "ppqip",
+    "nnb_build_arch": "",
+    "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfipppp",
+    "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
+    "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
+    "nnb_gemm_swiglu": "ppppiiiqqqqipp",
+    "nnb_gemm_rope": "pppppiiiqqqiiiipp",
+    "nnb_gemm_swiglu_bwd": "ppppiiiqqqqipp",
+    "nnb_gemm_ce_stats": "ppppiiiqqqipp",
+    "nnb_gemm_ce_loss": "pppppiiiqqipp",
+    "nnb_gemm_rs_bf16": "ppppppiiiiiiqqqiiipp",
+    "nnb_ag_gemm_bf16": "ppppppiiiiiiiqqiipp",
+    "nnb_gather_b_gemm_bf16": "pppppppiiiiqqqiiiqqipp",
+    "nnb_gemm_mxfp8": "pppppiiiqqqiiiipp",
+    "nnb_mxfp8_quantize_sw": "pqpqppqpiip",
+    "nnb_mxfp8_fake_quant": "ppqiqqp",
+    "nnb_mxfp8_quantize": "pppqiqqp",
+}
+_TYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "q": ctypes.c_longlong, "f": ctypes.c_float, "d": ctypes.c_double}
+
+
+@lru_cache(maxsize=None)
+def _launcher(name: str):
+    fn = getattr(lib(), name)
+    fn.argtypes = [_TYPES[c] for c in _SIGNATURES[name]]
+    return fn
+
+
 LAUNCHES = 0  # launchers called through `call` since import (the benchmark reports the delta)
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # torch.cuda.current_stream() without its Python objects
 
 
 def call(name: str, *args) -> None:
     """Call launcher `name`; raises with the library's message on a non-zero return."""
     global LAUNCHES
-    fn = getattr(lib(), name)
-    rc = fn(*args)
+    rc = _launcher(name)(*args)
     LAUNCHES += 1
     if rc != 0:
         msg = lib().nnb_last_error()
@@ -61,7 +121,7 @@ def call(name: str, *args) -> None:
 def call_rc(name: str, *args) -> int:
     """Like `call`, for launchers that answer 1 when they do not serve the problem (nothing was launched): returns 0 or 1."""
     global LAUNCHES
-    rc = getattr(lib(), name)(*args)
+    rc = _launcher(name)(*args)
     if rc == 0:
         LAUNCHES += 1
     elif rc != 1:
@@ -70,8 +130,13 @@ def call_rc(name: str, *args) -> int:
     return rc
 
 
-def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-i32, i64, f32, vp = ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p
+i32 = i64 = operator.index  # an integer, as it is (anything else raises)
+f32 = float
+
+
+def vp(address: int | None) -> int | None:
+    return address  # None is the null pointer

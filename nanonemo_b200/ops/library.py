@@ -32,12 +32,31 @@ from nanonemo_b200.ops import adamw as adamw_mod, attention, embed as embed_mod,
 NS = "nanonemo_b200"
 
 
+def _operator(fn):
+    """Register `fn` as the CUDA kernel of operator NS::<its name>, with the schema of its annotations. This is
+    ``torch.library.custom_op`` without the wrapper that checks every call's results for aliases of its arguments (the kernels
+    below return new tensors only), which took longer than a small launch: the 87 operator calls of a 201-token forward of the
+    114M model took 6.3 ms on the host with it and with ctypes objects for every argument (_lib.py), and 4.6 ms without."""
+    name = f"{NS}::{fn.__name__}"
+    torch.library.define(name, torch.library.infer_schema(fn, mutates_args=()), tags=(torch.Tag.pt2_compliant_tag,))
+    torch.library.impl(name, "cuda", torch.compiler.disable(fn))
+    return getattr(torch.ops.nanonemo_b200, fn.__name__).default
+
+
+def _fake(op):
+    return torch.library.register_fake(op.name())
+
+
+def _autograd(op, backward, setup_context):
+    torch.library.register_autograd(op.name(), backward, setup_context=setup_context)
+
+
 # ----------------------------------------------------------------------------- add + RMSNorm
 _DT = {0: torch.float32, 1: torch.bfloat16, 2: torch.float16}
 _DT_CODE = {v: k for k, v in _DT.items()}
 
 
-@torch.library.custom_op(f"{NS}::add_rms_norm", mutates_args=(), device_types="cuda")
+@_operator
 def add_rms_norm(x: Tensor, delta: Tensor | None, weight: Tensor, eps: float, y_code: int = -1) -> tuple[Tensor, Tensor, Tensor]:
     """(y, h, rstd): h = x + delta (x itself without a delta), y = rmsnorm(h) * weight in dtype code y_code (0 fp32, 1 bf16,
     2 fp16; -1 = the delta's dtype, or x's without a delta)."""
@@ -46,21 +65,21 @@ def add_rms_norm(x: Tensor, delta: Tensor | None, weight: Tensor, eps: float, y_
     return y, (h if delta is not None else h.clone()), rstd
 
 
-@add_rms_norm.register_fake
+@_fake(add_rms_norm)
 def _(x, delta, weight, eps, y_code=-1):
     y_dtype = _DT[y_code] if y_code >= 0 else (delta.dtype if delta is not None else x.dtype)
     return (x.new_empty(x.shape, dtype=y_dtype), torch.empty_like(x, memory_format=torch.contiguous_format),
             x.new_empty(x.numel() // x.shape[-1], dtype=torch.float32))
 
 
-@torch.library.custom_op(f"{NS}::add_rms_norm_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def add_rms_norm_bwd(dy: Tensor, dh: Tensor | None, h: Tensor, rstd: Tensor, weight: Tensor, delta_code: int) -> tuple[Tensor, Tensor, Tensor]:
     """(dx, ddelta, dw); ddelta has dtype code delta_code (when it equals the residual dtype it is a copy of dx)."""
     dx, ddelta, dw = rmsnorm.bwd(dy, h, rstd, weight, dh, _DT[delta_code])
     return dx, ddelta if ddelta is not dx else dx.clone(), dw
 
 
-@add_rms_norm_bwd.register_fake
+@_fake(add_rms_norm_bwd)
 def _(dy, dh, h, rstd, weight, delta_code):
     return torch.empty_like(h), h.new_empty(h.shape, dtype=_DT[delta_code]), weight.new_empty(weight.shape, dtype=torch.float32)
 
@@ -82,11 +101,11 @@ def _arn_backward(ctx, dy, dh, _drstd):
     return dx, (ddelta if ctx.has_delta else None), dw.to(weight.dtype), None, None
 
 
-add_rms_norm.register_autograd(_arn_backward, setup_context=_arn_setup)
+_autograd(add_rms_norm, _arn_backward, setup_context=_arn_setup)
 
 
 # ----------------------------------------------------------------------------- SwiGLU (packed gate || up)
-@torch.library.custom_op(f"{NS}::swiglu", mutates_args=(), device_types="cuda")
+@_operator
 def swiglu(gu: Tensor) -> Tensor:
     F = gu.shape[-1] // 2
     gu2 = swiglu_act._rows(gu)
@@ -95,12 +114,12 @@ def swiglu(gu: Tensor) -> Tensor:
     return out.view(*gu.shape[:-1], F)
 
 
-@swiglu.register_fake
+@_fake(swiglu)
 def _(gu):
     return gu.new_empty((*gu.shape[:-1], gu.shape[-1] // 2))
 
 
-@torch.library.custom_op(f"{NS}::swiglu_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def swiglu_bwd(dy: Tensor, gu: Tensor) -> Tensor:
     F = gu.shape[-1] // 2
     gu2, dy2 = swiglu_act._rows(gu), swiglu_act._rows(dy)
@@ -109,17 +128,17 @@ def swiglu_bwd(dy: Tensor, gu: Tensor) -> Tensor:
     return dgu.view(gu.shape)
 
 
-@swiglu_bwd.register_fake
+@_fake(swiglu_bwd)
 def _(dy, gu):
     return torch.empty_like(gu, memory_format=torch.contiguous_format)
 
 
-swiglu.register_autograd(lambda ctx, dy: swiglu_bwd(dy.contiguous(), ctx.saved_tensors[0]),
+_autograd(swiglu, lambda ctx, dy: swiglu_bwd(dy.contiguous(), ctx.saved_tensors[0]),
                          setup_context=lambda ctx, inputs, output: ctx.save_for_backward(inputs[0]))
 
 
 # ----------------------------------------------------------------------------- RoPE on the packed projection
-@torch.library.custom_op(f"{NS}::rope_qkv", mutates_args=(), device_types="cuda")
+@_operator
 def rope_qkv(qkv: Tensor, cos: Tensor, sin: Tensor, n_heads: int, n_kv_heads: int, head_dim: int, sign: float = 1.0) -> Tensor:
     B, T, C = qkv.shape
     x2 = qkv.reshape(B * T, C)
@@ -130,7 +149,7 @@ def rope_qkv(qkv: Tensor, cos: Tensor, sin: Tensor, n_heads: int, n_kv_heads: in
     return out.view(B, T, C)
 
 
-@rope_qkv.register_fake
+@_fake(rope_qkv)
 def _(qkv, cos, sin, n_heads, n_kv_heads, head_dim, sign=1.0):
     return torch.empty_like(qkv, memory_format=torch.contiguous_format)
 
@@ -147,7 +166,7 @@ def _rope_backward(ctx, dout):
     return rope_qkv(dout.contiguous(), cos, sin, H, KVH, hd, -sign), None, None, None, None, None, None
 
 
-rope_qkv.register_autograd(_rope_backward, setup_context=_rope_setup)
+_autograd(rope_qkv, _rope_backward, setup_context=_rope_setup)
 
 
 # ----------------------------------------------------------------------------- FlashAttention on the packed projection
@@ -157,7 +176,7 @@ def _split(qkv, H, KVH, hd):
             qkv[..., (H + KVH) * hd:].view(B, T, KVH, hd))
 
 
-@torch.library.custom_op(f"{NS}::flash_attn_packed", mutates_args=(), device_types="cuda")
+@_operator
 def flash_attn_packed(qkv: Tensor, n_heads: int, n_kv_heads: int, head_dim: int) -> tuple[Tensor, Tensor]:
     qkv = qkv.contiguous()
     B, T, _ = qkv.shape
@@ -167,13 +186,13 @@ def flash_attn_packed(qkv: Tensor, n_heads: int, n_kv_heads: int, head_dim: int)
     return o.view(B, T, n_heads * head_dim), lse
 
 
-@flash_attn_packed.register_fake
+@_fake(flash_attn_packed)
 def _(qkv, n_heads, n_kv_heads, head_dim):
     B, T, _ = qkv.shape
     return qkv.new_empty((B, T, n_heads * head_dim)), qkv.new_empty((B, n_heads, T), dtype=torch.float32)
 
 
-@torch.library.custom_op(f"{NS}::flash_attn_packed_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def flash_attn_packed_bwd(do: Tensor, qkv: Tensor, o: Tensor, lse: Tensor, n_heads: int, n_kv_heads: int, head_dim: int) -> Tensor:
     qkv, do = qkv.contiguous(), do.contiguous()
     B, T, _ = qkv.shape
@@ -184,7 +203,7 @@ def flash_attn_packed_bwd(do: Tensor, qkv: Tensor, o: Tensor, lse: Tensor, n_hea
     return dqkv
 
 
-@flash_attn_packed_bwd.register_fake
+@_fake(flash_attn_packed_bwd)
 def _(do, qkv, o, lse, n_heads, n_kv_heads, head_dim):
     return torch.empty_like(qkv, memory_format=torch.contiguous_format)
 
@@ -201,17 +220,17 @@ def _fa_backward(ctx, do, _dlse):
     return flash_attn_packed_bwd(do, qkv, o, lse, *ctx.meta), None, None, None
 
 
-flash_attn_packed.register_autograd(_fa_backward, setup_context=_fa_setup)
+_autograd(flash_attn_packed, _fa_backward, setup_context=_fa_setup)
 
 
 # ----------------------------------------------------------------------------- linear (tcgen05 GEMM), 16-bit weight
-@torch.library.custom_op(f"{NS}::matmul_nt", mutates_args=(), device_types="cuda")
+@_operator
 def matmul_nt(a: Tensor, b: Tensor, a_mn: bool = False, b_mn: bool = False, out_f32: bool = False) -> Tensor:
     """a @ b^T with the operand layouts of csrc/gemm.cu (a_mn / b_mn: the operand is stored transposed)."""
     return gemm_mod.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32 if out_f32 else None)
 
 
-@matmul_nt.register_fake
+@_fake(matmul_nt)
 def _(a, b, a_mn=False, b_mn=False, out_f32=False):
     M = a.shape[1] if a_mn else a.shape[0]
     N = b.shape[1] if b_mn else b.shape[0]
@@ -232,7 +251,7 @@ def _mm_backward(ctx, dy):
     return da, db, None, None, None
 
 
-matmul_nt.register_autograd(_mm_backward, setup_context=_mm_setup)
+_autograd(matmul_nt, _mm_backward, setup_context=_mm_setup)
 
 
 
@@ -242,13 +261,13 @@ def _w16(weight: Tensor, dtype: torch.dtype) -> Tensor:
     return weight if weight.dtype == dtype else weight.to(dtype)
 
 
-@torch.library.custom_op(f"{NS}::linear_w", mutates_args=(), device_types="cuda")
+@_operator
 def linear_w(x2: Tensor, weight: Tensor) -> Tensor:
     """x2 [M, K] (16-bit) @ weight [N, K]^T; an fp32 weight is cast to x2's dtype for the product."""
     return gemm_mod.gemm(x2, _w16(weight, x2.dtype))
 
 
-@linear_w.register_fake
+@_fake(linear_w)
 def _(x2, weight):
     return x2.new_empty((x2.shape[0], weight.shape[0]))
 
@@ -265,7 +284,7 @@ def _linw_backward(ctx, dy):
     return dx, dw.to(weight.dtype)
 
 
-linear_w.register_autograd(_linw_backward, setup_context=_linw_setup)
+_autograd(linear_w, _linw_backward, setup_context=_linw_setup)
 
 
 def linear(x: Tensor, weight: Tensor) -> Tensor:
@@ -277,7 +296,7 @@ def linear(x: Tensor, weight: Tensor) -> Tensor:
 
 
 # ----------------------------------------------------------------------------- RoPE on 2-D rows (any column count, in / out of place)
-@torch.library.custom_op(f"{NS}::rope_rows", mutates_args=(), device_types="cuda")
+@_operator
 def rope_rows(x2: Tensor, cos: Tensor, sin: Tensor, t_len: int, n_rot_heads: int, head_dim: int, sign: float) -> Tensor:
     """Rotate-half on the first n_rot_heads heads of every row (row m at position m % t_len), other columns copied."""
     x2 = x2 if x2.stride(-1) == 1 else x2.contiguous()
@@ -286,7 +305,7 @@ def rope_rows(x2: Tensor, cos: Tensor, sin: Tensor, t_len: int, n_rot_heads: int
     return out
 
 
-@rope_rows.register_fake
+@_fake(rope_rows)
 def _(x2, cos, sin, t_len, n_rot_heads, head_dim, sign):
     return torch.empty_like(x2, memory_format=torch.contiguous_format)
 
@@ -303,11 +322,11 @@ def _rr_backward(ctx, dout):
     return rope_rows(dout.contiguous(), cos, sin, t_len, n_rot, hd, -sign), None, None, None, None, None, None
 
 
-rope_rows.register_autograd(_rr_backward, setup_context=_rr_setup)
+_autograd(rope_rows, _rr_backward, setup_context=_rr_setup)
 
 
 # ----------------------------------------------------------------------------- GEMMs with a fused epilogue
-@torch.library.custom_op(f"{NS}::gemm_rope", mutates_args=(), device_types="cuda")
+@_operator
 def gemm_rope(x2: Tensor, weight: Tensor, cos: Tensor, sin: Tensor, t_len: int, rope_cols: int, head_dim: int) -> Tensor:
     """x2 @ weight^T with RoPE on columns [0, rope_cols) in the GEMM epilogue (plain GEMM + RoPE kernel for shapes the
     fused kernel does not serve: same result)."""
@@ -319,7 +338,7 @@ def gemm_rope(x2: Tensor, weight: Tensor, cos: Tensor, sin: Tensor, t_len: int, 
     return out
 
 
-@gemm_rope.register_fake
+@_fake(gemm_rope)
 def _(x2, weight, cos, sin, t_len, rope_cols, head_dim):
     return x2.new_empty((x2.shape[0], weight.shape[0]))
 
@@ -339,10 +358,10 @@ def _gr_backward(ctx, dout):
     return dx, dw.to(weight.dtype), None, None, None, None, None
 
 
-gemm_rope.register_autograd(_gr_backward, setup_context=_gr_setup)
+_autograd(gemm_rope, _gr_backward, setup_context=_gr_setup)
 
 
-@torch.library.custom_op(f"{NS}::gemm_swiglu", mutates_args=(), device_types="cuda")
+@_operator
 def gemm_swiglu(x2: Tensor, weight: Tensor) -> tuple[Tensor, Tensor]:
     """(gu, act): gu = x2 @ weight^T with gate columns first, act = silu(gate) * up written by the GEMM epilogue."""
     w16 = _w16(weight, x2.dtype)
@@ -356,7 +375,7 @@ def gemm_swiglu(x2: Tensor, weight: Tensor) -> tuple[Tensor, Tensor]:
     return gu, act
 
 
-@gemm_swiglu.register_fake
+@_fake(gemm_swiglu)
 def _(x2, weight):
     return x2.new_empty((x2.shape[0], weight.shape[0])), x2.new_empty((x2.shape[0], weight.shape[0] // 2))
 
@@ -378,11 +397,11 @@ def _gs_backward(ctx, dgu, dact):
     return dx, dw.to(weight.dtype)
 
 
-gemm_swiglu.register_autograd(_gs_backward, setup_context=_gs_setup)
+_autograd(gemm_swiglu, _gs_backward, setup_context=_gs_setup)
 
 
 # ----------------------------------------------------------------------------- embedding
-@torch.library.custom_op(f"{NS}::embedding", mutates_args=(), device_types="cuda")
+@_operator
 def embedding(idx: Tensor, weight: Tensor, fp32_out: bool = True) -> Tensor:
     """weight[idx] from the fp32 table, written in fp32 or bf16 (the dtype of the residual stream)."""
     w = weight if weight.dtype == torch.float32 else weight.float()
@@ -390,12 +409,12 @@ def embedding(idx: Tensor, weight: Tensor, fp32_out: bool = True) -> Tensor:
     return out
 
 
-@embedding.register_fake
+@_fake(embedding)
 def _(idx, weight, fp32_out=True):
     return weight.new_empty((*idx.shape, weight.shape[1]), dtype=torch.float32 if fp32_out else torch.bfloat16)
 
 
-@torch.library.custom_op(f"{NS}::embedding_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def embedding_bwd(idx: Tensor, dout: Tensor, vocab: int) -> Tensor:
     """fp32 [vocab, D] with dout's rows added at idx (rows that repeat are summed)."""
     flat = idx.reshape(-1)
@@ -405,7 +424,7 @@ def embedding_bwd(idx: Tensor, dout: Tensor, vocab: int) -> Tensor:
     return dW
 
 
-@embedding_bwd.register_fake
+@_fake(embedding_bwd)
 def _(idx, dout, vocab):
     return dout.new_empty((vocab, dout.shape[-1]), dtype=torch.float32)
 
@@ -421,11 +440,11 @@ def _emb_backward(ctx, dout):
     return None, embedding_bwd(idx, dout, ctx.vocab).to(ctx.w_dtype), None
 
 
-embedding.register_autograd(_emb_backward, setup_context=_emb_setup)
+_autograd(embedding, _emb_backward, setup_context=_emb_setup)
 
 
 # ----------------------------------------------------------------------------- fused linear + cross-entropy
-@torch.library.custom_op(f"{NS}::linear_ce", mutates_args=(), device_types="cuda")
+@_operator
 def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> tuple[Tensor, Tensor, Tensor]:
     """Mean cross-entropy of x2 @ weight^T against targets, and the gradients of that mean with respect to x2 (16-bit)
     and weight (fp32), all produced in the same pass (the logits exist one row chunk at a time, in 16 bits)."""
@@ -436,7 +455,7 @@ def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> t
     return loss_sum / x2.shape[0], dx, dW
 
 
-@linear_ce.register_fake
+@_fake(linear_ce)
 def _(x2, weight, targets, chunk_rows):
     return x2.new_empty((), dtype=torch.float32), torch.empty_like(x2), weight.new_empty(weight.shape, dtype=torch.float32)
 
@@ -454,17 +473,17 @@ def _lce_backward(ctx, dloss, _ddx, _ddw):
     return dx * dloss.to(dx.dtype), (dW * dloss).to(ctx.w_dtype), None, None
 
 
-linear_ce.register_autograd(_lce_backward, setup_context=_lce_setup)
+_autograd(linear_ce, _lce_backward, setup_context=_lce_setup)
 
 
-@torch.library.custom_op(f"{NS}::linear_ce_loss", mutates_args=(), device_types="cuda")
+@_operator
 def linear_ce_loss(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> Tensor:
     """The loss of ``linear_ce`` alone: no gradients, one product instead of three, no logits in memory."""
     tg = (targets if targets.dtype == torch.int64 else targets.long()).contiguous()
     return ce_mod.linear_ce_loss(x2, _w16(weight, x2.dtype).contiguous(), tg, chunk_rows) / x2.shape[0]
 
 
-@linear_ce_loss.register_fake
+@_fake(linear_ce_loss)
 def _(x2, weight, targets, chunk_rows):
     return x2.new_empty((), dtype=torch.float32)
 
@@ -497,7 +516,7 @@ def _(p, g, m, v, shadow, decay_flags, grad_norm_sq, lr, beta1, beta2, eps, weig
 
 
 # ----------------------------------------------------------------------------- SwiGLU on separate gate / up tensors
-@torch.library.custom_op(f"{NS}::swiglu_gu", mutates_args=(), device_types="cuda")
+@_operator
 def swiglu_gu(g: Tensor, u: Tensor) -> Tensor:
     g2, u2 = swiglu_act._rows(g), swiglu_act._rows(u)
     out = torch.empty((g2.shape[0], g2.shape[1]), dtype=g.dtype, device=g.device)
@@ -505,12 +524,12 @@ def swiglu_gu(g: Tensor, u: Tensor) -> Tensor:
     return out.view(g.shape)
 
 
-@swiglu_gu.register_fake
+@_fake(swiglu_gu)
 def _(g, u):
     return torch.empty_like(g, memory_format=torch.contiguous_format)
 
 
-@torch.library.custom_op(f"{NS}::swiglu_gu_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def swiglu_gu_bwd(dy: Tensor, g: Tensor, u: Tensor) -> tuple[Tensor, Tensor]:
     g2, u2, dy2 = swiglu_act._rows(g), swiglu_act._rows(u), swiglu_act._rows(dy)
     dg = torch.empty((g2.shape[0], g2.shape[1]), dtype=g.dtype, device=g.device)
@@ -519,12 +538,12 @@ def swiglu_gu_bwd(dy: Tensor, g: Tensor, u: Tensor) -> tuple[Tensor, Tensor]:
     return dg.view(g.shape), du.view(g.shape)
 
 
-@swiglu_gu_bwd.register_fake
+@_fake(swiglu_gu_bwd)
 def _(dy, g, u):
     return torch.empty_like(g, memory_format=torch.contiguous_format), torch.empty_like(g, memory_format=torch.contiguous_format)
 
 
-swiglu_gu.register_autograd(lambda ctx, dy: swiglu_gu_bwd(dy.contiguous(), *ctx.saved_tensors),
+_autograd(swiglu_gu, lambda ctx, dy: swiglu_gu_bwd(dy.contiguous(), *ctx.saved_tensors),
                             setup_context=lambda ctx, inputs, output: ctx.save_for_backward(*inputs))
 
 
@@ -536,7 +555,7 @@ def _bthd(t: Tensor) -> Tensor:
     return t if ok else t.contiguous()
 
 
-@torch.library.custom_op(f"{NS}::flash_attn", mutates_args=(), device_types="cuda")
+@_operator
 def flash_attn(q: Tensor, k: Tensor, v: Tensor) -> tuple[Tensor, Tensor]:
     """Causal GQA attention on bf16 q (B, H, T, hd), k / v (B, KVH, T, hd) -> (o (B, H, T, hd), lse (B, H, T))."""
     qt, kt, vt = _bthd(q), _bthd(k), _bthd(v)
@@ -546,13 +565,13 @@ def flash_attn(q: Tensor, k: Tensor, v: Tensor) -> tuple[Tensor, Tensor]:
     return o.transpose(1, 2), lse
 
 
-@flash_attn.register_fake
+@_fake(flash_attn)
 def _(q, k, v):
     B, H, T, hd = q.shape
     return q.new_empty((B, T, H, hd)).transpose(1, 2), q.new_empty((B, H, T), dtype=torch.float32)
 
 
-@torch.library.custom_op(f"{NS}::flash_attn_bwd", mutates_args=(), device_types="cuda")
+@_operator
 def flash_attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: Tensor) -> tuple[Tensor, Tensor, Tensor]:
     qt, kt, vt, ot, dot = _bthd(q), _bthd(k), _bthd(v), _bthd(o), _bthd(do)
     hd = qt.shape[-1]
@@ -563,7 +582,7 @@ def flash_attn_bwd(do: Tensor, q: Tensor, k: Tensor, v: Tensor, o: Tensor, lse: 
     return dq.transpose(1, 2), dk.transpose(1, 2), dv.transpose(1, 2)
 
 
-@flash_attn_bwd.register_fake
+@_fake(flash_attn_bwd)
 def _(do, q, k, v, o, lse):
     mk = lambda t: t.new_empty((t.shape[0], t.shape[2], t.shape[1], t.shape[3])).transpose(1, 2)
     return mk(q), mk(k), mk(v)
@@ -578,4 +597,4 @@ def _fl_backward(ctx, do, _dlse):
     return flash_attn_bwd(do.to(q.dtype), q, k, v, o, lse)
 
 
-flash_attn.register_autograd(_fl_backward, setup_context=_fl_setup)
+_autograd(flash_attn, _fl_backward, setup_context=_fl_setup)
