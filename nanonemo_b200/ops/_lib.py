@@ -67,6 +67,7 @@ _SIGNATURES = {
     "nnb_add_rmsnorm_fwd": "ppppppiifiiip",
     "nnb_rmsnorm_bwd_blocks": "",
     "nnb_add_rmsnorm_bwd": "pppppppppiiiiiip",
+    "nnb_scale": "pppqiip",
     "nnb_rope_packed": "ppppqiiiiqqfip",
     "nnb_swiglu_fwd": "pppqiqqqip",
     "nnb_swiglu_bwd": "pppppqiqqqqqip",

@@ -450,7 +450,7 @@ def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> t
     and weight (fp32), all produced in the same pass (the logits exist one row chunk at a time, in 16 bits)."""
     w16 = _w16(weight, x2.dtype)
     tg = (targets if targets.dtype == torch.int64 else targets.long()).contiguous()
-    dW = torch.zeros(weight.shape, dtype=torch.float32, device=x2.device)
+    dW = torch.empty(weight.shape, dtype=torch.float32, device=x2.device)
     loss_sum, dx = ce_mod.linear_ce_fwd(x2, w16.contiguous(), tg, chunk_rows, dW)
     return loss_sum / x2.shape[0], dx, dW
 
@@ -458,6 +458,29 @@ def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> t
 @_fake(linear_ce)
 def _(x2, weight, targets, chunk_rows):
     return x2.new_empty((), dtype=torch.float32), torch.empty_like(x2), weight.new_empty(weight.shape, dtype=torch.float32)
+
+
+@_operator
+def scaled(t: Tensor, scalar: Tensor) -> Tensor:
+    """t * scalar for a 0-dim fp32 scalar on the device."""
+    return ce_mod.scale(t, scalar)
+
+
+@_fake(scaled)
+def _(t, scalar):
+    return torch.empty_like(t, memory_format=torch.contiguous_format)
+
+
+def _scaled_setup(ctx, inputs, output):
+    ctx.save_for_backward(*inputs)
+
+
+def _scaled_backward(ctx, g):
+    t, scalar = ctx.saved_tensors
+    return scaled(g.contiguous(), scalar), (g.float() * t.float()).sum().to(scalar.dtype).reshape(scalar.shape)
+
+
+_autograd(scaled, _scaled_backward, setup_context=_scaled_setup)
 
 
 def _lce_setup(ctx, inputs, output):
@@ -470,7 +493,7 @@ def _lce_backward(ctx, dloss, _ddx, _ddw):
     dx, dW = ctx.saved_tensors
     if dloss is None:
         return None, None, None, None
-    return dx * dloss.to(dx.dtype), (dW * dloss).to(ctx.w_dtype), None, None
+    return scaled(dx, dloss), scaled(dW, dloss).to(ctx.w_dtype), None, None
 
 
 _autograd(linear_ce, _lce_backward, setup_context=_lce_setup)

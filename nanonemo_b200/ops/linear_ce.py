@@ -35,9 +35,19 @@ def ce_from_stats(logits: torch.Tensor, targets: torch.Tensor, tile_stats: torch
 FUSE_STATS = True  # head GEMM epilogue produces the softmax statistics (tests switch it off to compare the two routes)
 
 
+def scale(t: torch.Tensor, scalar: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``t * scalar`` (fp32 product, t's dtype) for a 0-dim fp32 device scalar, or ``out += t * scalar``."""
+    t = t if t.is_contiguous() else t.contiguous()
+    dst = out if out is not None else torch.empty_like(t)
+    code = 0 if t.dtype == torch.float32 else _CODE[t.dtype]
+    _lib.call("nnb_scale", _lib.ptr(t), _lib.ptr(scalar.float()), _lib.ptr(dst), _lib.i64(t.numel()), _lib.i32(code),
+              _lib.i32(int(out is not None)), _lib.vp(_lib.stream_ptr()))
+    return dst
+
+
 def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
-    """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); accumulates the
-    mean-loss weight gradient into dW_out (fp32 [V, D])."""
+    """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
+    mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
     N, D = x16.shape
     V = w16.shape[0]
     chunk_rows = min(chunk_rows, N)
@@ -55,7 +65,7 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
             gemm(xc, w16, out=lg)
             ce_inplace(lg, targets[r0:r1], loss_rows[r0:r1], 1.0 / N)
         gemm(lg, w16, b_mn=True, out=dx[r0:r1])
-        gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=True)
+        gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=r0 > 0)
     return loss_rows.sum(), dx
 
 
@@ -90,7 +100,7 @@ class _LinearCE(torch.autograd.Function):
         x16 = x16 if x16.is_contiguous() else x16.contiguous()
         tg = targets if targets.dtype == torch.int64 else targets.long()
         tg = tg if tg.is_contiguous() else tg.contiguous()
-        dW = torch.zeros(weight.shape, dtype=torch.float32, device=x.device)
+        dW = torch.empty(weight.shape, dtype=torch.float32, device=x.device)
         loss_sum, dx = linear_ce_fwd(x16, w16, tg, chunk_rows or DEFAULT_CHUNK_ROWS, dW)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype
@@ -99,14 +109,14 @@ class _LinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dx, dW, weight = ctx.saved_tensors
-        gx = (dx * dloss.to(dx.dtype)).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
+        gx = scale(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
         gw = None
         if ctx.needs_input_grad[1]:
             main = getattr(weight, "_main_grad", None)
             if main is not None and main.dtype == torch.float32:
-                main.addcmul_(dW, dloss)  # readiness of the tied weight is reported by the embedding backward
+                scale(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
             else:
-                gw = (dW * dloss).to(weight.dtype)
+                gw = scale(dW, dloss).to(weight.dtype)
         return gx, gw, None, None
 
 
@@ -159,7 +169,7 @@ class _VocabParallelLinearCE(torch.autograd.Function):
         Vl = w16.shape[0]
         rows = min(chunk_rows or DEFAULT_CHUNK_ROWS, N)
         dx = torch.empty_like(x16)
-        dW = torch.zeros(weight.shape, dtype=torch.float32, device=x.device)
+        dW = torch.empty(weight.shape, dtype=torch.float32, device=x.device)
         loss_rows = torch.empty(N, dtype=torch.float32, device=x.device)
         logits = torch.empty((rows, Vl), dtype=dt, device=x.device)
         for r0 in range(0, N, rows):
@@ -168,7 +178,7 @@ class _VocabParallelLinearCE(torch.autograd.Function):
             gemm(xc, w16, out=lg)
             vocab_parallel_ce_inplace(lg, tg[r0:r1], loss_rows[r0:r1], 1.0 / N, v0, Vl * tp.world, tp.all_gather, tp.world)
             gemm(lg, w16, b_mn=True, out=dx[r0:r1])
-            gemm(lg, xc, a_mn=True, b_mn=True, out=dW, accumulate=True)
+            gemm(lg, xc, a_mn=True, b_mn=True, out=dW, accumulate=r0 > 0)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype
         return loss_rows.sum() / N
@@ -176,14 +186,14 @@ class _VocabParallelLinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dx, dW, weight = ctx.saved_tensors
-        gx = (dx * dloss.to(dx.dtype)).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
+        gx = scale(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
         gw = None
         if ctx.needs_input_grad[1]:
             main = getattr(weight, "_main_grad", None)
             if main is not None and main.dtype == torch.float32:
-                main.add_(dW * dloss)  # readiness of the tied weight is reported by the embedding backward
+                scale(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
             else:
-                gw = (dW * dloss).to(weight.dtype)
+                gw = scale(dW, dloss).to(weight.dtype)
         return gx, gw, None, None, None, None
 
 

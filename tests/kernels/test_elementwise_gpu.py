@@ -162,3 +162,17 @@ def test_sumsq_and_adamw_match_torch(n):
         assert gbuf.abs().max() == 0
         torch.testing.assert_close(p, ref_p.data, rtol=1e-5, atol=1e-6)
         torch.testing.assert_close(shadow.float(), ref_p.data, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2048, 2051, 1 << 20])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_scale_by_a_device_scalar(n, dtype):
+    """One fp32 product (and sum) and one rounding: at most one unit in the last place beside the same thing done by PyTorch in fp32."""
+    from nanonemo_b200.ops.linear_ce import scale
+
+    torch.manual_seed(n)
+    t, s, out = torch.randn(n, device=DEV).to(dtype), torch.tensor(-0.37, device=DEV), torch.randn(n, device=DEV).to(dtype)
+    eps = torch.finfo(dtype).eps
+    torch.testing.assert_close(scale(t, s), (t.float() * s).to(dtype), rtol=eps, atol=0)
+    want = (out.float() + t.float() * s).to(dtype)
+    torch.testing.assert_close(scale(t, s, out=out), want, rtol=eps, atol=2 * torch.finfo(torch.float32).eps)

@@ -46,6 +46,8 @@ def test_opcheck_every_registered_operator():
     head = (torch.randn(512, 128, device=DEV) * 0.02).requires_grad_()
     tg = torch.randint(0, 512, (256,), device=DEV)
     torch.library.opcheck(L.linear_ce, (a, head, tg, 128))
+    torch.library.opcheck(L.linear_ce_loss, (a.detach(), head.detach(), tg, 128))
+    torch.library.opcheck(L.scaled, (torch.randn(33, device=DEV, requires_grad=True), torch.tensor(0.5, device=DEV, requires_grad=True)))
     n = 1024
     p, gr, m, vv = (torch.randn(n, device=DEV) for _ in range(4))
     vv.abs_()
