@@ -8,22 +8,37 @@
 #include "common.cuh"
 
 // ============================================================================ add + RMSNorm
-// y = rmsnorm(h) * w,  h = round_to_TX(x + delta);  rstd saved for backward. One warp per row;
-// lane l owns 8-element chunks l, l+32, ...; MAXC chunks per lane (N <= 256 * MAXC).
-template <typename TX, typename TD, typename TY, int MAXC>
+// Sum over the WPR warps that share a row (WPR 1 or 2; `pair` numbers the row's warps in the block). `slot` alternates from row to
+// row, so that one barrier per row is enough. Every lane gets the sum, added in the same order.
+template <int WPR>
+__device__ __forceinline__ float row_sum(float v, float (*s_part)[2][2], int pair, int slot) {
+  v = warp_sum(v);
+  if constexpr (WPR == 1) return v;
+  if ((threadIdx.x & 31) == 0) s_part[pair][slot][(threadIdx.x >> 5) & 1] = v;
+  asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+  return s_part[pair][slot][0] + s_part[pair][slot][1];
+}
+
+// y = rmsnorm(h) * w,  h = round_to_TX(x + delta);  rstd saved for backward. WPR warps per row (two for rows wider than 1024, so
+// that a lane never holds more than four chunks); lane l of them owns 8-element chunks l, l + 32 WPR, ...; MAXC chunks per lane.
+// HBM-bound. M = 32768, N = 2048, fp32 residual, bf16 delta and y, cold L2: 129 us with two warps a row, 158 with one
+// (floor 123); 8192 rows 41 and 49 us.
+template <typename TX, typename TD, typename TY, int MAXC, int WPR>
 __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restrict__ x, const TD* __restrict__ delta,
                                                               const float* __restrict__ w, TY* __restrict__ y,
                                                               TX* __restrict__ h, float* __restrict__ rstd, int M,
                                                               int N, float eps) {
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= M) return;
+  __shared__ float s_part[8 / WPR][2][2];
+  constexpr int kLanes = 32 * WPR;
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes, lane = threadIdx.x % kLanes;
+  if (row >= M) return;  // (all warps of a row together)
   const int nchunks = N >> 3;
   const size_t base = (size_t)row * N;
   float v[MAXC][8];
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < MAXC; ++c) {
-    const int ch = lane + 32 * c;
+    const int ch = lane + kLanes * c;
     if (ch < nchunks) {
       Chunk8<TX>::load(x + base + ch * 8, v[c]);
       if (delta != nullptr) {
@@ -37,12 +52,12 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restri
       for (int i = 0; i < 8; ++i) ss += v[c][i] * v[c][i];
     }
   }
-  ss = warp_sum(ss);
+  ss = row_sum<WPR>(ss, s_part, threadIdx.x / kLanes, 0);
   const float r = rsqrtf(ss / (float)N + eps);
   if (lane == 0) rstd[row] = r;
 #pragma unroll
   for (int c = 0; c < MAXC; ++c) {
-    const int ch = lane + 32 * c;
+    const int ch = lane + kLanes * c;
     if (ch < nchunks) {
       float g[8];
       Chunk8<float>::load(w + ch * 8, g);
@@ -58,15 +73,20 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restri
 // register file only holds one row), warps of a block are then summed and the block writes one partial row of dw, reduced in
 // index order by dw_reduce_kernel. Every load of a row (h, dy AND the incoming residual gradient) is issued before the first
 // use, so a warp has its whole ~8 KB in flight at once instead of paying the memory latency twice per row, and blocks are
-// 128 threads with at most 128 registers so that four of them (16 warps) share an SM.
-template <typename TX, typename TD, typename TY, int MAXC>
-__global__ void __launch_bounds__(128, MAXC <= 4 ? 4 : 2) add_rmsnorm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ h,
+// 128 threads with at most 128 registers so that four of them (16 warps) share an SM. Rows wider than 1024 take two warps: with one, a
+// row's loads did not fit the registers, the residual gradient was fetched late and only half the warps fitted. With the reduction
+// of dw, cold L2, fp32 residual, bf16 dy and ddelta: M = 32768, N = 2048 278 -> 198 us (floor 164), 8192 rows 99 -> 73 us.
+template <typename TX, typename TD, typename TY, int MAXC, int WPR>
+__global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ h,
                                                                  const float* __restrict__ rstd,
                                                                  const float* __restrict__ w, const TX* __restrict__ dres,
                                                                  TX* __restrict__ dx, TD* __restrict__ ddelta,
                                                                  float* __restrict__ dw_partial, int M, int N) {
-  extern __shared__ float s_mem[];  // [N] weight, then [warps][N] accumulators
-  const int lane = threadIdx.x & 31, warp_in_block = threadIdx.x >> 5, warps_per_block = blockDim.x >> 5;
+  extern __shared__ float s_mem[];  // [N] weight, then [rows in flight][N] accumulators
+  __shared__ float s_part[4 / WPR][2][2];
+  constexpr int kLanes = 32 * WPR;
+  const int lane = threadIdx.x % kLanes, warp_in_block = threadIdx.x / kLanes, warps_per_block = blockDim.x / kLanes;  // (groups of WPR warps)
+  int slot = 0;
   const int nchunks = N >> 3;
   float* s_w = s_mem;
   float* s_acc = s_mem + N + (size_t)warp_in_block * N;
@@ -76,24 +96,21 @@ __global__ void __launch_bounds__(128, MAXC <= 4 ? 4 : 2) add_rmsnorm_bwd_kernel
   const float inv_n = 1.f / (float)N;
   for (int row = blockIdx.x * warps_per_block + warp_in_block; row < M; row += gridDim.x * warps_per_block) {
     const size_t base = (size_t)row * N;
-    constexpr bool kEarly = MAXC <= 4;  // wider rows (N up to 2048) would spill: they fetch the residual gradient late
-    float n_[MAXC][8], dn[MAXC][8], res[kEarly ? MAXC : 1][8];
+    float n_[MAXC][8], dn[MAXC][8], res[MAXC][8];
 #pragma unroll
     for (int c = 0; c < MAXC; ++c) {
-      const int ch = lane + 32 * c;
+      const int ch = lane + kLanes * c;
       if (ch < nchunks) {
         Chunk8<TX>::load(h + base + ch * 8, n_[c]);
         Chunk8<TY>::load(dy + base + ch * 8, dn[c]);
-        if constexpr (kEarly) {
-          if (dres != nullptr) Chunk8<TX>::load(dres + base + ch * 8, res[c]);
-        }
+        if (dres != nullptr) Chunk8<TX>::load(dres + base + ch * 8, res[c]);
       }
     }
     const float r = rstd[row];
     float dot = 0.f;
 #pragma unroll
     for (int c = 0; c < MAXC; ++c) {
-      const int ch = lane + 32 * c;
+      const int ch = lane + kLanes * c;
       if (ch < nchunks) {
         float g[8], a[8];
         Chunk8<float>::load(s_w + ch * 8, g);
@@ -108,17 +125,15 @@ __global__ void __launch_bounds__(128, MAXC <= 4 ? 4 : 2) add_rmsnorm_bwd_kernel
         Chunk8<float>::store(s_acc + ch * 8, a);
       }
     }
-    dot = warp_sum(dot) * inv_n;
+    dot = row_sum<WPR>(dot, s_part, warp_in_block, slot) * inv_n;
+    slot ^= 1;
 #pragma unroll
     for (int c = 0; c < MAXC; ++c) {
-      const int ch = lane + 32 * c;
+      const int ch = lane + kLanes * c;
       if (ch < nchunks) {
         float o[8];
-        if constexpr (!kEarly) {
-          if (dres != nullptr) Chunk8<TX>::load(dres + base + ch * 8, res[0]);
-        }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = r * (dn[c][i] - n_[c][i] * dot) + (dres != nullptr ? res[kEarly ? c : 0][i] : 0.f);
+        for (int i = 0; i < 8; ++i) o[i] = r * (dn[c][i] - n_[c][i] * dot) + (dres != nullptr ? res[c][i] : 0.f);
         Chunk8<TX>::store(dx + base + ch * 8, o);
         if (ddelta != nullptr) Chunk8<TD>::store(ddelta + base + ch * 8, o);
       }
@@ -164,11 +179,10 @@ __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict_
 template <typename TX, typename TD, typename TY>
 static void rmsnorm_fwd_t(const void* x, const void* delta, const float* w, void* y, void* h, float* rstd, int M, int N,
                           float eps, cudaStream_t st) {
-  const int blocks = (M + 7) / 8;
-#define NNB_RMS_FWD(MAXC) \
-  add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC><<<blocks, 256, 0, st>>>((const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
-  if (N <= 1024) NNB_RMS_FWD(4);
-  else NNB_RMS_FWD(8);
+#define NNB_RMS_FWD(MAXC, WPR) \
+  add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC, WPR><<<(M * WPR + 7) / 8, 256, 0, st>>>((const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
+  if (N <= 1024) NNB_RMS_FWD(4, 1);
+  else NNB_RMS_FWD(4, 2);
 #undef NNB_RMS_FWD
 }
 
@@ -199,16 +213,16 @@ extern "C" int nnb_rmsnorm_bwd_blocks() { return 4 * nnb_num_sms(); }  // four 1
 template <typename TX, typename TD, typename TY>
 static int rmsnorm_bwd_t(const void* dy, const void* h, const float* rstd, const float* w, const void* dres, void* dx,
                          void* ddelta, float* partial, int blocks, int M, int N, cudaStream_t st) {
-  const size_t smem = (size_t)N * 5 * sizeof(float);  // the weight + one accumulator row per warp (4 warps)
-#define NNB_RMS_BWD(MAXC)                                                                                         \
+#define NNB_RMS_BWD(MAXC, WPR)                                                                                    \
   {                                                                                                               \
-    auto k = add_rmsnorm_bwd_kernel<TX, TD, TY, MAXC>;                                                            \
+    const size_t smem = (size_t)N * (1 + 4 / WPR) * sizeof(float); /* the weight, and an accumulator per row in flight */ \
+    auto k = add_rmsnorm_bwd_kernel<TX, TD, TY, MAXC, WPR>;                                                       \
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -3; \
     k<<<blocks, 128, smem, st>>>((const TY*)dy, (const TX*)h, rstd, w, (const TX*)dres, (TX*)dx, (TD*)ddelta, partial, M, N); \
   }
-  if (N <= 768) NNB_RMS_BWD(3)   // one row fits 3 chunks per lane: fewer registers, more resident warps
-  else if (N <= 1024) NNB_RMS_BWD(4)
-  else NNB_RMS_BWD(8)
+  if (N <= 768) NNB_RMS_BWD(3, 1)   // one row fits 3 chunks per lane: fewer registers, more resident warps
+  else if (N <= 1024) NNB_RMS_BWD(4, 1)
+  else NNB_RMS_BWD(4, 2)
 #undef NNB_RMS_BWD
   return 0;
 }
@@ -218,7 +232,8 @@ extern "C" int nnb_add_rmsnorm_bwd(const void* dy, const void* h, const void* rs
                                    void* dx, void* ddelta, void* dw, void* dw_partial, int M, int N, int x_dtype,
                                    int delta_dtype, int y_dtype, int accumulate_dw, cudaStream_t st) {
   NNB_REQUIRE(N % 8 == 0 && N <= 2048 && N > 0, "add_rmsnorm_bwd: N=%d must be a multiple of 8 and <= 2048", N);
-  const int blocks = min(nnb_rmsnorm_bwd_blocks(), (M + 3) / 4);
+  const int rows_per_block = N > 1024 ? 2 : 4;
+  const int blocks = min(nnb_rmsnorm_bwd_blocks(), (M + rows_per_block - 1) / rows_per_block);
   bool done = false;
   int rc = 0;
 #define X(cx, cd, cy, TX, TD, TY)                                                                      \

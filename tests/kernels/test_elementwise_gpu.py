@@ -15,7 +15,7 @@ def _ref_add_rms(x, delta, w, eps):
     return y, h
 
 
-@pytest.mark.parametrize("M,N", [(1, 8), (7, 768), (64, 768), (33, 1000), (16, 2048), (5, 72)])
+@pytest.mark.parametrize("M,N", [(1, 8), (7, 768), (64, 768), (33, 1000), (16, 2048), (5, 72), (1, 1032), (7, 1032), (2401, 1536), (1187, 2040), (2, 2048)])
 @pytest.mark.parametrize("xd,cd", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16),
                                    (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float16)])
 @pytest.mark.parametrize("has_delta", [True, False])
