@@ -745,6 +745,15 @@ extern "C" int nnb_gemm_swiglu(const void* X, const void* Wgu, void* GU, void* A
   return nnb_gemm2_launch(g, st);
 }
 
+// act of nnb_gemm_swiglu alone (the projection is not kept): a forward pass without gradients.
+extern "C" int nnb_gemm_swiglu_act(const void* X, const void* Wgu, void* ACT, int M, int F, int K, long long lda, long long ldw,
+                                   long long ldact, int dtype, void* status, cudaStream_t st) {
+  NnbGemm2Args g{};
+  if (int rc = fused_gemm_common(g, X, Wgu, nullptr, M, 2 * F, K, lda, ldw, 2 * F, dtype, status)) return rc;
+  g.epilogue = EPI_SWIGLU_ACT; g.E = ACT; g.lde = ldact;
+  return nnb_gemm2_launch(g, st);
+}
+
 // qkv[M, N] = x[M, K] @ w[N, K]^T with rotate-half RoPE applied to columns [0, rope_cols) (heads of head_dim columns, row m
 // at position m % t_len; cos / sin: fp32 [t_len, head_dim / 2]); the remaining columns (V) pass through.
 extern "C" int nnb_gemm_rope(const void* X, const void* W, void* QKV, const void* cos_t, const void* sin_t, int M, int N, int K,

@@ -24,6 +24,9 @@
 //   EPI_CE_STATS  LM head: besides the 16-bit logits, every (row, 256-column tile) gets its (max, sum of exp(x - max)), so
 //                 the cross-entropy kernel needs one sweep over the logits instead of two
 //                 (nanonemo/kernels/triton/linear_ce.py:21-41).
+//   EPI_SWIGLU_ACT  the same for a forward pass without gradients: nobody reads the projection, so only act leaves the tile, a
+//                 third of the bytes. One staging tile per 64 features instead of three: two epilogue groups and a sixth
+//                 operand stage fit. 32768 x 4096 x 768: 145 us, EPI_SWIGLU 192.
 //   EPI_CE_LOSS   LM head of a loss without gradients (validation): the statistics and the target's logit of every row, and no
 //                 logits at all. Against EPI_CE_STATS + the one-sweep kernel this drops the 16-bit logits' write, read and
 //                 rewrite; the accumulator goes straight from tensor memory to the statistics, so the staging tiles' shared
@@ -56,7 +59,7 @@ template <int EPI> struct Cfg {
   // The softmax statistics (an exponential per logit) get the same split, one staging tile per group.
   // (The SwiGLU forward stays with one group: a second one needs six staging tiles, which leaves four operand stages, and
   // measured slower: 0.201 vs 0.182 ms at M = 32768, N = 4096, K = 768.)
-  static constexpr int kEpiGroups = (EPI == EPI_SWIGLU_BWD || EPI == EPI_CE_STATS || EPI == EPI_CE_LOSS) ? 2 : 1;
+  static constexpr int kEpiGroups = (EPI == EPI_SWIGLU_BWD || EPI == EPI_CE_STATS || EPI == EPI_CE_LOSS || EPI == EPI_SWIGLU_ACT) ? 2 : 1;
   static constexpr int kThreads = 64 + kEpiGroups * kEpilogueThreads;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
@@ -241,7 +244,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tile_coords(tile, m_pair, n_blk);
         const int m_row0 = (m_pair * 2 + (int)rank) * BM;
         // SwiGLU: the leader stages gate rows, the peer the up rows (F further down) of the same 128 features
-        const int n_row0 = EPI == EPI_SWIGLU ? n_blk * (BN / 2) + (int)rank * p.epi_cols : n_blk * BN + (int)rank * (BN / 2);
+        const int n_row0 = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_ACT ? n_blk * (BN / 2) + (int)rank * p.epi_cols : n_blk * BN + (int)rank * (BN / 2);
         const int kb0 = ks * p.kblocks_per_split, kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const uint32_t s = it % kStages, ph = (it / kStages) & 1;
@@ -411,6 +414,35 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             tma_store_2d(&tmD, smem_u32(tiles), fcol, d_row);
             tma_store_2d(&tmD, smem_u32(tiles + BM * 128), F + fcol, d_row);
             tma_store_2d(&tmE, smem_u32(tiles + 2 * BM * 128), fcol, d_row);
+            tma_commit_group();
+          }
+          pending_stores = 1;
+        }
+      } else if constexpr (EPI == EPI_SWIGLU_ACT) {
+        // group g takes the 64 features of chunk g through its own staging tile; the arithmetic is EPI_SWIGLU's, on the rounded values
+        const int fcol = n_blk * (BN / 2) + grp * 64;
+        if (rows_live && fcol < p.epi_cols) {
+          uint8_t* tile_a = staging + grp * (BM * 128);
+          if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();
+          named_barrier_sync(epi_bar, kEpilogueThreads);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t g[32], u[32], wa[16];
+            tmem_ld_32x32b_x32(t_row + grp * 64 + h * 32, g);
+            tmem_ld_32x32b_x32(t_row + BN / 2 + grp * 64 + h * 32, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float2 gg = unpack16(pack16(__uint_as_float(g[2 * e]), __uint_as_float(g[2 * e + 1]), bf), bf);
+              const float2 uu = unpack16(pack16(__uint_as_float(u[2 * e]), __uint_as_float(u[2 * e + 1]), bf), bf);
+              wa[e] = pack16(gg.x / (1.f + __expf(-gg.x)) * uu.x, gg.y / (1.f + __expf(-gg.y)) * uu.y, bf);
+            }
+            stage32(tile_a + row * 128, sw, h * 4, wa);
+          }
+          fence_proxy_async_smem();
+          named_barrier_sync(epi_bar, kEpilogueThreads);
+          if (et == 0) {
+            tma_store_2d(&tmD, smem_u32(tile_a), fcol, d_row);
             tma_commit_group();
           }
           pending_stores = 1;
@@ -678,7 +710,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   p.m_pairs = (a.M + 2 * BM - 1) / (2 * BM);
   p.n_blocks = (a.N + BN - 1) / BN;
   p.kblocks_total = (a.K + BK - 1) / BK;
-  if (EPI == EPI_SWIGLU) {
+  if (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_ACT) {
     // a.N = 2 F (rows of the gate||up weight); one tile = 128 features = gate and up columns of the same features
     NNB_REQUIRE(!a.out_f32 && !a.a_mn && !a.b_mn && !a.accumulate && a.E != nullptr, "gemm_swiglu: plain K-major 16-bit problem expected");
     NNB_REQUIRE(a.N % 256 == 0, "gemm_swiglu: F = %d must be a multiple of 128", a.N / 2);
@@ -739,6 +771,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   // (EPI_SWIGLU_BWD writes d(gate) | d(up): its output, like the projection it reads through tmE, is 2 N columns wide)
   const int d_cols = EPI == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
   if (EPI == EPI_CE_LOSS) tmD = tmA;  // nothing is stored
+  else if (EPI == EPI_SWIGLU_ACT) { if (!nnb_make_tmap_2d(&tmD, in_dt, 2, a.E, a.M, a.N / 2, a.lde * 2, BM, 64, "gemm2 act")) return -4; }
   else if (!nnb_make_tmap_2d(&tmD, d_dt, d_bytes, a.D, a.M, d_cols, a.ldd * d_bytes, BM, d_box, "gemm2 D")) return -4;
   tmE = tmD;
   if (EPI == EPI_SWIGLU_BWD && !nnb_make_tmap_2d(&tmE, in_dt, 2, a.E, a.M, 2 * a.N, a.lde * 2, BM, 64, "gemm2 gate|up")) return -4;
@@ -765,6 +798,7 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st) {
     case EPI_CE_STATS: return NNB_LAUNCH2(EPI_CE_STATS);
     case EPI_SWIGLU_BWD: return NNB_LAUNCH2(EPI_SWIGLU_BWD);
     case EPI_CE_LOSS: return NNB_LAUNCH2(EPI_CE_LOSS);
+    case EPI_SWIGLU_ACT: return NNB_LAUNCH2(EPI_SWIGLU_ACT);
 #undef NNB_LAUNCH2
     default: nnb_set_error("gemm2: unknown epilogue %d", a.epilogue); return -1;
   }

@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 
 // Work fused into the epilogue while a tile leaves tensor memory (see gemm2.cu).
-enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4, EPI_CE_LOSS = 5 };
+enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4, EPI_CE_LOSS = 5, EPI_SWIGLU_ACT = 6 };
 
 struct NnbGemm2Args {
   const void *A, *B;
@@ -18,6 +18,7 @@ struct NnbGemm2Args {
   // EPI_SWIGLU: B = gate||up weight [2 F, K] (N = 2 F), D = projection [M, 2 F], E = act [M, F] with row stride lde
   void* E = nullptr;
   long long lde = 0;
+  // EPI_SWIGLU_ACT: the same without the projection (D is not written): act alone, for a forward pass without gradients
   // EPI_ROPE: rotate-half on columns [0, rope_cols) in heads of head_dim columns; row m uses table row m % t_len of the
   // fp32 tables [t_len, head_dim / 2]
   const void *cos_t = nullptr, *sin_t = nullptr;

@@ -80,6 +80,7 @@ _SIGNATURES = {
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
     "nnb_gemm_swiglu": "ppppiiiqqqqipp",
+    "nnb_gemm_swiglu_act": "pppiiiqqqipp",
     "nnb_gemm_rope": "pppppiiiqqqiiiipp",
     "nnb_gemm_swiglu_bwd": "ppppiiiqqqqipp",
     "nnb_gemm_ce_stats": "ppppiiiqqqipp",

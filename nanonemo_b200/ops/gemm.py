@@ -92,6 +92,19 @@ def gemm_swiglu(x2: torch.Tensor, w_gu: torch.Tensor):
     return (gu, act) if ok else None
 
 
+def gemm_swiglu_act(x2: torch.Tensor, w_gu: torch.Tensor):
+    """The activation of ``gemm_swiglu`` alone (the projection never reaches memory) -> act [M, F] or None."""
+    M, K = x2.shape
+    F = w_gu.shape[0] // 2
+    if M < 256 or F % 128 or w_gu.stride(1) != 1 or x2.stride(1) != 1:
+        return None
+    act = torch.empty((M, F), dtype=x2.dtype, device=x2.device)
+    ok = _fused_call("nnb_gemm_swiglu_act", _lib.ptr(x2), _lib.ptr(w_gu), _lib.ptr(act), _lib.i32(M), _lib.i32(F), _lib.i32(K),
+                     _lib.i64(x2.stride(0)), _lib.i64(w_gu.stride(0)), _lib.i64(F), _lib.i32(_CODE[x2.dtype]),
+                     _lib.ptr(status_tensor(x2.device)), _lib.vp(_lib.stream_ptr()))
+    return act if ok else None
+
+
 def gemm_swiglu_bwd(dy2: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor):
     """SwiGLU backward inside the down projection's input-gradient GEMM: dy2 [M, d] @ w_down [d, F] is the gradient of
     act = silu(gate) * up; the epilogue reads the saved projection gu [M, 2F] and writes d(gate) | d(up) [M, 2F] directly

@@ -34,6 +34,27 @@ def test_gemm_swiglu_epilogue(M, F_, K, dtype):
     _close(act, F.silu(g) * u, tol=1e-2)  # from the ROUNDED projection, as the stand-alone kernel computes it
 
 
+@pytest.mark.parametrize("M,F_,K", [(256, 128, 64), (512, 256, 768), (1000, 512, 264), (4096, 2048, 768), (384, 5632, 128), (257, 384, 8)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_swiglu_without_the_projection_gives_the_same_activation(M, F_, K, dtype):
+    """The same accumulator, the same rounding and the same arithmetic: bitwise equal, through the operator as well."""
+    from nanonemo_b200.ops import fused_block
+    from nanonemo_b200.ops.gemm import check_status, gemm_swiglu, gemm_swiglu_act
+
+    torch.manual_seed(M)
+    x, w = torch.randn(M, K, device=DEV).to(dtype), (torch.randn(2 * F_, K, device=DEV) / K ** 0.5).to(dtype)
+    full, act = gemm_swiglu(x, w), gemm_swiglu_act(x, w)
+    check_status()
+    assert torch.equal(act, full[1])
+    wd = (torch.randn(64, F_, device=DEV) / F_ ** 0.5).to(dtype)
+    with torch.autocast("cuda", dtype=dtype):
+        y = fused_block.mlp_swiglu(x.clone().requires_grad_(), w, wd)
+        with torch.no_grad():
+            quiet = fused_block.mlp_swiglu(x.clone().requires_grad_(), w, wd)
+    check_status()
+    assert y.requires_grad and not quiet.requires_grad and torch.equal(y.detach(), quiet)
+
+
 def test_gemm_swiglu_declines_shapes_it_does_not_serve():
     from nanonemo_b200.ops.gemm import gemm_swiglu
 
