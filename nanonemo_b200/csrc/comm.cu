@@ -416,11 +416,11 @@ extern "C" int nnb_comm_timeout_probe(void* flags, void* status, void* result, i
 extern "C" int nnb_comm_flag_words(int blocks) { return 2 * blocks * kMaxWorld; }
 
 // Threads per collective block (a multiple of 32 up to kCommThreads; NANONEMO_COMM_THREADS). The default of 128 keeps a block
-// at about 10 K registers, so that it fits on an SM next to ANY compute kernel of the training step, including the
-// 320-thread x 168-register attention backward and the GEMMs with two epilogue groups (53.8 K of the 64 K registers): a
-// collective that cannot share the SM either waits for those kernels or, once resident, keeps their CTAs off the SM while it
-// sits in a cross-GPU barrier. The launcher's `blocks` (two per SM by default) makes up for the smaller blocks wherever the
-// resident compute kernel leaves room for both.
+// at about 10 K registers, so that it fits on an SM next to the GEMMs, those with two epilogue groups included (53.8 K of the 64 K
+// registers): a collective that cannot share the SM either waits for those kernels or, once resident, keeps their CTAs off the SM
+// while it sits in a cross-GPU barrier. The attention backward is the exception: its 512 threads x 128 registers take an SM's whole
+// register file, so beside it a collective's blocks start as its CTAs retire (each lives for a fraction of a millisecond). The
+// launcher's `blocks` (two per SM by default) makes up for the smaller blocks wherever the resident kernel leaves room for both.
 static inline int comm_threads() {
   static int threads = [] {
     const char* e = getenv("NANONEMO_COMM_THREADS");

@@ -26,7 +26,7 @@ import torch
 
 from nanonemo_b200.ops import attention, rope, swiglu_act
 from nanonemo_b200.ops.gemm import (_rowmajor2d, compute_dtype, gemm, gemm_rope, gemm_swiglu, gemm_swiglu_act, gemm_swiglu_bwd,
-                                    linear_backward, shadow_of)
+                                    linear_backward, no_backward, shadow_of)
 
 
 def _rows16(x, dt):
@@ -184,7 +184,7 @@ class _MLPSwiGLU(torch.autograd.Function):
 
 def mlp_swiglu(x, w_gu, w_down):
     """x: (..., d); w_gu: [2 F, d] (gate rows first); w_down: [d, F] -> down(silu(x Wg^T) * (x Wu^T)), shape (..., d)."""
-    if not (torch.is_grad_enabled() and (x.requires_grad or w_gu.requires_grad or w_down.requires_grad)):
+    if no_backward(x, w_gu, w_down):
         dt = compute_dtype()  # no backward will ask for the projection: only the activation leaves its GEMM
         act = gemm_swiglu_act(_rows16(x, dt), shadow_of(w_gu, dt))
         if act is not None:

@@ -16,6 +16,7 @@ in fp32 directly into the flat gradient buffer when there is one.
 """
 
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from nanonemo_b200.ops import _lib
 
@@ -177,6 +178,14 @@ def shadow_of(weight: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     if sh is not None and sh.dtype == dtype:
         return sh
     return weight.detach().to(dtype)
+
+
+def no_backward(*tensors: torch.Tensor) -> bool:
+    """True when nothing can ask for a derivative of what is computed from these tensors: an operator may then skip what it would
+    keep for its backward. Forward-mode tangents count as asking (the autograd functions refuse them, and go on doing so)."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    return all(unpack_dual(t).tangent is None for t in tensors)
 
 
 class _Linear(torch.autograd.Function):

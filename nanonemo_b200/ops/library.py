@@ -515,7 +515,7 @@ def linear_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, chunk_rows:
     """x: [N, D]; weight: [V, D] (fp32 master or 16-bit); targets: [N] -> scalar mean loss (fp32)."""
     dt = gemm_mod.compute_dtype()
     x2 = x if x.dtype == dt else x.to(dt)
-    if not ce_mod.needs_grad(x, weight):
+    if not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
         return linear_ce_loss(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
     loss, _, _ = linear_ce(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
     return loss

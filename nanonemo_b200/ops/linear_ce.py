@@ -13,7 +13,7 @@ waves; the reference uses 512-row chunks on 8 GB parts).
 import torch
 
 from nanonemo_b200.ops import _lib
-from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_loss, gemm_ce_stats, shadow_of
+from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_loss, gemm_ce_stats, no_backward, shadow_of
 
 DEFAULT_CHUNK_ROWS = 32768
 
@@ -73,6 +73,7 @@ def linear_ce_loss(x16, w16, targets, chunk_rows):
     """Sum of row losses [fp32 scalar] when nobody asks for gradients (validation): one product per chunk instead of three, and
     its logits are reduced to softmax statistics before they leave the tensor core's accumulator."""
     N, V = x16.shape[0], w16.shape[0]
+    chunk_rows = min(chunk_rows, N)  # (no rows: refused by the loop below, as in linear_ce_fwd)
     loss_rows = torch.empty(N, dtype=torch.float32, device=x16.device)
     for r0 in range(0, N, chunk_rows):
         xc, tg = x16[r0:r0 + chunk_rows], targets[r0:r0 + chunk_rows]
@@ -85,10 +86,6 @@ def linear_ce_loss(x16, w16, targets, chunk_rows):
         _lib.call("nnb_ce_loss_from_stats", _lib.ptr(stats), _lib.i32(stats.shape[1]), _lib.ptr(target_logit), _lib.ptr(tg),
                   _lib.ptr(rows), _lib.i64(xc.shape[0]), _lib.i32(V), _lib.vp(_lib.stream_ptr()))
     return loss_rows.sum()
-
-
-def needs_grad(x, weight) -> bool:
-    return torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
 
 
 class _LinearCE(torch.autograd.Function):
@@ -122,7 +119,7 @@ class _LinearCE(torch.autograd.Function):
 
 def linear_cross_entropy(x, weight, targets, chunk_rows=None):
     """x: [N, D]; weight: [V, D] (fp32 master or 16-bit); targets: [N] int64 -> scalar mean loss (fp32)."""
-    if not needs_grad(x, weight):
+    if no_backward(x, weight):
         dt = compute_dtype()
         loss = linear_ce_loss(x.to(dt).contiguous(), shadow_of(weight, dt), targets.long().contiguous(), chunk_rows or DEFAULT_CHUNK_ROWS)
         return loss / x.shape[0]

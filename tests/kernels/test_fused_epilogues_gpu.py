@@ -55,6 +55,25 @@ def test_swiglu_without_the_projection_gives_the_same_activation(M, F_, K, dtype
     assert y.requires_grad and not quiet.requires_grad and torch.equal(y.detach(), quiet)
 
 
+def test_forward_mode_tangents_are_refused_without_gradients_too():
+    """The autograd functions have no forward-mode rule; the routes that skip them must not drop a tangent silently."""
+    from torch.autograd import forward_ad
+
+    from nanonemo_b200.ops import fused_block, linear_ce
+
+    x, w = torch.randn(256, 128, device=DEV).bfloat16(), (torch.randn(512, 128, device=DEV) * 0.1).bfloat16()
+    wd, t = (torch.randn(128, 256, device=DEV) * 0.1).bfloat16(), torch.randint(0, 512, (256,), device=DEV)
+    with torch.no_grad():
+        fused_block.mlp_swiglu(x, w, wd), linear_ce.linear_cross_entropy(x, w, t)  # plain inputs are served
+    with forward_ad.dual_level():
+        dual = forward_ad.make_dual(x, torch.randn_like(x))
+        for call in (lambda: fused_block.mlp_swiglu(dual, w, wd), lambda: linear_ce.linear_cross_entropy(dual, w, t)):
+            with pytest.raises((NotImplementedError, RuntimeError)):
+                call()
+    with pytest.raises(ValueError):
+        linear_ce.linear_cross_entropy(x[:0], w, t[:0])
+
+
 def test_gemm_swiglu_declines_shapes_it_does_not_serve():
     from nanonemo_b200.ops.gemm import gemm_swiglu
 
