@@ -2,7 +2,7 @@
 for the trainer's engine.
 
 They launch exactly the kernels the registered operators in ``ops/library.py`` launch; what they skip is the dispatcher round
-trip of a Python ``torch.library.custom_op`` (tens of microseconds per call, forward and backward). An eager training step of
+trip of a Python ``torch.library`` operator (tens of microseconds per call, forward and backward). An eager training step of
 the 114M model is 300 launches in 20-35 ms, and under tensor parallelism the host is the bottleneck, so the engine — any run
 that owns a flat parameter store, see ``enable()`` — takes these; everything else (plain modules, ``torch.compile``,
 ``opcheck``) takes the registered operators. Contracts: nanonemo/kernels/triton/{swiglu,rope}.py,
