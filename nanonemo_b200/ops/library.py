@@ -32,23 +32,31 @@ from nanonemo_b200.ops import adamw as adamw_mod, attention, embed as embed_mod,
 NS = "nanonemo_b200"
 
 
+_NO_FORMULA = {}  # operators that have no derivative formula (so far)
+
+
 def _operator(fn):
     """Register `fn` as the CUDA kernel of operator NS::<its name>, with the schema of its annotations. This is
     ``torch.library.custom_op`` without the wrapper that checks every call's results for aliases of its arguments (the kernels
     below return new tensors only), which took longer than a small launch: the 87 operator calls of a 201-token forward of the
-    114M model took 6.3 ms on the host with it and with ctypes objects for every argument (_lib.py), and 4.6 ms without."""
+    114M model took 6.3 ms on the host with it and with ctypes objects for every argument (_lib.py), and 4.6 ms without.
+    Like ``custom_op``, and unlike a bare definition, an operator without a formula stops a backward pass that reaches it: see
+    the end of this file."""
     name = f"{NS}::{fn.__name__}"
     torch.library.define(name, torch.library.infer_schema(fn, mutates_args=()), tags=(torch.Tag.pt2_compliant_tag,))
     torch.library.impl(name, "cuda", torch.compiler.disable(fn))
-    return getattr(torch.ops.nanonemo_b200, fn.__name__).default
+    op = getattr(torch.ops.nanonemo_b200, fn.__name__).default
+    _NO_FORMULA[op.name()] = op
+    return op
 
 
 def _fake(op):
     return torch.library.register_fake(op.name())
 
 
-def _autograd(op, backward, setup_context):
+def _autograd(op, backward, setup_context=None):
     torch.library.register_autograd(op.name(), backward, setup_context=setup_context)
+    _NO_FORMULA.pop(op.name())
 
 
 # ----------------------------------------------------------------------------- add + RMSNorm
@@ -621,3 +629,18 @@ def _fl_backward(ctx, do, _dlse):
 
 
 _autograd(flash_attn, _fl_backward, setup_context=_fl_setup)
+
+
+# ----------------------------------------------------------------------------- operators without a derivative
+# PyTorch lets an operator that has no formula through with a warning and drops its share of the derivative: a gradient of a
+# gradient (create_graph=True) would come back with its second-order part missing. These refuse instead. The formula costs a call
+# about 6 us on the host.
+def _refuse(op):
+    def backward(ctx, *grads):
+        raise RuntimeError(f"Trying to backward through {op.name()}, which has no derivative formula")
+
+    return backward
+
+
+for _op in list(_NO_FORMULA.values()):
+    _autograd(_op, _refuse(_op))
