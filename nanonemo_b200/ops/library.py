@@ -26,6 +26,7 @@ import math
 
 import torch
 from torch import Tensor
+from torch.autograd.forward_ad import unpack_dual
 
 from nanonemo_b200.ops import adamw as adamw_mod, attention, embed as embed_mod, gemm as gemm_mod, linear_ce as ce_mod, rmsnorm, rope, swiglu_act
 
@@ -501,7 +502,8 @@ def _lce_backward(ctx, dloss, _ddx, _ddw):
     dx, dW = ctx.saved_tensors
     if dloss is None:
         return None, None, None, None
-    return scaled(dx, dloss), scaled(dW, dloss).to(ctx.w_dtype), None, None
+    times = scaled if unpack_dual(dloss).tangent is None else ce_mod.times_upstream  # (`scaled` has no forward-mode formula)
+    return times(dx, dloss), times(dW, dloss).to(ctx.w_dtype), None, None
 
 
 _autograd(linear_ce, _lce_backward, setup_context=_lce_setup)

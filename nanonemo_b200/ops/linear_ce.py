@@ -45,6 +45,15 @@ def scale(t: torch.Tensor, scalar: torch.Tensor, out: torch.Tensor | None = None
     return dst
 
 
+def times_upstream(t: torch.Tensor, dloss: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``t * dloss`` in a backward pass (or ``out += t * dloss``): ``scale``, which sees values only, unless the upstream gradient
+    carries more than its value. A history (create_graph=True), a forward-mode tangent and a batch of gradients
+    (is_grads_batched=True hands in a wrapper without memory of its own) go through differentiable arithmetic."""
+    if no_backward(dloss) and torch._C._has_storage(dloss):
+        return scale(t, dloss, out)
+    return (t.float() * dloss).to(t.dtype) if out is None else out.addcmul_(t, dloss)
+
+
 def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
     mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
@@ -106,14 +115,14 @@ class _LinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dx, dW, weight = ctx.saved_tensors
-        gx = scale(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
+        gx = times_upstream(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
         gw = None
         if ctx.needs_input_grad[1]:
             main = getattr(weight, "_main_grad", None)
             if main is not None and main.dtype == torch.float32:
-                scale(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
+                times_upstream(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
             else:
-                gw = scale(dW, dloss).to(weight.dtype)
+                gw = times_upstream(dW, dloss).to(weight.dtype)
         return gx, gw, None, None
 
 
@@ -183,14 +192,14 @@ class _VocabParallelLinearCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         dx, dW, weight = ctx.saved_tensors
-        gx = scale(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
+        gx = times_upstream(dx, dloss).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
         gw = None
         if ctx.needs_input_grad[1]:
             main = getattr(weight, "_main_grad", None)
             if main is not None and main.dtype == torch.float32:
-                scale(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
+                times_upstream(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
             else:
-                gw = scale(dW, dloss).to(weight.dtype)
+                gw = times_upstream(dW, dloss).to(weight.dtype)
         return gx, gw, None, None, None, None
 
 
