@@ -36,8 +36,15 @@ FUSE_STATS = True  # head GEMM epilogue produces the softmax statistics (tests s
 
 
 def scale(t: torch.Tensor, scalar: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``t * scalar`` (fp32 product, t's dtype) for a 0-dim fp32 device scalar, or ``out += t * scalar``."""
+    """``t * scalar`` (fp32 product, t's dtype) for a one-element scalar on the same device, or ``out += t * scalar``."""
+    if scalar.numel() != 1 or scalar.device != t.device:  # the kernel reads one value at this address
+        raise ValueError(f"scale: one value on {t.device} expected, got shape {tuple(scalar.shape)} on {scalar.device}")
     t = t if t.is_contiguous() else t.contiguous()
+    if t.data_ptr() % 16:
+        t = t.clone()  # a view that starts between two 16-byte vectors
+    if out is not None and not (out.shape == t.shape and out.dtype == t.dtype and out.device == t.device and out.is_contiguous()
+                                and out.data_ptr() % 16 == 0):
+        return out.add_(t.float() * scalar)  # strided or unaligned gradient views; refuses what does not fit together
     dst = out if out is not None else torch.empty_like(t)
     code = 0 if t.dtype == torch.float32 else _CODE[t.dtype]
     _lib.call("nnb_scale", _lib.ptr(t), _lib.ptr(scalar.float()), _lib.ptr(dst), _lib.i64(t.numel()), _lib.i32(code),

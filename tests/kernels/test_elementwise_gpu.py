@@ -176,3 +176,8 @@ def test_scale_by_a_device_scalar(n, dtype):
     torch.testing.assert_close(scale(t, s), (t.float() * s).to(dtype), rtol=eps, atol=0)
     want = (out.float() + t.float() * s).to(dtype)
     torch.testing.assert_close(scale(t, s, out=out), want, rtol=eps, atol=2 * torch.finfo(torch.float32).eps)
+    rows = torch.randn(3, n + 5, device=DEV).to(dtype)  # views that the vector kernel cannot take: a strided sum, an odd start
+    strided, odd = rows[:, 1:n + 1], rows.view(-1)[1:n + 1]
+    want = (strided.float() + t.float() * s).to(dtype)
+    torch.testing.assert_close(scale(t.expand(3, n), s, out=strided), want, rtol=eps, atol=2 * torch.finfo(torch.float32).eps)
+    torch.testing.assert_close(scale(odd, s), (odd.float() * s).to(dtype), rtol=eps, atol=0)

@@ -109,3 +109,47 @@ def test_a_gradient_store_is_added_to(head):
     (head(x, w, t) * 0.5).backward()
     torch.testing.assert_close(w._main_grad, 1 + 0.5 * unit[1])
     assert w.grad is None
+
+
+@pytest.fixture
+def launched(monkeypatch):
+    """The arguments of the raw launches: (source, destination, elements, accumulate)."""
+    got = []
+
+    def call(name, src, scalar, dst, n, dtype, accumulate, stream):
+        assert name == "nnb_scale" and src % 16 == 0 and dst % 16 == 0
+        got.append((src, dst, n, accumulate))
+
+    monkeypatch.setattr(linear_ce._lib, "call", call)
+    monkeypatch.setattr(linear_ce._lib, "stream_ptr", lambda: 0)
+    return got
+
+
+def test_scale_launches_on_dense_aligned_memory_only(launched):
+    s, base = torch.tensor(0.5), torch.randn(12, 8)
+    dense = base[:4]
+    assert linear_ce.scale(dense, s).shape == (4, 8)
+    assert launched.pop()[::2] == (dense.data_ptr(), 32)
+    assert linear_ce.scale(dense, s, out=base[4:8]) is not None
+    assert launched.pop() == (dense.data_ptr(), base[4:8].data_ptr(), 32, 1)
+    offset = base.view(-1)[1:33]  # contiguous, four bytes past a vector: copied (`call` checks the addresses)
+    linear_ce.scale(offset, s)
+    assert launched.pop()[0] != offset.data_ptr()
+    for t, out in ((dense, torch.zeros(4, 16)[:, :8]), (dense, torch.zeros(8, 4).t()), (offset, torch.zeros(33)[1:]),
+                   (dense, torch.zeros(4, 8, dtype=torch.float64))):
+        assert linear_ce.scale(t, s, out=out) is out and not launched
+        torch.testing.assert_close(out.float(), t * 0.5)
+
+
+@pytest.mark.parametrize("out", [torch.zeros(4, 9), torch.zeros(3, 8), torch.zeros(8)])
+def test_scale_refuses_what_does_not_fit(launched, out):
+    with pytest.raises(RuntimeError):
+        linear_ce.scale(torch.randn(4, 8), torch.tensor(0.5), out=out)
+    assert not launched
+
+
+def test_scale_takes_one_value_on_the_same_device(launched):
+    for scalar in (torch.ones(2), torch.ones((), device="meta")):
+        with pytest.raises(ValueError):
+            linear_ce.scale(torch.randn(4, 8), scalar)
+    assert not launched
