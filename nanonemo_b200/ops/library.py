@@ -526,6 +526,8 @@ def linear_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, chunk_rows:
     dt = gemm_mod.compute_dtype()
     x2 = x if x.dtype == dt else x.to(dt)
     if not (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
+        if not torch.compiler.is_compiling() and not gemm_mod.no_backward(x, weight):
+            raise NotImplementedError("linear_cross_entropy has no forward-mode derivative")  # as with gradients
         return linear_ce_loss(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
     loss, _, _ = linear_ce(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
     return loss

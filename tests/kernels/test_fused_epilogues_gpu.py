@@ -59,6 +59,7 @@ def test_forward_mode_tangents_are_refused_without_gradients_too():
     """The autograd functions have no forward-mode rule; the routes that skip them must not drop a tangent silently."""
     from torch.autograd import forward_ad
 
+    from nanonemo_b200 import ops
     from nanonemo_b200.ops import fused_block, linear_ce
 
     x, w = torch.randn(256, 128, device=DEV).bfloat16(), (torch.randn(512, 128, device=DEV) * 0.1).bfloat16()
@@ -67,7 +68,8 @@ def test_forward_mode_tangents_are_refused_without_gradients_too():
         fused_block.mlp_swiglu(x, w, wd), linear_ce.linear_cross_entropy(x, w, t)  # plain inputs are served
     with forward_ad.dual_level():
         dual = forward_ad.make_dual(x, torch.randn_like(x))
-        for call in (lambda: fused_block.mlp_swiglu(dual, w, wd), lambda: linear_ce.linear_cross_entropy(dual, w, t)):
+        for call in (lambda: fused_block.mlp_swiglu(dual, w, wd), lambda: linear_ce.linear_cross_entropy(dual, w, t),
+                     lambda: ops.linear_cross_entropy(dual, w, t)):
             with pytest.raises((NotImplementedError, RuntimeError)):
                 call()
     with pytest.raises(ValueError):

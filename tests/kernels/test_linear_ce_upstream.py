@@ -102,6 +102,18 @@ def test_the_registered_head_carries_the_tangent_too():
             assert tangent is not None and tangent.shape == t.shape
 
 
+@pytest.mark.parametrize("which", [0, 1])
+@pytest.mark.parametrize("requires_grad", [False, True])
+def test_the_registered_head_refuses_tangents_of_its_inputs(which, requires_grad):
+    inputs = [torch.empty(s, dtype=torch.bfloat16, device="meta") for s in ((128, 64), (64, 64))]
+    targets = torch.zeros(128, dtype=torch.long, device="meta")
+    assert library.linear_cross_entropy(*inputs, targets).shape == ()
+    with forward_ad.dual_level():
+        inputs[which] = forward_ad.make_dual(inputs[which].requires_grad_(requires_grad), torch.empty_like(inputs[which]))
+        with pytest.raises(NotImplementedError):
+            library.linear_cross_entropy(*inputs, targets)
+
+
 def test_a_gradient_store_is_added_to(head):
     x, w, t = _inputs()
     unit = torch.autograd.grad(head(x, w, t), (x, w))
