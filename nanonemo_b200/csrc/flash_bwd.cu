@@ -44,12 +44,14 @@ namespace {
 using namespace sm100;
 
 constexpr int BQ = 128, BKV = 128, HD = 64;
-// Four warpgroups: TMA + MMA issuers (and two idle warps), drain, 2 x compute. The block is launched with 512 x 128 registers; the
+// Four warpgroups: TMA + MMA issuers (and two idle warps), drain, 2 x compute. The block is launched with 512 x 128 registers (checked before the first launch); the
 // compute warps keep 64 probabilities each and need more, so the others hand registers over: 104 + 104 + 2 x 152 = 4 x 128.
 constexpr int kThreads = 512;
 constexpr int kComputeThreads = 256, kDrainThreads = 128;
 constexpr int kDrainWarp0 = 4, kComputeWarp0 = 8;
-constexpr int kRegsIssue = 104, kRegsDrain = 104, kRegsCompute = 152;
+constexpr int kRegsIssue = 104, kRegsDrain = 104, kRegsCompute = 152, kRegsLaunch = 128;
+constexpr int kRegsShares = kRegsIssue + kRegsDrain + 2 * kRegsCompute;  // one warpgroup each, two for compute
+static_assert(kRegsShares == kThreads / 128 * kRegsLaunch, "the shares have to be the registers that the block is launched with");
 constexpr int kTile16 = 128 * 64 * 2;     // a [128 x 64] 16-bit tile = 16 KB
 constexpr int kStagesQ = 3;             // a stage is released when dK / dQ of its visit are done and refilled two visits ahead
 // shared memory map (bytes)
@@ -508,6 +510,25 @@ int nnb_flash_bwd_t_impl(int hd, const void* q, const void* k, const void* v, co
 extern "C" int nnb_flash_bwd_prof_read(unsigned long long* out) { return (int)cudaMemcpyFromSymbol(out, g_flash_prof, sizeof(g_flash_prof)); }
 #endif
 
+// Whether a block that is launched with `regs` registers a thread can hand them over as flash_bwd_kernel does. The increase waits,
+// without a limit, for registers that the other warpgroups give up: in a build with fewer of them (another compiler, a register
+// limit among its flags) it would never end, so the launcher refuses such a build.
+extern "C" int nnb_flash_bwd_registers(int regs) {
+  NNB_REQUIRE(regs * (kThreads / 128) >= kRegsShares, "flash_bwd: built with %d registers a thread, the hand-over needs %d", regs, kRegsLaunch);
+  return 0;
+}
+
+template <bool F16>
+static int configure_bwd() {
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, flash_bwd_kernel<F16>) != cudaSuccess ||
+      cudaFuncSetAttribute(flash_bwd_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
+    nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", kSmem);
+    return -3;
+  }
+  return nnb_flash_bwd_registers(a.numRegs);
+}
+
 // All tensors are [B, T, heads, 64] views given by element strides (contiguous last dim), bf16 or fp16 (one dtype for all).
 // lse: fp32 [B, H, T] from the forward pass; delta: fp32 [B, H, T] scratch (written here);
 // dq_acc: fp32 [B, T, H, hd] contiguous scratch (cleared by the delta pre-pass; partial tiles are reduce-added into it).
@@ -576,11 +597,8 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.rope_sin = static_cast<const float*>(rope_sin);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(flash_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(flash_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
-      nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", kSmem);
-      return -3;
-    }
+    if (int rc = configure_bwd<false>()) return rc;
+    if (int rc = configure_bwd<true>()) return rc;
     configured = true;
   }
   dim3 grid(KVH, B, (T + BKV - 1) / BKV);

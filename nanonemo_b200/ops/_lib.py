@@ -76,6 +76,7 @@ _SIGNATURES = {
     "nnb_warmup_add": "pppqp",
     "nnb_cast_from_f32": "ppqip",
     "nnb_build_arch": "",
+    "nnb_flash_bwd_registers": "i",
     "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfipppp",
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
