@@ -591,8 +591,10 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   const int sms = max_ctas > 0 ? min(max_ctas, nnb_num_sms()) : nnb_num_sms();
   // CTA-pair kernel (gemm2.cu): 256 x 256 tiles over two SMs, for every problem that has one. Measured (us, pair / 256-wide / 128-wide
   // single-CTA tiles, alternating runs): 8192 x 2048 x 5632 169 / 183 / 232, 8192^3 736 / 814 / 1237, 32768 x 2048 x 5632
-  // 472 / 507 / 780, 4096 x 768 x 50304 255 / 292 / 416, 16384 x 768 x 4096 87 / 99 / 134; below about 512 x 4096 x 768 all
-  // three take the 13-16 us of a launch. Weight gradients likewise (11264 x 2048 x 8192: 318 / 359).
+  // 472 / 507 / 780, 4096 x 768 x 50304 255 / 292 / 416, 16384 x 768 x 4096 87 / 99 / 134, 2048^3 23 / 24 / 30; weight gradients likewise
+  // (11264 x 2048 x 8192: 318 / 359; 2048 x 2048 x 8192: 57 / 64 / 90). It is not the best one for a 16-bit output whose 128-wide
+  // tiles fit one wave, where a tile's latency is all that counts: 1024 x 768 x 768 17 / 17 / 15, 1024 x 768 x 2048 26 / 26 / 22,
+  // 1024 x 2048 x 5632 44 / 46 / 38. The head's input gradient asks for the narrow tile there by its hint.
   static const bool pair_enabled = [] { const char* e = getenv("NANONEMO_GEMM_PAIR"); return !(e && e[0] == '0'); }();
   if (mode == 0 && (bn_hint == 512 || (bn_hint == 0 && pair_enabled && M >= 256 && N >= 256))) {
     const NnbGemm2Args g{A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, dtype, out_f32, accumulate, k_splits, max_ctas, status};

@@ -10,6 +10,8 @@ chunk's 16-bit logits are 3.3 GB of the 180 GB, and the three GEMMs fill all 148
 waves; the reference uses 512-row chunks on 8 GB parts).
 """
 
+from functools import lru_cache
+
 import torch
 
 from nanonemo_b200.ops import _lib
@@ -61,6 +63,19 @@ def times_upstream(t: torch.Tensor, dloss: torch.Tensor, out: torch.Tensor | Non
     return (t.float() * dloss).to(t.dtype) if out is None else out.addcmul_(t, dloss)
 
 
+@lru_cache(maxsize=None)
+def _sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def _dx_tile(rows: int, width: int, device) -> int:
+    """Tile hint of the head's input gradient [rows, width], whose K loop is the whole vocabulary: 128 x 128 tiles while one wave of SMs
+    holds them all, the dispatcher's choice (CTA pairs) beyond. In one wave every tile takes one K loop whatever its size, and
+    the smaller tile starts sooner: K = 50304, us, 128-wide / pair: 256 x 768 243 / 248, 1024 x 768 238 / 240, 2304 x 768
+    231 / 240, 512 x 2048 284 / 288; K = 32000: 512 x 768 165 / 170, 512 x 2048 222 / 232. In two waves: 3584 x 768 x 50304 451 / 246."""
+    return 128 if -(-rows // 128) * -(-width // 128) <= _sm_count(device) else 0
+
+
 def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
     mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
@@ -80,7 +95,7 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
         else:
             gemm(xc, w16, out=lg)
             ce_inplace(lg, targets[r0:r1], loss_rows[r0:r1], 1.0 / N)
-        gemm(lg, w16, b_mn=True, out=dx[r0:r1])
+        gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
         gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=r0 > 0)
     return loss_rows.sum(), dx
 
@@ -190,7 +205,7 @@ class _VocabParallelLinearCE(torch.autograd.Function):
             lg, xc = logits[: r1 - r0], x16[r0:r1]
             gemm(xc, w16, out=lg)
             vocab_parallel_ce_inplace(lg, tg[r0:r1], loss_rows[r0:r1], 1.0 / N, v0, Vl * tp.world, tp.all_gather, tp.world)
-            gemm(lg, w16, b_mn=True, out=dx[r0:r1])
+            gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
             gemm(lg, xc, a_mn=True, b_mn=True, out=dW, accumulate=r0 > 0)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype

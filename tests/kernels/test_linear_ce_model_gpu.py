@@ -30,6 +30,20 @@ def test_linear_ce_loss_and_grads(N, D, V, chunk):
         assert err <= 3e-2 * want.abs().max().item() + 1e-5, err
 
 
+@pytest.mark.parametrize("rows,width", [(3072, 768), (3073, 768), (1152, 2048), (1153, 2048)])
+def test_input_gradient_on_both_sides_of_its_tile_rule(rows, width):
+    """One wave of 128-wide tiles and one tile more, against fp64 of the same 16-bit operands: one rounding to 8 bits (2^-9) of sums
+    whose fp32 error is far below it; the absolute term is for results near zero."""
+    from nanonemo_b200.ops.gemm import check_status, gemm
+    from nanonemo_b200.ops.linear_ce import _dx_tile
+
+    torch.manual_seed(rows)
+    g, w = torch.randn(rows, 4096, device=DEV).bfloat16(), torch.randn(4096, width, device=DEV).bfloat16()
+    out = gemm(g, w, b_mn=True, bn=_dx_tile(rows, width, g.device))
+    check_status()
+    torch.testing.assert_close(out.double(), g.double() @ w.double(), rtol=2 ** -8, atol=1e-3)
+
+
 @pytest.mark.parametrize("N,D,V,chunk", [(256, 64, 128, None), (300, 256, 1088, None), (1000, 768, 50304, 384), (130, 64, 520, 64), (513, 128, 4160, 257)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_loss_without_gradients_equals_the_loss_with_them(N, D, V, chunk, dtype):

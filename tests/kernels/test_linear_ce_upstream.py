@@ -43,7 +43,7 @@ def head(request, monkeypatch):
         dW.copy_(dw)
         return loss, dx
 
-    def gemm(a, b, out=None, a_mn=False, b_mn=False, accumulate=False):
+    def gemm(a, b, out=None, a_mn=False, b_mn=False, accumulate=False, bn=0):
         out.copy_((a.float().t() if a_mn else a.float()) @ (b.float() if b_mn else b.float().t()))
 
     def ce_inplace(logits, targets, loss_rows, scale, v0, v_total, all_gather, world):
@@ -55,6 +55,7 @@ def head(request, monkeypatch):
     monkeypatch.setattr(linear_ce, "linear_ce_fwd", fwd)
     monkeypatch.setattr(linear_ce, "gemm", gemm)
     monkeypatch.setattr(linear_ce, "vocab_parallel_ce_inplace", ce_inplace)
+    monkeypatch.setattr(linear_ce, "_sm_count", lambda device: 148)
     if request.param == "engine":
         return linear_ce.linear_cross_entropy
     return lambda x, w, t: linear_ce.vocab_parallel_linear_cross_entropy(x, w, t, _Tp, 0)
@@ -165,3 +166,24 @@ def test_scale_takes_one_value_on_the_same_device(launched):
         with pytest.raises(ValueError):
             linear_ce.scale(torch.randn(4, 8), scalar)
     assert not launched
+
+
+@pytest.mark.parametrize("rows,width,hint", [(256, 768, 128), (3072, 768, 128), (3073, 768, 0), (1152, 2048, 128), (1153, 2048, 0), (16384, 64, 128),
+                                             (32768, 768, 0)])
+def test_the_input_gradient_takes_narrow_tiles_while_one_wave_holds_them(monkeypatch, rows, width, hint):
+    hints = []
+
+    def gemm(a, b, out=None, a_mn=False, b_mn=False, accumulate=False, bn=0):
+        if b_mn and not a_mn:
+            hints.append(bn)
+
+    monkeypatch.setattr(linear_ce, "gemm", gemm)
+    monkeypatch.setattr(linear_ce, "gemm_ce_stats", lambda *a: None)
+    monkeypatch.setattr(linear_ce, "ce_inplace", lambda *a: None)
+    monkeypatch.setattr(linear_ce, "vocab_parallel_ce_inplace", lambda *a: None)
+    monkeypatch.setattr(linear_ce, "_sm_count", lambda device: 148)
+    x, w = (torch.empty(n, width, dtype=torch.bfloat16, device="meta", requires_grad=True) for n in (rows, 512))
+    targets = torch.empty(rows, dtype=torch.long, device="meta")
+    linear_ce.linear_cross_entropy(x, w, targets)
+    linear_ce.vocab_parallel_linear_cross_entropy(x, w, targets, _Tp, 0)
+    assert hints == [hint, hint]
