@@ -60,6 +60,7 @@ struct Cfg {
 struct Params {
   int M, N, K;
   int m_blocks, n_blocks, k_splits, kblocks_total, kblocks_per_split;
+  int chain;            // CHAIN: k-blocks per accumulator
   int group_m;          // tile order: groups of group_m m-blocks are swept n-block by n-block (1 = row by row)
   int a_mn, b_mn;       // operand majors
   int out_f32;          // output dtype: 0 = 16-bit (same as inputs), 1 = fp32
@@ -95,7 +96,9 @@ struct DMaps {
   CUtensorMap m[8];       // mode 1: one output map per rank; otherwise m[0]
 };
 
-template <int BN, bool MX>
+// CHAIN (fp32 output, 128-wide tile): the accumulator is handed over every p.chain k-blocks and added to sums in registers (128 columns
+// a thread) while the tensor core fills the other one, as in the pair kernel and for its reason (EPI_CHAINED in gemm2.cu).
+template <int BN, bool MX, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ DMaps tmDs, const Params p) {
@@ -394,39 +397,43 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const uint32_t a_step = p.a_mn ? (16 * 128) >> 4 : 32 >> 4;  // descriptor start-address step per UMMA_K = 16
       const uint32_t b_step = p.b_mn ? (16 * 128) >> 4 : 32 >> 4;
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
-      for (int item = cta0; item < items && ok; item += nctas, ++tile_iter) {
+      const int chain = CHAIN ? p.chain : p.kblocks_per_split;  // k-blocks per accumulator
+      for (int item = cta0; item < items && ok; item += nctas) {
         const int ks = item % p.k_splits;
         const int kb0 = ks * p.kblocks_per_split, kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
-        const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
+        for (int c0 = kb0; c0 < kb1 && ok; c0 += chain, ++tile_iter) {
+          const int c1 = min(c0 + chain, kb1);
+          const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+          if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(stage_base + s * C::kStageBytes), sb = sa + C::kStageBytesA;
-          const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
-          if constexpr (MX) {
-            // scales of this stage: shared memory -> tensor memory (tcgen05 operations of one thread execute in order, so the
-            // copy neither overtakes the previous stage's MMAs nor is overtaken by the ones below)
-            const uint32_t sf_tmem = tmem_base + C::kSfCol;
-            tmem_cp_32x128b_warpx4_elect(el, sf_tmem, make_smem_desc_noswizzle(sa + C::kOperandBytes, 0, 128));
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          for (int kb = c0; kb < c1; ++kb) {
+            if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(stage_base + s * C::kStageBytes), sb = sa + C::kStageBytesA;
+            const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
+            if constexpr (MX) {
+              // scales of this stage: shared memory -> tensor memory (tcgen05 operations of one thread execute in order, so the
+              // copy neither overtakes the previous stage's MMAs nor is overtaken by the ones below)
+              const uint32_t sf_tmem = tmem_base + C::kSfCol;
+              tmem_cp_32x128b_warpx4_elect(el, sf_tmem, make_smem_desc_noswizzle(sa + C::kOperandBytes, 0, 128));
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j)
-              tmem_cp_32x128b_warpx4_elect(el, sf_tmem + 4 + 4 * j, make_smem_desc_noswizzle(sa + C::kOperandBytes + 512 + 512 * j, 0, 128));
+              for (int j = 0; j < BN / 128; ++j)
+                tmem_cp_32x128b_warpx4_elect(el, sf_tmem + 4 + 4 * j, make_smem_desc_noswizzle(sa + C::kOperandBytes + 512 + 512 * j, 0, 128));
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)  // 4 x K = 32 (32 bytes of every 128-byte row); scale byte k of each column
-              umma_mxf8_elect(el, d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), p.idesc | (k << 4) | (k << 29),
-                        sf_tmem | (k << 30), (sf_tmem + 4) | (k << 30), (kb > kb0 || k > 0) ? 1u : 0u);
-          } else {
+              for (uint32_t k = 0; k < 4; ++k)  // 4 x K = 32 (32 bytes of every 128-byte row); scale byte k of each column
+                umma_mxf8_elect(el, d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), p.idesc | (k << 4) | (k << 29),
+                          sf_tmem | (k << 30), (sf_tmem + 4) | (k << 30), (kb > c0 || k > 0) ? 1u : 0u);
+            } else {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k)
-              umma_f16_elect(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < BK / 16; ++k)
+                umma_f16_elect(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > c0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit_elect(el, bar_empty + 8 * s);  // the stage is free once these MMAs have read it
+            if (++s == C::kStages) { s = 0; ph ^= 1; }
           }
-          umma_commit_elect(el, bar_empty + 8 * s);  // the stage is free once these MMAs have read it
-          if (++s == C::kStages) { s = 0; ph ^= 1; }
+          if (ok) umma_commit_elect(el, bar_tfull + 8 * acc);  // accumulator complete
         }
-        if (ok) umma_commit_elect(el, bar_tfull + 8 * acc);  // accumulator complete
       }
     }
   } else {
@@ -446,6 +453,58 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int owner = p.mode == 1 ? m_blk / p.mblocks_per_rank : 0;
       const int d_row = p.mode == 1 ? (m_blk - owner * p.mblocks_per_rank) * BM : m_blk * BM;
       const CUtensorMap* tmD = &tmDs.m[owner];
+      if constexpr (CHAIN) {
+        const int kb0 = item % p.k_splits * p.kblocks_per_split, kbs = min(p.kblocks_per_split, p.kblocks_total - kb0);
+        const int chains = (kbs + p.chain - 1) / p.chain;
+        float sum[BN / 32][32];
+#pragma unroll
+        for (int e = 0; e < BN; ++e) sum[e >> 5][e & 31] = 0.f;
+        bool left = false;
+        for (int i = 0; i < chains; ++i, ++tile_iter) {
+          const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+          const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag);
+          if (!ok) { fail_role = 3; fail_item = item; }
+          if (named_barrier_or(1, kEpilogueThreads, !ok)) { left = true; break; }  // all leave together
+          tc_fence_after();
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+#pragma unroll
+          for (int j = 0; j < BN / 32; ++j) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(t_row + j * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sum[j][e] += __uint_as_float(r[e]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
+        }
+        if (left) break;
+        --tile_iter;  // (the loop's own step)
+#pragma unroll
+        for (int j = 0; j < BN / 32; ++j) {
+          const int col = n_blk * BN + j * 32;
+          if (col < p.N) {
+            uint8_t* buf = staging + (gchunk & 1) * (BM * 128);
+            ++gchunk;
+            if (et == 0 && pending_stores >= 2) tma_wait_group_read<1>();  // the store that last read `buf` is done
+            named_barrier_sync(1, kEpilogueThreads);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<float4*>(buf + row * 128 + ((u ^ (row & 7)) << 4)) =
+                  make_float4(sum[j][4 * u], sum[j][4 * u + 1], sum[j][4 * u + 2], sum[j][4 * u + 3]);
+            fence_proxy_async_smem();
+            named_barrier_sync(1, kEpilogueThreads);
+            if (et == 0) {
+              if (p.reduce_add) tma_reduce_add_2d(tmD, smem_u32(buf), col, d_row);
+              else tma_store_2d(tmD, smem_u32(buf), col, d_row);
+              tma_commit_group();
+            }
+            if (pending_stores < 2) ++pending_stores;
+          }
+        }
+        continue;
+      }
       const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
       const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag);
       if (!ok) { fail_role = 3; fail_item = item; }
@@ -548,9 +607,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
 }
 
-template <int BN, bool MX = false>
+template <int BN, bool MX = false, bool CHAIN = false>
 int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const DMaps& tmDs, const Params& p, int grid, cudaStream_t st) {
-  auto kern = gemm_tcgen05_kernel<BN, MX>;
+  auto kern = gemm_tcgen05_kernel<BN, MX, CHAIN>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, MX>::kSmemBytes) != cudaSuccess) {
@@ -632,7 +691,7 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   if (out_f32 && mode == 0) {
     if (k_splits > 0) splits = k_splits;
     else {
-      splits = nnb_pick_k_splits((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total, 0.5, (double)M * N * 4, accumulate != 0);
+      splits = nnb_even_k_splits((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total);  // (no chains: 256 columns a thread)
     }
     splits = max(1, min(splits, p.kblocks_total));
   }
@@ -868,7 +927,7 @@ extern "C" int nnb_gemm_mxfp8(const void* A, const void* sfa, const void* B, con
   if (out_f32) {
     if (k_splits > 0) splits = k_splits;
     else {
-      splits = nnb_pick_k_splits((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total, 0.3, (double)M * N * 4, accumulate != 0);
+      nnb_plan_k((long long)p.m_blocks * p.n_blocks, sms, p.kblocks_total, 0.3, (double)M * N * 4, accumulate != 0, splits, p.chain);
     }
     splits = max(1, min(splits, p.kblocks_total));
   }
@@ -900,7 +959,8 @@ extern "C" int nnb_gemm_mxfp8(const void* A, const void* sfa, const void* B, con
     else cudaMemset2DAsync(D, ldd * 4, 0, (size_t)N * 4, M, st);
   }
   const int items = p.m_blocks * p.n_blocks * p.k_splits;
-  const int rc = launch<BN, true>(tmA, tmB, tmDs, p, min(items, sms), st);
+  const int rc = p.chain > 0 ? launch<BN, true, true>(tmA, tmB, tmDs, p, min(items, sms), st)
+                         : launch<BN, true>(tmA, tmB, tmDs, p, min(items, sms), st);
   if (rc != 0) return rc;
   NNB_LAUNCH_OK("gemm_mxfp8");
   return 0;

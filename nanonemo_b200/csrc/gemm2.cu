@@ -31,6 +31,12 @@
 //                 logits at all. Against EPI_CE_STATS + the one-sweep kernel this drops the 16-bit logits' write, read and
 //                 rewrite; the accumulator goes straight from tensor memory to the statistics, so the staging tiles' shared
 //                 memory holds a seventh operand stage instead.
+//   EPI_CHAINED   no fusion, fp32 output of a long K loop that is not cut into splits: the accumulator is handed over every p.chain
+//                 k-blocks and added to sums in registers (128 columns a thread, two epilogue groups) while the tensor core fills
+//                 the other one. The tensor core's own additions lose more than an fp32 addition does, and what they lose grows
+//                 with the length of the chain: normal bf16 operands, K = 8192, one chain is 9.1e-6 off 64 bits (2-norm), chains
+//                 of 16 k-blocks 1.0e-6, of 8 4.8e-7 (torch.matmul in fp32: 9.5e-7). Reduce-adding that many splits to memory
+//                 instead costs the output's bytes each time: see nnb_plan_k.
 // All of them compute on the values ROUNDED to the 16-bit output type, so they match the unfused kernels bit for bit.
 #include "gemm2.cuh"
 
@@ -48,10 +54,11 @@ constexpr int kEpilogueThreads = 128;  // one epilogue GROUP: four warps, one pe
 constexpr int kStageBytesA = BM * BK * 2, kStageBytesB = (BN / 2) * BK * 2, kStageBytes = kStageBytesA + kStageBytesB;
 constexpr int kTmemCols = 512;
 // The SwiGLU epilogue fills three staging tiles per 64-feature round (gate, up, act); its backward keeps two (gate, up)
-// tile pairs in flight: both pay for the staging with one stage of the operand ring.
+// tile pairs in flight, the chained fp32 output two tiles per group: they pay for the staging with one stage of the operand ring
+// (chained, 2048 x 5632 x 4096: 93 us, with two tiles and six stages 112; 11264 x 2048 x 2048 87 / 89, 3072 x 2048 x 8192 84 / 81).
 template <int EPI> struct Cfg {
-  static constexpr int kStages = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD) ? 5 : (EPI == EPI_CE_LOSS ? 7 : 6);
-  static constexpr int kStagingTiles = EPI == EPI_SWIGLU ? 3 : (EPI == EPI_SWIGLU_BWD ? 4 : (EPI == EPI_CE_LOSS ? 0 : 2));
+  static constexpr int kStages = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD || EPI == EPI_CHAINED) ? 5 : (EPI == EPI_CE_LOSS ? 7 : 6);
+  static constexpr int kStagingTiles = EPI == EPI_SWIGLU ? 3 : ((EPI == EPI_SWIGLU_BWD || EPI == EPI_CHAINED) ? 4 : (EPI == EPI_CE_LOSS ? 0 : 2));
   static constexpr int kStagingBytes = kStagingTiles * BM * 128;
   // Epilogue groups of four warps. The SwiGLU backward does the most arithmetic per accumulator element (a sigmoid and both
   // products, operands read from shared memory): two groups take alternate 64-column chunks, each with its own staging
@@ -59,7 +66,8 @@ template <int EPI> struct Cfg {
   // The softmax statistics (an exponential per logit) get the same split, one staging tile per group.
   // (The SwiGLU forward stays with one group: a second one needs six staging tiles, which leaves four operand stages, and
   // measured slower: 0.201 vs 0.182 ms at M = 32768, N = 4096, K = 768.)
-  static constexpr int kEpiGroups = (EPI == EPI_SWIGLU_BWD || EPI == EPI_CE_STATS || EPI == EPI_CE_LOSS || EPI == EPI_SWIGLU_ACT) ? 2 : 1;
+  // EPI_CHAINED takes two groups because a thread then holds the sums of 128 columns.
+  static constexpr int kEpiGroups = (EPI == EPI_NONE || EPI == EPI_SWIGLU || EPI == EPI_ROPE) ? 1 : 2;
   static constexpr int kThreads = 64 + kEpiGroups * kEpilogueThreads;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
@@ -67,6 +75,7 @@ template <int EPI> struct Cfg {
 struct Params2 {
   int M, N, K;
   int m_pairs, n_blocks, k_splits, kblocks_total, kblocks_per_split;
+  int chain;    // EPI_CHAINED: k-blocks per accumulator
   int group_m;  // tile order: groups of group_m 256-row blocks are swept n-block by n-block
   int a_mn, b_mn, out_f32, reduce_add, out_bf16;
   uint32_t idesc;
@@ -276,28 +285,32 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const uint32_t a_step = p.a_mn ? (16 * 128) >> 4 : 32 >> 4, b_step = p.b_mn ? (16 * 128) >> 4 : 32 >> 4;
       const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, b_lbo = p.b_mn ? BK * 128 : 16;
       const uint32_t peer_empty = map_to_cta(bar_empty, 1), peer_tfull = map_to_cta(bar_tfull, 1);
-      for (int item = pair0; item < items && ok; item += npairs, ++tile_iter) {
+      const int chain = EPI == EPI_CHAINED ? p.chain : p.kblocks_per_split;  // k-blocks per accumulator
+      for (int item = pair0; item < items && ok; item += npairs) {
         const int ks = item % p.k_splits;
         const int kb0 = ks * p.kblocks_per_split, kb1 = min(kb0 + p.kblocks_per_split, p.kblocks_total);
-        const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
+        for (int c0 = kb0; c0 < kb1 && ok; c0 += chain, ++tile_iter) {
+          const int c1 = min(c0 + chain, kb1);
+          const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+          if (!mbar_wait(bar_tempty + 8 * acc, acc_ph ^ 1, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(stage_base + s * kStageBytes), sb = sa + kStageBytesA;
-          const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          for (int kb = c0; kb < c1; ++kb) {
+            if (!mbar_wait(bar_full + 8 * s, ph, abort_flag)) { ok = false; fail_role = 2; fail_item = lane == 0 ? item : -1; break; }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(stage_base + s * kStageBytes), sb = sa + kStageBytesA;
+            const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_f16_pair(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(el, bar_empty + 8 * s);    // this CTA's stage is free once the MMAs have read it
-          umma_commit_pair(el, peer_empty + 8 * s);   // ... and so is the peer's
-          if (++s == kStages) { s = 0; ph ^= 1; }
-        }
-        if (ok) {
-          umma_commit_pair(el, bar_tfull + 8 * acc);
-          umma_commit_pair(el, peer_tfull + 8 * acc);
+            for (int k = 0; k < BK / 16; ++k)
+              umma_f16_pair(el, d_tmem, da + (uint64_t)(k * a_step), db + (uint64_t)(k * b_step), p.idesc, (kb > c0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(el, bar_empty + 8 * s);    // this CTA's stage is free once the MMAs have read it
+            umma_commit_pair(el, peer_empty + 8 * s);   // ... and so is the peer's
+            if (++s == kStages) { s = 0; ph ^= 1; }
+          }
+          if (ok) {
+            umma_commit_pair(el, bar_tfull + 8 * acc);
+            umma_commit_pair(el, peer_tfull + 8 * acc);
+          }
         }
       }
     }
@@ -318,6 +331,65 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       int m_pair, n_blk;
       tile_coords(tile, m_pair, n_blk);
       const int d_row = (m_pair * 2 + (int)rank) * BM;
+      if constexpr (EPI == EPI_CHAINED) {
+        // group g holds the sums of 32-column chunks g, g + 2, g + 4, g + 6 of this thread's row, chain after chain, then stores them
+        const bool live = d_row < p.M;
+        const int kb0 = item % p.k_splits * p.kblocks_per_split, kbs = min(p.kblocks_per_split, p.kblocks_total - kb0);
+        const int chains = (kbs + p.chain - 1) / p.chain;
+        float sum[4][32];
+#pragma unroll
+        for (int e = 0; e < 128; ++e) sum[e >> 5][e & 31] = 0.f;
+        bool left = false;
+        for (int i = 0; i < chains; ++i, ++tile_iter) {
+          const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+          const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag);
+          if (!ok) { fail_role = 3; fail_item = item; }
+          if (named_barrier_or(epi_bar, kEpilogueThreads, !ok)) { left = true; break; }  // the group leaves together
+          tc_fence_after();
+          if (live) {
+            const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + grp * 32;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              uint32_t r[16];
+              tmem_ld_32x32b_x16(t_row + (j >> 1) * 64 + (j & 1) * 16, r);
+              tmem_ld_wait(r);
+#pragma unroll
+              for (int e = 0; e < 16; ++e) sum[j >> 1][(j & 1) * 16 + e] += __uint_as_float(r[e]);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (rank == 0) mbar_arrive(bar_tempty + 8 * acc);
+            else mbar_arrive_cluster(leader_tempty + 8 * acc);
+          }
+        }
+        if (left) break;
+        --tile_iter;  // (the loop's own step)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int col = n_blk * BN + grp * 32 + j * 64;
+          if (live && col < p.N) {
+            uint8_t* buf = staging + (grp * 2 + (int)(gchunk & 1)) * (BM * 128);  // (counted by stores: a tile may have fewer than four)
+            ++gchunk;
+            if (et == 0 && pending_stores >= 2) tma_wait_group_read<1>();  // the store that last read `buf` is done
+            named_barrier_sync(epi_bar, kEpilogueThreads);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<float4*>(buf + row * 128 + ((u ^ (row & 7)) << 4)) =
+                  make_float4(sum[j][4 * u], sum[j][4 * u + 1], sum[j][4 * u + 2], sum[j][4 * u + 3]);
+            fence_proxy_async_smem();
+            named_barrier_sync(epi_bar, kEpilogueThreads);
+            if (et == 0) {
+              if (p.reduce_add) tma_reduce_add_2d(&tmD, smem_u32(buf), col, d_row);
+              else tma_store_2d(&tmD, smem_u32(buf), col, d_row);
+              tma_commit_group();
+            }
+            if (pending_stores < 2) ++pending_stores;
+          }
+        }
+        continue;
+      }
       const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
       long long tgt_col = -1;  // EPI_CE_LOSS: this row's target relative to the tile's first column
       if constexpr (EPI == EPI_CE_LOSS) {
@@ -737,14 +809,8 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
                 "gemm_swiglu_bwd: 16-bit output, F a multiple of 64 and an aligned saved projection expected");
     p.epi_cols = a.N;
   }
-  int splits = 1;
-  if (a.out_f32) {
-    if (a.k_splits > 0) splits = a.k_splits;
-    else {
-      splits = nnb_pick_k_splits((long long)p.m_pairs * p.n_blocks, pairs, p.kblocks_total, 0.5, (double)a.M * a.N * 4, a.accumulate != 0);
-    }
-    splits = max(1, min(splits, p.kblocks_total));
-  }
+  const int splits = a.out_f32 ? max(1, min(a.k_splits, p.kblocks_total)) : 1;
+  p.chain = a.chain;
   p.kblocks_per_split = (p.kblocks_total + splits - 1) / splits;
   p.k_splits = (p.kblocks_total + p.kblocks_per_split - 1) / p.kblocks_per_split;
   p.group_m = 1;
@@ -790,8 +856,17 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
 }  // namespace
 
 int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st) {
-  switch (a.epilogue) {
 #define NNB_LAUNCH2(E) (a.dtype == NNB_BF16 ? launch2<E, true>(a, st) : launch2<E, false>(a, st))
+  if (a.epilogue == EPI_NONE && a.out_f32 && a.k_splits <= 0) {
+    const int sms = a.max_ctas > 0 ? min(a.max_ctas, nnb_num_sms()) : nnb_num_sms();
+    const int resident = a.dtype == NNB_BF16 ? max_resident_pairs<EPI_NONE, true>() : max_resident_pairs<EPI_NONE, false>();
+    const long long tiles = (long long)((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + BN - 1) / BN);
+    NnbGemm2Args f = a;
+    nnb_plan_k(tiles, max(1, min(sms / 2, resident)), (a.K + BK - 1) / BK, 0.5, (double)a.M * a.N * 4, a.accumulate != 0, f.k_splits, f.chain);
+    if (f.chain > 0) return a.dtype == NNB_BF16 ? launch2<EPI_CHAINED, true>(f, st) : launch2<EPI_CHAINED, false>(f, st);
+    return a.dtype == NNB_BF16 ? launch2<EPI_NONE, true>(f, st) : launch2<EPI_NONE, false>(f, st);
+  }
+  switch (a.epilogue) {
     case EPI_NONE: return NNB_LAUNCH2(EPI_NONE);
     case EPI_SWIGLU: return NNB_LAUNCH2(EPI_SWIGLU);
     case EPI_ROPE: return NNB_LAUNCH2(EPI_ROPE);
@@ -799,7 +874,7 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st) {
     case EPI_SWIGLU_BWD: return NNB_LAUNCH2(EPI_SWIGLU_BWD);
     case EPI_CE_LOSS: return NNB_LAUNCH2(EPI_CE_LOSS);
     case EPI_SWIGLU_ACT: return NNB_LAUNCH2(EPI_SWIGLU_ACT);
-#undef NNB_LAUNCH2
     default: nnb_set_error("gemm2: unknown epilogue %d", a.epilogue); return -1;
   }
+#undef NNB_LAUNCH2
 }

@@ -3,7 +3,8 @@
 #include <cuda_runtime.h>
 
 // Work fused into the epilogue while a tile leaves tensor memory (see gemm2.cu).
-enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4, EPI_CE_LOSS = 5, EPI_SWIGLU_ACT = 6 };
+enum NnbGemm2Epilogue : int { EPI_NONE = 0, EPI_SWIGLU = 1, EPI_ROPE = 2, EPI_CE_STATS = 3, EPI_SWIGLU_BWD = 4, EPI_CE_LOSS = 5, EPI_SWIGLU_ACT = 6,
+                              EPI_CHAINED = 7 /* never asked for: see nnb_plan_k */ };
 
 struct NnbGemm2Args {
   const void *A, *B;
@@ -32,24 +33,48 @@ struct NnbGemm2Args {
   // targets[m] (int64) and is left alone where that column does not exist
   const void* targets = nullptr;
   void* target_logit = nullptr;
+  int chain = 0;  // EPI_CHAINED: k-blocks per accumulator
 };
 
 // Returns 0 on success, 1 when the shape is not served by the pair kernel (caller falls back), < 0 on error.
 int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st);
 
-// K splits of an fp32-output product of `tiles` tiles on `workers` persistent CTAs (or pairs). Splitting evens out the last wave
-// (ceil(tiles s / workers) / s of a whole tile's K loop) but adds the output's bytes once more per split, and a cleared output
-// where the product does not accumulate. Measured: a k-block of a tile takes `us_per_kblock`, a megabyte reduce-added about
-// 0.1 us. With that traffic left out of the count, 50304 x 2048 x 8192 took 8 splits and 1859 us (1 split: 1320), 11264 x 2048 x
-// 8192 486 us (318); 4096 x 768 x 32768 keeps its 3 splits (142 us, 1 split: 186), 768 x 768 x 32768 its 8 (39, 172).
-inline int nnb_pick_k_splits(long long tiles, int workers, int kblocks, double us_per_kblock, double out_bytes, bool accumulate) {
-  const double us_tile = kblocks * us_per_kblock, us_out = out_bytes * 1e-7;
+// K splits that even out the last wave of `tiles` tiles on `workers` persistent CTAs (or pairs), whatever traffic they add. This is how
+// long an accumulator's chain may get: with it as the limit a product is as exact as if it were cut into these splits.
+inline int nnb_even_k_splits(long long tiles, int workers, int kblocks) {
   const int s_max = kblocks / 4 < 1 ? 1 : (kblocks / 4 > 32 ? 32 : kblocks / 4);
   int best_s = 1;
   double best = 1e30;
   for (int s = 1; s <= s_max; ++s) {
-    const double cost = (double)((tiles * s + workers - 1) / workers) / s * us_tile + s * us_out + (s > 1 && !accumulate ? us_out + 2.0 : 0.0);
+    const double cost = (double)((tiles * s + workers - 1) / workers) / s + 0.002 * s;
     if (cost < best - 1e-9) { best = cost; best_s = s; }
   }
   return best_s;
+}
+
+// How the K loop of an fp32-output product is cut: into `splits` that are reduce-added to memory, each of them into chains of `chain`
+// k-blocks that are added up in registers (0: the whole split is one chain). For kernels that hold a thread's sums in registers.
+// Splitting evens out the last wave (ceil(tiles s / workers) / s of a whole tile's K loop) but adds the output's bytes once more per
+// split, and a cleared output where the product does not accumulate. Measured: a k-block of a tile takes `us_per_kblock`, a
+// megabyte reduce-added about 0.1 us. Of counts within 1 % of the least cost the smallest is taken: they measured up to 13 % faster
+// and never more than 1 % slower (2048 x 2048 x 16384: 1 split 100 us, 8 splits 114; 1280 x 768 x 32768: 9 splits 61, 14 64).
+// Fewer splits alone would lengthen the accumulators' chains, and the error grows with them (see EPI_CHAINED): the chains stay
+// as short as the even splits would make them. bf16, accumulating, us and error off 64 bits, even splits / fewer splits without
+// chains / as here: 11264 x 2048 x 8192 386 us 6.0e-7 / 245 us 9.1e-6 / 259 us 6.0e-7; 2048 x 2048 x 8192 81 us 1.0e-6 / 63 us 9.1e-6 /
+// 62 us 1.0e-6; 3072 x 2048 x 4096 77 us 4.1e-7 / 48 us 1.4e-6 / 55 us 4.0e-7; 50304 x 2048 x 1024 360 us 3.2e-7 / 204 us 9.9e-7 /
+// 259 us 3.2e-7; MXFP8 11264 x 2048 x 8192 302 us 7.8e-8 / 222 us 4.7e-7 / 228 us 7.9e-8.
+inline void nnb_plan_k(long long tiles, int workers, int kblocks, double us_per_kblock, double out_bytes, bool accumulate, int& splits,
+                       int& chain) {
+  const double us_tile = kblocks * us_per_kblock, us_out = out_bytes * 1e-7;
+  const int s_max = kblocks / 4 < 1 ? 1 : (kblocks / 4 > 32 ? 32 : kblocks / 4);
+  auto cost = [&](int s) {
+    return (double)((tiles * s + workers - 1) / workers) / s * us_tile + s * us_out + (s > 1 && !accumulate ? us_out + 2.0 : 0.0);
+  };
+  double best = 1e30;
+  for (int s = 1; s <= s_max; ++s) best = cost(s) < best ? cost(s) : best;
+  splits = 1;
+  while (cost(splits) > 1.01 * best) ++splits;
+  const int even = nnb_even_k_splits(tiles, workers, kblocks);
+  const int limit = (kblocks + even - 1) / even;
+  chain = limit < (kblocks + splits - 1) / splits ? limit : 0;
 }

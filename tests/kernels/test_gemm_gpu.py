@@ -111,6 +111,26 @@ def test_default_dispatch(M, N, K):
         _check(out, ref, K)
 
 
+@pytest.mark.parametrize("accumulate", [True, False])
+@pytest.mark.parametrize("M,N,K,chain", [(2048, 2048, 8192, 16), (2176, 2056, 4104, 7), (2432, 2048, 4104, 6), (11264, 2048, 2048, 7), (2304, 2080, 2048, 4),
+                                         (4096, 768, 1024, 6)])
+def test_fp32_products_keep_their_accumulation_chains_short(M, N, K, chain, accumulate):
+    """`chain`: k-blocks that one accumulator sums (the K loop cut into even splits). It loses about 7.1e-8 of the product's 2-norm per
+    k-block (9.1e-6 in a chain of 128); adding the chains up in fp32 costs a few 1e-8 each, and the cleared or existing output one
+    rounding. Sizes with a shorter last chain, a last tile of eight columns, and an odd number of 128-row blocks."""
+    from nanonemo_b200.ops.gemm import check_status, gemm
+
+    torch.manual_seed(M + K)
+    at, bt = torch.randn(K, M, device=DEV).bfloat16(), torch.randn(K, N, device=DEV).bfloat16()
+    out = torch.zeros(M, N, device=DEV)
+    gemm(at, bt, a_mn=True, b_mn=True, out=out, accumulate=accumulate)
+    check_status()
+    ref = at.double().t() @ bt.double()
+    assert (out.double() - ref).norm() <= (7.5e-8 * chain + 2.5e-7) * ref.norm()
+    again = gemm(at, bt, a_mn=True, b_mn=True, out=torch.full_like(out, 1.0), accumulate=True)
+    assert (again.double() - 1 - ref).norm() <= (7.5e-8 * chain + 2.5e-7) * ref.norm()
+
+
 def test_strided_views_and_bn128():
     from nanonemo_b200.ops.gemm import check_status, gemm
 
