@@ -53,6 +53,13 @@ def test_first_derivatives_stay(name):
         assert g.shape == t.shape and g.dtype == t.dtype and not g.requires_grad
 
 
+@pytest.mark.parametrize("name", FORWARD)
+def test_gradients_of_several_upstream_gradients_at_once(name):
+    y, inputs = FORWARD[name]()
+    for g, t in zip(torch.autograd.grad(y, inputs, y.new_empty((3, *y.shape)), is_grads_batched=True), inputs):
+        assert g.shape == (3, *t.shape)
+
+
 @pytest.mark.parametrize("name", BACKWARD)
 def test_an_operator_without_a_formula_stops_a_backward_pass(name):
     out = BACKWARD[name]()
