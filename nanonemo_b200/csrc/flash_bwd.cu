@@ -5,7 +5,7 @@
 // written once and need no atomics (as in the reference kernel, nanonemo/kernels/cuda/flash_attn.cu:
 // 176-340, which keeps them in registers). Per visit, five tensor-core products:
 //     S  = Q K^T            dP = dO V^T                       (M = queries, N = keys, K = head_dim)
-//     P  = exp(S*scale - L) ; dS = P * (dP - D) * scale       (128 compute threads, one per query row)
+//     P  = exp(S*scale - L) ; dS = P * (dP - D) * scale       (256 compute threads, two per query row)
 //     dV += P^T dO          dK += dS^T Q                      (M = keys, N = head_dim, K = queries)
 //     dQ  = dS K                                              (M = queries, N = head_dim, K = keys)
 // P and dS are written once to shared memory as bf16 [query][key] tiles with the 128-byte swizzle; the
@@ -32,7 +32,7 @@
 // register. Now the visit is about 3180: A 1700 (1024 of it the exponentials on the special-function unit), B 770, and the products
 // issue in 1780 (about 1660 at the tensor core's rate). What is left is A's latency and shared memory: 368 KB a visit, 2900 cycles.
 // Whole backward at T4096: 950 -> 696 us, at B32 T1024 360 -> 299 us (of which 50 are the two elementwise kernels).
-// All waits are bounded.
+// All waits are bounded, except the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers).
 #include <cstdlib>
 #include <type_traits>
 
