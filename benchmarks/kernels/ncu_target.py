@@ -1,8 +1,8 @@
 """Small profiler target: a few launches of one kernel family at a shape larger than L2 but holding only
 a few hundred MB, so an `ncu --set full` capture ends by itself in about a minute.
 
-    python benchmarks/kernels/ncu_target.py {gemm,gemm_single,gemm_mxfp8,gemm_swiglu,gemm_swiglu_bwd,gemm_rope,flash,flash128,rmsnorm,swiglu,rope,
-                                             ce,adamw,embedding,quantize}[,more targets] [iters]
+    python benchmarks/kernels/ncu_target.py {gemm,gemm_single,gemm_mxfp8,gemm_swiglu,gemm_swiglu_bwd,gemm_rope,gemm_swiglu_act,
+                                             gemm_wgrad,flash,flash128,rmsnorm,rmsnorm_wide,swiglu,rope,ce,ce_loss,adamw,embedding,quantize}[,more targets] [iters]
 """
 
 import sys
@@ -46,6 +46,17 @@ def build(kind: str):
         dy, w_down = torch.randn(M, 768, device=dev, dtype=bf), torch.randn(768, 2048, device=dev, dtype=bf) * 0.03
         gu = torch.randn(M, 4096, device=dev, dtype=bf)
         fn = lambda: gemm_swiglu_bwd(dy, w_down, gu)  # down projection's dgrad with the SwiGLU backward epilogue (gemm2_tcgen05_kernel<4>)
+    elif kind == "gemm_swiglu_act":
+        from nanonemo_b200.ops.gemm import gemm_swiglu_act
+
+        a, b = torch.randn(M, 768, device=dev, dtype=bf), torch.randn(4096, 768, device=dev, dtype=bf)
+        fn = lambda: gemm_swiglu_act(a, b)  # feed-forward without gradients: the activation alone is stored (gemm2_tcgen05_kernel<6>)
+    elif kind == "gemm_wgrad":
+        from nanonemo_b200.ops.gemm import gemm
+
+        dy, x = torch.randn(8192, 11264, device=dev, dtype=bf), torch.randn(8192, 2048, device=dev, dtype=bf)
+        dw = torch.zeros(11264, 2048, device=dev)
+        fn = lambda: gemm(dy, x, a_mn=True, b_mn=True, out=dw, accumulate=True)  # 1.3B weight gradient, sums in registers (gemm2_tcgen05_kernel<7>)
     elif kind == "gemm_rope":
         from nanonemo_b200.models.layers import rope_cache
         from nanonemo_b200.ops.gemm import gemm_rope
@@ -73,6 +84,11 @@ def build(kind: str):
         d = torch.randn(M, 768, device=dev, dtype=bf, requires_grad=True)
         w = torch.ones(768, device=dev, requires_grad=True)
         fn = lambda: sum(t.float().sum() for t in ops.add_rms_norm(x, d, w, 1e-5, impl="sm100")).backward()
+    elif kind == "rmsnorm_wide":  # two warps per row
+        x = torch.randn(M, 2048, device=dev, requires_grad=True)
+        d = torch.randn(M, 2048, device=dev, dtype=bf, requires_grad=True)
+        w = torch.ones(2048, device=dev, requires_grad=True)
+        fn = lambda: sum(t.float().sum() for t in ops.add_rms_norm(x, d, w, 1e-5, impl="sm100")).backward()
     elif kind == "swiglu":
         gu = torch.randn(M, 4096, device=dev, dtype=bf, requires_grad=True)
         fn = lambda: ops.swiglu_packed(gu, impl="sm100").sum().backward()
@@ -87,6 +103,10 @@ def build(kind: str):
         w = (torch.randn(50304, 768, device=dev) * 0.02).requires_grad_()
         t = torch.randint(0, 50257, (4096,), device=dev)
         fn = lambda: ops.linear_cross_entropy(x, w, t).backward()
+    elif kind == "ce_loss":
+        x, w = torch.randn(4096, 768, device=dev, dtype=bf), torch.randn(50304, 768, device=dev, dtype=bf) * 0.02
+        t = torch.randint(0, 50257, (4096,), device=dev)
+        fn = lambda: ops.linear_cross_entropy(x, w, t)  # no gradients: gemm2_tcgen05_kernel<5> and ce_loss_from_stats_kernel
     elif kind == "adamw":
         from nanonemo_b200.ops.adamw import adamw_flat, sumsq
 

@@ -39,8 +39,8 @@ _NO_FORMULA = {}  # operators that have no derivative formula (so far)
 def _operator(fn):
     """Register `fn` as the CUDA kernel of operator NS::<its name>, with the schema of its annotations. This is
     ``torch.library.custom_op`` without the wrapper that checks every call's results for aliases of its arguments (the kernels
-    below return new tensors only), which took longer than a small launch: the 87 operator calls of a 201-token forward of the
-    114M model took 6.3 ms on the host with it and with ctypes objects for every argument (_lib.py), and 4.6 ms without.
+    below return new tensors only). With custom_op and all else as here, a 201-token forward of the 114M model (87 operator calls)
+    takes 5.2 ms instead of 4.55, add + RMSNorm forward and backward 211 us instead of 188.
     Like ``custom_op``, and unlike a bare definition, an operator without a formula stops a backward pass that reaches it: see
     the end of this file."""
     name = f"{NS}::{fn.__name__}"
