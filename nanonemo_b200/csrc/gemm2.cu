@@ -9,7 +9,7 @@
 //   * TMA loads of both CTAs completing on the leader's "full" barrier (cta_group::2 form of the load),
 //   * tcgen05.commit.cta_group::2 arriving on the "empty" / "accumulator full" barriers of BOTH CTAs (one commit per CTA),
 //   * the peer's epilogue warps arriving remotely on the leader's "accumulator empty" barrier.
-// Roles per CTA as in gemm.cu: warp 0 TMA producer, warp 1 MMA issuer (leader only; both allocate TMEM), warps 2..5
+// Roles per CTA as in gemm.cu: warp 0 TMA producer, warp 1 MMA issuer (leader only; both allocate TMEM), warps 2.. (4 or 8)
 // epilogue (tcgen05.ld -> swizzled staging -> TMA store / reduce-add). All waits are bounded.
 // Replaces the cuBLAS calls behind nn.Linear in the reference (nanonemo/model/layers.py:80-83, 128-130).
 //
@@ -26,7 +26,7 @@
 //                 (nanonemo/kernels/triton/linear_ce.py:21-41).
 //   EPI_SWIGLU_ACT  the same for a forward pass without gradients: nobody reads the projection, so only act leaves the tile, a
 //                 third of the bytes. One staging tile per 64 features instead of three: two epilogue groups and a sixth
-//                 operand stage fit. 32768 x 4096 x 768: 145 us, EPI_SWIGLU 192.
+//                 operand stage fit. 32768 x 4096 x 768: 133 us, EPI_SWIGLU 168.
 //   EPI_CE_LOSS   LM head of a loss without gradients (validation): the statistics and the target's logit of every row, and no
 //                 logits at all. Against EPI_CE_STATS + the one-sweep kernel this drops the 16-bit logits' write, read and
 //                 rewrite; the accumulator goes straight from tensor memory to the statistics, so the staging tiles' shared
@@ -53,22 +53,28 @@ constexpr int BK = 64;
 constexpr int kEpilogueThreads = 128;  // one epilogue GROUP: four warps, one per tensor-memory lane quadrant
 constexpr int kStageBytesA = BM * BK * 2, kStageBytesB = (BN / 2) * BK * 2, kStageBytes = kStageBytesA + kStageBytesB;
 constexpr int kTmemCols = 512;
-// The SwiGLU epilogue fills three staging tiles per 64-feature round (gate, up, act); its backward keeps two (gate, up)
-// tile pairs in flight, the chained fp32 output two tiles per group: they pay for the staging with one stage of the operand ring
+// The SwiGLU epilogue fills three staging tiles per 64-feature round (gate, up, act); its backward has a ring of two (gate, up)
+// tile pairs (three and a stage less: 139 us instead of 141 at K = 768, 182 instead of 176 at K = 2048, M 8192, F 5632), the chained
+// fp32 output two tiles per group: they pay for the staging with one stage of the operand ring
 // (chained, 2048 x 5632 x 4096: 93 us, with two tiles and six stages 112; 11264 x 2048 x 2048 87 / 89, 3072 x 2048 x 8192 84 / 81).
 template <int EPI> struct Cfg {
   static constexpr int kStages = (EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD || EPI == EPI_CHAINED) ? 5 : (EPI == EPI_CE_LOSS ? 7 : 6);
   static constexpr int kStagingTiles = EPI == EPI_SWIGLU ? 3 : ((EPI == EPI_SWIGLU_BWD || EPI == EPI_CHAINED) ? 4 : (EPI == EPI_CE_LOSS ? 0 : 2));
   static constexpr int kStagingBytes = kStagingTiles * BM * 128;
-  // Epilogue groups of four warps. The SwiGLU backward does the most arithmetic per accumulator element (a sigmoid and both
-  // products, operands read from shared memory): two groups take alternate 64-column chunks, each with its own staging
-  // pair, barrier and elected thread, so one group's stores and loads overlap the other's arithmetic.
-  // The softmax statistics (an exponential per logit) get the same split, one staging tile per group.
-  // (The SwiGLU forward stays with one group: a second one needs six staging tiles, which leaves four operand stages, and
-  // measured slower: 0.201 vs 0.182 ms at M = 32768, N = 4096, K = 768.)
-  // EPI_CHAINED takes two groups because a thread then holds the sums of 128 columns.
-  static constexpr int kEpiGroups = (EPI == EPI_NONE || EPI == EPI_SWIGLU || EPI == EPI_ROPE) ? 1 : 2;
-  static constexpr int kThreads = 64 + kEpiGroups * kEpilogueThreads;
+  // Epilogue warps. A group shares staging tiles, a named barrier and a thread that issues its TMA traffic.
+  //   one group of four warps  the plain epilogue: a thread per accumulator row.
+  //   two groups of four       each has staging tiles of its own and takes alternate 64-column chunks: softmax statistics (an exponential
+  //                            per logit), activation only, and EPI_CHAINED, where a thread holds the sums of 128 columns.
+  //   one group of eight       two threads a row, half the columns of a round each, in the SAME staging tiles: the arithmetic of a
+  //                            round is spread over twice the warps without a second set of tiles, which would cost an operand
+  //                            stage, and is done before the tiles are waited for, so it overlaps the stores of the round before.
+  //                            SwiGLU forward 176 -> 168 us (32768 x 4096 x 768), RoPE 65 -> 61 (32768 x 1280 x 768) and at
+  //                            head_dim 128 91 -> 80 (8192 x 3072 x 2048), SwiGLU backward 162 -> 141 (32768 x 2048 x 768).
+  static constexpr int kEpiGroups = (EPI == EPI_NONE || EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD || EPI == EPI_ROPE) ? 1 : 2;
+  static constexpr int kGroupThreads = EPI == EPI_SWIGLU || EPI == EPI_SWIGLU_BWD || EPI == EPI_ROPE ? 2 * kEpilogueThreads : kEpilogueThreads;
+  static constexpr int kEpiThreads = kEpiGroups * kGroupThreads;
+  static constexpr int kThreads = 64 + kEpiThreads + (EPI == EPI_SWIGLU_BWD ? 32 : 0);  // (SwiGLU backward: a warp for the epilogue's loads and stores)
+  static constexpr int kPairs = kStagingTiles / 2;  // SwiGLU backward: ring of (gate, up) tile pairs
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
 };
 
@@ -112,22 +118,30 @@ __device__ __forceinline__ void stage32(uint8_t* my_row, int sw, int u0, const u
   for (int j = 0; j < 4; ++j)
     *reinterpret_cast<uint4*>(my_row + (((u0 + j) ^ sw) << 4)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
 }
-// Rotate-half on 32 (lo, hi) column pairs of one token: lo' = lo c - hi s, hi' = lo s + hi c, computed on the rounded values.
-__device__ __forceinline__ void rope32(uint32_t (&lo)[32], uint32_t (&hi)[32], const float (&cc)[32], const float (&ss)[32], bool bf) {
+// Rotate-half on 16 (lo, hi) column pairs of one token: lo' = lo c - hi s, hi' = lo s + hi c, computed on the rounded values.
+__device__ __forceinline__ void rope16(uint32_t (&lo)[16], uint32_t (&hi)[16], const float (&cc)[16], const float (&ss)[16], bool bf) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
+  for (int i = 0; i < 16; ++i) {
     const float a = round16(__uint_as_float(lo[i]), bf), b = round16(__uint_as_float(hi[i]), bf);
     lo[i] = __float_as_uint(a * cc[i] - b * ss[i]);
     hi[i] = __float_as_uint(a * ss[i] + b * cc[i]);
   }
 }
-// 32 consecutive fp32 table entries of one token (16-byte aligned: the tables have 32 or 64 entries per row).
-__device__ __forceinline__ void load_table32(const float* __restrict__ src, float (&dst)[32]) {
+// 16 consecutive fp32 table entries of one token (16-byte aligned: the tables have 32 or 64 entries per row).
+__device__ __forceinline__ void load_table16(const float* __restrict__ src, float (&dst)[16]) {
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) {
+  for (int i = 0; i < 16; i += 4) {
     const float4 v = __ldg(reinterpret_cast<const float4*>(src + i));
     dst[i] = v.x; dst[i + 1] = v.y; dst[i + 2] = v.z; dst[i + 3] = v.w;
   }
+}
+// 16 consecutive columns of this thread's row into 16-byte units [u0, u0 + 2) of a swizzled staging row.
+__device__ __forceinline__ void stage16(uint8_t* my_row, int sw, int u0, const uint32_t (&r)[16], bool bf) {
+  uint32_t w[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) w[e] = pack16(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]), bf);
+  *reinterpret_cast<uint4*>(my_row + ((u0 ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4*>(my_row + (((u0 + 1) ^ sw) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 __device__ __forceinline__ void pack32(const uint32_t (&r)[32], uint32_t (&w)[16], bool bf) {
 #pragma unroll
@@ -191,8 +205,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + kStagingBytes);
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kStages;
   const uint32_t bar_tfull = bar_empty + 8 * kStages, bar_tempty = bar_tfull + 16;
-  const uint32_t bar_in = bar_tempty + 16;  // EPI_SWIGLU_BWD: the (gate, up) tiles of staging pair 0 / 1 have landed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 6);
+  const uint32_t bar_in = bar_tempty + 16, bar_out = bar_in + 24;  // EPI_SWIGLU_BWD: a (gate, up) pair has landed / has been worked off
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* epi_abort_base = abort_flag + 1;  // one word per epilogue group
 
@@ -205,8 +219,11 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(bar_tfull + 8 * a, 1);
-      mbar_init(bar_tempty + 8 * a, 2 * Cfg<EPI>::kEpiGroups * (kEpilogueThreads / 32));  // leader: epilogue warps of both CTAs
+      mbar_init(bar_tempty + 8 * a, 2 * Cfg<EPI>::kEpiThreads / 32);  // leader: epilogue warps of both CTAs
+    }
+    for (int a = 0; a < 3; ++a) {
       mbar_init(bar_in + 8 * a, 1);
+      mbar_init(bar_out + 8 * a, Cfg<EPI>::kEpiThreads / 32);
     }
     *abort_flag = 0;
     epi_abort_base[0] = 0;
@@ -314,16 +331,76 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
       }
     }
+  } else if (EPI == EPI_SWIGLU_BWD && warp == 2 + Cfg<EPI>::kEpiThreads / 32) {
+    // ------------------------------------------------------------------ I/O warp of the SwiGLU backward (both CTAs)
+    // Fetches the (gate, up) tiles of every 64-column chunk into a ring of pairs and stores what the epilogue warps leave in them, so
+    // that neither a load's latency nor a store's drain stops a warp that computes (when the warps did both themselves, a third of an
+    // epilogue's 16,000 cycles a tile were such waits). The chunks of the NEXT tile are pulled into L2 a whole tile ahead of their use.
+    // (The values straight into registers, 32 bytes of its own row a thread: 195 us, 32 cache lines an access are too many.)
+    if (lane == 0) {
+      constexpr uint32_t kPairs = Cfg<EPI>::kPairs;
+      struct Cursor { int item, c, chunks, col, row; };
+      auto enter = [&](Cursor& u, int item) {  // the first chunk at or after `item`
+        for (u.c = u.chunks = 0; item < items; item += npairs) {
+          int m_pair, n_blk;
+          tile_coords(item / p.k_splits, m_pair, n_blk);
+          u.row = (m_pair * 2 + (int)rank) * BM;
+          u.col = n_blk * BN;
+          u.chunks = u.row < p.M ? min(BN / 64, (p.N - u.col) / 64) : 0;
+          if (u.chunks > 0) break;
+        }
+        u.item = item;
+      };
+      auto step = [&](Cursor& u) { if (++u.c == u.chunks) enter(u, u.item + npairs); };
+      Cursor load, store, ahead;
+      auto fetch = [&](uint32_t pair) {
+        const uint32_t bar = bar_in + 8 * pair, dst = smem_u32(staging + pair * 2 * BM * 128);
+        mbar_expect_tx(bar, 2 * BM * 128);
+        tma_load_2d(dst, &tmE, bar, load.col + load.c * 64, load.row);
+        tma_load_2d(dst + BM * 128, &tmE, bar, p.N + load.col + load.c * 64, load.row);
+        if (load.c == 0) {
+          enter(ahead, load.item + npairs);
+          for (; ahead.c < ahead.chunks; ++ahead.c) {
+            tma_prefetch_l2_2d(&tmE, ahead.col + ahead.c * 64, ahead.row);
+            tma_prefetch_l2_2d(&tmE, p.N + ahead.col + ahead.c * 64, ahead.row);
+          }
+        }
+        step(load);
+      };
+      enter(load, pair0);
+      store = load;
+      uint32_t loaded = 0, stored = 0;
+      for (; loaded < kPairs && load.item < items; ++loaded) fetch(loaded);
+      for (; store.item < items; ++stored) {
+        const uint32_t pair = stored % kPairs;
+        if (!mbar_wait(bar_out + 8 * pair, (stored / kPairs) & 1, abort_flag)) { fail_role = 3; fail_item = store.item; break; }
+        const uint32_t src = smem_u32(staging + pair * 2 * BM * 128);
+        tma_store_2d(&tmD, src, store.col + store.c * 64, store.row);
+        tma_store_2d(&tmD, src + BM * 128, p.N + store.col + store.c * 64, store.row);
+        tma_commit_group();
+        step(store);
+        if (load.item < items) {
+          tma_wait_group_read<0>();  // the pair is free again
+          fetch(pair);
+          ++loaded;
+        }
+      }
+      // whatever was requested has to have landed before the shared memory is given up (after a wait that ran out, too)
+      volatile int unset = 0;
+      for (uint32_t k = stored; k < loaded; ++k) mbar_wait(bar_in + 8 * (k % kPairs), (k / kPairs) & 1, const_cast<int*>(&unset));
+      tma_wait_group<0>();
+    }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------------ epilogue (warps 2.., both CTAs)
     const int q = warp & 3;
     const int row = q * 32 + lane;
-    const int grp = Cfg<EPI>::kEpiGroups == 1 ? 0 : (threadIdx.x - 64) / kEpilogueThreads;  // epilogue group
-    const int et = (threadIdx.x - 64) % kEpilogueThreads;           // thread within the group; et == 0 issues its TMA traffic
+    constexpr int kGroup = Cfg<EPI>::kGroupThreads;
+    const int grp = Cfg<EPI>::kEpiGroups == 1 ? 0 : (threadIdx.x - 64) / kGroup;  // epilogue group
+    const int et = (threadIdx.x - 64) % kGroup;                     // thread within the group; et == 0 issues its TMA traffic
+    const int half = et / kEpilogueThreads;                         // groups of eight warps: which of the row's two threads this is
     const int epi_bar = 1 + grp;                                    // the group's named barrier
     volatile int* epi_abort = epi_abort_base + grp;
     uint32_t tile_iter = 0, gchunk = 0;
-    uint32_t in_count = 0;  // EPI_SWIGLU_BWD: loads this group has consumed from its staging pair (parity of the next wait)
     int pending_stores = 0;
     const uint32_t leader_tempty = map_to_cta(bar_tempty, 0);
     for (int item = pair0; item < items; item += npairs, ++tile_iter) {
@@ -344,7 +421,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
           const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag);
           if (!ok) { fail_role = 3; fail_item = item; }
-          if (named_barrier_or(epi_bar, kEpilogueThreads, !ok)) { left = true; break; }  // the group leaves together
+          if (named_barrier_or(epi_bar, kGroup, !ok)) { left = true; break; }  // the group leaves together
           tc_fence_after();
           if (live) {
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + grp * 32;
@@ -373,13 +450,13 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             uint8_t* buf = staging + (grp * 2 + (int)(gchunk & 1)) * (BM * 128);  // (counted by stores: a tile may have fewer than four)
             ++gchunk;
             if (et == 0 && pending_stores >= 2) tma_wait_group_read<1>();  // the store that last read `buf` is done
-            named_barrier_sync(epi_bar, kEpilogueThreads);
+            named_barrier_sync(epi_bar, kGroup);
 #pragma unroll
             for (int u = 0; u < 8; ++u)
               *reinterpret_cast<float4*>(buf + row * 128 + ((u ^ (row & 7)) << 4)) =
                   make_float4(sum[j][4 * u], sum[j][4 * u + 1], sum[j][4 * u + 2], sum[j][4 * u + 3]);
             fence_proxy_async_smem();
-            named_barrier_sync(epi_bar, kEpilogueThreads);
+            named_barrier_sync(epi_bar, kGroup);
             if (et == 0) {
               if (p.reduce_add) tma_reduce_add_2d(&tmD, smem_u32(buf), col, d_row);
               else tma_store_2d(&tmD, smem_u32(buf), col, d_row);
@@ -391,101 +468,112 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         continue;
       }
       const uint32_t acc = tile_iter & 1, acc_ph = (tile_iter >> 1) & 1;
+      if constexpr (EPI == EPI_SWIGLU_BWD) {
+        // accumulator = d(act). The saved gate and up values arrive in pairs of 64-column tiles (see the I/O warp); a row's two
+        // threads turn 32 columns each into d(gate) | d(up) in place:
+        //   s = sigmoid(g), d(gate) = d(act) u s (1 + g (1 - s)), d(up) = d(act) g s
+        // Every warp goes its own way: it hands over to the I/O warp and to the MMA warp through mbarriers only.
+        const int chunks = d_row < p.M ? min(BN / 64, (p.N - n_blk * BN) / 64) : 0, sw = row & 7;
+        if (!__all_sync(0xffffffffu, mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag))) { fail_role = 3; fail_item = item; break; }
+        tc_fence_after();
+        bool ok = true;
+        for (int c = 0; c < chunks; ++c, ++gchunk) {
+          const uint32_t pair = gchunk % Cfg<EPI>::kPairs, ph = (gchunk / Cfg<EPI>::kPairs) & 1;
+          uint32_t d[32];
+          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + c * 64 + half * 32, d);
+          tmem_ld_wait();
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_in + 8 * pair, ph, abort_flag));
+          if (!ok) { fail_role = 3; fail_item = item; break; }
+          uint8_t* row_g = staging + (pair * 2 * BM + row) * 128;
+          uint8_t* row_u = row_g + BM * 128;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint4* pg = reinterpret_cast<uint4*>(row_g + (((half * 4 + j) ^ sw) << 4));
+            uint4* pu = reinterpret_cast<uint4*>(row_u + (((half * 4 + j) ^ sw) << 4));
+            const uint4 gw = *pg, uw = *pu;
+            const uint32_t gin[4] = {gw.x, gw.y, gw.z, gw.w}, uin[4] = {uw.x, uw.y, uw.z, uw.w};
+            uint32_t og[4], ou[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float d0 = __uint_as_float(d[j * 8 + 2 * e]), d1 = __uint_as_float(d[j * 8 + 2 * e + 1]);
+              const float2 g2 = unpack16(gin[e], BF16), u2 = unpack16(uin[e], BF16);
+              const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
+              og[e] = pack16(d0 * u2.x * s0 * (1.f + g2.x * (1.f - s0)), d1 * u2.y * s1 * (1.f + g2.y * (1.f - s1)), BF16);
+              ou[e] = pack16(d0 * g2.x * s0, d1 * g2.y * s1, BF16);
+            }
+            *pg = make_uint4(og[0], og[1], og[2], og[3]);
+            *pu = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_out + 8 * pair);
+        }
+        if (!ok) break;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (rank == 0) mbar_arrive(bar_tempty + 8 * acc);
+          else mbar_arrive_cluster(leader_tempty + 8 * acc);
+        }
+        continue;
+      }
       long long tgt_col = -1;  // EPI_CE_LOSS: this row's target relative to the tile's first column
       if constexpr (EPI == EPI_CE_LOSS) {
         if (d_row + row < p.M) tgt_col = p.targets[d_row + row] - (long long)n_blk * BN;
       }
-      float rope_c[32], rope_s[32];  // EPI_ROPE, head_dim 64: this token's table row, fetched while the tile is still being multiplied
+      // EPI_ROPE: the table entries of this thread's token, fetched while the tile is still being multiplied: 16 at head_dim 64, 32 at 128
+      float rope_c[2][16], rope_s[2][16];
       if constexpr (EPI == EPI_ROPE) {
-        if (p.half_dim == 32 && n_blk * BN < p.epi_cols) {
-          const int t = (d_row + row) % p.t_len;
-          load_table32(p.cos_t + (size_t)t * 32, rope_c);
-          load_table32(p.sin_t + (size_t)t * 32, rope_s);
-        }
-      }
-      // EPI_SWIGLU_BWD: the saved (gate, up) values of this tile arrive by TMA in 64-column chunks; group g takes chunks g,
-      // g + 2 into staging pair g. Its first chunk is requested here, while the tile is still being multiplied.
-      int bwd_chunks = 0;
-      auto load_gu_chunk = [&](int c) {  // the group's thread et == 0 only; its staging pair must not be the source of a store in flight
-        const uint32_t bar = bar_in + 8 * grp, dst = smem_u32(staging + grp * 2 * (BM * 128));
-        mbar_expect_tx(bar, 2 * BM * 128);
-        tma_load_2d(dst, &tmE, bar, n_blk * BN + c * 64, d_row);
-        tma_load_2d(dst + BM * 128, &tmE, bar, p.N + n_blk * BN + c * 64, d_row);
-      };
-      if constexpr (EPI == EPI_SWIGLU_BWD) {
-        if (d_row < p.M) bwd_chunks = min(BN / 64, (p.N - n_blk * BN) / 64);
-        if (et == 0) {
-          if (grp < bwd_chunks) {
-            if (pending_stores > 0) tma_wait_group_read<0>();
-            load_gu_chunk(grp);
-          }
-          // The group's loads form a chain (a pair is reloaded only after its stores have drained), so their latency is
-          // exposed: pull this tile's later chunk and the NEXT tile's chunks into L2 now, a whole tile ahead of their use.
-          auto prefetch_gu = [&](int nb, int r0, int c) {
-            tma_prefetch_l2_2d(&tmE, nb * BN + c * 64, r0);
-            tma_prefetch_l2_2d(&tmE, p.N + nb * BN + c * 64, r0);
-          };
-          if (grp + 2 < bwd_chunks) prefetch_gu(n_blk, d_row, grp + 2);
-          if (item + npairs < items) {
-            int m2, n2;
-            tile_coords((item + npairs) / p.k_splits, m2, n2);
-            const int r2 = (m2 * 2 + (int)rank) * BM;
-            const int ch2 = r2 < p.M ? min(BN / 64, (p.N - n2 * BN) / 64) : 0;
-            for (int c = grp; c < ch2; c += 2) prefetch_gu(n2, r2, c);
+        if (n_blk * BN < p.epi_cols) {
+          const size_t at = (size_t)((d_row + row) % p.t_len) * p.half_dim;
+          load_table16(p.cos_t + at + half * 16, rope_c[0]);
+          load_table16(p.sin_t + at + half * 16, rope_s[0]);
+          if (p.half_dim == 64) {
+            load_table16(p.cos_t + at + 32 + half * 16, rope_c[1]);
+            load_table16(p.sin_t + at + 32 + half * 16, rope_s[1]);
           }
         }
       }
       const bool ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, abort_flag);
       if (!ok) { fail_role = 3; fail_item = item; }
       if (et == 0) *epi_abort = *abort_flag;
-      named_barrier_sync(epi_bar, kEpilogueThreads);
-      if (*epi_abort) {
-        if constexpr (EPI == EPI_SWIGLU_BWD) {  // the tile loads requested above must have landed before shared memory is given up
-          if (grp < bwd_chunks) mbar_wait(bar_in + 8 * grp, (in_count++) & 1, abort_flag);
-        }
-        break;
-      }
+      named_barrier_sync(epi_bar, kGroup);
+      if (*epi_abort) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       const bool rows_live = d_row < p.M;  // an odd number of 128-row blocks leaves the peer's last block outside the matrix
       constexpr bool bf = BF16;
       const int sw = row & 7;
       if constexpr (EPI == EPI_SWIGLU) {
-        // accumulator columns [0, 128) = gate, [128, 256) = up of features n_blk * 128 ...; 64 features per round, all three
-        // staging tiles (gate | up | act) filled in two half rounds of 32 columns, then three TMA stores
+        // accumulator columns [0, 128) = gate, [128, 256) = up of features n_blk * 128 ...; 64 features per round, a row's two
+        // threads take 32 of them each into the three staging tiles (gate | up | act), then three TMA stores. The arithmetic of a
+        // round is done before the tiles are waited for, so that it overlaps the stores of the round before.
         const int F = p.epi_cols;
-        uint8_t* tiles = staging + grp * 3 * (BM * 128);  // this group's gate | up | act staging tiles
-        for (int c = grp; c < 2 && rows_live; c += Cfg<EPI>::kEpiGroups) {
+        for (int c = 0; c < 2 && rows_live; ++c) {
           const int fcol = n_blk * (BN / 2) + c * 64;
           if (fcol >= F) break;
-          if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
-          uint8_t* row_g = tiles + row * 128;
-          uint8_t* row_u = row_g + BM * 128;
-          uint8_t* row_a = row_u + BM * 128;
+          uint32_t g[32], u[32], wg[16], wu[16], wa[16];
+          tmem_ld_32x32b_x32(t_row + c * 64 + half * 32, g);
+          tmem_ld_32x32b_x32(t_row + BN / 2 + c * 64 + half * 32, u);
+          tmem_ld_wait();
+          pack32(g, wg, bf);
+          pack32(u, wu, bf);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t g[32], u[32], wg[16], wu[16], wa[16];
-            tmem_ld_32x32b_x32(t_row + c * 64 + h * 32, g);
-            tmem_ld_32x32b_x32(t_row + BN / 2 + c * 64 + h * 32, u);
-            tmem_ld_wait();
-            pack32(g, wg, bf);
-            pack32(u, wu, bf);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const float2 gg = unpack16(wg[e], bf), uu = unpack16(wu[e], bf);
-              wa[e] = pack16(gg.x / (1.f + __expf(-gg.x)) * uu.x, gg.y / (1.f + __expf(-gg.y)) * uu.y, bf);
-            }
-            stage32(row_g, sw, h * 4, wg);
-            stage32(row_u, sw, h * 4, wu);
-            stage32(row_a, sw, h * 4, wa);
+          for (int e = 0; e < 16; ++e) {
+            const float2 gg = unpack16(wg[e], bf), uu = unpack16(wu[e], bf);
+            wa[e] = pack16(gg.x / (1.f + __expf(-gg.x)) * uu.x, gg.y / (1.f + __expf(-gg.y)) * uu.y, bf);
           }
+          if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();  // the previous round has left the tiles
+          named_barrier_sync(epi_bar, kGroup);
+          stage32(staging + row * 128, sw, half * 4, wg);
+          stage32(staging + (BM + row) * 128, sw, half * 4, wu);
+          stage32(staging + (2 * BM + row) * 128, sw, half * 4, wa);
           fence_proxy_async_smem();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          named_barrier_sync(epi_bar, kGroup);
           if (et == 0) {
-            tma_store_2d(&tmD, smem_u32(tiles), fcol, d_row);
-            tma_store_2d(&tmD, smem_u32(tiles + BM * 128), F + fcol, d_row);
-            tma_store_2d(&tmE, smem_u32(tiles + 2 * BM * 128), fcol, d_row);
+            tma_store_2d(&tmD, smem_u32(staging), fcol, d_row);
+            tma_store_2d(&tmD, smem_u32(staging + BM * 128), F + fcol, d_row);
+            tma_store_2d(&tmE, smem_u32(staging + 2 * BM * 128), fcol, d_row);
             tma_commit_group();
           }
           pending_stores = 1;
@@ -496,7 +584,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         if (rows_live && fcol < p.epi_cols) {
           uint8_t* tile_a = staging + grp * (BM * 128);
           if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          named_barrier_sync(epi_bar, kGroup);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t g[32], u[32], wa[16];
@@ -512,124 +600,50 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             stage32(tile_a + row * 128, sw, h * 4, wa);
           }
           fence_proxy_async_smem();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          named_barrier_sync(epi_bar, kGroup);
           if (et == 0) {
             tma_store_2d(&tmD, smem_u32(tile_a), fcol, d_row);
             tma_commit_group();
           }
           pending_stores = 1;
         }
-      } else if constexpr (EPI == EPI_SWIGLU_BWD) {
-        // accumulator = d(act); the group's staging pair holds gate | up of the chunk's 64 features for this CTA's 128 rows
-        // (same swizzled layout the stores use). Each thread turns its own row's slots into d(gate) | d(up) in place:
-        //   s = sigmoid(g), d(gate) = d(act) u s (1 + g (1 - s)), d(up) = d(act) g s
-        // then the two tiles are stored at columns col and F + col of the projection's gradient.
-        for (int c = grp; c < bwd_chunks; c += 2) {
-          uint8_t* g_tile = staging + grp * 2 * (BM * 128);
-          if (!mbar_wait(bar_in + 8 * grp, (in_count++) & 1, abort_flag)) { fail_role = 3; fail_item = item; }
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32b_x32(t_row + c * 64, r0);
-          tmem_ld_32x32b_x32(t_row + c * 64 + 32, r1);
-          tmem_ld_wait();
-          uint8_t* row_g = g_tile + row * 128;
-          uint8_t* row_u = row_g + BM * 128;
+      } else if constexpr (EPI == EPI_ROPE) {
+        // 128 columns a round, in two staging tiles; of every 32 column pairs a row's two threads rotate 16 each. head_dim 64: two
+        // heads, the partners are the 32-column halves of one tile; head_dim 128: one head, column i of the first tile rotates
+        // with column i of the second.
+        const bool wide = p.half_dim == 64;
+        const int lo1 = wide ? 32 : 64, to_hi = wide ? 64 : 32;  // first column of the second 32 pairs; distance of the partners
+        for (int g = 0; g < BN / 128 && rows_live; ++g) {
+          const int gcol = n_blk * BN + g * 128;  // (at head_dim 64 the second head may lie outside the matrix)
+          if (gcol >= p.N) break;
+          uint32_t lo[2][16], hi[2][16];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            uint4* pg = reinterpret_cast<uint4*>(row_g + ((j ^ sw) << 4));
-            uint4* pu = reinterpret_cast<uint4*>(row_u + ((j ^ sw) << 4));
-            const uint4 gw = *pg, uw = *pu;
-            const uint32_t gin[4] = {gw.x, gw.y, gw.z, gw.w}, uin[4] = {uw.x, uw.y, uw.z, uw.w};
-            uint32_t og[4], ou[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int i = (j & 3) * 8 + 2 * e;
-              const float d0 = __uint_as_float(j < 4 ? r0[i] : r1[i]), d1 = __uint_as_float(j < 4 ? r0[i + 1] : r1[i + 1]);
-              const float2 g2 = unpack16(gin[e], bf), u2 = unpack16(uin[e], bf);
-              const float s0 = 1.f / (1.f + __expf(-g2.x)), s1 = 1.f / (1.f + __expf(-g2.y));
-              og[e] = pack16(d0 * u2.x * s0 * (1.f + g2.x * (1.f - s0)), d1 * u2.y * s1 * (1.f + g2.y * (1.f - s1)), bf);
-              ou[e] = pack16(d0 * g2.x * s0, d1 * g2.y * s1, bf);
-            }
-            *pg = make_uint4(og[0], og[1], og[2], og[3]);
-            *pu = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+          for (int h = 0; h < 2; ++h) {
+            tmem_ld_32x32b_x16(t_row + g * 128 + h * lo1 + half * 16, lo[h]);
+            tmem_ld_32x32b_x16(t_row + g * 128 + h * lo1 + to_hi + half * 16, hi[h]);
           }
+          tmem_ld_wait();
+          if (gcol < p.epi_cols) rope16(lo[0], hi[0], rope_c[0], rope_s[0], bf);
+          if (wide) {
+            if (gcol < p.epi_cols) rope16(lo[1], hi[1], rope_c[1], rope_s[1], bf);
+          } else if (gcol + 64 < p.epi_cols) {
+            rope16(lo[1], hi[1], rope_c[0], rope_s[0], bf);
+          }
+          if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();
+          named_barrier_sync(epi_bar, kGroup);
+          uint8_t *row0 = staging + row * 128, *row1 = row0 + BM * 128;
+          stage16(row0, sw, half * 2, lo[0], bf);
+          stage16(wide ? row0 : row1, sw, (wide ? 4 : 0) + half * 2, lo[1], bf);
+          stage16(wide ? row1 : row0, sw, (wide ? 0 : 4) + half * 2, hi[0], bf);
+          stage16(row1, sw, 4 + half * 2, hi[1], bf);
           fence_proxy_async_smem();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          named_barrier_sync(epi_bar, kGroup);
           if (et == 0) {
-            const int col = n_blk * BN + c * 64;
-            tma_store_2d(&tmD, smem_u32(g_tile), col, d_row);
-            tma_store_2d(&tmD, smem_u32(g_tile + BM * 128), p.N + col, d_row);
+            tma_store_2d(&tmD, smem_u32(staging), gcol, d_row);
+            if (gcol + 64 < p.N) tma_store_2d(&tmD, smem_u32(staging + BM * 128), gcol + 64, d_row);
             tma_commit_group();
-            if (c + 2 < bwd_chunks) {
-              tma_wait_group_read<0>();  // the stores just issued have left this pair: it can take the chunk after next
-              load_gu_chunk(c + 2);
-            }
           }
           pending_stores = 1;
-        }
-      } else if constexpr (EPI == EPI_ROPE) {
-        if (p.half_dim == 32) {
-          // head_dim 64: a 64-column chunk is one head; its two 32-column halves are the rotation partners
-          for (int c = 0; c < BN / 64 && rows_live; ++c) {
-            const int gcol = n_blk * BN + c * 64;
-            if (gcol >= p.N) break;
-            uint8_t* buf = staging + (gchunk & 1) * (BM * 128);
-            ++gchunk;
-            if (et == 0 && pending_stores >= 2) tma_wait_group_read<1>();
-            named_barrier_sync(epi_bar, kEpilogueThreads);
-            uint32_t r0[32], r1[32], w0[16], w1[16];
-            tmem_ld_32x32b_x32(t_row + c * 64, r0);
-            tmem_ld_32x32b_x32(t_row + c * 64 + 32, r1);
-            tmem_ld_wait();
-            if (gcol < p.epi_cols) rope32(r0, r1, rope_c, rope_s, bf);
-            pack32(r0, w0, bf);
-            pack32(r1, w1, bf);
-            stage32(buf + row * 128, sw, 0, w0);
-            stage32(buf + row * 128, sw, 4, w1);
-            fence_proxy_async_smem();
-            named_barrier_sync(epi_bar, kEpilogueThreads);
-            if (et == 0) {
-              tma_store_2d(&tmD, smem_u32(buf), gcol, d_row);
-              tma_commit_group();
-            }
-            if (pending_stores < 2) ++pending_stores;
-          }
-        } else {
-          // head_dim 128: a head is two chunks; column i of the first rotates with column i of the second, so both
-          // staging tiles are filled together (32 column pairs per half round) and stored as two tiles
-          const int t = (d_row + row) % p.t_len;
-          for (int g = 0; g < BN / 128 && rows_live; ++g) {
-            const int gcol = n_blk * BN + g * 128;
-            if (gcol >= p.N) break;
-            if (et == 0 && pending_stores > 0) tma_wait_group_read<0>();
-            named_barrier_sync(epi_bar, kEpilogueThreads);
-            uint8_t* row_lo = staging + row * 128;
-            uint8_t* row_hi = row_lo + BM * 128;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              uint32_t lo[32], hi[32], w0[16], w1[16];
-              tmem_ld_32x32b_x32(t_row + g * 128 + h * 32, lo);
-              tmem_ld_32x32b_x32(t_row + g * 128 + 64 + h * 32, hi);
-              tmem_ld_wait();
-              if (gcol < p.epi_cols) {
-                float cc[32], ss[32];
-                load_table32(p.cos_t + (size_t)t * 64 + h * 32, cc);
-                load_table32(p.sin_t + (size_t)t * 64 + h * 32, ss);
-                rope32(lo, hi, cc, ss, bf);
-              }
-              pack32(lo, w0, bf);
-              pack32(hi, w1, bf);
-              stage32(row_lo, sw, h * 4, w0);
-              stage32(row_hi, sw, h * 4, w1);
-            }
-            fence_proxy_async_smem();
-            named_barrier_sync(epi_bar, kEpilogueThreads);
-            if (et == 0) {
-              tma_store_2d(&tmD, smem_u32(staging), gcol, d_row);
-              tma_store_2d(&tmD, smem_u32(staging + BM * 128), gcol + 64, d_row);
-              tma_commit_group();
-            }
-            pending_stores = 2;
-          }
         }
       } else {
         const int cols_per_chunk = p.out_f32 ? 32 : 64;
@@ -648,7 +662,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           } else if (et == 0 && pending_stores >= 2) {
             tma_wait_group_read<1>();
           }
-          if (kStore) named_barrier_sync(epi_bar, kEpilogueThreads);
+          if (kStore) named_barrier_sync(epi_bar, kGroup);
           uint8_t* my_row = buf + row * 128;
           if (p.out_f32) {
             uint32_t r[32];
@@ -698,7 +712,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
           if constexpr (!kStore) continue;
           fence_proxy_async_smem();
-          named_barrier_sync(epi_bar, kEpilogueThreads);
+          named_barrier_sync(epi_bar, kGroup);
           if (et == 0) {
             if (p.reduce_add) tma_reduce_add_2d(&tmD, smem_u32(buf), n_blk * BN + col0, d_row);
             else tma_store_2d(&tmD, smem_u32(buf), n_blk * BN + col0, d_row);

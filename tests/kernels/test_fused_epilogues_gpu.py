@@ -243,6 +243,54 @@ def test_gemm_swiglu_backward_epilogue(M, F_, K, dtype):
     assert torch.equal(dgu, gemm_swiglu_bwd(dy, w_down, gu))
 
 
+@pytest.mark.parametrize("M,F_,K", [(128 * 151 + 1, 2048, 64), (128 * 150, 1856, 72), (257, 64 * 77, 128)])
+def test_swiglu_epilogues_over_many_tiles_and_ragged_edges(M, F_, K):
+    """Several tiles per CTA pair, a last row block without a partner, a last column tile of one to three chunks, both directions:
+    every element within the rounding of a 16-bit result of a K-long fp32 sum, so that no tile of the ring can stand in for another."""
+    from nanonemo_b200.ops.gemm import check_status, gemm, gemm_swiglu, gemm_swiglu_bwd
+
+    torch.manual_seed(M)
+    dy, gu = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(M, 2 * F_, device=DEV).bfloat16()
+    w = (torch.randn(K, F_, device=DEV) / math.sqrt(K)).bfloat16()
+    if F_ % 128 == 0:
+        wg = (torch.randn(2 * F_, K, device=DEV) / math.sqrt(K)).bfloat16()
+        proj, act = gemm_swiglu(dy, wg)
+        assert torch.equal(proj, gemm(dy, wg))  # the same accumulator, stored by another epilogue
+        g, u = proj.float().split(F_, dim=1)
+        ref = F.silu(g) * u
+        assert ((act.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6).all()  # one rounding to bf16 (2^-9), and fast exp and division
+        del proj, g, u, ref
+    out = gemm_swiglu_bwd(dy, w, gu)
+    check_status()
+    dact = dy.float() @ w.float()  # (TF32 is off: an fp32 sum)
+    g, u = gu.float().split(F_, dim=1)
+    s = torch.sigmoid(g)
+    for got, ref in ((out[:, :F_], dact * u * s * (1 + g * (1 - s))), (out[:, F_:], dact * g * s)):
+        # one rounding to bf16; an fp32 sum of K products of size 1 / sqrt(K) is off by K^1/2 2^-24 at most here, times the factors' size
+        bound = 2 ** -8 * ref.abs() + 2e-5 * (1 + u.abs()) * (1 + g.abs())
+        assert ((got.float() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,T,H,KVH,hd", [(3, 333, 4, 1, 64), (70, 128, 2, 1, 64), (5, 257, 2, 1, 128)])
+def test_gemm_rope_epilogue_with_an_odd_number_of_rotated_heads(B, T, H, KVH, hd):
+    """The last rotated head shares its 128 columns with one that passes through; rows end inside a tile, tokens wrap inside one."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+    from nanonemo_b200.ops.gemm import check_status, gemm, gemm_rope
+
+    torch.manual_seed(T)
+    N, rot = (H + 2 * KVH) * hd, (H + KVH) * hd
+    x, w = torch.randn(B * T, 192, device=DEV).bfloat16(), (torch.randn(N, 192, device=DEV) / 14).bfloat16()
+    cos, sin = (t.contiguous() for t in rope_cache(hd, T, device=DEV))
+    out, plain = gemm_rope(x, w, cos, sin, T, rot, hd), gemm(x, w)
+    check_status()
+    assert torch.equal(out[:, rot:], plain[:, rot:])
+    ref = ops.rope_qkv(plain.float().view(B, T, N), cos, sin, H, KVH, hd, impl="torch").view(B * T, N)
+    half = hd // 2
+    pair = plain.float().view(B * T, -1, 2, half).abs().sum(2, keepdim=True).expand(-1, -1, 2, -1).reshape(B * T, N)
+    assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6 * pair).all()  # one rounding to bf16, fp32 arithmetic
+
+
 def test_mlp_node_matches_unfused_composition():
     """The one-node feed-forward (SwiGLU backward inside the down projection's dgrad) against linear -> swiglu -> linear built
     from the separate operators, and against fp32 PyTorch: output, input gradient and both weight gradients."""
