@@ -6,7 +6,9 @@ Each translation unit is compiled with ``nvcc -gencode arch=compute_100a,code=sm
 (nvcc cross-compiles without a GPU) and the objects are linked into ``libnanonemo_b200.so`` next to
 the sources, where ``nanonemo_b200.ops._lib`` loads it. Only the CUDA runtime and the driver API
 (resolved at run time through cudaGetDriverEntryPoint) are needed: no torch headers, so a full
-rebuild takes seconds. Objects are rebuilt when their source or a header is newer.
+rebuild takes seconds. Objects are rebuilt when their source or a header is newer. The one file that
+does use torch's headers, ``binding.cpp``, becomes ``nanonemo_b200/ops/_native.so`` (g++, 20 seconds)
+and links against that library.
 """
 
 import argparse
@@ -18,6 +20,7 @@ from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 LIB = HERE / "libnanonemo_b200.so"
+NATIVE = HERE.parent / "ops" / "_native.so"
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler", "-fPIC", "-DNNB_ARCH=100",
               "--expt-relaxed-constexpr", "-Xptxas", "-v"]
@@ -74,7 +77,27 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_native(force)
     return LIB
+
+
+def build_native(force: bool = False) -> Path:
+    """The C++ binding (binding.cpp) against the torch of this interpreter, next to the modules that use it."""
+    import sysconfig
+
+    from torch.utils import cpp_extension
+
+    src, out = HERE / "binding.cpp", NATIVE
+    if force or _stale(out, [src]):
+        include = [*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"]]
+        lib_dirs = cpp_extension.library_paths("cuda")
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native",
+               *(f"-I{p}" for p in include), str(src), "-o", str(out), *(f"-L{p}" for p in lib_dirs), f"-L{HERE}", "-lnanonemo_b200", "-lc10",
+               "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN/../csrc"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"binding.cpp failed:\n{r.stdout}\n{r.stderr}")
+    return out
 
 
 def main(argv=None):

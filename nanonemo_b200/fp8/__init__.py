@@ -20,7 +20,7 @@ from contextlib import contextmanager
 import torch
 
 from nanonemo_b200.ops import _lib
-from nanonemo_b200.ops.gemm import gemm, shadow_of, status_tensor
+from nanonemo_b200.ops.gemm import gemm, shadow_of
 
 
 def fake_quant(x: torch.Tensor) -> torch.Tensor:
@@ -54,20 +54,7 @@ def quantize_mx(x: torch.Tensor, rowwise: bool = True, colwise: bool = False):
     """x [R, C] bf16, R and C multiples of 128 -> (q, sf, qt, sft): q [R, C] e4m3 bytes with blocks along C, qt [C, R] (the
     transpose) with blocks along R, each with its e8m0 scales in the 512-byte-chunk layout the GEMM reads (chunk
     [row / 128][k / 128]; see ``scales_to_plain``). Entries of a pair that was not requested are None."""
-    assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.stride(1) == 1
-    R, C = x.shape
-    dev = x.device
-    q = sf = qt = sft = None
-    if rowwise:
-        q = torch.empty((R, C), dtype=torch.uint8, device=dev)
-        sf = torch.empty((R // 128) * (C // 128) * 512, dtype=torch.uint8, device=dev)
-    if colwise:
-        qt = torch.empty((C, R), dtype=torch.uint8, device=dev)
-        sft = torch.empty((C // 128) * (R // 128) * 512, dtype=torch.uint8, device=dev)
-    _lib.call("nnb_mxfp8_quantize_sw", _lib.ptr(x), _lib.i64(x.stride(0)), _lib.ptr(q) if rowwise else _lib.vp(None), _lib.i64(C),
-              _lib.ptr(sf) if rowwise else _lib.vp(None), _lib.ptr(qt) if colwise else _lib.vp(None), _lib.i64(R),
-              _lib.ptr(sft) if colwise else _lib.vp(None), _lib.i32(R), _lib.i32(C), _lib.vp(_lib.stream_ptr()))
-    return q, sf, qt, sft
+    return _lib.native().quantize_mx(x, rowwise, colwise)
 
 
 def scales_to_plain(sf: torch.Tensor, rows: int, k: int) -> torch.Tensor:
@@ -78,18 +65,7 @@ def scales_to_plain(sf: torch.Tensor, rows: int, k: int) -> torch.Tensor:
 
 def gemm_mxfp8(aq, asf, bq, bsf, out=None, out_dtype=torch.bfloat16, accumulate=False, k_splits=0):
     """(aq [M, K], asf) x (bq [N, K], bsf)^T -> [M, N] bf16 or fp32 on the block-scaled tensor-core path."""
-    M, K = aq.shape
-    N = bq.shape[0]
-    assert bq.shape[1] == K and aq.dtype == bq.dtype == torch.uint8
-    if out is None:
-        assert not accumulate
-        out = torch.empty((M, N), dtype=out_dtype, device=aq.device)
-    assert out.shape == (M, N) and out.stride(1) == 1 and out.dtype in (torch.bfloat16, torch.float32)
-    _lib.call("nnb_gemm_mxfp8", _lib.ptr(aq), _lib.ptr(asf), _lib.ptr(bq), _lib.ptr(bsf), _lib.ptr(out), _lib.i32(M), _lib.i32(N),
-              _lib.i32(K), _lib.i64(aq.stride(0)), _lib.i64(bq.stride(0)), _lib.i64(out.stride(0)),
-              _lib.i32(int(out.dtype == torch.float32)), _lib.i32(int(accumulate)), _lib.i32(k_splits), _lib.i32(0),
-              _lib.ptr(status_tensor(aq.device)), _lib.vp(_lib.stream_ptr()))
-    return out
+    return _lib.native().gemm_mxfp8(aq, asf, bq, bsf, out, out_dtype, accumulate, k_splits)
 
 
 # Quantised copies of a weight are made once per optimizer step, not once per forward: every micro-batch of the step, and

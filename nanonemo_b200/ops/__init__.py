@@ -3,12 +3,13 @@
 (``impl="sm100"``) from ``nanonemo_b200/csrc``. There is no third backend and no runtime probing:
 asking for ``sm100`` without the built library, or off a CUDA device, raises.
 
-The sm100 kernels are bound once, as ``torch.library`` custom operators with fake implementations and autograd
-formulas (``ops/library.py``), and that is what these functions call. The exception is the trainer's engine: a
-parameter that lives in a flat parameter store (it carries ``_main_grad``) runs its operators as ``autograd.Function``s
-that accumulate the weight gradient in place in the flat fp32 buffer and tell the strategy when it is complete — what a
-functional operator may not do — and once such a store exists the weightless operators take the direct functions of
-``ops/direct.py`` too (no dispatcher round trip on the hot path). Both routes launch the same kernels.
+A plain call (exact tensors on CUDA, no tangents, no mode, transform or tracer active) of ``linear``, ``add_rms_norm``, ``flash_attn``,
+``qkv_rope_attention`` and ``mlp_swiglu`` runs natively (csrc/binding.cpp): checks, allocation, launches and the autograd node without
+Python in between. Everything else takes the operators registered with ``torch.library``, with fake implementations and autograd
+formulas (``ops/library.py``) or, for a parameter that lives in the trainer's flat parameter store (it carries ``_main_grad``), the
+``autograd.Function``s that accumulate the weight gradient in place in the flat fp32 buffer and tell the strategy when it is
+complete — what a functional operator may not do. Once such a store exists the weightless operators take the direct functions of
+``ops/direct.py`` too (no dispatcher round trip on the hot path). All routes launch the same kernels.
 
 Operator contracts follow the reference kernels (nanonemo/kernels/triton/*.py,
 nanonemo/kernels/cuda/*.py): ``add_rms_norm(x, delta, w, eps) -> (y, h)``, RoPE on Q and K in one
@@ -18,6 +19,8 @@ launch, ``swiglu``, ``flash_attn(q, k, v)`` reading KV heads directly, ``linear_
 import torch
 import torch.nn.functional as F
 from torch.nn.attention import SDPBackend, sdpa_kernel
+
+from nanonemo_b200.ops import _lib
 
 _ATTN_DTYPES = (torch.bfloat16, torch.float16)  # operand formats of the tensor-core attention kernels
 
@@ -89,6 +92,9 @@ def linear(x, weight, impl="torch"):
         from nanonemo_b200.fp8 import linear_mxfp8
 
         return linear_mxfp8(x, weight)
+    y = _lib.operator_call("linear", x, weight)
+    if y is not NotImplemented:
+        return y
     if in_flat_store(weight) or getattr(weight, "_shadow", None) is not None:
         from nanonemo_b200.ops.gemm import linear_sm100
 
@@ -102,6 +108,9 @@ def add_rms_norm(x, delta, weight, eps, impl="torch"):
     if impl == "torch":
         return add_rms_norm_torch(x, delta, weight, eps)
     _need_cuda(x, "add_rms_norm")
+    out = _lib.operator_call("add_rms_norm", x, delta, weight, eps)
+    if out is not NotImplemented:
+        return out
     from nanonemo_b200.ops import rmsnorm
 
     if in_flat_store(weight):
@@ -177,6 +186,9 @@ def flash_attn(q, k, v, impl="sm100"):
     if impl == "torch":
         return attention_torch(q, k, v)
     _need_cuda(q, "flash_attn")
+    o = _lib.operator_call("flash_attn", q, k, v)
+    if o is not NotImplemented:
+        return o
     from nanonemo_b200.ops import library
 
     dt = q.dtype if q.dtype in _ATTN_DTYPES else torch.bfloat16  # 16-bit operands of one dtype; fp32 goes through bf16 and back
@@ -213,6 +225,9 @@ def fused_ok() -> bool:
 def qkv_rope_attention(x, weight, cos, sin, n_heads, n_kv_heads, head_dim):
     """Packed QKV projection + RoPE (GEMM epilogue) + causal GQA attention (sm100 only)."""
     _need_cuda(x, "qkv_rope_attention")
+    y = _lib.operator_call("qkv_rope_attention", x, weight, cos, sin, n_heads, n_kv_heads, head_dim)
+    if y is not NotImplemented:
+        return y
     if in_flat_store(weight) or getattr(weight, "_shadow", None) is not None:
         from nanonemo_b200.ops.fused_block import qkv_rope_attention as f
 
@@ -249,6 +264,9 @@ def mlp_swiglu(x, w_gu, w_down):
     shadow) it is one autograd node whose backward computes the activation's backward in a GEMM epilogue; elsewhere it is
     the registered gate||up operator followed by the registered linear."""
     _need_cuda(x, "mlp_swiglu")
+    y = _lib.operator_call("mlp_swiglu", x, w_gu, w_down)
+    if y is not NotImplemented:
+        return y
     engine = lambda w: in_flat_store(w) or getattr(w, "_shadow", None) is not None
     if engine(w_gu) and engine(w_down) and getattr(w_gu, "_gather_in_gemm", None) is None:
         from nanonemo_b200.ops.fused_block import mlp_swiglu as f

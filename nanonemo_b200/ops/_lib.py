@@ -9,8 +9,11 @@ library sits in the source tree. Every launcher returns 0 on success or a negati
 """
 
 import ctypes
+import importlib
 import operator
 import os
+import sys
+import types
 from functools import lru_cache
 from pathlib import Path
 
@@ -39,6 +42,18 @@ def lib():
         raise RuntimeError(f"{LIB_PATH} is missing: build it with `python -m nanonemo_b200.csrc.build` "
                            "(the sm100 operators have no fallback)")
     return handle
+
+
+@lru_cache(maxsize=1)
+def native():
+    """The C++ binding (csrc/binding.cpp): raw launches and operators that run without Python in between."""
+    lib()  # (says how to build it when it is missing)
+    return importlib.import_module("nanonemo_b200.ops._native")
+
+
+def operator_call(name: str, *args):
+    """Operator `name` of the binding, or NotImplemented where the call is not a plain one (see csrc/binding.cpp)."""
+    return NotImplemented if torch.compiler.is_compiling() else getattr(native(), name)(*args)
 
 
 # Argument types of every launcher (p pointer, i int, q long long, f float, d double), in the order of its C declaration. With
@@ -104,7 +119,20 @@ def _launcher(name: str):
     return fn
 
 
-LAUNCHES = 0  # launchers called through `call` since import (the benchmark reports the delta)
+_python_launches = 0  # launchers called through `call` since import; the binding counts its own
+
+
+class _Module(types.ModuleType):
+    @property
+    def LAUNCHES(self) -> int:  # all launches since import (the benchmark reports the delta)
+        return self._python_launches + (native().launches() if native.cache_info().currsize else 0)
+
+    @LAUNCHES.setter
+    def LAUNCHES(self, n: int):
+        self._python_launches += n - self.LAUNCHES
+
+
+sys.modules[__name__].__class__ = _Module
 
 
 def stream_ptr() -> int:
@@ -113,9 +141,9 @@ def stream_ptr() -> int:
 
 def call(name: str, *args) -> None:
     """Call launcher `name`; raises with the library's message on a non-zero return."""
-    global LAUNCHES
+    global _python_launches
     rc = _launcher(name)(*args)
-    LAUNCHES += 1
+    _python_launches += 1
     if rc != 0:
         msg = lib().nnb_last_error()
         raise RuntimeError(f"{name} failed (code {rc}): {msg.decode() if msg else 'no message'}")
@@ -123,10 +151,10 @@ def call(name: str, *args) -> None:
 
 def call_rc(name: str, *args) -> int:
     """Like `call`, for launchers that answer 1 when they do not serve the problem (nothing was launched): returns 0 or 1."""
-    global LAUNCHES
+    global _python_launches
     rc = _launcher(name)(*args)
     if rc == 0:
-        LAUNCHES += 1
+        _python_launches += 1
     elif rc != 1:
         msg = lib().nnb_last_error()
         raise RuntimeError(f"{name} failed (code {rc}): {msg.decode() if msg else 'no message'}")

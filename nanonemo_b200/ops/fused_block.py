@@ -24,7 +24,7 @@ import os
 
 import torch
 
-from nanonemo_b200.ops import attention, rope, swiglu_act
+from nanonemo_b200.ops import _lib, attention, rope, swiglu_act
 from nanonemo_b200.ops.gemm import (_rowmajor2d, compute_dtype, gemm, gemm_rope, gemm_swiglu, gemm_swiglu_act, gemm_swiglu_bwd,
                                     linear_backward, no_backward, shadow_of)
 
@@ -97,6 +97,9 @@ class _QKVRopeAttention(torch.autograd.Function):
 
 def qkv_rope_attention(x, weight, cos, sin, n_heads, n_kv_heads, head_dim):
     """x: (B, T, d); weight: [(H + 2 KVH) hd, d] (fp32 master or 16-bit) -> attention output (B, T, H hd), bf16 compute."""
+    y = _lib.operator_call("qkv_rope_attention", x, weight, cos, sin, n_heads, n_kv_heads, head_dim)
+    if y is not NotImplemented:
+        return y
     return _QKVRopeAttention.apply(x, weight, cos, sin, n_heads, n_kv_heads, head_dim)
 
 
@@ -184,6 +187,9 @@ class _MLPSwiGLU(torch.autograd.Function):
 
 def mlp_swiglu(x, w_gu, w_down):
     """x: (..., d); w_gu: [2 F, d] (gate rows first); w_down: [d, F] -> down(silu(x Wg^T) * (x Wu^T)), shape (..., d)."""
+    y = _lib.operator_call("mlp_swiglu", x, w_gu, w_down) if FUSE_SWIGLU_BWD else NotImplemented
+    if y is not NotImplemented:
+        return y
     if no_backward(x, w_gu, w_down):
         dt = compute_dtype()  # no backward will ask for the projection: only the activation leaves its GEMM
         act = gemm_swiglu_act(_rows16(x, dt), shadow_of(w_gu, dt))

@@ -21,21 +21,17 @@ from torch.autograd.forward_ad import unpack_dual
 from nanonemo_b200.ops import _lib
 
 _CODE = {torch.bfloat16: 1, torch.float16: 2}
-_status: dict = {}
 
 
 def status_tensor(device) -> torch.Tensor:
-    key = (device.type, device.index)
-    t = _status.get(key)
-    if t is None:
-        t = torch.zeros(4, dtype=torch.int32, device=device)
-        _status[key] = t
-    return t
+    """The status words of the bounded waits on a device (one tensor per device, owned by the binding)."""
+    device = torch.device(device)
+    return _lib.native().status_tensor(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def check_status(device=None):
     """Raise if any GEMM launched so far on `device` gave up on a bounded wait (synchronises)."""
-    for key, t in _status.items():
+    for t in _lib.native().status_tensors():
         code, role, block, item = t.tolist()
         if code != 0:
             t.zero_()
@@ -54,23 +50,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          out_dtype: torch.dtype | None = None, accumulate: bool = False, k_splits: int = 0, bn: int = 0,
          max_ctas: int = 0) -> torch.Tensor:
     """a: [M, K] (or [K, M] when a_mn); b: [N, K] (or [K, N] when b_mn) -> out [M, N]."""
-    a, b = _rowmajor2d(a), _rowmajor2d(b)
-    assert a.dtype == b.dtype and a.dtype in _CODE, f"gemm needs matching bf16/fp16 inputs, got {a.dtype}/{b.dtype}"
-    K, M = (a.shape if a_mn else a.shape[::-1])
-    Kb, N = (b.shape if b_mn else b.shape[::-1])
-    assert K == Kb, f"inner dimensions differ: {K} vs {Kb}"
-    out_dtype = out_dtype or (out.dtype if out is not None else a.dtype)
-    assert out_dtype in (a.dtype, torch.float32)
-    if out is None:
-        assert not accumulate
-        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    assert out.shape == (M, N) and out.stride(1) == 1 and out.dtype == out_dtype
-    _lib.call("nnb_gemm_bf16", _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.i32(M), _lib.i32(N), _lib.i32(K),
-              _lib.i64(a.stride(0)), _lib.i64(b.stride(0)), _lib.i64(out.stride(0)), _lib.i32(int(a_mn)), _lib.i32(int(b_mn)),
-              _lib.i32(_CODE[a.dtype]), _lib.i32(int(out_dtype == torch.float32)), _lib.i32(int(accumulate)),
-              _lib.i32(k_splits), _lib.i32(bn), _lib.i32(max_ctas), _lib.ptr(status_tensor(a.device)),
-              _lib.vp(_lib.stream_ptr()))
-    return out
+    return _lib.native().gemm(a, b, a_mn, b_mn, out, out_dtype, accumulate, k_splits, bn, max_ctas)
 
 
 def _fused_call(name: str, *args) -> bool:
@@ -81,59 +61,25 @@ def _fused_call(name: str, *args) -> bool:
 
 def gemm_swiglu(x2: torch.Tensor, w_gu: torch.Tensor):
     """x2 [M, K] @ w_gu [2F, K]^T with the SwiGLU activation in the epilogue -> (gu [M, 2F], act [M, F]) or None."""
-    M, K = x2.shape
-    F = w_gu.shape[0] // 2
-    if M < 256 or F % 128 or w_gu.stride(1) != 1 or x2.stride(1) != 1:
-        return None
-    gu = torch.empty((M, 2 * F), dtype=x2.dtype, device=x2.device)
-    act = torch.empty((M, F), dtype=x2.dtype, device=x2.device)
-    ok = _fused_call("nnb_gemm_swiglu", _lib.ptr(x2), _lib.ptr(w_gu), _lib.ptr(gu), _lib.ptr(act), _lib.i32(M), _lib.i32(F),
-                     _lib.i32(K), _lib.i64(x2.stride(0)), _lib.i64(w_gu.stride(0)), _lib.i64(2 * F), _lib.i64(F),
-                     _lib.i32(_CODE[x2.dtype]), _lib.ptr(status_tensor(x2.device)), _lib.vp(_lib.stream_ptr()))
-    return (gu, act) if ok else None
+    return _lib.native().gemm_swiglu(x2, w_gu)
 
 
 def gemm_swiglu_act(x2: torch.Tensor, w_gu: torch.Tensor):
     """The activation of ``gemm_swiglu`` alone (the projection never reaches memory) -> act [M, F] or None."""
-    M, K = x2.shape
-    F = w_gu.shape[0] // 2
-    if M < 256 or F % 128 or w_gu.stride(1) != 1 or x2.stride(1) != 1:
-        return None
-    act = torch.empty((M, F), dtype=x2.dtype, device=x2.device)
-    ok = _fused_call("nnb_gemm_swiglu_act", _lib.ptr(x2), _lib.ptr(w_gu), _lib.ptr(act), _lib.i32(M), _lib.i32(F), _lib.i32(K),
-                     _lib.i64(x2.stride(0)), _lib.i64(w_gu.stride(0)), _lib.i64(F), _lib.i32(_CODE[x2.dtype]),
-                     _lib.ptr(status_tensor(x2.device)), _lib.vp(_lib.stream_ptr()))
-    return act if ok else None
+    return _lib.native().gemm_swiglu_act(x2, w_gu)
 
 
 def gemm_swiglu_bwd(dy2: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor):
     """SwiGLU backward inside the down projection's input-gradient GEMM: dy2 [M, d] @ w_down [d, F] is the gradient of
     act = silu(gate) * up; the epilogue reads the saved projection gu [M, 2F] and writes d(gate) | d(up) [M, 2F] directly
     (the gradient of act is never stored) -> dgu or None when the CTA-pair kernel does not serve the shape."""
-    M, K = dy2.shape
-    F = w_down.shape[1]
-    if (M < 256 or F < 128 or F % 64 or gu.shape != (M, 2 * F) or gu.stride(1) != 1 or gu.stride(0) % 8 or w_down.stride(1) != 1
-            or dy2.stride(1) != 1 or gu.dtype != dy2.dtype or w_down.dtype != dy2.dtype):
-        return None
-    dgu = torch.empty((M, 2 * F), dtype=gu.dtype, device=gu.device)
-    ok = _fused_call("nnb_gemm_swiglu_bwd", _lib.ptr(dy2), _lib.ptr(w_down), _lib.ptr(gu), _lib.ptr(dgu), _lib.i32(M), _lib.i32(F),
-                     _lib.i32(K), _lib.i64(dy2.stride(0)), _lib.i64(w_down.stride(0)), _lib.i64(gu.stride(0)), _lib.i64(2 * F),
-                     _lib.i32(_CODE[dy2.dtype]), _lib.ptr(status_tensor(dy2.device)), _lib.vp(_lib.stream_ptr()))
-    return dgu if ok else None
+    return _lib.native().gemm_swiglu_bwd(dy2, w_down, gu)
 
 
 def gemm_rope(x2: torch.Tensor, w: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, t_len: int, rope_cols: int, head_dim: int):
     """x2 [M, K] @ w [N, K]^T with rotate-half RoPE on columns [0, rope_cols) in the epilogue (row m at position
     m % t_len; cos / sin fp32 [t_len, head_dim / 2] contiguous) -> [M, N] or None."""
-    M, K = x2.shape
-    N = w.shape[0]
-    if M < 256 or N < 128 or head_dim not in (64, 128) or N % head_dim or rope_cols % head_dim:
-        return None
-    out = torch.empty((M, N), dtype=x2.dtype, device=x2.device)
-    ok = _fused_call("nnb_gemm_rope", _lib.ptr(x2), _lib.ptr(w), _lib.ptr(out), _lib.ptr(cos), _lib.ptr(sin), _lib.i32(M), _lib.i32(N),
-                     _lib.i32(K), _lib.i64(x2.stride(0)), _lib.i64(w.stride(0)), _lib.i64(N), _lib.i32(t_len), _lib.i32(rope_cols),
-                     _lib.i32(head_dim), _lib.i32(_CODE[x2.dtype]), _lib.ptr(status_tensor(x2.device)), _lib.vp(_lib.stream_ptr()))
-    return out if ok else None
+    return _lib.native().gemm_rope(x2, w, cos, sin, t_len, rope_cols, head_dim)
 
 
 def gemm_ce_stats(x2: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
@@ -239,7 +185,8 @@ def linear_backward(dy2, x2, weight, w16, need_dx: bool, need_dw: bool):
 
 
 def linear_sm100(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    return _Linear.apply(x, weight)
+    y = _lib.operator_call("linear", x, weight)
+    return y if y is not NotImplemented else _Linear.apply(x, weight)
 
 
 # ----------------------------------------------------------------------------- GEMMs fused with a collective

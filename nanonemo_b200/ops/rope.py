@@ -11,14 +11,9 @@ import torch
 
 from nanonemo_b200.ops import _lib
 
-_CODE = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
-
 
 def rope_packed_raw(x2, out2, cos, sin, T, n_rot_heads, hd, n_copy_cols, sign):
-    M = x2.shape[0]
-    _lib.call("nnb_rope_packed", _lib.ptr(x2), _lib.ptr(out2), _lib.ptr(cos), _lib.ptr(sin), _lib.i64(M), _lib.i32(T),
-              _lib.i32(n_rot_heads), _lib.i32(hd), _lib.i32(n_copy_cols), _lib.i64(x2.stride(0)), _lib.i64(out2.stride(0)),
-              _lib.f32(sign), _lib.i32(_CODE[x2.dtype]), _lib.vp(_lib.stream_ptr()))
+    _lib.native().rope_packed(x2, out2, cos, sin, T, n_rot_heads, hd, n_copy_cols, sign)
 
 
 def _tables(cos, sin, T):

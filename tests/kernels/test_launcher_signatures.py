@@ -27,3 +27,13 @@ def test_every_launcher_that_is_called_by_name_has_a_signature():
     root = Path(_lib.__file__).resolve().parents[1]
     called = {n for f in root.rglob("*.py") for n in re.findall(r'"(nnb_\w+)"', f.read_text())}
     assert called <= set(_lib._SIGNATURES), called - set(_lib._SIGNATURES)
+
+
+def test_the_native_binding_declares_the_launchers_as_the_sources_do():
+    text = (Path(_lib.__file__).resolve().parents[1] / "csrc" / "binding.cpp").read_text()
+    protos = re.findall(r"^int (nnb_\w+)\(([^)]*)\);", text, re.M)
+    assert protos
+    for name, args in protos:
+        args = [a.strip() for a in args.split(",") if a.strip()]
+        sig = "".join("p" if "*" in a or a == "cudaStream_t" else CODES[a] for a in args)
+        assert sig == _lib._SIGNATURES[name], name

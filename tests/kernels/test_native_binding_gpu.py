@@ -1,0 +1,290 @@
+"""The native operators against the registered operators and Python autograd functions that served every call before them: the same
+results over the forms a call can have, and everything that is not a plain call (modes, transforms, tangents) still goes there."""
+
+import math
+
+import pytest
+import torch
+from torch.autograd import forward_ad
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture
+def python_route(monkeypatch):
+    """Run a function with the native operators switched off."""
+    from nanonemo_b200.ops import _lib
+
+    def run(fn):
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "operator_call", lambda *a: NotImplemented)
+            return fn()
+
+    return run
+
+
+def _native(name, *args):
+    from nanonemo_b200.ops import _lib
+
+    out = _lib.operator_call(name, *args)
+    assert out is not NotImplemented, f"{name} did not take a plain call"
+    return out
+
+
+def _run(fn, leaves, grads):
+    out = fn()
+    out = out if isinstance(out, tuple) else (out,)
+    pairs = [(o, g) for o, g in zip(out, grads) if g is not None and o.requires_grad]
+    got = torch.autograd.grad([o for o, _ in pairs], leaves, [g for _, g in pairs], allow_unused=True) if pairs else ()
+    return (*[o.detach() for o in out], *got)
+
+
+def _same(a, b):
+    assert len(a) == len(b)
+    for x, y in zip(a, b):
+        assert (x is None) == (y is None)
+        if x is not None:
+            assert x.dtype == y.dtype and x.shape == y.shape and x.device == y.device
+            assert torch.equal(x, y)  # the same launches: bitwise
+
+
+def _rand(*shape, dtype=torch.float32, grad=True):
+    return (torch.randn(*shape, device=DEV) * 0.5).to(dtype).requires_grad_(grad)
+
+
+@pytest.mark.parametrize("amp", [None, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("x_shape", [(7, 64), (300, 64), (2, 65, 64), (5, 3, 1, 64)])
+@pytest.mark.parametrize("x_dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.float32)])
+def test_linear(python_route, amp, x_shape, x_dtype, w_dtype):
+    from nanonemo_b200 import ops
+
+    torch.manual_seed(0)
+    x, w = _rand(*x_shape, dtype=x_dtype), _rand(136, 64, dtype=w_dtype)
+    dy = torch.randn(*x_shape[:-1], 272, device=DEV)[..., ::2]  # strided upstream gradient
+    with torch.autocast("cuda", dtype=amp or torch.bfloat16, enabled=amp is not None):
+        _native("linear", x, w)
+        fn = lambda: _run(lambda: ops.linear(x, w, impl="sm100"), (x, w), (dy.to(amp or torch.bfloat16),))  # noqa: E731
+        _same(fn(), python_route(fn))
+
+
+def test_linear_on_strided_and_unaligned_inputs(python_route):
+    from nanonemo_b200 import ops
+
+    base, w = torch.randn(130, 200, device=DEV).bfloat16(), _rand(72, 64)
+    for x in (base[:, :64], base[:, 3:67], base.t()[:64].t(), base[::2, 8:72], torch.randn(64, 130, device=DEV).t(), base[:1, :64].expand(130, 64)):
+        x = x.detach().requires_grad_()
+        for dy in (torch.randn(x.shape[0], 72, device=DEV).bfloat16(), torch.ones((), device=DEV).bfloat16().expand(x.shape[0], 72),
+                   torch.randn(72, x.shape[0], device=DEV).bfloat16().t(), torch.randn(x.shape[0], 80, device=DEV).bfloat16()[:, 3:75]):
+            _native("linear", x, w)
+            fn = lambda: _run(lambda: ops.linear(x, w, impl="sm100"), (x, w), (dy,))  # noqa: E731, B023
+            _same(fn(), python_route(fn))
+
+
+@pytest.mark.parametrize("with_delta", [False, True])
+@pytest.mark.parametrize("x_dtype,d_dtype,amp", [(torch.float32, torch.bfloat16, True), (torch.float32, torch.float32, False), (torch.bfloat16, torch.bfloat16, False),
+                                                 (torch.float16, torch.float32, False), (torch.float32, torch.float32, True)])
+@pytest.mark.parametrize("use", [(True, True), (True, False), (False, True)])
+def test_add_rms_norm(python_route, with_delta, x_dtype, d_dtype, amp, use):
+    from nanonemo_b200 import ops
+
+    torch.manual_seed(1)
+    x, w = _rand(3, 37, 264, dtype=x_dtype), (1 + 0.1 * torch.randn(264, device=DEV)).requires_grad_()
+    delta = _rand(3, 37, 528, dtype=d_dtype, grad=False)[..., ::2].requires_grad_() if with_delta else None
+    with torch.autocast("cuda", dtype=torch.bfloat16, enabled=amp):
+        y, h = _native("add_rms_norm", x, delta, w, 1e-5)
+        grads = (torch.randn_like(y) if use[0] else None, torch.randn_like(h).transpose(0, 1).contiguous().transpose(0, 1) if use[1] else None)
+        fn = lambda: _run(lambda: ops.add_rms_norm(x, delta, w, 1e-5, impl="sm100"), [t for t in (x, delta, w) if t is not None], grads)  # noqa: E731
+        _same(fn(), python_route(fn))
+
+
+@pytest.mark.parametrize("B,T,H,KVH,hd", [(1, 65, 2, 1, 64), (2, 130, 4, 4, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("layout", ["bthd", "bhtd", "odd"])
+def test_flash_attn(python_route, B, T, H, KVH, hd, dtype, layout):
+    from nanonemo_b200 import ops
+
+    torch.manual_seed(2)
+
+    def make(heads):
+        if layout == "bthd":
+            return torch.randn(B, T, heads, hd, device=DEV).to(dtype).transpose(1, 2)
+        if layout == "bhtd":
+            return torch.randn(B, heads, T, hd, device=DEV).to(dtype)
+        return torch.randn(B, T, heads, hd + 4, device=DEV).to(dtype)[..., 3:hd + 3].transpose(1, 2)  # neither aligned nor dense
+
+    q, k, v = (make(n).detach().requires_grad_() for n in (H, KVH, KVH))
+    do = make(H)
+    _native("flash_attn", q, k, v)
+    fn = lambda: _run(lambda: ops.flash_attn(q, k, v), (q, k, v), (do,))  # noqa: E731
+    a, b = fn(), python_route(fn)
+    _same(a[:1] + a[2:], b[:1] + b[2:])
+    # dQ is summed in fp32 by atomic adds in any order, then rounded once
+    assert ((a[1].float() - b[1].float()).abs() <= 2 ** -7 * b[1].float().abs() + 1e-4).all()
+
+
+def _engine(*ws):
+    for w in ws:
+        w._shadow, w._main_grad = w.detach().bfloat16(), torch.zeros_like(w)
+        w._told = []
+        w._grad_ready_cb = lambda p, done: p._told.append(done)
+
+
+@pytest.mark.parametrize("M", [128, 320])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_engine_nodes_add_into_the_flat_gradient_and_report_it(python_route, M, hd):
+    """Both sides of the 256 rows from which the fused GEMM epilogues serve; x in fp32 and bf16."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+
+    torch.manual_seed(3)
+    d, F, H, KVH = 192, 256, 2, 1
+    cos, sin = rope_cache(hd, 1024, device=DEV)
+    for dtype in (torch.float32, torch.bfloat16):
+        x = _rand(2, M // 2, d, dtype=dtype)
+        wq, gu, down, norm = _rand((H + 2 * KVH) * hd, d), _rand(2 * F, d), _rand(d, F), (torch.rand(d, device=DEV) + 0.5).requires_grad_()
+        calls = {"qkv": ((wq,), lambda: ops.qkv_rope_attention(x, wq, cos, sin, H, KVH, hd)), "mlp": ((gu, down), lambda: ops.mlp_swiglu(x, gu, down)),  # noqa: B023
+                 "linear": ((wq,), lambda: ops.linear(x, wq, impl="sm100")), "norm": ((norm,), lambda: ops.add_rms_norm(x, None, norm, 1e-5, impl="sm100")[0])}  # noqa: B023
+        for name, (ws, fn) in calls.items():
+            got = []
+            for run in (lambda f: f(), python_route):
+                _engine(*ws)
+                out = run(fn)
+                g = torch.linspace(-1, 1, out.numel(), device=DEV).view(out.shape).to(out.dtype)
+                dx, *dw = torch.autograd.grad(out, (x, *ws), g, allow_unused=True)
+                assert all(t is None for t in dw) and all(w._told == [True] for w in ws), name
+                got.append((out.detach(), dx, *(w._main_grad for w in ws)))
+            for a, b in zip(*got):  # the weight gradients of these sizes are cut into splits that are added in any order; dQ likewise
+                assert a.dtype == b.dtype
+                assert (a.float() - b.float()).norm() <= (2 ** -8 if a.dtype != torch.float32 or name == "qkv" else 1e-6) * b.float().norm(), name
+
+
+def test_calls_without_gradients_match_the_registered_operators(python_route):
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+
+    torch.manual_seed(4)
+    cos, sin = rope_cache(64, 512, device=DEV)
+    for rows in (33, 300):
+        x, wq, gu, down = _rand(1, rows, 128, grad=False), _rand(256, 128), _rand(512, 128), _rand(128, 256)
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            fn = lambda: (ops.qkv_rope_attention(x, wq, cos, sin, 2, 1, 64), ops.mlp_swiglu(x, gu, down), ops.linear(x, wq, impl="sm100"),  # noqa: E731, B023
+                          *ops.add_rms_norm(x, None, down[:, 0].contiguous(), 1e-5, impl="sm100"))  # noqa: B023
+            _same(fn(), python_route(fn))
+
+
+def _cases():
+    from nanonemo_b200 import ops
+
+    torch.manual_seed(5)
+    x, w, n = _rand(66, 64, dtype=torch.bfloat16), _rand(72, 64), torch.ones(64, device=DEV).requires_grad_()
+    q = _rand(1, 2, 66, 64, dtype=torch.bfloat16)
+    return [(lambda a: ops.linear(a, w, impl="sm100"), x), (lambda a: ops.add_rms_norm(a, a.detach(), n, 1e-5, impl="sm100")[0], x), (lambda a: ops.flash_attn(a, a.detach(), a.detach()), q)]
+
+
+def test_second_derivatives_batched_gradients_and_hooks_behave_as_before(python_route):
+    for fn, x in _cases():
+        out = fn(x)
+        g = torch.randn_like(out)
+        plain = torch.autograd.grad(out, x, g)[0]
+
+        def second():  # create_graph=True, and one more derivative: the gradient, or the refusal, of the registered operators
+            try:
+                (d,) = torch.autograd.grad(fn(x), x, g, create_graph=True)  # noqa: B023
+                return d.detach(), torch.autograd.grad(d.float().sum(), x)[0]  # noqa: B023
+            except (RuntimeError, AssertionError) as e:
+                return type(e)
+
+        a, b = second(), python_route(second)
+        assert all(torch.allclose(s.float(), t.float(), rtol=2e-2, atol=1e-3) for s, t in zip(a, b)) if isinstance(b, tuple) else a is b
+        batched = torch.autograd.grad(fn(x), x, torch.stack((g, 2 * g)), is_grads_batched=True)[0]
+        assert batched.shape == (2, *x.shape) and torch.allclose(batched[0].float(), plain.float(), rtol=2e-2, atol=1e-3)
+        # saved tensors pass through hooks, and what was saved is checked for in-place changes
+        packed = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(1) or t.cpu(), lambda t: t.to(DEV)):
+            out = fn(x)
+        assert packed and torch.allclose(torch.autograd.grad(out, x, g)[0].float(), plain.float(), rtol=2e-2, atol=1e-3)
+    from nanonemo_b200 import ops
+
+    y, w = torch.randn(66, 64, device=DEV).bfloat16().requires_grad_(), _rand(72, 64)
+    z = y * 1
+    out = ops.linear(z, w, impl="sm100")
+    with torch.no_grad():
+        z.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out, w, torch.ones_like(out))
+
+
+def test_outputs_may_be_changed_in_place():
+    for fn, x in _cases()[:2]:  # (attention keeps its output for the backward)
+        fn(x).mul_(2).float().sum().backward()
+        assert x.grad is not None
+
+
+def test_anything_but_a_plain_call_takes_the_other_route(python_route):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from nanonemo_b200.ops import _lib
+
+    x, w = _rand(66, 64, dtype=torch.bfloat16), _rand(72, 64)
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert _lib.operator_call("linear", x, w) is not NotImplemented
+    assert _lib.operator_call("linear", x.cpu(), w.cpu()) is NotImplemented
+    assert _lib.operator_call("linear", x.detach().as_subclass(Sub), w) is NotImplemented
+    with Mode():
+        assert _lib.operator_call("linear", x, w) is NotImplemented
+    with torch.device(DEV):
+        assert _lib.operator_call("linear", x, w) is NotImplemented
+    with forward_ad.dual_level():
+        assert _lib.operator_call("linear", forward_ad.make_dual(x.detach(), torch.ones_like(x)), w) is NotImplemented
+    seen = []
+    torch.func.vmap(lambda a: seen.append(_lib.operator_call("linear", a, w)) or a)(x[None])
+    torch.func.grad(lambda a: seen.append(_lib.operator_call("linear", a, w)) or a.float().sum())(x.detach())
+    assert seen == [NotImplemented, NotImplemented]
+    for fn, x in _cases():  # torch.func.grad through the front end: as the registered operators have it
+        f = lambda a: fn(a).float().sum()  # noqa: E731, B023
+        try:
+            ref = python_route(lambda: torch.func.grad(f)(x.detach()))  # noqa: B023
+        except RuntimeError as e:
+            with pytest.raises(type(e)):
+                torch.func.grad(f)(x.detach())
+        else:
+            assert torch.allclose(torch.func.grad(f)(x.detach()).float(), ref.float(), rtol=2e-2, atol=1e-3)
+
+
+def test_wrong_calls_are_refused_with_the_same_errors(python_route):
+    from nanonemo_b200 import ops
+    from nanonemo_b200.ops.gemm import gemm
+
+    x, w = _rand(66, 64, dtype=torch.bfloat16), _rand(72, 64)
+    q = _rand(1, 2, 66, 64, dtype=torch.bfloat16)
+    calls = [lambda: ops.linear(x, w[:, :32], impl="sm100"), lambda: ops.linear(x, w[:, :60], impl="sm100"), lambda: ops.flash_attn(q[..., :32], q[..., :32], q[..., :32]),
+             lambda: ops.add_rms_norm(x[:, :60], None, w[0, :60], 1e-5, impl="sm100"), lambda: ops.add_rms_norm(x.double(), None, w[0], 1e-5, impl="sm100")]
+    for call in calls:
+        with pytest.raises(Exception) as ref:
+            python_route(call)
+        with pytest.raises(ref.type):
+            call()
+    with pytest.raises(AssertionError):
+        gemm(x.detach(), w.detach())  # dtypes differ
+    with pytest.raises(AssertionError):
+        gemm(x.detach(), x.detach()[:, :32])
+
+
+def test_launches_are_counted_once():
+    from nanonemo_b200 import ops
+    from nanonemo_b200.ops import _lib
+
+    x, w = _rand(66, 64, dtype=torch.bfloat16), _rand(72, 64, dtype=torch.bfloat16)
+    before = _lib.LAUNCHES
+    y = ops.linear(x, w, impl="sm100")
+    torch.autograd.grad(y, (x, w), torch.ones_like(y))
+    assert _lib.LAUNCHES - before == 3
+    assert math.isfinite(y.float().sum().item())
