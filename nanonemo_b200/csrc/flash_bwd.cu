@@ -3,35 +3,34 @@
 // One CTA owns 128 keys of one (batch, KV head) and visits every (query head of the group, query tile)
 // at or after its keys; dK and dV of the tile accumulate in TMEM over the whole GQA group, so they are
 // written once and need no atomics (as in the reference kernel, nanonemo/kernels/cuda/flash_attn.cu:
-// 176-340, which keeps them in registers). Per visit, five tensor-core products:
-//     S  = Q K^T            dP = dO V^T                       (M = queries, N = keys, K = head_dim)
-//     P  = exp(S*scale - L) ; dS = P * (dP - D) * scale       (256 compute threads, two per query row)
+// 176-340, which keeps them in registers). Per visit, five tensor-core products, on TRANSPOSED score tiles:
+//     S^T = K Q^T           dP^T = V dO^T                     (M = keys, N = queries, K = head_dim)
+//     P^T = exp(S^T*scale - L) ; dS^T = P^T * (dP^T - D) * scale   (256 compute threads, two per key row)
 //     dV += P^T dO          dK += dS^T Q                      (M = keys, N = head_dim, K = queries)
 //     dQ  = dS K                                              (M = queries, N = head_dim, K = keys)
-// P and dS are written once to shared memory as bf16 [query][key] tiles with the 128-byte swizzle; the
-// same bytes serve as the K-major A operand of dQ and, read through an MN-major descriptor, as the
-// transposed A operand of dV / dK. Q and dO tiles arrive by TMA and are read both K-major (S, dP) and
-// MN-major (dK, dV) without any transposed copy. dQ partial tiles leave through a swizzled fp32
-// staging tile and a TMA reduce-add (cp.reduce.async.bulk.tensor .add.f32) into an fp32 buffer that a
-// small kernel converts at the end. D = rowsum(dO * O) is a pre-pass kernel in this file.
-// 512 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4..7 drain dQ, warps 8..15 compute: two threads per query row,
-// one for keys 0..63 of the tile and one for keys 64..127 (same TMEM lanes, different columns).
+// Keys as rows are how dV and dK want their A operand: P^T and dS^T go back into tensor memory over the scores and products they came
+// from, as 16-bit values, and are multiplied from there. Only dS^T also goes to shared memory ([key][query], 128-byte swizzle), as the
+// MN-major A operand of dQ. K is read K-major (S^T) and MN-major (dQ), Q and dO K-major (scores) and MN-major (dK, dV), without any
+// transposed copy. dQ partial tiles leave through a swizzled fp32 staging tile and a TMA reduce-add
+// (cp.reduce.async.bulk.tensor .add.f32) into an fp32 buffer that a small kernel converts at the end. D = rowsum(dO * O) is a pre-pass
+// kernel in this file.
+// 512 threads: warp 0 TMA producer, warp 1 MMA issuer, warp 2 fetches L and D of the visits' queries, warps 4..7 drain dQ, warps 8..15
+// compute: two threads per key row, one for queries 0..63 of the tile and one for queries 64..127 (same TMEM lanes, different columns).
 //
-// Software pipeline. The score tile is double buffered in tensor memory (S0 | S1 | dP | dV | dK = 512 columns; the dQ
-// partial product of a visit is accumulated into the first 64 columns of THAT visit's S buffer, which is free once P has
-// been computed from it). The compute warps only do  A: P = exp(S scale - L)  and  B: dS = P (dP - D) scale;  the dQ tile
-// leaves through four warps of its own, and a visit's L and D are fetched one visit ahead:
+// Software pipeline. The score tile is double buffered in tensor memory (S0 | S1 | dP | dV | dK = 512 columns). Within a visit's score
+// buffer P^T takes the outer 32 columns on either side and the dQ partial product the 64 between them. The compute warps only do
+// A: P^T = exp(S^T scale - L)  and  B: dS^T = P^T (dP^T - D) scale;  the dQ tile leaves through four warps of its own:
 //     compute :  A(n)                    B(n)                     A(n+1)   ...
 //     tensor  :        S(n+1)   dV(n)          dQ(n) dK(n) dP(n+1)
 //     drain   :  dQ(n-1)                                          dQ(n)
 // S(n+1) needs only the drained buffer, so it is issued before dV(n) and is complete long before A(n+1); dP(n+1) before
 // B(n+1). No block barrier is left in the loop: the compute warps meet the tensor core through mbarriers alone.
-// What bounded a visit, by clock counters of one thread per role (cycles, B8 H12/4 T4096): with dQ drained by the compute warps
-// and the L / D loads in their chain 4286 (wait for S and the loads 890, A 1531, drain 949, wait for dP 206, B 709), and the one-lane
-// MMA issuer needed 2760 for the 32 products of a visit, up to 115 each, because every descriptor had to be moved to a uniform
-// register. Now the visit is about 3180: A 1700 (1024 of it the exponentials on the special-function unit), B 770, and the products
-// issue in 1780 (about 1660 at the tensor core's rate). What is left is A's latency and shared memory: 368 KB a visit, 2900 cycles.
-// Whole backward at T4096: 950 -> 696 us, at B32 T1024 360 -> 299 us (of which 50 are the two elementwise kernels).
+// What bounds a visit, by clock counters of one thread per role (cycles): with the queries as rows, and P and dS both written to and read
+// from shared memory, 2980 (waits 690, A 1660, B 620) beside 368 KB of shared-memory traffic, 2900 cycles; now 272 KB, and about
+// 3050 (waits 480, A 1700, of it 1024 exponentials on the special-function unit, B 850): one chain through A and B, whose latency two
+// warps a scheduler do not hide. (A quarter or half of the exponentials as polynomials on the multiply-add pipe: no change.) Whole backward,
+// us, queries as rows / keys as rows: B32 H12/4 T1024 303 / 283, B128 T256 184 / 174, B64 H8/8 T200 84 / 80, B2 H12/4 T333 35 / 33, B8 H12/4 T4096
+// 697 / 702, where the card's power limit (1.63 GHz under this kernel) evens them out.
 // All waits are bounded, except the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers).
 #include <cstdlib>
 #include <type_traits>
@@ -56,13 +55,16 @@ constexpr int kTile16 = 128 * 64 * 2;     // a [128 x 64] 16-bit tile = 16 KB
 constexpr int kStagesQ = 3;             // a stage is released when dK / dQ of its visit are done and refilled two visits ahead
 // shared memory map (bytes)
 constexpr int kOffK = 0, kOffV = kTile16, kOffQdO = 2 * kTile16;               // ring of (Q | dO)
-constexpr int kOffP = kOffQdO + kStagesQ * 2 * kTile16, kOffdS = kOffP + 2 * kTile16;
+constexpr int kOffdS = kOffQdO + kStagesQ * 2 * kTile16;                       // dS^T: [128 keys] x two groups of 64 queries
 constexpr int kOffStage = kOffdS + 2 * kTile16;                                // fp32 [128 x 64] = 32 KB
 constexpr int kOffBars = kOffStage + 2 * kTile16;
-constexpr int kSmem = kOffBars + 256 + 1024;
+constexpr int kOffLD = kOffBars + 256;                                         // float [2 parities][2 (-L log2e, -D scale)][128]
+constexpr int kSmem = kOffLD + 2 * 2 * BQ * 4 + 1024;
 // tensor memory columns
 constexpr int kColS = 0 /* two buffers: + 128 * (visit & 1) */, kColdP = 256, kColdV = 384, kColdK = 448, kTmemCols = 512;
-constexpr int kColdQ = kColS;            // dQ(n) lands in columns [0, 64) of S buffer (n & 1), after P(n) has been taken from it
+// A visit's S^T buffer also holds its P^T, the queries 0..63 in columns [0, 32) and 64..127 in [96, 128), and between them its dQ
+constexpr int kColdQ = kColS + 32;
+__device__ __forceinline__ uint32_t col_of_queries(int k) { return k < 4 ? 8 * k : 96 + 8 * (k - 4); }  // 16 queries from 16 k, of P^T and dS^T
 
 struct BParams {
   int B, H, KVH, T, n_q_tiles, group;
@@ -88,12 +90,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBars);
-  // barriers: kv_full, q_full[3], q_empty[3], s_full[2], dp_full, p_written, ds_written, dq_full, dq_read, p_free, all_done
+  // barriers: kv_full, q_full[3], q_empty[3], s_full[2], dp_full, p_written, ds_written, dq_full, dq_read, ld_full[2], ld_empty[2], all_done
   const uint32_t bar_kv = smem_u32(bars), bar_qf = bar_kv + 8, bar_qe = bar_qf + 8 * kStagesQ;
   const uint32_t bar_s = bar_qe + 8 * kStagesQ, bar_dp = bar_s + 16, bar_p = bar_dp + 8, bar_ds = bar_p + 8;
-  const uint32_t bar_dq = bar_ds + 8, bar_dqr = bar_dq + 8, bar_pf = bar_dqr + 8, bar_fin = bar_pf + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kStagesQ + 9);
+  const uint32_t bar_dq = bar_ds + 8, bar_dqr = bar_dq + 8, bar_lf = bar_dqr + 8, bar_le = bar_lf + 16, bar_fin = bar_le + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kStagesQ + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* s_ld = reinterpret_cast<float*>(smem + kOffLD);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Longest-job-first over the whole grid: key tile 0 is visited by every query tile, the last one by a single tile, and the
@@ -117,7 +120,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     mbar_init(bar_ds, kComputeThreads);
     mbar_init(bar_dq, 1);
     mbar_init(bar_dqr, kDrainThreads);
-    mbar_init(bar_pf, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_lf + 8 * i, 32);
+      mbar_init(bar_le + 8 * i, kComputeThreads);
+    }
     mbar_init(bar_fin, 1);
     *abort_flag = 0;
     fence_barrier_init();
@@ -154,24 +160,24 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ---------------------------------------------------------------- MMA issuer (warp-uniform: see umma_f16_elect)
       const bool el = elect_one();
       bool ok = mbar_wait(bar_kv, 0, abort_flag);
-      const uint32_t sK = s_base + kOffK, sV = s_base + kOffV, sP = s_base + kOffP, sdS = s_base + kOffdS;
+      const uint32_t sK = s_base + kOffK, sV = s_base + kOffV, sdS = s_base + kOffdS;
       // ring positions of visits n (cur) and n + 1 (nxt) and the phase of nxt, counted along instead of divided out
       uint32_t cur = 0, nxt = 0, nxt_ph = 0;
       auto stage_at = [&](uint32_t s) { return s_base + kOffQdO + s * 2 * kTile16; };
-      // S(n) = Q K^T into score buffer n & 1 (K-major operands, 4 k-steps of 16 over head_dim)
+      // S^T(n) = K Q^T into score buffer n & 1 (K-major operands, 4 k-steps of 16 over head_dim)
       auto issue_s = [&](int n, uint32_t s) {
         const uint32_t sQ = stage_at(s);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_f16_elect(el, tmem_base + kColS + (n & 1) * BKV, make_smem_desc(sQ + k * 32, 16, 1024), make_smem_desc(sK + k * 32, 16, 1024), p.idesc_s, k > 0);
+          umma_f16_elect(el, tmem_base + kColS + (n & 1) * BKV, make_smem_desc(sK + k * 32, 16, 1024), make_smem_desc(sQ + k * 32, 16, 1024), p.idesc_s, k > 0);
         umma_commit_elect(el, bar_s + 8 * (n & 1));
       };
-      // dP(n) = dO V^T
+      // dP^T(n) = V dO^T
       auto issue_dp = [&](uint32_t s) {
         const uint32_t sdO = stage_at(s) + kTile16;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_f16_elect(el, tmem_base + kColdP, make_smem_desc(sdO + k * 32, 16, 1024), make_smem_desc(sV + k * 32, 16, 1024), p.idesc_s, k > 0);
+          umma_f16_elect(el, tmem_base + kColdP, make_smem_desc(sV + k * 32, 16, 1024), make_smem_desc(sdO + k * 32, 16, 1024), p.idesc_s, k > 0);
         umma_commit_elect(el, bar_dp);
       };
       if (ok && iters > 0) {
@@ -185,43 +191,70 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int n = 0; n < iters && ok; ++n) {
         const uint32_t sQ = stage_at(cur), sdO = sQ + kTile16;
         if (++nxt == kStagesQ) { nxt = 0; nxt_ph ^= 1; }
-        // S(n + 1) goes into the other score buffer, whose scores were read before bar_p(n - 1) and whose first columns held
-        // dQ(n - 1): wait until that was drained. (Waited for in every visit, so that bar_dq is never two phases ahead of the drain.)
+        // S^T(n + 1) goes into the other score buffer: its scores were read before bar_p(n - 1), its P^T(n - 1) is read by dV(n - 1),
+        // which is ahead in order, and its dQ(n - 1) must have been drained. (Waited for in every visit, so that bar_dq is never two
+        // phases ahead of the drain.)
         if (n >= 1 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }
         if (n + 1 < iters) {
           if (!mbar_wait(bar_qf + 8 * nxt, nxt_ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
           issue_s(n + 1, nxt);
         }
-        if (!mbar_wait(bar_p, n & 1, abort_flag)) { ok = false; break; }     // P(n) is in shared memory, S(n) has been read
+        if (!mbar_wait(bar_p, n & 1, abort_flag)) { ok = false; break; }     // P^T(n) is in tensor memory, S^T(n) has been read
         tc_fence_after();
-        // dV += P^T dO: A = [query][key] tile read MN-major (M = keys: two 64-key groups 16 KB apart), B = [query][hd]
-        // tile read MN-major; 8 k-steps of 16 query rows (2048 bytes each).
+        // dV += P^T dO: A = P^T in tensor memory (16 queries = 8 columns per k-step), B = [query][hd] tile read MN-major (16 query rows =
+        // 2048 bytes per step)
+        const uint32_t buf = tmem_base + kColS + (n & 1) * BQ, tdS = tmem_base + kColdP;
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k)
-          umma_f16_elect(el, tmem_base + kColdV, make_smem_desc(sP + k * 2048, kTile16, 1024), make_smem_desc(sdO + k * 2048, kTile16, 1024),
-                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
-        umma_commit_elect(el, bar_pf);   // P may be overwritten
-        if (!mbar_wait(bar_ds, n & 1, abort_flag)) { ok = false; break; }    // dS(n) is in shared memory, dP(n) has been read
+          umma_f16_ts_elect(el, tmem_base + kColdV, buf + col_of_queries(k), make_smem_desc(sdO + k * 2048, kTile16, 1024), p.idesc_dkv,
+                            (n > 0 || k > 0) ? 1u : 0u);
+        if (!mbar_wait(bar_ds, n & 1, abort_flag)) { ok = false; break; }    // dS^T(n) is written, dP^T(n) has been read
         tc_fence_after();
-        // dQ(n) = dS K into the score buffer of this visit: A = dS K-major over keys (two 64-key blocks), B = K tile read
-        // MN-major (16 key rows per step)
+        // dQ(n) = dS K into the middle of the score buffer of this visit: A = [key][query] tile read MN-major (M = queries: two groups of 64,
+        // 16 KB apart), B = K tile read MN-major; 8 k-steps of 16 key rows
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k)
-          umma_f16_elect(el, tmem_base + kColdQ + (n & 1) * BKV, make_smem_desc(sdS + (k / 4) * kTile16 + (k % 4) * 32, 16, 1024),
-                   make_smem_desc(sK + k * 2048, kTile16, 1024), p.idesc_dq, k > 0);
-        umma_commit_elect(el, bar_dq);        // before dK(n): the drain runs beside dK(n) and dP(n + 1)
-        // dK += dS^T Q (operands as for dV)
+          umma_f16_elect(el, tmem_base + kColdQ + (n & 1) * BQ, make_smem_desc(sdS + k * 2048, kTile16, 1024), make_smem_desc(sK + k * 2048, kTile16, 1024),
+                   p.idesc_dq, k > 0);
+        umma_commit_elect(el, bar_dq);        // before dK(n): the drain runs beside dK(n) and dP^T(n + 1)
+        // dK += dS^T Q, operands as for dV
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k)
-          umma_f16_elect(el, tmem_base + kColdK, make_smem_desc(sdS + k * 2048, kTile16, 1024), make_smem_desc(sQ + k * 2048, kTile16, 1024),
-                   p.idesc_dkv, (n > 0 || k > 0) ? 1u : 0u);
+          umma_f16_ts_elect(el, tmem_base + kColdK, tdS + col_of_queries(k), make_smem_desc(sQ + k * 2048, kTile16, 1024), p.idesc_dkv,
+                            (n > 0 || k > 0) ? 1u : 0u);
         umma_commit_elect(el, bar_qe + 8 * cur);
-        if (n + 1 < iters) issue_dp(nxt);   // dP(n) was consumed (bar_ds), Q / dO of visit n + 1 were awaited above
+        if (n + 1 < iters) issue_dp(nxt);   // over dS^T(n), which dK(n), ahead in order, reads; Q / dO of visit n + 1 were awaited above
         else umma_commit_elect(el, bar_fin);            // one-shot: every product has been accumulated
         cur = nxt;
       }
       if (!ok && lane == 0) fail_role = 2;
+    }
+    if (warp == 2) {
+      // ---------------------------------------------------------------- L and D of a visit's 128 queries, up to two visits ahead:
+      // -L log2(e) and -D scale, the addends of the packed multiply-adds
+      constexpr float kLog2e = 1.4426950408889634f;
+      const float* gL = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T;
+      const float* gD = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T;
+      int qt = first_qt;
+      for (int n = 0; n < iters; ++n) {
+        float l[4], d[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int qi = qt * BQ + i * 32 + lane;
+          l[i] = qi < p.T ? -gL[qi] * kLog2e : 0.f;
+          d[i] = qi < p.T ? -gD[qi] * p.scale : 0.f;
+        }
+        if (++qt == p.n_q_tiles) { qt = first_qt; gL += p.T; gD += p.T; }
+        if (n >= 2 && !mbar_wait(bar_le + 8 * (n & 1), ((n >> 1) - 1) & 1, abort_flag)) { fail_role = 5; break; }
+        float* dst = s_ld + (n & 1) * 2 * BQ + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          dst[i * 32] = l[i];
+          dst[BQ + i * 32] = d[i];
+        }
+        mbar_arrive(bar_lf + 8 * (n & 1));
+      }
     }
   } else if (warp < kComputeWarp0) {
     regs_dec<kRegsDrain>();
@@ -238,8 +271,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
       if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }  // all leave together
       uint32_t r0[32], r1[32];
-      tmem_ld_32x32b_x32(t_row + (m & 1) * BKV, r0);
-      tmem_ld_32x32b_x32(t_row + (m & 1) * BKV + 32, r1);
+      tmem_ld_32x32b_x32(t_row + (m & 1) * BQ, r0);
+      tmem_ld_32x32b_x32(t_row + (m & 1) * BQ + 32, r1);
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(bar_dqr);
@@ -260,111 +293,99 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (leader) tma_wait_group<0>();
   } else {
     regs_inc<kRegsCompute>();
-    // ------------------------------------------------------------------ compute warps (two threads per query row)
-    const int half = (warp - kComputeWarp0) >> 2;  // 0: keys 0..63 / dV; 1: keys 64..127 / dK
+    // ------------------------------------------------------------------ compute warps (two threads per key row)
+    const int half = (warp - kComputeWarp0) >> 2;  // 0: queries 0..63 / dV; 1: queries 64..127 / dK
     const int q = warp & 3, row = q * 32 + lane, sw = row & 7;
     const bool leader = half == 0 && row == 0;
     const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
-    uint8_t* my_p = smem + kOffP + half * kTile16 + row * 128;
     uint8_t* my_ds = smem + kOffdS + half * kTile16 + row * 128;
-    const int key0 = kt * BKV + half * 64;
+    const int key = kt * BKV + row;
+    // A thread works on 32 of its 64 queries and then on the others, in steps of 16. Each 32 leave their P^T (and dS^T) in 16 columns that
+    // this thread has read already: for the upper half that takes its last 32 queries first.
+    const int first = half * 32;
+    auto query = [&](int c) { return (c < 2 ? first : 32 - first) + (c & 1) * 16; };  // first query of step c
     bool ok = true;
     NNB_PROF_DECL;
-    constexpr float kLog2e = 1.4426950408889634f;
-    // L and D of this thread's query row, fetched one visit ahead: their latency hides behind a whole visit
-    float L_next = 0.f, D_next = 0.f;
-    int qt = first_qt, qt_next = first_qt;
-    const float* stat_L = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T + row;
-    const float* stat_D = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T + row;
-    auto fetch_ld = [&]() {  // of the visit at qt_next, and steps to the one after it
-      const bool live = qt_next * BQ + row < p.T;
-      L_next = live ? __ldg(stat_L + qt_next * BQ) : 0.f;
-      D_next = live ? __ldg(stat_D + qt_next * BQ) : 0.f;
-      if (++qt_next == p.n_q_tiles) {
-        qt_next = first_qt;
-        stat_L += p.T;
-        stat_D += p.T;
-      }
-    };
-    fetch_ld();
+    int qt = first_qt;
     const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
     for (int n = 0; n < iters && ok; ++n) {
       NNB_PROF_T0;
-      const int qi = qt * BQ + row;
-      const bool row_ok = qi < p.T;
-      const float L = L_next * kLog2e, Ds = D_next * p.scale;
-      const uint64_t nL2 = pack_f32x2(-L, -L), nDs2 = pack_f32x2(-Ds, -Ds);
-      if (n + 1 < iters) fetch_ld();
-      // Only tiles on the diagonal, past the end of the sequence, or with padded query rows need the
+      const int q0 = qt * BQ + half * 64;
+      if (++qt == p.n_q_tiles) qt = first_qt;
+      // Only tiles on the diagonal, past the end of the sequence, or with padded key rows need the
       // per-element mask; every other tile takes the branch-free version.
-      const bool need_mask = key0 + 63 > qt * BQ || key0 + 63 >= p.T || qt * BQ + BQ > p.T;
-      const uint32_t t_s = t_lane + kColS + (n & 1) * BKV + half * 64;
-      float prob[64];  // P of this thread's 64 keys, kept in fp32 from phase A to phase B
-      // ---- phase A: P = exp2(S scale log2e - L log2e)
+      const bool need_mask = q0 < kt * BKV + BKV - 1 || q0 + 64 > p.T || kt * BKV + BKV > p.T;
+      const uint32_t t_buf = t_lane + kColS + (n & 1) * BQ, t_s = t_buf + half * 64, t_dp = t_lane + kColdP + half * 64;
+      const float* sL = s_ld + (n & 1) * 2 * BQ + half * 64;
+      float prob[64];  // P^T of this thread's 64 queries, kept in fp32 from phase A to phase B
+      // ---- phase A: P^T = exp2(S^T scale log2e - L log2e)
+      if (!mbar_wait(bar_lf + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
       if (!mbar_wait(bar_s + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
-      if (n > 0 && !mbar_wait(bar_pf, (n - 1) & 1, abort_flag)) { ok = false; break; }  // dV(n - 1) has read P
       tc_fence_after();
       NNB_PROF_ADD(0);
       auto phase_a = [&](auto masked) {
         constexpr bool kMask = decltype(masked)::value;
-        uint32_t rs[2][16];  // 16 columns at a time, the next load in flight while these are worked on
-        tmem_ld_32x32b_x16(t_s, rs[0]);
+        uint32_t rs[2][16], pk[16];  // 16 columns at a time, the next load in flight while these are worked on
+        tmem_ld_32x32b_x16(t_s + query(0), rs[0]);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          const ulonglong2* l4 = reinterpret_cast<const ulonglong2*>(sL + query(c));
+          const ulonglong2 l[4] = {l4[0], l4[1], l4[2], l4[3]};  // (arrive while the scores are waited for)
           tmem_ld_wait(rs[c & 1]);
-          if (c < 3) tmem_ld_32x32b_x16(t_s + (c + 1) * 16, rs[(c + 1) & 1]);
-          uint32_t pk[8];
+          if (c < 3) tmem_ld_32x32b_x16(t_s + query(c + 1), rs[(c + 1) & 1]);
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
             const uint64_t s2 = pack_f32x2(__uint_as_float(rs[c & 1][i]), __uint_as_float(rs[c & 1][i + 1]));
-            const float2 e = unpack_f32x2(fma_f32x2(s2, scale_log2_2, nL2));
+            const float2 e = unpack_f32x2(fma_f32x2(s2, scale_log2_2, (i & 2) ? l[i / 4].y : l[i / 4].x));
             float p0 = exp2f(e.x), p1 = exp2f(e.y);
             if (kMask) {
-              const int key = key0 + c * 16 + i;
-              p0 = (row_ok && key <= qi && key < p.T) ? p0 : 0.f;
-              p1 = (row_ok && key + 1 <= qi && key + 1 < p.T) ? p1 : 0.f;
+              const int qi = q0 + query(c) + i;
+              p0 = (key <= qi && qi < p.T && key < p.T) ? p0 : 0.f;
+              p1 = (key <= qi + 1 && qi + 1 < p.T && key < p.T) ? p1 : 0.f;
             }
             prob[c * 16 + i] = p0;
             prob[c * 16 + i + 1] = p1;
-            pk[i >> 1] = pack2_16<F16>(p0, p1);
+            pk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(p0, p1);
           }
-#pragma unroll
-          for (int jj = 0; jj < 2; ++jj)
-            *reinterpret_cast<uint4*>(my_p + (((c * 2 + jj) ^ sw) << 4)) = make_uint4(pk[4 * jj], pk[4 * jj + 1], pk[4 * jj + 2], pk[4 * jj + 3]);
+          if (c & 1) tmem_st_32x32b_x16(t_buf + half * 96 + query(c - 1) / 2, pk);
         }
       };
       if (need_mask) phase_a(std::true_type{});
       else phase_a(std::false_type{});
-      fence_proxy_async_smem();
+      tmem_st_wait();
       tc_fence_before();
       mbar_arrive(bar_p);
       NNB_PROF_ADD(1);
-      // ---- phase B: dS = P (dP scale - D scale)
-      // (dP(n) was issued after dK(n - 1) and dQ(n - 1): once it is complete they have read dS)
+      // ---- phase B: dS^T = P^T (dP^T scale - D scale)
+      // (dP^T(n) was issued after dK(n - 1) and dQ(n - 1): once it is complete they have read dS^T)
       if (!mbar_wait(bar_dp, n & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       NNB_PROF_ADD(2);
-      uint32_t rp[2][16];
-      tmem_ld_32x32b_x16(t_lane + kColdP + half * 64, rp[0]);
+      uint32_t rp[2][16], dk[16];
+      tmem_ld_32x32b_x16(t_dp + query(0), rp[0]);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
+        const ulonglong2* d4 = reinterpret_cast<const ulonglong2*>(sL + BQ + query(c));
+        const ulonglong2 d[4] = {d4[0], d4[1], d4[2], d4[3]};
         tmem_ld_wait(rp[c & 1]);
-        if (c < 3) tmem_ld_32x32b_x16(t_lane + kColdP + half * 64 + (c + 1) * 16, rp[(c + 1) & 1]);
-        uint32_t dk[8];
+        if (c < 3) tmem_ld_32x32b_x16(t_dp + query(c + 1), rp[(c + 1) & 1]);
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
-          const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c & 1][i]), __uint_as_float(rp[c & 1][i + 1])), scale2, nDs2);
-          const float2 d = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i], prob[c * 16 + i + 1]), t));
-          dk[i >> 1] = pack2_16<F16>(d.x, d.y);
+          const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c & 1][i]), __uint_as_float(rp[c & 1][i + 1])), scale2, (i & 2) ? d[i / 4].y : d[i / 4].x);
+          const float2 g = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i], prob[c * 16 + i + 1]), t));
+          dk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(g.x, g.y);
         }
 #pragma unroll
         for (int jj = 0; jj < 2; ++jj)
-          *reinterpret_cast<uint4*>(my_ds + (((c * 2 + jj) ^ sw) << 4)) = make_uint4(dk[4 * jj], dk[4 * jj + 1], dk[4 * jj + 2], dk[4 * jj + 3]);
+          *reinterpret_cast<uint4*>(my_ds + (((query(c) / 8 + jj) ^ sw) << 4)) =
+              make_uint4(dk[(c & 1) * 8 + 4 * jj], dk[(c & 1) * 8 + 4 * jj + 1], dk[(c & 1) * 8 + 4 * jj + 2], dk[(c & 1) * 8 + 4 * jj + 3]);
+        if (c & 1) tmem_st_32x32b_x16(t_lane + kColdP + half * 96 + query(c - 1) / 2, dk);
       }
+      mbar_arrive(bar_le + 8 * (n & 1));
       fence_proxy_async_smem();
+      tmem_st_wait();
       tc_fence_before();
       mbar_arrive(bar_ds);
-      if (++qt == p.n_q_tiles) qt = first_qt;
       NNB_PROF_ADD(3);
     }
     if (ok && iters > 0 && !mbar_wait(bar_fin, 0, abort_flag)) ok = false;
@@ -374,9 +395,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       fail_role = 3;
     }
     NNB_PROF_FLUSH_N(iters);
-    // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the P / dS tiles) -> TMA store
+    // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the dS^T tiles) -> TMA store
     if (ok && iters > 0) {
-      uint8_t* dst = (half == 0 ? smem + kOffP : smem + kOffdS) + row * 128;
+      uint8_t* dst = my_ds;
       uint32_t r0[32], r1[32];
       tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
       tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
@@ -410,8 +431,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       fence_proxy_async_smem();
       named_barrier_sync(2, kComputeThreads);
       if (leader) {
-        tma_store_4d(&tmdV, s_base + kOffP, 0, kvh, kt * BKV, b);
-        tma_store_4d(&tmdK, s_base + kOffdS, 0, kvh, kt * BKV, b);
+        tma_store_4d(&tmdV, s_base + kOffdS, 0, kvh, kt * BKV, b);
+        tma_store_4d(&tmdK, s_base + kOffdS + kTile16, 0, kvh, kt * BKV, b);
         tma_commit_group();
       }
     }
@@ -546,8 +567,8 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   const bool f16 = dtype == NNB_F16;
   NNB_REQUIRE(H % KVH == 0 && B > 0 && T > 0, "flash_bwd: bad shape");
   // head_dim 128 runs on the transposed-tile kernel (flash_bwd_t.cu). It also serves head_dim 64
-  // (NANONEMO_FLASH_BWD=transposed), but there the 128 x 128 formulation of this file measured faster (299 vs 361 us at
-  // B32 H12/4 T1024; 696 vs 1058 us at B8 T4096): with 64-wide tiles every product has N = 64 and is bound by shared-memory operand reads.
+  // (NANONEMO_FLASH_BWD=transposed), but there the 128 x 128 tiles of this file measured faster (283 vs 361 us at
+  // B32 H12/4 T1024; 702 vs 1058 us at B8 T4096): with 64-wide tiles every product has N = 64 and is bound by shared-memory operand reads.
   static const bool square = [] { const char* e = getenv("NANONEMO_FLASH_BWD"); return !(e && e[0] == 't'); }();
   NNB_REQUIRE((rope_cos == nullptr) == (rope_sin == nullptr), "flash_bwd: give both RoPE tables or neither");
   NNB_REQUIRE(rope_cos == nullptr || (hd == HD && square && nnb_aligned16(rope_cos) && nnb_aligned16(rope_sin)),
@@ -589,9 +610,9 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.lse = static_cast<const float*>(lse);
   p.delta = static_cast<const float*>(delta);
   const int fmt = f16 ? 0 : 1;
-  p.idesc_s = sm100::make_idesc_f16(fmt, 0, 0, BQ, BKV);
-  p.idesc_dkv = sm100::make_idesc_f16(fmt, 1, 1, BKV, HD);
-  p.idesc_dq = sm100::make_idesc_f16(fmt, 0, 1, BQ, HD);
+  p.idesc_s = sm100::make_idesc_f16(fmt, 0, 0, BKV, BQ);
+  p.idesc_dkv = sm100::make_idesc_f16(fmt, 0, 1, BKV, HD);
+  p.idesc_dq = sm100::make_idesc_f16(fmt, 1, 1, BQ, HD);
   p.status = static_cast<int*>(status);
   p.rope_cos = static_cast<const float*>(rope_cos);
   p.rope_sin = static_cast<const float*>(rope_sin);
