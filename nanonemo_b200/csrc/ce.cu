@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(kCeThreads) ce_grad_from_stats_kernel(T* __res
                                                                         const float* __restrict__ tile_stats, int n_tiles,
                                                                         float* __restrict__ loss_rows, int V, long long ld,
                                                                         float grad_scale) {
+  nnb_after_previous(logits, targets, tile_stats, loss_rows);
+  nnb_release_next();
   constexpr float kLog2e = 1.4426950408889634f;
   __shared__ float s_m[kCeThreads / 32], s_s[kCeThreads / 32];
   const long long row = blockIdx.x;
@@ -175,6 +177,8 @@ __global__ void __launch_bounds__(kCeThreads) ce_loss_from_stats_kernel(const fl
                                                                         const float* __restrict__ target_logit,
                                                                         const long long* __restrict__ targets,
                                                                         float* __restrict__ loss_rows, long long R, int V) {
+  nnb_after_previous(tile_stats, target_logit, targets, loss_rows);
+  nnb_release_next();
   constexpr float kLog2e = 1.4426950408889634f;
   const long long row = (long long)blockIdx.x * (kCeThreads / 32) + (threadIdx.x >> 5);
   if (row >= R) return;
@@ -276,7 +280,7 @@ extern "C" int nnb_ce_grad_from_stats(void* logits, const void* targets, const v
   NNB_REQUIRE(ld % 8 == 0 && nnb_aligned16(logits) && nnb_aligned16(tile_stats), "ce_from_stats: rows must be 16-byte aligned");
   if (R == 0) return 0;
   NNB_DISPATCH_16(dtype, T, {
-    ce_grad_from_stats_kernel<T><<<(unsigned)R, kCeThreads, 0, st>>>((T*)logits, (const long long*)targets, (const float*)tile_stats,
+    nnb_launch(ce_grad_from_stats_kernel<T>, (unsigned)R, kCeThreads, 0, st, (T*)logits, (const long long*)targets, (const float*)tile_stats,
                                                                      n_tiles, (float*)loss_rows, V, ld, grad_scale);
   });
   NNB_LAUNCH_OK("ce_grad_from_stats");
@@ -289,8 +293,7 @@ extern "C" int nnb_ce_loss_from_stats(const void* tile_stats, int n_tiles, const
   NNB_REQUIRE(n_tiles > 0 && V > 0 && (reinterpret_cast<uintptr_t>(tile_stats) & 7) == 0, "ce_loss_from_stats: bad statistics");
   if (R == 0) return 0;
   constexpr int rows = kCeThreads / 32;
-  ce_loss_from_stats_kernel<<<(unsigned)((R + rows - 1) / rows), kCeThreads, 0, st>>>(
-      (const float*)tile_stats, n_tiles, (const float*)target_logit, (const long long*)targets, (float*)loss_rows, R, V);
+  nnb_launch(ce_loss_from_stats_kernel, (unsigned)((R + rows - 1) / rows), kCeThreads, 0, st, (const float*)tile_stats, n_tiles, (const float*)target_logit, (const long long*)targets, (float*)loss_rows, R, V);
   NNB_LAUNCH_OK("ce_loss_from_stats");
   return 0;
 }

@@ -40,9 +40,48 @@ static inline int nnb_num_sms() {
   return sms;
 }
 
+// Launch that may begin while the previous kernel of the stream is still running its last blocks: blocks are placed as SMs fall free, set
+// themselves up (barriers, tensor memory, descriptors) and stop in nnb_after_previous(), which EVERY kernel launched this way calls
+// before it touches global memory. What it returns to is what stream order gives: the previous kernel, and with it everything before
+// it, has finished and its writes are visible. A kernel lets its successor in with nnb_release_next() when its own work is nearly
+// handed out, not earlier: blocks that wait hold their SM's resources, which kernels of other streams may want.
+// An eager step of the 114M model in two micro-batches of 4096 tokens is 574 launches with 1.7 us of idle GPU before each: 12.0 ms
+// in plain launches, 11.1 in these (8192 tokens in fp8: 11.6 and 11.1).
+// `cluster`: CTAs of a cluster along x, 1 for a kernel without clusters (or with its own __cluster_dims__).
+template <typename... K, typename... A>
+static inline void nnb_launch_clusters(void (*kernel)(K...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);  // (its error is read by NNB_LAUNCH_OK)
+}
+template <typename... K, typename... A>
+static inline void nnb_launch(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  nnb_launch_clusters(kernel, 1, grid, block, smem, st, args...);
+}
+
 static inline bool nnb_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 #ifdef __CUDACC__
+// See nnb_launch_clusters. The pointers through which the kernel reads are named here: their values then come out of the statement after
+// the wait, so that no load (read-only loads obey no memory clobber) can be moved above it.
+template <typename... P>
+__device__ __forceinline__ void nnb_after_previous(P&... pointers) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ((void)[&] { asm volatile("" : "+l"(pointers)); }(), ...);
+}
+__device__ __forceinline__ void nnb_release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- 8-element (one "chunk") loads/stores converting to/from fp32 registers
 template <typename T>
 struct Chunk8;

@@ -28,6 +28,8 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restri
                                                               const float* __restrict__ w, TY* __restrict__ y,
                                                               TX* __restrict__ h, float* __restrict__ rstd, int M,
                                                               int N, float eps) {
+  nnb_after_previous(x, delta, w, y, h, rstd);
+  nnb_release_next();
   __shared__ float s_part[8 / WPR][2][2];
   constexpr int kLanes = 32 * WPR;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes, lane = threadIdx.x % kLanes;
@@ -90,8 +92,9 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
   const int nchunks = N >> 3;
   float* s_w = s_mem;
   float* s_acc = s_mem + N + (size_t)warp_in_block * N;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) s_w[i] = w[i];
   for (int i = threadIdx.x; i < N * warps_per_block; i += blockDim.x) s_mem[N + i] = 0.f;
+  nnb_after_previous(dy, h, rstd, w, dres, dx, ddelta, dw_partial);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) s_w[i] = w[i];
   __syncthreads();
   const float inv_n = 1.f / (float)N;
   for (int row = blockIdx.x * warps_per_block + warp_in_block; row < M; row += gridDim.x * warps_per_block) {
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
       }
     }
   }
+  nnb_release_next();
   __syncthreads();
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     float s = 0.f;
@@ -151,6 +155,8 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
 // (fixed order within a thread, then a fixed-order combine: the result does not depend on scheduling).
 __global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int rows,
                                                         int N, int accumulate) {
+  nnb_after_previous(partial, dw);
+  nnb_release_next();
   __shared__ float s_red[8][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx;
@@ -180,7 +186,7 @@ template <typename TX, typename TD, typename TY>
 static void rmsnorm_fwd_t(const void* x, const void* delta, const float* w, void* y, void* h, float* rstd, int M, int N,
                           float eps, cudaStream_t st) {
 #define NNB_RMS_FWD(MAXC, WPR) \
-  add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC, WPR><<<(M * WPR + 7) / 8, 256, 0, st>>>((const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
+  nnb_launch(add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC, WPR>, (M * WPR + 7) / 8, 256, 0, st, (const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
   if (N <= 1024) NNB_RMS_FWD(4, 1);
   else NNB_RMS_FWD(4, 2);
 #undef NNB_RMS_FWD
@@ -218,7 +224,7 @@ static int rmsnorm_bwd_t(const void* dy, const void* h, const float* rstd, const
     const size_t smem = (size_t)N * (1 + 4 / WPR) * sizeof(float); /* the weight, and an accumulator per row in flight */ \
     auto k = add_rmsnorm_bwd_kernel<TX, TD, TY, MAXC, WPR>;                                                       \
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -3; \
-    k<<<blocks, 128, smem, st>>>((const TY*)dy, (const TX*)h, rstd, w, (const TX*)dres, (TX*)dx, (TD*)ddelta, partial, M, N); \
+    nnb_launch(k, blocks, 128, smem, st, (const TY*)dy, (const TX*)h, rstd, w, (const TX*)dres, (TX*)dx, (TD*)ddelta, partial, M, N); \
   }
   if (N <= 768) NNB_RMS_BWD(3, 1)   // one row fits 3 chunks per lane: fewer registers, more resident warps
   else if (N <= 1024) NNB_RMS_BWD(4, 1)
@@ -247,7 +253,7 @@ extern "C" int nnb_add_rmsnorm_bwd(const void* dy, const void* h, const void* rs
   NNB_REQUIRE(done, "add_rmsnorm_bwd: unsupported dtype combination (x=%d, delta=%d, y=%d)", x_dtype, delta_dtype, y_dtype);
   NNB_REQUIRE(rc == 0, "add_rmsnorm_bwd: cannot raise the shared-memory limit");
   NNB_LAUNCH_OK("add_rmsnorm_bwd");
-  dw_reduce_kernel<<<(N + 31) / 32, 256, 0, st>>>((const float*)dw_partial, (float*)dw, blocks, N, accumulate_dw);
+  nnb_launch(dw_reduce_kernel, (N + 31) / 32, 256, 0, st, (const float*)dw_partial, (float*)dw, blocks, N, accumulate_dw);
   NNB_LAUNCH_OK("rmsnorm_dw_reduce");
   return 0;
 }
@@ -260,6 +266,8 @@ extern "C" int nnb_add_rmsnorm_bwd(const void* dy, const void* h, const void* rs
 template <typename T, bool ACC>
 __global__ void __launch_bounds__(256) scale_kernel(const T* __restrict__ src, const float* __restrict__ scalar, T* __restrict__ dst,
                                                     long long n) {
+  nnb_after_previous(src, scalar, dst);
+  nnb_release_next();
   const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   const float s = scalar[0];
@@ -285,8 +293,8 @@ extern "C" int nnb_scale(const void* src, const void* scalar, void* dst, long lo
   if (n == 0) return 0;
   const unsigned blocks = (unsigned)((n + 2047) / 2048);
 #define NNB_SCALE(T)                                                                                              \
-  if (accumulate) scale_kernel<T, true><<<blocks, 256, 0, st>>>((const T*)src, (const float*)scalar, (T*)dst, n); \
-  else scale_kernel<T, false><<<blocks, 256, 0, st>>>((const T*)src, (const float*)scalar, (T*)dst, n)
+  if (accumulate) nnb_launch(scale_kernel<T, true>, blocks, 256, 0, st, (const T*)src, (const float*)scalar, (T*)dst, n); \
+  else nnb_launch(scale_kernel<T, false>, blocks, 256, 0, st, (const T*)src, (const float*)scalar, (T*)dst, n)
   if (dtype == NNB_F32) { NNB_SCALE(float); }
   else if (dtype == NNB_BF16) { NNB_SCALE(__nv_bfloat16); }
   else { NNB_SCALE(__half); }
@@ -302,6 +310,8 @@ template <typename T>
 __global__ void rope_packed_kernel(const T* __restrict__ in, T* __restrict__ out, const float* __restrict__ cos_t,
                                    const float* __restrict__ sin_t, long long M, int T_len, int n_rot_heads, int hd,
                                    int n_copy_cols, long long in_stride, long long out_stride, float sin_sign) {
+  nnb_after_previous(in, out, cos_t, sin_t);
+  nnb_release_next();
   const int half = hd >> 1, vec_per_half = half >> 3;
   const int rot_items = n_rot_heads * vec_per_half, copy_items = n_copy_cols >> 3;
   const int items = rot_items + copy_items;
@@ -347,7 +357,7 @@ extern "C" int nnb_rope_packed(const void* in, void* out, const void* cos_t, con
   const long long items = M * ((long long)n_rot_heads * (hd / 16) + n_copy_cols / 8);
   const int blocks = (int)min((items + 255) / 256, (long long)nnb_num_sms() * 16);
   NNB_DISPATCH(dtype, T, {
-    rope_packed_kernel<T><<<blocks, 256, 0, st>>>((const T*)in, (T*)out, (const float*)cos_t, (const float*)sin_t, M,
+    nnb_launch(rope_packed_kernel<T>, blocks, 256, 0, st, (const T*)in, (T*)out, (const float*)cos_t, (const float*)sin_t, M,
                                                   T_len, n_rot_heads, hd, n_copy_cols, in_stride, out_stride, sin_sign);
   });
   NNB_LAUNCH_OK("rope_packed");
@@ -359,6 +369,8 @@ extern "C" int nnb_rope_packed(const void* in, void* out, const void* cos_t, con
 template <typename T>
 __global__ void swiglu_fwd_kernel(const T* __restrict__ g, const T* __restrict__ u, T* __restrict__ out, long long M,
                                   int F, long long g_stride, long long u_stride, long long o_stride) {
+  nnb_after_previous(g, u, out);
+  nnb_release_next();
   const int vec = F >> 3;
   const long long total = M * vec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -379,6 +391,8 @@ template <typename T>
 __global__ void swiglu_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ g, const T* __restrict__ u,
                                   T* __restrict__ dg, T* __restrict__ du, long long M, int F, long long dy_stride,
                                   long long g_stride, long long u_stride, long long dg_stride, long long du_stride) {
+  nnb_after_previous(dy, g, u, dg, du);
+  nnb_release_next();
   const int vec = F >> 3;
   const long long total = M * vec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -407,7 +421,7 @@ extern "C" int nnb_swiglu_fwd(const void* g, const void* u, void* out, long long
   if (M == 0) return 0;
   const int blocks = (int)min((M * (F / 8) + 255) / 256, (long long)nnb_num_sms() * 16);
   NNB_DISPATCH(dtype, T, {
-    swiglu_fwd_kernel<T><<<blocks, 256, 0, st>>>((const T*)g, (const T*)u, (T*)out, M, F, g_stride, u_stride, o_stride);
+    nnb_launch(swiglu_fwd_kernel<T>, blocks, 256, 0, st, (const T*)g, (const T*)u, (T*)out, M, F, g_stride, u_stride, o_stride);
   });
   NNB_LAUNCH_OK("swiglu_fwd");
   return 0;
@@ -421,7 +435,7 @@ extern "C" int nnb_swiglu_bwd(const void* dy, const void* g, const void* u, void
   if (M == 0) return 0;
   const int blocks = (int)min((M * (F / 8) + 255) / 256, (long long)nnb_num_sms() * 16);
   NNB_DISPATCH(dtype, T, {
-    swiglu_bwd_kernel<T><<<blocks, 256, 0, st>>>((const T*)dy, (const T*)g, (const T*)u, (T*)dg, (T*)du, M, F, dy_stride,
+    nnb_launch(swiglu_bwd_kernel<T>, blocks, 256, 0, st, (const T*)dy, (const T*)g, (const T*)u, (T*)dg, (T*)du, M, F, dy_stride,
                                                  g_stride, u_stride, dg_stride, du_stride);
   });
   NNB_LAUNCH_OK("swiglu_bwd");
@@ -433,6 +447,8 @@ extern "C" int nnb_swiglu_bwd(const void* dy, const void* g, const void* u, void
 template <typename TO>
 __global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const float* __restrict__ W,
                                      TO* __restrict__ out, long long M, int D, int vocab) {
+  nnb_after_previous(idx, W, out);
+  nnb_release_next();
   const int vec = D >> 3;
   const long long total = M * vec;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -452,6 +468,8 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ idx, const fl
 template <typename TO>
 __global__ void embedding_bwd_kernel(const long long* __restrict__ idx, const TO* __restrict__ dout,
                                      float* __restrict__ dW, long long M, int D, int vocab) {
+  nnb_after_previous(idx, dout, dW);
+  nnb_release_next();
   const int vec = D >> 3;
   const long long total = M * vec;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -474,7 +492,7 @@ extern "C" int nnb_embedding_fwd(const void* idx, const void* W, void* out, long
   if (M == 0) return 0;
   const int blocks = (int)min((M * (D / 8) + 255) / 256, (long long)nnb_num_sms() * 16);
   NNB_DISPATCH(out_dtype, TO, {
-    embedding_fwd_kernel<TO><<<blocks, 256, 0, st>>>((const long long*)idx, (const float*)W, (TO*)out, M, D, vocab);
+    nnb_launch(embedding_fwd_kernel<TO>, blocks, 256, 0, st, (const long long*)idx, (const float*)W, (TO*)out, M, D, vocab);
   });
   NNB_LAUNCH_OK("embedding_fwd");
   return 0;
@@ -486,7 +504,7 @@ extern "C" int nnb_embedding_bwd(const void* idx, const void* dout, void* dW, lo
   if (M == 0) return 0;
   const int blocks = (int)min((M * (D / 8) + 255) / 256, (long long)nnb_num_sms() * 16);
   NNB_DISPATCH(dout_dtype, TO, {
-    embedding_bwd_kernel<TO><<<blocks, 256, 0, st>>>((const long long*)idx, (const TO*)dout, (float*)dW, M, D, vocab);
+    nnb_launch(embedding_bwd_kernel<TO>, blocks, 256, 0, st, (const long long*)idx, (const TO*)dout, (float*)dW, M, D, vocab);
   });
   NNB_LAUNCH_OK("embedding_bwd");
   return 0;

@@ -137,6 +137,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const float *g_lse = p.lse, *g_delta = p.delta, *g_cos = p.rope_cos, *g_sin = p.rope_sin;
+  nnb_after_previous(g_lse, g_delta, g_cos, g_sin);
   int fail_role = 0;
 
   if (warp < kDrainWarp0) {
@@ -155,6 +157,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tma_load_4d(dst, &tmQ, bar_qf + 8 * s, 0, hq, qt * BQ, b);
         tma_load_4d(dst + kTile16, &tmdO, bar_qf + 8 * s, 0, hq, qt * BQ, b);
       }
+      nnb_release_next();
     }
     if (warp == 1) {
       // ---------------------------------------------------------------- MMA issuer (warp-uniform: see umma_f16_elect)
@@ -234,8 +237,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ---------------------------------------------------------------- L and D of a visit's 128 queries, up to two visits ahead:
       // -L log2(e) and -D scale, the addends of the packed multiply-adds
       constexpr float kLog2e = 1.4426950408889634f;
-      const float* gL = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T;
-      const float* gD = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T;
+      const float* gL = g_lse + ((size_t)b * p.H + kvh * p.group) * p.T;
+      const float* gD = g_delta + ((size_t)b * p.H + kvh * p.group) * p.T;
       int qt = first_qt;
       for (int n = 0; n < iters; ++n) {
         float l[4], d[4];
@@ -404,8 +407,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_ld_wait();
       if (half == 1 && p.rope_cos != nullptr && kt * BKV + row < p.T) {
         // dK of key position t leaves through the transpose of the forward rotation: lo' = lo c + hi s, hi' = hi c - lo s
-        const float* cr = p.rope_cos + (size_t)(kt * BKV + row) * (HD / 2);
-        const float* sr = p.rope_sin + (size_t)(kt * BKV + row) * (HD / 2);
+        const float* cr = g_cos + (size_t)(kt * BKV + row) * (HD / 2);
+        const float* sr = g_sin + (size_t)(kt * BKV + row) * (HD / 2);
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
           const float4 c4 = __ldg(reinterpret_cast<const float4*>(cr + i)), s4 = __ldg(reinterpret_cast<const float4*>(sr + i));
@@ -460,6 +463,8 @@ template <typename T16>
 __global__ void flash_delta_kernel(const T16* __restrict__ o, const T16* __restrict__ d_o,
                                    float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int H, long long o_sb, long long o_st,
                                    long long o_sh, long long do_sb, long long do_st, long long do_sh) {
+  nnb_after_previous(o, d_o, delta, dq_acc);
+  nnb_release_next();
   const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long w = gid >> 3;
   const int sub = threadIdx.x & 7;
@@ -492,6 +497,8 @@ template <typename T16>
 __global__ void flash_dq_convert_kernel(const float* __restrict__ acc, T16* __restrict__ dq, long long rows, int H,
                                         int T, long long sb, long long st, long long sh, const float* __restrict__ rope_cos,
                                         const float* __restrict__ rope_sin) {
+  nnb_after_previous(acc, dq, rope_cos, rope_sin);
+  nnb_release_next();
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // one thread per 8 + 8 elements
   const long long total = rows * (HD / 16);
   if (idx >= total) return;
@@ -594,10 +601,10 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   const long long rows = (long long)B * T * H;
   const unsigned delta_blocks = (unsigned)((rows * 8 + 255) / 256);
   if (f16)
-    flash_delta_kernel<__half><<<delta_blocks, 256, 0, st>>>((const __half*)o, (const __half*)d_o, (float*)delta, (float*)dq_acc, B, T, H, o_sb,
+    nnb_launch(flash_delta_kernel<__half>, delta_blocks, 256, 0, st, (const __half*)o, (const __half*)d_o, (float*)delta, (float*)dq_acc, B, T, H, o_sb,
                                                             o_st, o_sh, do_sb, do_st, do_sh);
   else
-    flash_delta_kernel<__nv_bfloat16><<<delta_blocks, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, (float*)delta,
+    nnb_launch(flash_delta_kernel<__nv_bfloat16>, delta_blocks, 256, 0, st, (const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, (float*)delta,
                                                                    (float*)dq_acc, B, T, H, o_sb, o_st, o_sh, do_sb, do_st, do_sh);
   NNB_LAUNCH_OK("flash_delta");
 
@@ -623,15 +630,15 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
     configured = true;
   }
   dim3 grid(KVH, B, (T + BKV - 1) / BKV);
-  if (f16) flash_bwd_kernel<true><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
-  else flash_bwd_kernel<false><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  if (f16) nnb_launch(flash_bwd_kernel<true>, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  else nnb_launch(flash_bwd_kernel<false>, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd");
   const unsigned conv_blocks = (unsigned)((rows * (HD / 16) + 255) / 256);
   if (f16)
-    flash_dq_convert_kernel<__half><<<conv_blocks, 256, 0, st>>>((const float*)dq_acc, (__half*)dq, rows, H, T, dq_sb, dq_st, dq_sh, p.rope_cos,
+    nnb_launch(flash_dq_convert_kernel<__half>, conv_blocks, 256, 0, st, (const float*)dq_acc, (__half*)dq, rows, H, T, dq_sb, dq_st, dq_sh, p.rope_cos,
                                                                 p.rope_sin);
   else
-    flash_dq_convert_kernel<__nv_bfloat16><<<conv_blocks, 256, 0, st>>>((const float*)dq_acc, (__nv_bfloat16*)dq, rows, H, T, dq_sb, dq_st, dq_sh,
+    nnb_launch(flash_dq_convert_kernel<__nv_bfloat16>, conv_blocks, 256, 0, st, (const float*)dq_acc, (__nv_bfloat16*)dq, rows, H, T, dq_sb, dq_st, dq_sh,
                                                                        p.rope_cos, p.rope_sin);
   NNB_LAUNCH_OK("flash_dq_convert");
   return 0;

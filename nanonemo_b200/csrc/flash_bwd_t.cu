@@ -120,6 +120,8 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const float *g_lse = p.lse, *g_delta = p.delta;
+  nnb_after_previous(g_lse, g_delta);
   int fail_role = 0;
 
   if (warp == 0) {
@@ -143,6 +145,7 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           tma_load_4d(dst + (NH + g) * kHalfQ, &tmdO, bar_qf + 8 * s, g * 64, hq, qb * BQ, b);
         }
       }
+      nnb_release_next();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (every lane runs the loop, one lane's instructions count)
@@ -220,8 +223,8 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // ------------------------------------------------------------------ L and D of a visit's 64 queries, up to two visits ahead:
     // -L log2(e) and -D scale, the addends of the packed multiply-adds
     constexpr float kLog2e = 1.4426950408889634f;
-    const float* gL = p.lse + ((size_t)b * p.H + kvh * p.group) * p.T;
-    const float* gD = p.delta + ((size_t)b * p.H + kvh * p.group) * p.T;
+    const float* gL = g_lse + ((size_t)b * p.H + kvh * p.group) * p.T;
+    const float* gD = g_delta + ((size_t)b * p.H + kvh * p.group) * p.T;
     int qb = first_qb;
     for (int n = 0; n < iters; ++n) {
       float v[4];
@@ -436,6 +439,8 @@ template <int HD, typename T16>
 __global__ void flash_delta_t_kernel(const T16* __restrict__ o, const T16* __restrict__ d_o,
                                      float* __restrict__ delta, float* __restrict__ dq_acc, int B, int T, int H, long long o_sb, long long o_st,
                                      long long o_sh, long long do_sb, long long do_st, long long do_sh) {
+  nnb_after_previous(o, d_o, delta, dq_acc);
+  nnb_release_next();
   constexpr int L = HD / 8;
   const long long gid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long w = gid / L;
@@ -466,6 +471,8 @@ __global__ void flash_delta_t_kernel(const T16* __restrict__ o, const T16* __res
 template <int HD, typename T16>
 __global__ void flash_dq_convert_t_kernel(const float* __restrict__ acc, T16* __restrict__ dq, long long rows, int H,
                                           int T, long long sb, long long st, long long sh) {
+  nnb_after_previous(acc, dq);
+  nnb_release_next();
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // one thread per 8 elements
   const long long total = rows * (HD / 8);
   if (idx >= total) return;
@@ -499,8 +506,7 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
   if (!nnb_make_tmap_4d(&tdv, dt, 2, dv, HD, KVH, T, B, dvs[2] * 2, dvs[1] * 2, dvs[0] * 2, 64, 1, BKV, "flash_bwd dV")) return -4;
 
   const long long rows = (long long)B * T * H;
-  flash_delta_t_kernel<HD, T16><<<(unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st>>>(
-      (const T16*)o, (const T16*)d_o, (float*)delta, (float*)dq_acc, B, T, H, os[0], os[1], os[2], dos[0], dos[1], dos[2]);
+  nnb_launch(flash_delta_t_kernel<HD, T16>, (unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st, (const T16*)o, (const T16*)d_o, (float*)delta, (float*)dq_acc, B, T, H, os[0], os[1], os[2], dos[0], dos[1], dos[2]);
   NNB_LAUNCH_OK("flash_delta");
   BParams p{};
   p.B = B; p.H = H; p.KVH = KVH; p.T = T;
@@ -524,9 +530,9 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
     configured = true;
   }
   dim3 grid(KVH, B, (T + BKV - 1) / BKV);
-  flash_bwd_t_kernel<HD, F16><<<grid, kThreads, C::kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  nnb_launch(flash_bwd_t_kernel<HD, F16>, grid, kThreads, C::kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd_t");
-  flash_dq_convert_t_kernel<HD, T16><<<(unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st>>>((const float*)dq_acc, (T16*)dq, rows, H, T,
+  nnb_launch(flash_dq_convert_t_kernel<HD, T16>, (unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st, (const float*)dq_acc, (T16*)dq, rows, H, T,
                                                                                                 dqs[0], dqs[1], dqs[2]);
   NNB_LAUNCH_OK("flash_dq_convert");
   return 0;

@@ -123,6 +123,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  nnb_after_previous();  // (all its reads of global memory are TMA loads)
   int fail_role = 0;
 
   if (warp == 0) {
@@ -143,6 +144,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) tma_load_4d(sv + c * (BN * 128), &tmV, bar_v + 8 * s, c * 64, kvh, j * BN, b);
       }
+      nnb_release_next();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (warp-uniform: see umma_f16_elect)
@@ -217,7 +219,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     configured = true;
   }
   dim3 grid(p.H, p.B, p.n_q_tiles);
-  kern<<<grid, kThreads, FCfg<HD>::kSmem, st>>>(tq, tk, tv, to, p);
+  nnb_launch(kern, grid, kThreads, FCfg<HD>::kSmem, st, tq, tk, tv, to, p);
   return 0;
 }
 

@@ -144,6 +144,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  nnb_after_previous();  // (its pointers are read through TMA, or across ranks with acquire loads)
 
   const int items = p.m_blocks * p.n_blocks * p.k_splits;
   int fail_role = 0, fail_item = -1;
@@ -381,6 +382,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
         }
       }
+      if (p.mode == 0) nnb_release_next();  // the last operands are on their way
       if (!ok) {
         // give the copies already in flight a bounded chance to land before the CTA exits
         const uint32_t first = it > (uint32_t)C::kStages ? it - C::kStages : 0;
@@ -618,7 +620,9 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const DMaps& tmDs, co
     }
     configured = true;
   }
-  kern<<<grid, kThreads, Cfg<BN, MX>::kSmemBytes, st>>>(tmA, tmB, tmDs, p);
+  // (the fused collectives meet other ranks: they start and end in stream order, as ever)
+  if (p.mode == 0) nnb_launch(kern, grid, kThreads, Cfg<BN, MX>::kSmemBytes, st, tmA, tmB, tmDs, p);
+  else kern<<<grid, kThreads, Cfg<BN, MX>::kSmemBytes, st>>>(tmA, tmB, tmDs, p);
   return 0;
 }
 

@@ -246,6 +246,9 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   cluster_sync_all();  // both CTAs' barriers exist before anybody signals the peer
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const float *cos_t = p.cos_t, *sin_t = p.sin_t;
+  const long long* targets = p.targets;
+  nnb_after_previous(cos_t, sin_t, targets);
 
   const int items = p.m_pairs * p.n_blocks * p.k_splits;
   const int pair0 = (int)blockIdx.x >> 1, npairs = (int)gridDim.x >> 1;
@@ -292,6 +295,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
         }
       }
+      nnb_release_next();  // the last operands are on their way
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only; warp-uniform, see umma_f16_elect)
@@ -352,7 +356,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         u.item = item;
       };
       auto step = [&](Cursor& u) { if (++u.c == u.chunks) enter(u, u.item + npairs); };
-      Cursor load, store, ahead;
+      Cursor load{}, store{}, ahead{};
       auto fetch = [&](uint32_t pair) {
         const uint32_t bar = bar_in + 8 * pair, dst = smem_u32(staging + pair * 2 * BM * 128);
         mbar_expect_tx(bar, 2 * BM * 128);
@@ -519,18 +523,18 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
       long long tgt_col = -1;  // EPI_CE_LOSS: this row's target relative to the tile's first column
       if constexpr (EPI == EPI_CE_LOSS) {
-        if (d_row + row < p.M) tgt_col = p.targets[d_row + row] - (long long)n_blk * BN;
+        if (d_row + row < p.M) tgt_col = targets[d_row + row] - (long long)n_blk * BN;
       }
       // EPI_ROPE: the table entries of this thread's token, fetched while the tile is still being multiplied: 16 at head_dim 64, 32 at 128
       float rope_c[2][16], rope_s[2][16];
       if constexpr (EPI == EPI_ROPE) {
         if (n_blk * BN < p.epi_cols) {
           const size_t at = (size_t)((d_row + row) % p.t_len) * p.half_dim;
-          load_table16(p.cos_t + at + half * 16, rope_c[0]);
-          load_table16(p.sin_t + at + half * 16, rope_s[0]);
+          load_table16(cos_t + at + half * 16, rope_c[0]);
+          load_table16(sin_t + at + half * 16, rope_s[0]);
           if (p.half_dim == 64) {
-            load_table16(p.cos_t + at + 32 + half * 16, rope_c[1]);
-            load_table16(p.sin_t + at + 32 + half * 16, rope_s[1]);
+            load_table16(cos_t + at + 32 + half * 16, rope_c[1]);
+            load_table16(sin_t + at + 32 + half * 16, rope_s[1]);
           }
         }
       }
@@ -862,7 +866,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   }
   const int items = p.m_pairs * p.n_blocks * p.k_splits;
   const int grid = 2 * min(items, pairs);
-  gemm2_tcgen05_kernel<EPI, BF16><<<grid, Cfg<EPI>::kThreads, Cfg<EPI>::kSmemBytes, st>>>(tmA, tmB, tmD, tmE, p);
+  nnb_launch(gemm2_tcgen05_kernel<EPI, BF16>, grid, Cfg<EPI>::kThreads, Cfg<EPI>::kSmemBytes, st, tmA, tmB, tmD, tmE, p);
   NNB_LAUNCH_OK("gemm2_tcgen05");
   return 0;
 }

@@ -81,6 +81,8 @@ template <bool ROW, bool COL>
 __global__ void __launch_bounds__(256) mxfp8_tile_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
                                                          long long ldq, uint8_t* __restrict__ sf, uint8_t* __restrict__ qt,
                                                          long long ldqt, uint8_t* __restrict__ sft, int R, int C) {
+  nnb_after_previous(x, q, sf, qt, sft);
+  nnb_release_next();
   __shared__ __align__(16) __nv_bfloat16 tile[kTile][kTile + kTilePad];
   const int c0 = blockIdx.x * kTile, r0 = blockIdx.y * kTile;
   for (int i = threadIdx.x; i < kTile * (kTile / 8); i += 256) {
@@ -165,7 +167,7 @@ extern "C" int nnb_mxfp8_quantize_sw(const void* x, long long ldx, void* q, long
   NNB_REQUIRE(!row || (sf != nullptr && ldq % 16 == 0 && nnb_aligned16(q)), "mxfp8_quantize_sw: bad row-wise output");
   NNB_REQUIRE(!col || (sft != nullptr && ldqt % 16 == 0 && nnb_aligned16(qt)), "mxfp8_quantize_sw: bad transposed output");
   const dim3 grid(C / 128, R / 128);
-#define NNB_MX_LAUNCH(ROW, COL) mxfp8_tile_kernel<ROW, COL><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (uint8_t*)q, ldq, \
+#define NNB_MX_LAUNCH(ROW, COL) nnb_launch(mxfp8_tile_kernel<ROW, COL>, grid, 256, 0, st, (const __nv_bfloat16*)x, ldx, (uint8_t*)q, ldq, \
     (uint8_t*)sf, (uint8_t*)qt, ldqt, (uint8_t*)sft, R, C)
   if (row && col) NNB_MX_LAUNCH(true, true);
   else if (row) NNB_MX_LAUNCH(true, false);
