@@ -78,7 +78,22 @@ struct BParams {
   // the projection before RoPE, so no separate inverse-RoPE pass over the packed gradient is needed.
   const float* rope_cos;
   const float* rope_sin;
+  // A cluster of `split` CTAs shares one key tile: each takes a part of its visits, and they add up their dK and dV at the end.
+  int split;
+  void *dk, *dv;                          // split > 1: written directly, strides as the launcher's
+  long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh;
 };
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 load_cluster(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
 
 template <bool F16>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -102,10 +117,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // Longest-job-first over the whole grid: key tile 0 is visited by every query tile, the last one by a single tile, and the
   // key tile is the slowest-varying block index, so the heavy CTAs all start first and the kernel ends on the short ones.
   const int kt = blockIdx.z;          // key tile
-  const int kvh = blockIdx.x, b = blockIdx.y;
+  const int part = blockIdx.x % p.split, kvh = blockIdx.x / p.split, b = blockIdx.y;  // (part = rank in the cluster)
   const int first_qt = (kt * BKV) / BQ;                     // first query tile that can see these keys
   const int n_qt = p.n_q_tiles - first_qt;                  // query tiles per head of the group
-  const int iters = n_qt * p.group;
+  // visits are numbered head by head; this CTA's are [visit0, visit0 + iters)
+  const int visit0 = n_qt * p.group * part / p.split, iters = n_qt * p.group * (part + 1) / p.split - visit0;
+  const int head0 = kvh * p.group + visit0 / n_qt, qt0 = first_qt + visit0 % n_qt;
 
   if (threadIdx.x == 0) {
     mbar_init(bar_kv, 1);
@@ -149,7 +166,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tma_load_4d(s_base + kOffK, &tmK, bar_kv, 0, kvh, kt * BKV, b);
       tma_load_4d(s_base + kOffV, &tmV, bar_kv, 0, kvh, kt * BKV, b);
       for (int n = 0; n < iters; ++n) {
-        const int hq = kvh * p.group + n / n_qt, qt = first_qt + n % n_qt;
+        const int hq = kvh * p.group + (visit0 + n) / n_qt, qt = first_qt + (visit0 + n) % n_qt;
         const uint32_t s = n % kStagesQ, ph = (n / kStagesQ) & 1;
         if (!mbar_wait(bar_qe + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
         const uint32_t dst = s_base + kOffQdO + s * 2 * kTile16;
@@ -237,9 +254,9 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ---------------------------------------------------------------- L and D of a visit's 128 queries, up to two visits ahead:
       // -L log2(e) and -D scale, the addends of the packed multiply-adds
       constexpr float kLog2e = 1.4426950408889634f;
-      const float* gL = g_lse + ((size_t)b * p.H + kvh * p.group) * p.T;
-      const float* gD = g_delta + ((size_t)b * p.H + kvh * p.group) * p.T;
-      int qt = first_qt;
+      const float* gL = g_lse + ((size_t)b * p.H + head0) * p.T;
+      const float* gD = g_delta + ((size_t)b * p.H + head0) * p.T;
+      int qt = qt0;
       for (int n = 0; n < iters; ++n) {
         float l[4], d[4];
 #pragma unroll
@@ -259,6 +276,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive(bar_lf + 8 * (n & 1));
       }
     }
+    __syncwarp();
+    if (p.split > 1) {  // every thread of the cluster meets twice: see the compute warps
+      cluster_sync();
+      cluster_sync();
+    }
   } else if (warp < kComputeWarp0) {
     regs_dec<kRegsDrain>();
     // ------------------------------------------------------------------ drain warps: the dQ partial tile of every visit
@@ -267,7 +289,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const bool leader = warp == kDrainWarp0 && lane == 0;
     const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColdQ;
     uint8_t* my_stage = smem + kOffStage + row * 128;
-    int hq = kvh * p.group, qt = first_qt;
+    int hq = head0, qt = qt0;
     for (int m = 0; m < iters; ++m) {
       const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
       tc_fence_after();
@@ -294,6 +316,11 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (++qt == p.n_q_tiles) { qt = first_qt; ++hq; }
     }
     if (leader) tma_wait_group<0>();
+    __syncwarp();
+    if (p.split > 1) {
+      cluster_sync();
+      cluster_sync();
+    }
   } else {
     regs_inc<kRegsCompute>();
     // ------------------------------------------------------------------ compute warps (two threads per key row)
@@ -309,7 +336,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     auto query = [&](int c) { return (c < 2 ? first : 32 - first) + (c & 1) * 16; };  // first query of step c
     bool ok = true;
     NNB_PROF_DECL;
-    int qt = first_qt;
+    int qt = qt0;
     const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
     for (int n = 0; n < iters && ok; ++n) {
       NNB_PROF_T0;
@@ -398,13 +425,18 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       fail_role = 3;
     }
     NNB_PROF_FLUSH_N(iters);
-    // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the dS^T tiles) -> TMA store
-    if (ok && iters > 0) {
-      uint8_t* dst = my_ds;
+    // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the dS^T tiles) -> TMA store; in a cluster
+    // TMEM -> fp32 tiles in the ring, which every CTA of the cluster then reads for the rows it adds up and stores
+    if (ok && (iters > 0 || p.split > 1)) {
       uint32_t r0[32], r1[32];
-      tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
-      tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
-      tmem_ld_wait();
+      if (iters > 0) {
+        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
+        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r0[i] = r1[i] = 0u;
+      }
       if (half == 1 && p.rope_cos != nullptr && kt * BKV + row < p.T) {
         // dK of key position t leaves through the transpose of the forward rotation: lo' = lo c + hi s, hi' = hi c - lo s
         const float* cr = g_cos + (size_t)(kt * BKV + row) * (HD / 2);
@@ -421,25 +453,57 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
+      if (p.split > 1) {
+        uint8_t* mine = smem + kOffQdO + half * 2 * kTile16 + row * 256;  // [128 x 64] fp32, 16-byte units swizzled by the row
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = (jj & 3) * 8 + 2 * e;
-          w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
+        for (int u = 0; u < 8; ++u) {
+          *reinterpret_cast<uint4*>(mine + ((u ^ sw) << 4)) = make_uint4(r0[4 * u], r0[4 * u + 1], r0[4 * u + 2], r0[4 * u + 3]);
+          *reinterpret_cast<uint4*>(mine + 128 + ((u ^ sw) << 4)) = make_uint4(r1[4 * u], r1[4 * u + 1], r1[4 * u + 2], r1[4 * u + 3]);
         }
-        *reinterpret_cast<uint4*>(dst + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = (jj & 3) * 8 + 2 * e;
+            w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
+          }
+          *reinterpret_cast<uint4*>(my_ds + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        fence_proxy_async_smem();
+        named_barrier_sync(2, kComputeThreads);
       }
-      fence_proxy_async_smem();
-      named_barrier_sync(2, kComputeThreads);
-      if (leader) {
+      if (leader && p.split == 1) {
         tma_store_4d(&tmdV, s_base + kOffdS, 0, kvh, kt * BKV, b);
         tma_store_4d(&tmdK, s_base + kOffdS + kTile16, 0, kvh, kt * BKV, b);
         tma_commit_group();
       }
     }
     if (leader) tma_wait_group<0>();
+    if (p.split > 1) {
+      __syncwarp();
+      cluster_sync();  // every CTA's tiles are written
+      // 2 tensors x 128 rows x 16 units of four values, 256 units at a time, dealt out to the CTAs; added in the order of the parts
+      if (ok) {
+        const uint32_t tiles = s_base + kOffQdO;
+        for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < 2 * BKV * 16; u += kComputeThreads * p.split) {
+          const int which = u >> 11, r = (u >> 4) & (BKV - 1), c = u & 15, t = kt * BKV + r;
+          const uint32_t at = tiles + which * 2 * kTile16 + r * 256 + (c >> 3) * 128 + (((c & 7) ^ (r & 7)) << 4);
+          float4 v = load_cluster(at, 0);
+          for (int k = 1; k < p.split; ++k) {
+            const float4 w = load_cluster(at, k);
+            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+          }
+          if (t < p.T) {
+            uint16_t* out = which == 0 ? static_cast<uint16_t*>(p.dv) + b * p.dv_sb + t * p.dv_st + kvh * p.dv_sh
+                                       : static_cast<uint16_t*>(p.dk) + b * p.dk_sb + t * p.dk_st + kvh * p.dk_sh;
+            *reinterpret_cast<uint2*>(out + c * 4) = make_uint2(pack2_16<F16>(v.x, v.y), pack2_16<F16>(v.z, v.w));
+          }
+        }
+      }
+      cluster_sync();  // ... and read
+    }
   }
 
   if (fail_role != 0 && p.status != nullptr) {
@@ -546,6 +610,19 @@ extern "C" int nnb_flash_bwd_registers(int regs) {
   return 0;
 }
 
+// CTAs per key tile. Where the grid leaves SMs idle the kernel takes as long as its longest CTA, the one of the first keys: its visits are
+// then shared by a cluster of two or four, until it is at most a quarter longer than an SM's share of all visits. Full grids keep
+// one CTA a tile: the parts would only add their set-up and the exchange of their sums. Whole backward, us, one CTA / shared:
+// B4 H12/4 T1024 66 / 57 (two),
+// B1 57 / 31 (four), B2 H12/4 T333 31 / 25, B1 H6/1 T4096 342 / 104.
+static int visits_split(int T, int kv_heads, int group) {
+  const int tiles = (T + BKV - 1) / BKV;
+  const long long all = (long long)kv_heads * group * tiles * (tiles + 1) / 2;
+  int split = 1;
+  while (split < 4 && 4ll * tiles * group * nnb_num_sms() > 5 * all * split) split *= 2;
+  return split;
+}
+
 template <bool F16>
 static int configure_bwd() {
   cudaFuncAttributes a;
@@ -629,9 +706,12 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
     if (int rc = configure_bwd<true>()) return rc;
     configured = true;
   }
-  dim3 grid(KVH, B, (T + BKV - 1) / BKV);
-  if (f16) nnb_launch(flash_bwd_kernel<true>, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
-  else nnb_launch(flash_bwd_kernel<false>, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  p.split = visits_split(T, KVH * B, p.group);
+  p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
+  p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
+  dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
+  if (f16) nnb_launch_clusters(flash_bwd_kernel<true>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  else nnb_launch_clusters(flash_bwd_kernel<false>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd");
   const unsigned conv_blocks = (unsigned)((rows * (HD / 16) + 255) / 256);
   if (f16)
