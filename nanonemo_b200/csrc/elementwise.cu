@@ -151,26 +151,39 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
   }
 }
 
-// dw[c] (+)= sum over partial rows; 32 columns per block, 8 threads per column stride over the rows
-// (fixed order within a thread, then a fixed-order combine: the result does not depend on scheduling).
-__global__ void __launch_bounds__(256) dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int rows,
-                                                        int N, int accumulate) {
+// dw[c] (+)= sum over partial rows; 32 columns per block, 128 rows at a time (a warp: 4 rows x 32 columns in 16-byte loads), in a fixed
+// order within a thread and between them: the result does not depend on scheduling. Bound by latency (592 rows of 768 are 1.8 MB in L2,
+// read by 24 blocks): with 8 rows at a time and 4-byte loads, 74 dependent rounds, it took 7.9 us after the kernel before it, now 5.2.
+__global__ void __launch_bounds__(1024) dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int rows,
+                                                         int N, int accumulate) {
   nnb_after_previous(partial, dw);
   nnb_release_next();
-  __shared__ float s_red[8][33];
-  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-  const int col = blockIdx.x * 32 + cx;
-  float s = 0.f;
-  if (col < N)
-    for (int r = ry; r < rows; r += 8) s += partial[(size_t)r * N + col];
-  s_red[ry][cx] = s;
-  __syncthreads();
-  if (ry == 0 && col < N) {
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t += s_red[i][cx];
-    dw[col] = accumulate ? dw[col] + t : t;
+  __shared__ float s_red[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + (lane & 7) * 4;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (col < N) {
+#pragma unroll 5
+    for (int r = warp * 4 + (lane >> 3); r < rows; r += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(partial + (size_t)r * N + col);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
   }
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+    s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+  }
+  if (lane < 8) {
+    float* d = &s_red[warp][lane * 4];
+    d[0] = s.x; d[1] = s.y; d[2] = s.z; d[3] = s.w;
+  }
+  __syncthreads();
+  const float t = warp_sum(s_red[lane][warp]);  // a warp per column
+  const int c = blockIdx.x * 32 + warp;
+  if (lane == 0 && c < N) dw[c] = accumulate ? dw[c] + t : t;
 }
 
 // Supported dtype triples (residual TX, delta TD, output TY): the compute dtype C for delta and y,
@@ -253,7 +266,7 @@ extern "C" int nnb_add_rmsnorm_bwd(const void* dy, const void* h, const void* rs
   NNB_REQUIRE(done, "add_rmsnorm_bwd: unsupported dtype combination (x=%d, delta=%d, y=%d)", x_dtype, delta_dtype, y_dtype);
   NNB_REQUIRE(rc == 0, "add_rmsnorm_bwd: cannot raise the shared-memory limit");
   NNB_LAUNCH_OK("add_rmsnorm_bwd");
-  nnb_launch(dw_reduce_kernel, (N + 31) / 32, 256, 0, st, (const float*)dw_partial, (float*)dw, blocks, N, accumulate_dw);
+  nnb_launch(dw_reduce_kernel, (N + 31) / 32, 1024, 0, st, (const float*)dw_partial, (float*)dw, blocks, N, accumulate_dw);
   NNB_LAUNCH_OK("rmsnorm_dw_reduce");
   return 0;
 }
