@@ -77,6 +77,21 @@ __device__ __forceinline__ uint32_t quant4(const float* v, float inv) {
   return (uint32_t)lo | ((uint32_t)hi << 16);
 }
 
+// N elements of one scale block, given its largest magnitude: the biased exponent goes to *biased, the bytes to w.
+template <int N>
+__device__ __forceinline__ void quant_block(const float (&v)[N], float amax, uint8_t* biased, uint32_t (&w)[N / 4]) {
+  float scale = block_scale_e8m0(amax, biased);
+  if (scale == 0.f) scale = __int_as_float(1 << 23);
+  const float inv = 1.f / scale;
+#pragma unroll
+  for (int k = 0; k < N / 4; ++k) w[k] = quant4(v + 4 * k, inv);
+}
+
+// Both directions work on the tile with all 256 threads. Rows: eight lanes hold a row's 128 columns as they come from memory, 16 each
+// (two lanes share a scale), and store them as one 128-byte line. Columns: a thread takes 32 rows of two neighbouring columns out of
+// shared memory (four-byte accesses, no bank conflicts) and writes each as one 32-byte sector. When one half of the threads did whole
+// rows, 16 bytes of 32 different lines a store, and the other whole columns in two-byte reads, the 144 calls of an optimizer step (8192
+// rows of 768 to 4096) took 20.3 us on average behind the kernel before, now 12.1.
 template <bool ROW, bool COL>
 __global__ void __launch_bounds__(256) mxfp8_tile_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q,
                                                          long long ldq, uint8_t* __restrict__ sf, uint8_t* __restrict__ qt,
@@ -85,70 +100,63 @@ __global__ void __launch_bounds__(256) mxfp8_tile_kernel(const __nv_bfloat16* __
   nnb_release_next();
   __shared__ __align__(16) __nv_bfloat16 tile[kTile][kTile + kTilePad];
   const int c0 = blockIdx.x * kTile, r0 = blockIdx.y * kTile;
-  for (int i = threadIdx.x; i < kTile * (kTile / 8); i += 256) {
-    const int r = i >> 4, cc = (i & 15) * 8;
-    *reinterpret_cast<uint4*>(&tile[r][cc]) = *reinterpret_cast<const uint4*>(x + (long long)(r0 + r) * ldx + c0 + cc);
+  const int seg = threadIdx.x & 7;
+  uint4 raw[4][2];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)(r0 + k * 32 + (threadIdx.x >> 3)) * ldx + c0 + seg * 16);
+    raw[k][0] = src[0];
+    raw[k][1] = src[1];
   }
-  __syncthreads();
-  const int t = threadIdx.x & 127;
-  const bool do_row = ROW && (!COL || threadIdx.x < 128), do_col = COL && (!ROW || threadIdx.x >= 128);
-  if (do_row) {
-    // row r0 + t: four blocks of 32 columns
-    uint32_t sfw = 0;
-    uint8_t* out = q + (long long)(r0 + t) * ldq + c0;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      float v[32];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(&tile[t][b * 32 + j * 8]);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(h[e]);
-          v[j * 8 + 2 * e] = f.x; v[j * 8 + 2 * e + 1] = f.y;
-        }
-      }
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
-      uint8_t sb;
-      float scale = block_scale_e8m0(amax, &sb);
-      if (scale == 0.f) scale = __int_as_float(1 << 23);
-      const float inv = 1.f / scale;
-      sfw |= (uint32_t)sb << (8 * b);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        *reinterpret_cast<uint4*>(out + b * 32 + j * 16) = make_uint4(quant4(v + j * 16, inv), quant4(v + j * 16 + 4, inv),
-                                                                       quant4(v + j * 16 + 8, inv), quant4(v + j * 16 + 12, inv));
+  for (int k = 0; k < 4; ++k) {
+    const int r = k * 32 + (threadIdx.x >> 3);
+    if (COL) {
+      uint4* dst = reinterpret_cast<uint4*>(&tile[r][seg * 16]);
+      dst[0] = raw[k][0];
+      dst[1] = raw[k][1];
     }
-    const long long chunk = (long long)blockIdx.y * (C / kTile) + blockIdx.x;
-    *reinterpret_cast<uint32_t*>(sf + chunk * 512 + (t & 31) * 16 + (t >> 5) * 4) = sfw;
-  }
-  if (do_col) {
-    // column c0 + t = row c0 + t of the transpose: four blocks of 32 rows
-    uint32_t sfw = 0;
-    uint8_t* out = qt + (long long)(c0 + t) * ldqt + r0;
+    if (ROW) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(raw[k]);
+      float v[16], amax = 0.f;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      float v[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __bfloat162float(tile[b * 32 + i][t]);
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
+      for (int e = 0; e < 8; ++e) {
+        const float2 f = __bfloat1622float2(h[e]);
+        v[2 * e] = f.x; v[2 * e + 1] = f.y;
+        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+      }
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+      uint32_t w[4];
       uint8_t sb;
-      float scale = block_scale_e8m0(amax, &sb);
-      if (scale == 0.f) scale = __int_as_float(1 << 23);
-      const float inv = 1.f / scale;
-      sfw |= (uint32_t)sb << (8 * b);
+      quant_block(v, amax, &sb, w);
+      *reinterpret_cast<uint4*>(q + (long long)(r0 + r) * ldq + c0 + seg * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+      const long long chunk = (long long)blockIdx.y * (C / kTile) + blockIdx.x;
+      if ((seg & 1) == 0) sf[chunk * 512 + (r & 31) * 16 + (r >> 5) * 4 + (seg >> 1)] = sb;
+    }
+  }
+  if (COL) {
+    __syncthreads();
+    // columns c and c + 1 = rows c0 + c and c0 + c + 1 of the transpose, block b of 32 rows
+    const int c = (threadIdx.x & 63) * 2, b = threadIdx.x >> 6;
+    float v[2][32], amax[2] = {0.f, 0.f};
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-        *reinterpret_cast<uint4*>(out + b * 32 + j * 16) = make_uint4(quant4(v + j * 16, inv), quant4(v + j * 16 + 4, inv),
-                                                                       quant4(v + j * 16 + 8, inv), quant4(v + j * 16 + 12, inv));
+    for (int i = 0; i < 32; ++i) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&tile[b * 32 + i][c]));
+      v[0][i] = f.x; v[1][i] = f.y;
+      amax[0] = fmaxf(amax[0], fabsf(f.x));
+      amax[1] = fmaxf(amax[1], fabsf(f.y));
     }
     const long long chunk = (long long)blockIdx.x * (R / kTile) + blockIdx.y;
-    *reinterpret_cast<uint32_t*>(sft + chunk * 512 + (t & 31) * 16 + (t >> 5) * 4) = sfw;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint32_t w[8];
+      uint8_t sb;
+      quant_block(v[u], amax[u], &sb, w);
+      uint4* out = reinterpret_cast<uint4*>(qt + (long long)(c0 + c + u) * ldqt + r0 + b * 32);
+      out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      out[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      sft[chunk * 512 + ((c + u) & 31) * 16 + ((c + u) >> 5) * 4 + b] = sb;
+    }
   }
 }
 
