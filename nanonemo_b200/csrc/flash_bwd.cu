@@ -84,18 +84,7 @@ struct BParams {
   long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh;
 };
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 load_cluster(uint32_t smem_addr, uint32_t rank) {
-  uint32_t a;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-
-template <bool F16>
+template <bool F16, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -117,11 +106,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // Longest-job-first over the whole grid: key tile 0 is visited by every query tile, the last one by a single tile, and the
   // key tile is the slowest-varying block index, so the heavy CTAs all start first and the kernel ends on the short ones.
   const int kt = blockIdx.z;          // key tile
-  const int part = blockIdx.x % p.split, kvh = blockIdx.x / p.split, b = blockIdx.y;  // (part = rank in the cluster)
+  const int split = SPLIT ? p.split : 1;
+  const int part = blockIdx.x % split, kvh = blockIdx.x / split, b = blockIdx.y;  // (part = rank in the cluster)
   const int first_qt = (kt * BKV) / BQ;                     // first query tile that can see these keys
   const int n_qt = p.n_q_tiles - first_qt;                  // query tiles per head of the group
   // visits are numbered head by head; this CTA's are [visit0, visit0 + iters)
-  const int visit0 = n_qt * p.group * part / p.split, iters = n_qt * p.group * (part + 1) / p.split - visit0;
+  const int visit0 = n_qt * p.group * part / split, iters = n_qt * p.group * (part + 1) / split - visit0;
   const int head0 = kvh * p.group + visit0 / n_qt, qt0 = first_qt + visit0 % n_qt;
 
   if (threadIdx.x == 0) {
@@ -277,7 +267,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
     __syncwarp();
-    if (p.split > 1) {  // every thread of the cluster meets twice: see the compute warps
+    if constexpr (SPLIT) {  // every thread of the cluster meets twice: see the compute warps
       cluster_sync();
       cluster_sync();
     }
@@ -317,7 +307,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     if (leader) tma_wait_group<0>();
     __syncwarp();
-    if (p.split > 1) {
+    if constexpr (SPLIT) {
       cluster_sync();
       cluster_sync();
     }
@@ -427,7 +417,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     NNB_PROF_FLUSH_N(iters);
     // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the dS^T tiles) -> TMA store; in a cluster
     // TMEM -> fp32 tiles in the ring, which every CTA of the cluster then reads for the rows it adds up and stores
-    if (ok && (iters > 0 || p.split > 1)) {
+    if (ok && (iters > 0 || SPLIT)) {
       uint32_t r0[32], r1[32];
       if (iters > 0) {
         tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
@@ -453,7 +443,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      if (p.split > 1) {
+      if constexpr (SPLIT) {
         uint8_t* mine = smem + kOffQdO + half * 2 * kTile16 + row * 256;  // [128 x 64] fp32, 16-byte units swizzled by the row
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -474,24 +464,24 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         fence_proxy_async_smem();
         named_barrier_sync(2, kComputeThreads);
       }
-      if (leader && p.split == 1) {
+      if (leader && !SPLIT) {
         tma_store_4d(&tmdV, s_base + kOffdS, 0, kvh, kt * BKV, b);
         tma_store_4d(&tmdK, s_base + kOffdS + kTile16, 0, kvh, kt * BKV, b);
         tma_commit_group();
       }
     }
     if (leader) tma_wait_group<0>();
-    if (p.split > 1) {
+    if constexpr (SPLIT) {
       __syncwarp();
       cluster_sync();  // every CTA's tiles are written
       // 2 tensors x 128 rows x 16 units of four values, 256 units at a time, dealt out to the CTAs; added in the order of the parts
       if (ok) {
         const uint32_t tiles = s_base + kOffQdO;
-        for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < 2 * BKV * 16; u += kComputeThreads * p.split) {
+        for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < 2 * BKV * 16; u += kComputeThreads * split) {
           const int which = u >> 11, r = (u >> 4) & (BKV - 1), c = u & 15, t = kt * BKV + r;
           const uint32_t at = tiles + which * 2 * kTile16 + r * 256 + (c >> 3) * 128 + (((c & 7) ^ (r & 7)) << 4);
           float4 v = load_cluster(at, 0);
-          for (int k = 1; k < p.split; ++k) {
+          for (int k = 1; k < split; ++k) {
             const float4 w = load_cluster(at, k);
             v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
           }
@@ -610,24 +600,11 @@ extern "C" int nnb_flash_bwd_registers(int regs) {
   return 0;
 }
 
-// CTAs per key tile. Where the grid leaves SMs idle the kernel takes as long as its longest CTA, the one of the first keys: its visits are
-// then shared by a cluster of two or four, until it is at most a quarter longer than an SM's share of all visits. Full grids keep
-// one CTA a tile: the parts would only add their set-up and the exchange of their sums. Whole backward, us, one CTA / shared:
-// B4 H12/4 T1024 66 / 57 (two),
-// B1 57 / 31 (four), B2 H12/4 T333 31 / 25, B1 H6/1 T4096 342 / 104.
-static int visits_split(int T, int kv_heads, int group) {
-  const int tiles = (T + BKV - 1) / BKV;
-  const long long all = (long long)kv_heads * group * tiles * (tiles + 1) / 2;
-  int split = 1;
-  while (split < 4 && 4ll * tiles * group * nnb_num_sms() > 5 * all * split) split *= 2;
-  return split;
-}
-
-template <bool F16>
+template <bool F16, bool SPLIT>
 static int configure_bwd() {
   cudaFuncAttributes a;
-  if (cudaFuncGetAttributes(&a, flash_bwd_kernel<F16>) != cudaSuccess ||
-      cudaFuncSetAttribute(flash_bwd_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
+  if (cudaFuncGetAttributes(&a, flash_bwd_kernel<F16, SPLIT>) != cudaSuccess ||
+      cudaFuncSetAttribute(flash_bwd_kernel<F16, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
     nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", kSmem);
     return -3;
   }
@@ -702,16 +679,20 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.rope_sin = static_cast<const float*>(rope_sin);
   static bool configured = false;
   if (!configured) {
-    if (int rc = configure_bwd<false>()) return rc;
-    if (int rc = configure_bwd<true>()) return rc;
+    int rc = configure_bwd<false, false>();
+    if (rc == 0) rc = configure_bwd<false, true>();
+    if (rc == 0) rc = configure_bwd<true, false>();
+    if (rc == 0) rc = configure_bwd<true, true>();
+    if (rc != 0) return rc;
     configured = true;
   }
-  p.split = visits_split(T, KVH * B, p.group);
+  p.split = nnb_visits_split(T, BQ, KVH * B, p.group);
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
-  if (f16) nnb_launch_clusters(flash_bwd_kernel<true>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
-  else nnb_launch_clusters(flash_bwd_kernel<false>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  const auto kernel = f16 ? (p.split > 1 ? flash_bwd_kernel<true, true> : flash_bwd_kernel<true, false>)
+                          : (p.split > 1 ? flash_bwd_kernel<false, true> : flash_bwd_kernel<false, false>);
+  nnb_launch_clusters(kernel, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd");
   const unsigned conv_blocks = (unsigned)((rows * (HD / 16) + 255) / 256);
   if (f16)

@@ -63,9 +63,13 @@ struct BParams {
   const float* delta;
   uint32_t idesc_s, idesc_dkv, idesc_dq;
   int* status;
+  // A cluster of `split` CTAs shares one key tile: each takes a part of its visits, and they add up their dK and dV at the end.
+  int split;
+  void* out[2];          // split > 1: dV, dK, written directly
+  long long out_s[2][3];  // element strides {batch, t, head}
 };
 
-template <int HD, bool F16>
+template <int HD, bool F16, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -86,10 +90,13 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   float* s_ld = reinterpret_cast<float*>(smem + C::kOffLD);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.z, kvh = blockIdx.x, b = blockIdx.y;  // key tile slowest: the heavy CTAs (early keys) are scheduled first
+  const int split = SPLIT ? p.split : 1, part = blockIdx.x % split;  // (part = rank in the cluster)
+  const int kt = blockIdx.z, kvh = blockIdx.x / split, b = blockIdx.y;  // key tile slowest: the heavy CTAs (early keys) are scheduled first
   const int first_qb = (kt * BKV) / BQ;
   const int n_qb = p.n_q_blocks - first_qb;
-  const int iters = n_qb * p.group;
+  // visits are numbered head by head; this CTA's are [visit0, visit0 + iters)
+  const int visit0 = n_qb * p.group * part / split, iters = n_qb * p.group * (part + 1) / split - visit0;
+  const int head0 = kvh * p.group + visit0 / n_qb, qb0 = first_qb + visit0 % n_qb;
 
   if (threadIdx.x == 0) {
     mbar_init(bar_kv, 1);
@@ -134,7 +141,7 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tma_load_4d(s_base + C::kOffV + g * kHalfK, &tmV, bar_kv, g * 64, kvh, kt * BKV, b);
       }
       for (int n = 0; n < iters; ++n) {
-        const int hq = kvh * p.group + n / n_qb, qb = first_qb + n % n_qb;
+        const int hq = kvh * p.group + (visit0 + n) / n_qb, qb = first_qb + (visit0 + n) % n_qb;
         const uint32_t s = n % S, ph = (n / S) & 1;
         if (!mbar_wait(bar_qe + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
         const uint32_t dst = s_base + C::kOffQdO + s * C::kStageQdO;
@@ -223,9 +230,9 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // ------------------------------------------------------------------ L and D of a visit's 64 queries, up to two visits ahead:
     // -L log2(e) and -D scale, the addends of the packed multiply-adds
     constexpr float kLog2e = 1.4426950408889634f;
-    const float* gL = g_lse + ((size_t)b * p.H + kvh * p.group) * p.T;
-    const float* gD = g_delta + ((size_t)b * p.H + kvh * p.group) * p.T;
-    int qb = first_qb;
+    const float* gL = g_lse + ((size_t)b * p.H + head0) * p.T;
+    const float* gD = g_delta + ((size_t)b * p.H + head0) * p.T;
+    int qb = qb0;
     for (int n = 0; n < iters; ++n) {
       float v[4];
 #pragma unroll
@@ -248,7 +255,7 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const bool leader = warp == kDrainWarp0 && lane == 0;
     const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16) + C::kColdQ;
     float* stage = reinterpret_cast<float*>(smem + C::kOffStage);
-    int hq = kvh * p.group, qb = first_qb;
+    int hq = head0, qb = qb0;
     for (int m = 0; m < iters; ++m) {
       const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
       tc_fence_after();
@@ -288,7 +295,7 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
     bool ok = true;
     NNB_PROF_DECL;
-    int qb = first_qb;
+    int qb = qb0;
     for (int n = 0; n < iters; ++n) {
       NNB_PROF_T0;
       const int q0 = qb * BQ;
@@ -383,7 +390,49 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     NNB_PROF_FLUSH_N(iters);
     // dV then dK of this key tile: TMEM -> bf16 staging (the (Q | dO) ring: every load has been consumed) -> TMA store
-    if (ok && iters > 0) {
+    if constexpr (SPLIT) {
+      // In a cluster: dV, then dK, as fp32 [128 x HD] in the ring (16-byte units swizzled by the row), from where every CTA reads the
+      // units that it adds up, in the order of the parts, and stores. All threads of the cluster meet four times.
+      const uint32_t tile = s_base + C::kOffQdO;
+      for (int which = 0; which < 2; ++which) {
+        if (ok) {
+          uint8_t* mine = smem + C::kOffQdO + row * (HD * 4);
+#pragma unroll
+          for (int g = 0; g < NH; ++g) {  // this thread's half of every 64-wide head_dim group
+            uint32_t r[32];
+            if (iters > 0) {
+              tmem_ld_32x32b_x32(t_lane + (which == 0 ? C::kColdV : C::kColdK) + g * 64 + half * 32, r);
+              tmem_ld_wait();
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<uint4*>(mine + g * 256 + half * 128 + ((u ^ sw) << 4)) = make_uint4(r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+          }
+        }
+        __syncwarp();
+        cluster_sync();  // every CTA's tile is written
+        if (ok) {
+          for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < BKV * (HD / 4); u += kComputeThreads * split) {
+            const int r = u / (HD / 4), c = u % (HD / 4), t = kt * BKV + r;
+            const uint32_t at = tile + r * (HD * 4) + (c >> 3) * 128 + (((c & 7) ^ (r & 7)) << 4);
+            float4 v = load_cluster(at, 0);
+            for (int k = 1; k < split; ++k) {
+              const float4 w = load_cluster(at, k);
+              v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+            }
+            if (t < p.T) {
+              uint16_t* out = static_cast<uint16_t*>(p.out[which]) + b * p.out_s[which][0] + t * p.out_s[which][1] + kvh * p.out_s[which][2];
+              *reinterpret_cast<uint2*>(out + c * 4) = make_uint2(pack2_16<F16>(v.x, v.y), pack2_16<F16>(v.z, v.w));
+            }
+          }
+        }
+        __syncwarp();
+        cluster_sync();  // ... and read
+      }
+    } else if (ok && iters > 0) {
 #pragma unroll
       for (int u = half; u < 2 * NH; u += 2) {
         const int which = u / NH, g = u % NH;  // 0 = dV, 1 = dK; 64-wide head_dim group
@@ -416,6 +465,10 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
     if (leader) tma_wait_group<0>();
+  }
+  if (SPLIT && warp < kComputeWarp0) {  // (the compute warps met the others above)
+    __syncwarp();
+    for (int i = 0; i < 4; ++i) cluster_sync();
   }
 
   if (fail_role != 0 && p.status != nullptr) {
@@ -523,14 +576,22 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
   p.status = static_cast<int*>(status);
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(flash_bwd_t_kernel<HD, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(flash_bwd_t_kernel<HD, F16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(flash_bwd_t_kernel<HD, F16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem) != cudaSuccess) {
       nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", C::kSmem);
       return -3;
     }
     configured = true;
   }
-  dim3 grid(KVH, B, (T + BKV - 1) / BKV);
-  nnb_launch(flash_bwd_t_kernel<HD, F16>, grid, kThreads, C::kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  p.split = nnb_visits_split(T, BQ, KVH * B, p.group);
+  p.out[0] = dv;
+  p.out[1] = dk;
+  for (int i = 0; i < 3; ++i) {
+    p.out_s[0][i] = dvs[i];
+    p.out_s[1][i] = dks[i];
+  }
+  dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
+  nnb_launch_clusters(p.split > 1 ? flash_bwd_t_kernel<HD, F16, true> : flash_bwd_t_kernel<HD, F16, false>, p.split, grid, kThreads, C::kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd_t");
   nnb_launch(flash_dq_convert_t_kernel<HD, T16>, (unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st, (const float*)dq_acc, (T16*)dq, rows, H, T,
                                                                                                 dqs[0], dqs[1], dqs[2]);

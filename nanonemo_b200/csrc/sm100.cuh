@@ -111,6 +111,20 @@ static inline bool nnb_make_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, in
   return true;
 }
 
+// Attention backward: CTAs per tile of 128 keys. Where the grid leaves SMs idle the kernel takes as long as its longest CTA, the one of the
+// first keys: its visits are then shared by a cluster of two or four, until it is at most a quarter longer than an SM's share of all
+// visits. Full grids keep one CTA a tile: the parts would only add their set-up and the exchange of their sums. Whole backward, us, one
+// CTA / shared: B4 H12/4 T1024 66 / 57 (two), B1 57 / 31 (four), B2 H12/4 T333 31 / 25, B1 H6/1 T4096 342 / 104; head_dim 128:
+// B1 H16/4 T2048 206 / 94, B4 T512 72 / 58. The kernels have an instance of their own for it: with the split as a run-time value the full
+// grid of B8 H16/4 T2048 took 478 instead of 467.
+static inline int nnb_visits_split(int T, int query_rows, int kv_heads, int group) {
+  const long long tiles = (T + 127) / 128, per_tile = 128 / query_rows;  // a CTA visits `query_rows` queries at a time
+  const long long longest = ((long long)T + query_rows - 1) / query_rows * group, all = kv_heads * group * per_tile * tiles * (tiles + 1) / 2;
+  int split = 1;
+  while (split < 4 && 4 * longest * nnb_num_sms() > 5 * all * split) split *= 2;
+  return split;
+}
+
 // Optional phase timers (clock64) of one thread of CTA (0,0,0); compiled in only with -DNNB_PROFILE.
 #ifdef NNB_PROFILE
 static __device__ unsigned long long g_flash_prof[8];
@@ -318,6 +332,19 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
+// ---- clusters
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Four values of the same place in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ float4 load_cluster(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
 }
 
 // ---- descriptors

@@ -148,32 +148,33 @@ def test_mixed_operand_dtypes_are_refused():
 
 @pytest.mark.parametrize("B,T,H,KVH", [(1, 128, 1, 1), (1, 1, 3, 3), (1, 300, 2, 2), (2, 333, 12, 4), (1, 1000, 6, 1), (40, 130, 8, 4), (3, 1153, 5, 5)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, H, KVH, dtype):
+@pytest.mark.parametrize("hd", [64, 128])
+def test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, H, KVH, dtype, hd):
     """One, two and four CTAs a key tile, some of them without a visit: dK and dV are those of fp32 math to the rounding of 16-bit
     probabilities, the same in every run, and nothing beyond the last key is written."""
     from nanonemo_b200.ops import attention
     from nanonemo_b200.ops.gemm import check_status
 
     torch.manual_seed(T + H)
-    q, k, v, do = (torch.randn(B, T, n, 64, device="cuda").to(dtype) for n in (H, KVH, KVH, H))
-    o = torch.empty_like(q)
-    lse = attention.fwd_raw(q, k, v, o, 0.125)
+    q, k, v, do = (torch.randn(B, T, n, hd, device="cuda").to(dtype) for n in (H, KVH, KVH, H))
+    o, scale = torch.empty_like(q), hd ** -0.5
+    lse = attention.fwd_raw(q, k, v, o, scale)
     got = []
     for _ in range(2):
-        pad = torch.full((B, T + 1, KVH, 2, 64), 7.0, device="cuda", dtype=dtype)  # dK and dV interleaved, a row more than they need
+        pad = torch.full((B, T + 1, KVH, 2, hd), 7.0, device="cuda", dtype=dtype)  # dK and dV interleaved, a row more than they need
         dq, dk, dv = torch.empty_like(q), pad[:, :T, :, 0], pad[:, :T, :, 1]
-        attention.bwd_raw(q, k, v, o, lse, do, dq, dk, dv, 0.125)
+        attention.bwd_raw(q, k, v, o, lse, do, dq, dk, dv, scale)
         check_status()
         assert (pad[:, T] == 7).all()
         got.append((dq, dk.clone(), dv.clone()))
     assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][2], got[1][2])
     qf, kf, vf = (t.float().transpose(1, 2).requires_grad_() for t in (q, k, v))
     group = H // KVH
-    s = (qf @ kf.repeat_interleave(group, 1).transpose(-1, -2)) * 0.125
+    s = (qf @ kf.repeat_interleave(group, 1).transpose(-1, -2)) * scale
     p = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), float("-inf")).softmax(-1)
     refs = torch.autograd.grad(p @ vf.repeat_interleave(group, 1), (qf, kf, vf), do.float().transpose(1, 2))
     eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11  # P, dS, O and the results are each rounded to half of this at most
     for g, r in zip(got[0], refs):
         r = r.transpose(1, 2)
-        scale = max(r.norm().item(), 1e-3 * r.numel() ** 0.5)  # (one query: its gradients vanish, dP and D cancel to their roundings)
-        assert (g.float() - r).norm().item() <= 2 * eps * scale
+        size = max(r.norm().item(), 1e-3 * r.numel() ** 0.5)  # (one query: its gradients vanish, dP and D cancel to their roundings)
+        assert (g.float() - r).norm().item() <= 2 * eps * size
