@@ -33,6 +33,7 @@
 // 697 / 702, where the card's power limit (1.63 GHz under this kernel) evens them out.
 // All waits are bounded, except the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers).
 #include <cstdlib>
+#include <initializer_list>
 #include <type_traits>
 
 #define NNB_PROF_THREAD 256  // a compute thread
@@ -84,7 +85,7 @@ struct BParams {
   long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh;
 };
 
-template <bool F16, bool SPLIT>
+template <bool F16, bool SPLIT = false>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -600,15 +601,18 @@ extern "C" int nnb_flash_bwd_registers(int regs) {
   return 0;
 }
 
-template <bool F16, bool SPLIT>
+template <bool F16>
 static int configure_bwd() {
-  cudaFuncAttributes a;
-  if (cudaFuncGetAttributes(&a, flash_bwd_kernel<F16, SPLIT>) != cudaSuccess ||
-      cudaFuncSetAttribute(flash_bwd_kernel<F16, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
-    nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", kSmem);
-    return -3;
+  for (auto kernel : {flash_bwd_kernel<F16>, flash_bwd_kernel<F16, true>}) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
+      nnb_set_error("flash_bwd: cannot reserve %d bytes of shared memory", kSmem);
+      return -3;
+    }
+    if (int rc = nnb_flash_bwd_registers(a.numRegs)) return rc;
   }
-  return nnb_flash_bwd_registers(a.numRegs);
+  return 0;
 }
 
 // All tensors are [B, T, heads, 64] views given by element strides (contiguous last dim), bf16 or fp16 (one dtype for all).
@@ -679,20 +683,18 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.rope_sin = static_cast<const float*>(rope_sin);
   static bool configured = false;
   if (!configured) {
-    int rc = configure_bwd<false, false>();
-    if (rc == 0) rc = configure_bwd<false, true>();
-    if (rc == 0) rc = configure_bwd<true, false>();
-    if (rc == 0) rc = configure_bwd<true, true>();
-    if (rc != 0) return rc;
+    if (int rc = configure_bwd<false>()) return rc;
+    if (int rc = configure_bwd<true>()) return rc;
     configured = true;
   }
   p.split = nnb_visits_split(T, BQ, KVH * B, p.group);
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
-  const auto kernel = f16 ? (p.split > 1 ? flash_bwd_kernel<true, true> : flash_bwd_kernel<true, false>)
-                          : (p.split > 1 ? flash_bwd_kernel<false, true> : flash_bwd_kernel<false, false>);
-  nnb_launch_clusters(kernel, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  if (p.split > 1)
+    nnb_launch_clusters(f16 ? flash_bwd_kernel<true, true> : flash_bwd_kernel<false, true>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  else if (f16) flash_bwd_kernel<true><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
+  else flash_bwd_kernel<false><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd");
   const unsigned conv_blocks = (unsigned)((rows * (HD / 16) + 255) / 256);
   if (f16)
