@@ -1,6 +1,6 @@
 """Causal grouped-query FlashAttention on tcgen05/TMEM (csrc/flash_fwd.cu, csrc/flash_bwd.cu).
 
-Raw launchers; the differentiable operators are registered in ``ops/library.py``: ``flash_attn(q, k, v)`` takes
+Raw launches (through csrc/binding.cpp); the differentiable operators are there and in ``ops/library.py``: ``flash_attn(q, k, v)`` takes
 (B, H, T, hd) / (B, KVH, T, hd) tensors with any strides whose last dim is contiguous (transposed views of a
 (B, T, H, hd) projection are the common case) and returns (B, H, T, hd); ``flash_attn_packed(qkv, H, KVH, hd)`` reads
 the three operands straight out of the packed (B, T, (H + 2 KVH) hd) projection and writes (B, T, H hd), and its

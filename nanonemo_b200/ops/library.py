@@ -3,10 +3,11 @@ for each, so they compose with ``torch.compile(fullgraph=True)``, ``opcheck`` an
 layer of the reference (nanonemo/kernels/cuda/rmsnorm.py:1-69, flash_attn.py:1-60: ``custom_op`` + ``register_fake`` +
 ``register_autograd``), on top of the ahead-of-time built library instead of a per-process JIT.
 
-These operators ARE the model's sm100 path: ``nanonemo_b200.ops`` routes every call here unless the parameter involved
-lives in a flat parameter store (``weight._main_grad``), where the trainer's variants accumulate weight gradients in
-place in the flat buffer and report gradient readiness to the strategy — side effects a functional operator cannot
-have. Both routes call the same launchers.
+``nanonemo_b200.ops`` routes here what the native operators (csrc/binding.cpp) leave: operators that they do not have, and every call
+that is not a plain one (tracing, transforms, tensor subclasses, tangents), unless the parameter involved lives in a flat parameter
+store (``weight._main_grad``), where the trainer's variants accumulate weight gradients in place in the flat buffer and report
+gradient readiness to the strategy — side effects a functional operator cannot have. The native operators' backward nodes come
+here too under create_graph=True and for batched gradients. All routes call the same launchers.
 
     torch.ops.nanonemo_b200.add_rms_norm(x, delta, weight, eps)              -> (y, h, rstd)
     torch.ops.nanonemo_b200.swiglu(gu)                                       -> act
