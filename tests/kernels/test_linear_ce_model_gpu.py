@@ -178,3 +178,21 @@ def test_cuda_graph_training_matches_eager(tmp_path):
                          total_tokens=1024 * 10, peak_lr=1e-3, precision="bf16", eval_every=100, eval_batches=1, cuda_graph=graph)
         out[name] = [r["loss"] for r in train(ModelConfig.sm100(**SMALL), tc, device="cuda:0") if "loss" in r]
     assert out["graph"] == pytest.approx(out["eager"], abs=2e-2)
+
+
+@pytest.mark.parametrize("rows,width,vocab", [(1, 64, 64), (130, 768, 5000), (1000, 512, 32000), (2432, 768, 5000), (4096, 768, 5000), (6144, 768, 2056)])
+def test_the_heads_input_gradient_in_splits_and_directly(rows, width, vocab):
+    """Both sides of the rule (one wave of narrow tiles or of pairs, filled and not): one rounding to 16 bits of a sum that is off by
+    less than a tenth of it."""
+    from nanonemo_b200.ops import linear_ce
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(rows)
+    g, w = (torch.randn(rows, vocab, device="cuda") * 0.01).bfloat16(), (torch.randn(vocab, width, device="cuda") * 0.02).bfloat16()
+    out = torch.full((rows + 1, width), 7.0, device="cuda", dtype=torch.bfloat16)
+    linear_ce._input_gradient(g, w, out[:rows])
+    check_status()
+    assert (out[rows] == 7).all()
+    ref = g.double() @ w.double()
+    rounding = (ref.bfloat16().double() - ref).norm()
+    assert (out[:rows].double() - ref).norm() <= 1.1 * rounding

@@ -288,3 +288,20 @@ def test_launches_are_counted_once():
     torch.autograd.grad(y, (x, w), torch.ones_like(y))
     assert _lib.LAUNCHES - before == 3
     assert math.isfinite(y.float().sum().item())
+
+
+def test_inference_mode(python_route):
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+
+    torch.manual_seed(6)
+    cos, sin = rope_cache(64, 512, device=DEV)
+    x, wq, gu, down, n = _rand(1, 300, 128, grad=False), _rand(256, 128), _rand(512, 128), _rand(128, 256), torch.ones(128, device=DEV).requires_grad_()
+    q = _rand(1, 2, 66, 64, dtype=torch.bfloat16, grad=False)
+
+    def fn():
+        y, h = ops.add_rms_norm(x, x.bfloat16(), n, 1e-5, impl="sm100")
+        return (ops.qkv_rope_attention(y, wq, cos, sin, 2, 1, 64), ops.mlp_swiglu(y, gu, down), ops.linear(y, wq, impl="sm100"), y, h, ops.flash_attn(q, q, q))
+
+    with torch.inference_mode(), torch.autocast("cuda", dtype=torch.bfloat16):
+        _same(fn(), python_route(fn))
