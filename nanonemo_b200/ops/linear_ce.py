@@ -76,23 +76,6 @@ def _dx_tile(rows: int, width: int, device) -> int:
     return 128 if -(-rows // 128) * -(-width // 128) <= _sm_count(device) else 0
 
 
-def _input_gradient(g: torch.Tensor, w16: torch.Tensor, out: torch.Tensor) -> None:
-    """out [rows, width] (16-bit) = g @ w16, the head's input gradient: one long K loop (the vocabulary) per tile. Where the tiles keep
-    fewer than four fifths of the SMs busy the loop is cut into splits that add up an fp32 matrix, which is then rounded once (error
-    against 64 bits the same to three digits); fuller grids write 16-bit tiles directly. us, direct / in splits: 128-wide tiles 256 x
-    768 x 50304 225 / 41, 1000 x 768 227 / 94, 2048 x 768 234 / 174, 500 x 2048 237 / 129, and where they fill the SMs 3000 x 768 242 /
-    246; CTA pairs 4096 x 768 250 / 211, 8192 x 768 532 / 442, and where they fill 6144 x 768 295 / 303, 2048 x 2048 268 / 336."""
-    rows, width = out.shape
-    sms, bn = _sm_count(g.device), _dx_tile(rows, width, g.device)
-    tiles, units = (-(-rows // 128) * -(-width // 128), sms) if bn == 128 else (-(-rows // 256) * -(-width // 256), sms // 2)
-    if 5 * tiles < 4 * units * -(-tiles // units):
-        total = torch.empty((rows, width), dtype=torch.float32, device=g.device)
-        gemm(g, w16, b_mn=True, out=total, bn=bn)
-        out.copy_(total)
-    else:
-        gemm(g, w16, b_mn=True, out=out, bn=bn)
-
-
 def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
     mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
@@ -112,7 +95,7 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
         else:
             gemm(xc, w16, out=lg)
             ce_inplace(lg, targets[r0:r1], loss_rows[r0:r1], 1.0 / N)
-        _input_gradient(lg, w16, dx[r0:r1])
+        gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
         gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=r0 > 0)
     return loss_rows.sum(), dx
 
@@ -222,7 +205,7 @@ class _VocabParallelLinearCE(torch.autograd.Function):
             lg, xc = logits[: r1 - r0], x16[r0:r1]
             gemm(xc, w16, out=lg)
             vocab_parallel_ce_inplace(lg, tg[r0:r1], loss_rows[r0:r1], 1.0 / N, v0, Vl * tp.world, tp.all_gather, tp.world)
-            _input_gradient(lg, w16, dx[r0:r1])
+            gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
             gemm(lg, xc, a_mn=True, b_mn=True, out=dW, accumulate=r0 > 0)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype
