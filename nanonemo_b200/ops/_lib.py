@@ -48,7 +48,9 @@ def lib():
 def native():
     """The C++ binding (csrc/binding.cpp): raw launches and operators that run without Python in between."""
     lib()  # (says how to build it when it is missing)
-    return importlib.import_module("nanonemo_b200.ops._native")
+    binding = importlib.import_module("nanonemo_b200.ops._native")
+    importlib.import_module("nanonemo_b200.ops.library")  # the operators that its backward nodes look up by name
+    return binding
 
 
 def operator_call(name: str, *args):

@@ -305,3 +305,28 @@ def test_inference_mode(python_route):
 
     with torch.inference_mode(), torch.autocast("cuda", dtype=torch.bfloat16):
         _same(fn(), python_route(fn))
+
+
+_FIRST_CALLS = """
+import torch
+from nanonemo_b200 import ops
+torch.manual_seed(0)
+x, w, n = (torch.randn(*s, device="cuda", requires_grad=True) for s in ((66, 64), (72, 64), (64,)))
+q = torch.randn(1, 2, 66, 64, device="cuda").bfloat16().requires_grad_()
+for fn, leaf in ((lambda: ops.linear(x, w, impl="sm100"), x), (lambda: ops.add_rms_norm(x, None, n, 1e-5, impl="sm100")[0], x), (lambda: ops.flash_attn(q, q.detach(), q.detach()), q)):
+    g = torch.randn_like(fn())
+    (plain,) = torch.autograd.grad(fn(), leaf, g)
+    (two,) = torch.autograd.grad(fn(), leaf, torch.stack((g, 2 * g)), is_grads_batched=True)
+    assert torch.allclose(two[0].float(), plain.float(), rtol=2e-2, atol=1e-3)
+for fn, leaf in ((lambda: ops.add_rms_norm(x, None, n, 1e-5, impl="sm100")[0], x), (lambda: ops.flash_attn(q, q.detach(), q.detach()), q)):
+    assert torch.autograd.grad(fn().float().sum(), leaf, create_graph=True)[0].requires_grad
+"""
+
+
+def test_backward_nodes_find_the_registered_operators_in_a_new_process():
+    """Nothing but `ops` imported and no call made that would have registered them."""
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", _FIRST_CALLS], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
