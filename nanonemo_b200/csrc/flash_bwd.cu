@@ -31,7 +31,8 @@
 // warps a scheduler do not hide. (A quarter or half of the exponentials as polynomials on the multiply-add pipe: no change.) Whole backward,
 // us, queries as rows / keys as rows: B32 H12/4 T1024 303 / 283, B128 T256 184 / 174, B64 H8/8 T200 84 / 80, B2 H12/4 T333 35 / 33, B8 H12/4 T4096
 // 697 / 702, where the card's power limit (1.63 GHz under this kernel) evens them out.
-// All waits are bounded, except the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers).
+// All waits are bounded, except two: the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers), and, in a
+// cluster, the two barriers of all its threads at the end, which every role of every CTA reaches, after a wait that ran out too.
 #include <cstdlib>
 #include <initializer_list>
 #include <type_traits>
@@ -267,7 +268,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive(bar_lf + 8 * (n & 1));
       }
     }
-    __syncwarp();
     if constexpr (SPLIT) {  // every thread of the cluster meets twice: see the compute warps
       cluster_sync();
       cluster_sync();
@@ -307,7 +307,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (++qt == p.n_q_tiles) { qt = first_qt; ++hq; }
     }
     if (leader) tma_wait_group<0>();
-    __syncwarp();
     if constexpr (SPLIT) {
       cluster_sync();
       cluster_sync();
@@ -473,7 +472,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     if (leader) tma_wait_group<0>();
     if constexpr (SPLIT) {
-      __syncwarp();
       cluster_sync();  // every CTA's tiles are written
       // 2 tensors x 128 rows x 16 units of four values, 256 units at a time, dealt out to the CTAs; added in the order of the parts
       if (ok) {

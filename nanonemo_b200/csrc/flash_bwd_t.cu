@@ -412,7 +412,6 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               *reinterpret_cast<uint4*>(mine + g * 256 + half * 128 + ((u ^ sw) << 4)) = make_uint4(r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
           }
         }
-        __syncwarp();
         cluster_sync();  // every CTA's tile is written
         if (ok) {
           for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < BKV * (HD / 4); u += kComputeThreads * split) {
@@ -429,7 +428,6 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             }
           }
         }
-        __syncwarp();
         cluster_sync();  // ... and read
       }
     } else if (ok && iters > 0) {
@@ -467,7 +465,6 @@ flash_bwd_t_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (leader) tma_wait_group<0>();
   }
   if (SPLIT && warp < kComputeWarp0) {  // (the compute warps met the others above)
-    __syncwarp();
     for (int i = 0; i < 4; ++i) cluster_sync();
   }
 

@@ -335,7 +335,10 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
 }
 
 // ---- clusters
+// All threads of the cluster meet. The aligned form wants every warp to arrive as one: the barrier gathers its lanes first, whatever branches
+// they come from. It has no limit; a caller reaches it on every path, each role after its own bounded waits.
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Four values of the same place in the shared memory of CTA `rank` of the cluster.
