@@ -630,17 +630,21 @@ py::object qkv_rope_attention(py::handle x_, py::handle weight_, py::handle cos_
   return py::cast(y);
 }
 
-// The SwiGLU feed-forward as one node (engine weights, or calls without gradients)
+// (gu, act) of the gate and up projection, gu only where it is kept or has to be made: in one launch, or in two where the fused kernel does not serve
+std::pair<Tensor, Tensor> gate_up(const Tensor& x2, const Tensor& w16, bool keep) {
+  auto r = gemm_swiglu(x2, w16, keep);
+  if (r.second.defined()) return r;
+  const int64_t F = w16.size(0) / 2;
+  r = {gemm_nt(x2, w16), empty({x2.size(0), F}, w16.scalar_type(), x2)};
+  swiglu_fwd(r.first.narrow(1, 0, F), r.first.narrow(1, F, F), r.second);
+  return r;
+}
+
+// The SwiGLU feed-forward as one node (engine weights)
 struct MLPFn : torch::autograd::Function<MLPFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_gu, const Tensor& w_down, const Tensor& gu16, const Tensor& down16) {
     const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), gu16.scalar_type()));
-    const int64_t F = w_gu.size(0) / 2;
-    auto [gu, act] = gemm_swiglu(x2, gu16, true);
-    if (!act.defined()) {
-      gu = gemm_nt(x2, gu16);
-      act = empty({x2.size(0), F}, gu16.scalar_type(), x);
-      swiglu_fwd(gu.narrow(1, 0, F), gu.narrow(1, F, F), act);
-    }
+    auto [gu, act] = gate_up(x2, gu16, true);
     Tensor y = gemm_nt(act, down16);
     ctx->save_for_backward({x2, w_gu, w_down, gu, act});
     ctx->saved_data["gu16"] = gu16;
@@ -680,12 +684,13 @@ py::object mlp_swiglu(py::handle x_, py::handle gu_, py::handle down_) {
   {
     py::gil_scoped_release nogil;
     const at::ScalarType dt = compute_dtype();
-    if (!grad) {  // nobody will ask for the projection: only the activation leaves its GEMM
-      const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), dt)), gu16 = gu.in(w_gu, dt);
-      Tensor act = gemm_swiglu(x2, gu16, false).second;
-      if (act.defined()) y = gemm_nt(act, down.in(w_down, dt)).view(with_last(x.sizes(), w_down.size(0)));
+    const Tensor gu16 = gu.in(w_gu, dt), down16 = down.in(w_down, dt);  // (cast once, whichever launches follow)
+    if (grad) {
+      y = MLPFn::apply(x, w_gu, w_down, gu16, down16);
+    } else {  // nobody will ask for the projection: where one launch serves, only the activation leaves it
+      const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), dt));
+      y = gemm_nt(gate_up(x2, gu16, false).second, down16).view(with_last(x.sizes(), w_down.size(0)));
     }
-    if (!y.defined()) y = MLPFn::apply(x, w_gu, w_down, gu.in(w_gu, dt), down.in(w_down, dt));
   }
   return py::cast(y);
 }
