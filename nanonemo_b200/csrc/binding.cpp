@@ -327,7 +327,9 @@ struct Weight {
   Tensor in(const Tensor& w, at::ScalarType dt) const { return shadow.defined() && shadow.scalar_type() == dt ? shadow : as_dtype(w.detach(), dt); }
 };
 
-// dW of an engine weight goes into the flat gradient buffer, and the strategy hears of it. Everything is read from the weight's
+// dW of an engine weight goes into the flat gradient buffer, and the strategy hears of it, in every backward pass through a weight that is
+// trained, also one that asks for other gradients only: as with the Python autograd functions, whose needs_input_grad is fixed in the
+// forward pass (needs_input_grad here is what the running pass asks for). Everything is read from the weight's
 // Python object when the backward runs (a saved-tensor hook may have put another tensor in its place).
 struct MainGrad {
   Tensor main;
@@ -404,6 +406,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     ctx->saved_data["x_sizes"] = x.sizes().vec();
     ctx->saved_data["x_dtype"] = (int64_t)x.scalar_type();
     ctx->saved_data["engine"] = engine;
+    ctx->saved_data["trained"] = weight.requires_grad();
     return fresh([&] { return y.view(with_last(x.sizes(), weight.size(0))); });
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -412,7 +415,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const bool engine = ctx->saved_data["engine"].toBool();
     const auto x_sizes = ctx->saved_data["x_sizes"].toIntVector();
     const auto x_dtype = (at::ScalarType)ctx->saved_data["x_dtype"].toInt();
-    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = engine ? ctx->saved_data["trained"].toBool() : ctx->needs_input_grad(1);
     Tensor dy2 = as_dtype(rows2d(grads[0]), x2.scalar_type()), dx, dw;
     if (!engine && through_dispatcher(grads[0])) {
       dy2 = dy2.contiguous();
@@ -579,6 +582,7 @@ struct QKVRopeAttentionFn : torch::autograd::Function<QKVRopeAttentionFn> {
     ctx->saved_data["w16"] = w16;
     ctx->saved_data["meta"] = std::vector<int64_t>{B, T, H, KVH, hd, (int64_t)x.scalar_type()};
     ctx->saved_data["x_sizes"] = x.sizes().vec();
+    ctx->saved_data["trained"] = weight.requires_grad();
     return fresh([&] { return o.view({B, T, H * hd}); });
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -601,7 +605,7 @@ struct QKVRopeAttentionFn : torch::autograd::Function<QKVRopeAttentionFn> {
     }
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) dx = as_dtype(gemm_nt(dqkv, ctx->saved_data["w16"].toTensor(), true).view(ctx->saved_data["x_sizes"].toIntVector()), (at::ScalarType)m[5]);
-    if (ctx->needs_input_grad(1)) dw = weight_gradient(dqkv, x2, weight, true);
+    if (ctx->saved_data["trained"].toBool()) dw = weight_gradient(dqkv, x2, weight, true);
     return {dx, dw, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -651,6 +655,7 @@ struct MLPFn : torch::autograd::Function<MLPFn> {
     ctx->saved_data["down16"] = down16;
     ctx->saved_data["x_sizes"] = x.sizes().vec();
     ctx->saved_data["x_dtype"] = (int64_t)x.scalar_type();
+    ctx->saved_data["trained"] = std::vector<int64_t>{w_gu.requires_grad(), w_down.requires_grad()};
     return fresh([&] { return y.view(with_last(x.sizes(), w_down.size(0))); });
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -666,10 +671,11 @@ struct MLPFn : torch::autograd::Function<MLPFn> {
       dgu = at::empty_like(gu);
       swiglu_bwd(dact, gu.narrow(1, 0, F), gu.narrow(1, F, F), dgu.narrow(1, 0, F), dgu.narrow(1, F, F));
     }
+    const auto trained = ctx->saved_data["trained"].toIntVector();
     Tensor dx, dw_gu, dw_down;
-    if (ctx->needs_input_grad(2)) dw_down = weight_gradient(dy2, act, w_down, true);
+    if (trained[1]) dw_down = weight_gradient(dy2, act, w_down, true);
     if (ctx->needs_input_grad(0)) dx = as_dtype(gemm_nt(dgu, gu16, true).view(ctx->saved_data["x_sizes"].toIntVector()), (at::ScalarType)ctx->saved_data["x_dtype"].toInt());
-    if (ctx->needs_input_grad(1)) dw_gu = weight_gradient(dgu, x2, w_gu, true);
+    if (trained[0]) dw_gu = weight_gradient(dgu, x2, w_gu, true);
     return {dx, dw_gu, dw_down, Tensor(), Tensor()};
   }
 };

@@ -159,6 +159,31 @@ def test_engine_nodes_add_into_the_flat_gradient_and_report_it(python_route, M, 
                 assert (a.float() - b.float()).norm() <= (2 ** -8 if a.dtype != torch.float32 or name == "qkv" else 1e-6) * b.float().norm(), name
 
 
+def test_engine_nodes_add_their_weight_gradients_whatever_a_backward_pass_asks_for(python_route):
+    """autograd.grad of the input alone, and a weight that is not trained."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+
+    torch.manual_seed(8)
+    cos, sin = rope_cache(64, 1024, device=DEV)
+    x = _rand(2, 160, 192, dtype=torch.bfloat16)
+    wq, gu, down, norm = _rand(256, 192), _rand(512, 192), _rand(192, 256), torch.ones(192, device=DEV).requires_grad_()
+    frozen, frozen_gu = _rand(256, 192, grad=False), _rand(512, 192, grad=False)
+    calls = [((wq,), lambda: ops.qkv_rope_attention(x, wq, cos, sin, 2, 1, 64)), ((gu, down), lambda: ops.mlp_swiglu(x, gu, down)), ((wq,), lambda: ops.linear(x, wq, impl="sm100")),
+             ((norm,), lambda: ops.add_rms_norm(x, None, norm, 1e-5, impl="sm100")[0]), ((frozen,), lambda: ops.linear(x, frozen, impl="sm100")),
+             ((frozen,), lambda: ops.qkv_rope_attention(x, frozen, cos, sin, 2, 1, 64)), ((frozen_gu, down), lambda: ops.mlp_swiglu(x, frozen_gu, down))]
+    for ws, fn in calls:
+        got = []
+        for run in (lambda f: f(), python_route):
+            _engine(*ws)
+            out = run(fn)
+            torch.autograd.grad(out, x, torch.linspace(-1, 1, out.numel(), device=DEV).view(out.shape).to(out.dtype))
+            got.append([(w._told, w._main_grad) for w in ws])
+        for w, (told, a), (ref_told, b) in zip(ws, *got):
+            assert told == ref_told == ([True] if w.requires_grad else [])
+            assert (a - b).norm() <= 2 ** -8 * b.norm() and (b.norm() > 0) == w.requires_grad  # (dQ is summed in any order, then rounded)
+
+
 def test_calls_without_gradients_match_the_registered_operators(python_route):
     from nanonemo_b200 import ops
     from nanonemo_b200.models.layers import rope_cache
