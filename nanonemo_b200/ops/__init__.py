@@ -264,14 +264,14 @@ def mlp_swiglu(x, w_gu, w_down):
     shadow) it is one autograd node whose backward computes the activation's backward in a GEMM epilogue; elsewhere it is
     the registered gate||up operator followed by the registered linear."""
     _need_cuda(x, "mlp_swiglu")
-    y = _lib.operator_call("mlp_swiglu", x, w_gu, w_down)
+    from nanonemo_b200.ops import fused_block
+
+    y = fused_block.native_mlp(x, w_gu, w_down)
     if y is not NotImplemented:
         return y
     engine = lambda w: in_flat_store(w) or getattr(w, "_shadow", None) is not None
     if engine(w_gu) and engine(w_down) and getattr(w_gu, "_gather_in_gemm", None) is None:
-        from nanonemo_b200.ops.fused_block import mlp_swiglu as f
-
-        return f(x, w_gu, w_down)
+        return fused_block.mlp_swiglu(x, w_gu, w_down)
     return linear(linear_swiglu(x, w_gu), w_down, impl="sm100")
 
 

@@ -146,6 +146,11 @@ def linear_swiglu(x, weight):
 FUSE_SWIGLU_BWD = os.environ.get("NANONEMO_FUSE_SWIGLU_BWD", "1") != "0"
 
 
+def native_mlp(x, w_gu, w_down):
+    """The native feed-forward, whose backward always tries the fused kernel: not where that is switched off."""
+    return _lib.operator_call("mlp_swiglu", x, w_gu, w_down) if FUSE_SWIGLU_BWD else NotImplemented
+
+
 class _MLPSwiGLU(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_gu, w_down):
@@ -187,7 +192,7 @@ class _MLPSwiGLU(torch.autograd.Function):
 
 def mlp_swiglu(x, w_gu, w_down):
     """x: (..., d); w_gu: [2 F, d] (gate rows first); w_down: [d, F] -> down(silu(x Wg^T) * (x Wu^T)), shape (..., d)."""
-    y = _lib.operator_call("mlp_swiglu", x, w_gu, w_down) if FUSE_SWIGLU_BWD else NotImplemented
+    y = native_mlp(x, w_gu, w_down)
     if y is not NotImplemented:
         return y
     if no_backward(x, w_gu, w_down):

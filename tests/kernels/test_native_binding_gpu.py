@@ -337,6 +337,26 @@ def test_calls_without_gradients_cast_no_more_than_the_registered_operators(pyth
         assert casts(fn) == weights + 1 <= python_route(lambda: casts(fn))  # noqa: B023
 
 
+def test_the_fused_swiglu_backward_can_be_switched_off_on_the_models_path(monkeypatch):
+    from nanonemo_b200 import ops
+    from nanonemo_b200.ops import _lib, fused_block
+
+    torch.manual_seed(7)
+    x, gu, down = _rand(300, 128), _rand(512, 128), _rand(128, 256)
+    launches, got = [], []
+    for fused in (True, False):
+        monkeypatch.setattr(fused_block, "FUSE_SWIGLU_BWD", fused)
+        _engine(gu, down)
+        before = _lib.LAUNCHES
+        out = ops.mlp_swiglu(x, gu, down)
+        (dx,) = torch.autograd.grad(out, x, torch.ones_like(out))
+        launches.append(_lib.LAUNCHES - before)
+        got.append((out.detach(), dx, gu._main_grad))
+    assert launches[1] == launches[0] + 1  # d(act) and the activation's backward apart
+    for a, b in zip(*got):  # d(act) is rounded to 16 bits between the two
+        assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
+
+
 def test_inference_mode(python_route):
     from nanonemo_b200 import ops
     from nanonemo_b200.models.layers import rope_cache
