@@ -599,6 +599,9 @@ extern "C" int nnb_flash_bwd_registers(int regs) {
   return 0;
 }
 
+// The rule on its own (head_dim 64: 128 queries a visit, 128: 64), for tests.
+extern "C" int nnb_flash_bwd_split(int T, int query_rows, long long kv_heads, int group, int sms) { return nnb_visits_split(T, query_rows, kv_heads, group, sms); }
+
 template <bool F16>
 static int configure_bwd() {
   for (auto kernel : {flash_bwd_kernel<F16>, flash_bwd_kernel<F16, true>}) {
@@ -685,7 +688,7 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
     if (int rc = configure_bwd<true>()) return rc;
     configured = true;
   }
-  p.split = nnb_visits_split(T, BQ, KVH * B, p.group);
+  p.split = nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);

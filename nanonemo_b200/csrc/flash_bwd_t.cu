@@ -580,7 +580,7 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
     }
     configured = true;
   }
-  p.split = nnb_visits_split(T, BQ, KVH * B, p.group);
+  p.split = nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
   p.out[0] = dv;
   p.out[1] = dk;
   for (int i = 0; i < 3; ++i) {

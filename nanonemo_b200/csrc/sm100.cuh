@@ -111,18 +111,41 @@ static inline bool nnb_make_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, in
   return true;
 }
 
-// Attention backward: CTAs per tile of 128 keys. Where the grid leaves SMs idle the kernel takes as long as its longest CTA, the one of the
-// first keys: its visits are then shared by a cluster of two or four, until it is at most a quarter longer than an SM's share of all
-// visits. Full grids keep one CTA a tile: the parts would only add their set-up and the exchange of their sums. Whole backward, us, one
-// CTA / shared: B4 H12/4 T1024 66 / 57 (two), B1 57 / 31 (four), B2 H12/4 T333 31 / 25, B1 H6/1 T4096 342 / 104; head_dim 128:
-// B1 H16/4 T2048 206 / 94, B4 T512 72 / 58. The kernels have an instance of their own for it: with the split as a run-time value the full
-// grid of B8 H16/4 T2048 took 478 instead of 467.
-static inline int nnb_visits_split(int T, int query_rows, int kv_heads, int group) {
-  const long long tiles = (T + 127) / 128, per_tile = 128 / query_rows;  // a CTA visits `query_rows` queries at a time
-  const long long longest = ((long long)T + query_rows - 1) / query_rows * group, all = kv_heads * group * per_tile * tiles * (tiles + 1) / 2;
-  int split = 1;
-  while (split < 4 && 4 * longest * nnb_num_sms() > 5 * all * split) split *= 2;
-  return split;
+// Attention backward: CTAs (a cluster: one, two or four) per tile of 128 keys. A CTA keeps an SM to itself and visits `query_rows` queries at a
+// time; one a tile, the kernel of a small grid takes as long as the CTA of the first keys while other SMs are idle. In a cluster each
+// takes a part of the tile's visits, at a price: sums that meet at the end (as long as 256 queries), and set-up that the next CTA of an
+// SM waits for (384). What a split takes is estimated as the largest of: all work over all SMs; the longest CTA; and, where there
+// are more CTAs than SMs, those that share an SM at best. A larger split has to be better by 15 %. Two waves and more stay as they are.
+// Of 460 grids timed with one, two and four (both head sizes, 1 to 320 tiles, 1 to 192 visits of the longest) one gets slower than with one
+// CTA, by 2 %, and the choice is within 12 % of the best; a rule that only compared the longest CTA with all work made 119 of the
+// first 380 slower, by up to 1.75 times. Whole backward, us, one / two / four: head_dim 64 B1 H6/1 T4096 342 / - / 104, B1 H12/4 T1024 57 / 41 / 31, B2 T2048
+// 104 / 76 / 98, B4 T1024 66 / 59 / 78, B10 T512 47 / 64 / 80, B8 H8/8 T64 16 / 21 / 29; head_dim 128 B1 H16/4 T2048 209 / 128 / 94, B4
+// T512 72 / 55 / 57, B14 T256 55 / 68 / 88. The kernels have an instance of their own for clusters: with the split as a run-time value
+// the full grid of B8 H16/4 T2048 took 478 instead of 467.
+static inline int nnb_visits_split(int T, int query_rows, long long kv_heads, int group, int sms) {
+  const long long tiles = (T + 127) / 128, q_tiles = (T + query_rows - 1) / query_rows, per_tile = 128 / query_rows;
+  const long long all = kv_heads * group * (tiles * q_tiles - per_tile * tiles * (tiles - 1) / 2), meet = 256 / query_rows, setup = 384 / query_rows;
+  if (kv_heads * tiles >= 2 * sms) return 1;
+  // in visits, times the number of SMs
+  auto takes = [&](int split) {
+    const long long ctas = kv_heads * split, m = split > 1 ? meet : 0, u = split > 1 ? setup : 0;  // ctas: of one key tile
+    long long t = all + u * ctas * tiles;
+    for (long long k = 0; k * sms < ctas * tiles; ++k) {  // the k sms + 1 longest CTAs: k + 1 of them share an SM
+      const long long part = ((q_tiles - k * sms / ctas * per_tile) * group + split - 1) / split, here = sms * ((k + 1) * part + k * u + m);
+      if (here > t) t = here;
+    }
+    return t;
+  };
+  int best = 1;
+  long long best_takes = takes(1);
+  for (int split = 2; split <= 4 && split <= q_tiles * group; split *= 2) {
+    const long long t = takes(split);
+    if (23 * t < 20 * best_takes) {
+      best = split;
+      best_takes = t;
+    }
+  }
+  return best;
 }
 
 // Optional phase timers (clock64) of one thread of CTA (0,0,0); compiled in only with -DNNB_PROFILE.

@@ -94,6 +94,7 @@ _SIGNATURES = {
     "nnb_cast_from_f32": "ppqip",
     "nnb_build_arch": "",
     "nnb_flash_bwd_registers": "i",
+    "nnb_flash_bwd_split": "iiqii",
     "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfipppp",
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",

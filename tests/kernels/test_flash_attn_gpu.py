@@ -1,5 +1,7 @@
 """FlashAttention (tcgen05) against PyTorch attention in fp32: MHA / GQA, odd T, hd 64 / 128."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -178,3 +180,13 @@ def test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, H, KVH, dtype
         r = r.transpose(1, 2)
         size = max(r.norm().item(), 1e-3 * r.numel() ** 0.5)  # (one query: its gradients vanish, dP and D cancel to their roundings)
         assert (g.float() - r).norm().item() <= 2 * eps * size
+
+
+@pytest.mark.parametrize("B,T,H,KVH,hd", [(4, 1001, 12, 4, 64), (4, 513, 16, 4, 128)])
+def test_backward_whose_key_tiles_are_shared_by_two_ctas(B, T, H, KVH, hd):
+    """Odd T: the last tile ends inside a warp of the exchange."""
+    from nanonemo_b200.ops import _lib
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _lib.lib().nnb_flash_bwd_split(T, 128 if hd == 64 else 64, ctypes.c_longlong(B * KVH), H // KVH, sms) == 2
+    test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, H, KVH, torch.bfloat16, hd)
