@@ -556,7 +556,7 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
   if (!nnb_make_tmap_4d(&tdv, dt, 2, dv, HD, KVH, T, B, dvs[2] * 2, dvs[1] * 2, dvs[0] * 2, 64, 1, BKV, "flash_bwd dV")) return -4;
 
   const long long rows = (long long)B * T * H;
-  nnb_launch(flash_delta_t_kernel<HD, T16>, (unsigned)((rows * (HD / 8) + 255) / 256), 256, 0, st, (const T16*)o, (const T16*)d_o, (float*)delta, (float*)dq_acc, B, T, H, os[0], os[1], os[2], dos[0], dos[1], dos[2]);
+  nnb_launch_pre_pass(rows * HD, flash_delta_t_kernel<HD, T16>, (unsigned)((rows * (HD / 8) + 255) / 256), 256, st, (const T16*)o, (const T16*)d_o, (float*)delta, (float*)dq_acc, B, T, H, os[0], os[1], os[2], dos[0], dos[1], dos[2]);
   NNB_LAUNCH_OK("flash_delta");
   BParams p{};
   p.B = B; p.H = H; p.KVH = KVH; p.T = T;

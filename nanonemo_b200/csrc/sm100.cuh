@@ -148,6 +148,18 @@ static inline int nnb_visits_split(int T, int query_rows, long long kv_heads, in
   return best;
 }
 
+// The attention backward's pre-pass (D of every row, and the dQ buffer cleared). From 2^24 values of O on (34 MB in 16 bits) it is launched in
+// plain stream order: with its first blocks placed one by one as the forward's CTAs leave, the pass itself, bound by memory, took 56 us
+// instead of 46 and the backward kernel behind it 474 instead of 463 (B8 H16/4 T2048 head_dim 128); below that the early start gains more.
+// Forward + backward in a row, us, early / in order: head_dim 128 B1 H16/4 T2048 114 / 116, B4 T512 61.3 / 62.7, B3 T2048 296 / 296, B4
+// 371 / 363, B5 454 / 459, B8 751 / 719, B32 T512 348 / 332, B64 T256 274 / 261; head_dim 64 B4 H12/4 T1024 68 / 72, B8 H16/4 T2048 425 / 419,
+// B64 T512 397 / 392, B8 H12/4 T4096 1127 / 1130.
+template <typename... K, typename... A>
+static inline void nnb_launch_pre_pass(long long values, void (*kernel)(K...), unsigned blocks, unsigned threads, cudaStream_t st, const A&... args) {
+  if (values < (1ll << 24)) nnb_launch(kernel, blocks, threads, 0, st, args...);
+  else kernel<<<blocks, threads, 0, st>>>(static_cast<K>(args)...);
+}
+
 // Optional phase timers (clock64) of one thread of CTA (0,0,0); compiled in only with -DNNB_PROFILE.
 #ifdef NNB_PROFILE
 static __device__ unsigned long long g_flash_prof[8];

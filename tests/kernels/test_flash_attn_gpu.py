@@ -190,3 +190,8 @@ def test_backward_whose_key_tiles_are_shared_by_two_ctas(B, T, H, KVH, hd):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert _lib.lib().nnb_flash_bwd_split(T, 128 if hd == 64 else 64, ctypes.c_longlong(B * KVH), H // KVH, sms) == 2
     test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, H, KVH, torch.bfloat16, hd)
+
+
+@pytest.mark.parametrize("B,T,hd", [(32, 255, 128), (32, 256, 128), (64, 255, 64), (64, 256, 64)])
+def test_backward_on_both_sides_of_the_size_from_which_its_pre_pass_is_launched_in_order(B, T, hd):
+    test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, 16, 4, torch.float16, hd)
