@@ -82,13 +82,17 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def build_native(force: bool = False) -> Path:
-    """The C++ binding (binding.cpp) against the torch of this interpreter, next to the modules that use it."""
+    """The C++ binding (binding.cpp) against the torch of this interpreter, next to the modules that use it. Built again when that
+    is another interpreter or torch than the last time."""
     import sysconfig
 
+    import torch
     from torch.utils import cpp_extension
 
-    src, out = HERE / "binding.cpp", NATIVE
-    if force or _stale(out, [src]):
+    src, out, stamp = HERE / "binding.cpp", NATIVE, HERE / "build" / "native.against"
+    against = f"python {sys.version} torch {torch.__version__} {torch.__file__}"
+    if force or _stale(out, [src]) or not stamp.exists() or stamp.read_text() != against:
+        stamp.unlink(missing_ok=True)
         include = [*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"]]
         lib_dirs = cpp_extension.library_paths("cuda")
         cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_native",
@@ -97,6 +101,8 @@ def build_native(force: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"binding.cpp failed:\n{r.stdout}\n{r.stderr}")
+        stamp.parent.mkdir(exist_ok=True)
+        stamp.write_text(against)
     return out
 
 

@@ -48,7 +48,11 @@ def lib():
 def native():
     """The C++ binding (csrc/binding.cpp): raw launches and operators that run without Python in between."""
     lib()  # (says how to build it when it is missing)
-    binding = importlib.import_module("nanonemo_b200.ops._native")
+    try:
+        binding = importlib.import_module("nanonemo_b200.ops._native")
+    except ImportError as e:
+        raise RuntimeError(f"nanonemo_b200/ops/_native.so is missing or was built against another torch ({e}): build it with "
+                           "`python -m nanonemo_b200.csrc.build` (the sm100 operators have no fallback)") from e
     importlib.import_module("nanonemo_b200.ops.library")  # the operators that its backward nodes look up by name
     return binding
 
