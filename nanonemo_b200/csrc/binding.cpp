@@ -53,7 +53,7 @@ int nnb_rope_packed(const void*, void*, const void*, const void*, long long, int
 int nnb_swiglu_fwd(const void*, const void*, void*, long long, int, long long, long long, long long, int, cudaStream_t);
 int nnb_swiglu_bwd(const void*, const void*, const void*, void*, void*, long long, int, long long, long long, long long, long long, long long, int, cudaStream_t);
 int nnb_flash_fwd(const void*, const void*, const void*, void*, void*, int, int, int, int, int, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, float, int, void*, cudaStream_t);
-int nnb_flash_bwd(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, void*, int, int, int, int, int, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, float, int, const void*, const void*, void*, cudaStream_t);
+int nnb_flash_bwd(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, void*, int, int, int, int, int, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, long long, float, int, const void*, const void*, int, void*, cudaStream_t);
 }
 
 namespace {
@@ -247,14 +247,14 @@ Tensor flash_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor
   return lse;
 }
 void flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& dout, const Tensor& dq, const Tensor& dk, const Tensor& dv, double scale,
-               const optional<Tensor>& cos, const optional<Tensor>& sin) {
+               const optional<Tensor>& cos, const optional<Tensor>& sin, bool in_order) {
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), hd = q.size(3), KVH = k.size(2);
   const int code = attention_code({&q, &k, &v, &o, &dout, &dq, &dk, &dv});
   const Tensor delta = empty({B, H, T}, at::kFloat, q);     // rowsum(dO * O), computed by the launcher's pre-pass
   const Tensor dq_acc = empty({B, T, H, hd}, at::kFloat, q);  // cleared by the pre-pass
   launched(nnb_flash_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(), dq.data_ptr(), dk.data_ptr(),
                          dv.data_ptr(), (int)B, (int)T, (int)H, (int)KVH, (int)hd, NNB_STRIDES(q), NNB_STRIDES(k), NNB_STRIDES(v), NNB_STRIDES(o), NNB_STRIDES(dout), NNB_STRIDES(dq),
-                         NNB_STRIDES(dk), NNB_STRIDES(dv), (float)scale, code, cos ? cos->data_ptr() : nullptr, sin ? sin->data_ptr() : nullptr, status_of(q), stream()),
+                         NNB_STRIDES(dk), NNB_STRIDES(dv), (float)scale, code, cos ? cos->data_ptr() : nullptr, sin ? sin->data_ptr() : nullptr, in_order, status_of(q), stream()),
            "nnb_flash_bwd");
 }
 
@@ -536,7 +536,7 @@ struct FlashAttnFn : torch::autograd::Function<FlashAttnFn> {
     }
     const Tensor qt = bthd(s[0]), kt = bthd(s[1]), vt = bthd(s[2]), ot = bthd(s[3]), dt = bthd(dout);
     const Tensor dq = empty(qt.sizes(), qt.scalar_type(), qt), dk = empty(kt.sizes(), qt.scalar_type(), qt), dv = empty(vt.sizes(), qt.scalar_type(), qt);
-    flash_bwd(qt, kt, vt, ot, s[4], dt, dq, dk, dv, 1.0 / std::sqrt((double)qt.size(3)), std::nullopt, std::nullopt);
+    flash_bwd(qt, kt, vt, ot, s[4], dt, dq, dk, dv, 1.0 / std::sqrt((double)qt.size(3)), std::nullopt, std::nullopt, false);
     return {dq.transpose(1, 2), dk.transpose(1, 2), dv.transpose(1, 2)};
   }
 };
@@ -598,9 +598,9 @@ struct QKVRopeAttentionFn : torch::autograd::Function<QKVRopeAttentionFn> {
     const double scale = 1.0 / std::sqrt((double)hd);
     const char* route = std::getenv("NANONEMO_FLASH_BWD");
     if (hd == 64 && !(route && route[0] == 't')) {  // this backward kernel un-rotates dQ and dK itself
-      flash_bwd(p.q, p.k, p.v, o, lse, dout, d.q, d.k, d.v, scale, cos, sin);
+      flash_bwd(p.q, p.k, p.v, o, lse, dout, d.q, d.k, d.v, scale, cos, sin, false);
     } else {
-      flash_bwd(p.q, p.k, p.v, o, lse, dout, d.q, d.k, d.v, scale, std::nullopt, std::nullopt);
+      flash_bwd(p.q, p.k, p.v, o, lse, dout, d.q, d.k, d.v, scale, std::nullopt, std::nullopt, false);
       rope_packed(dqkv, dqkv, cos, sin, T, H + KVH, hd, 0, -1.0);
     }
     Tensor dx, dw;

@@ -585,7 +585,7 @@ __global__ void flash_dq_convert_kernel(const float* __restrict__ acc, T16* __re
 int nnb_flash_bwd_t_impl(int hd, const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse, void* delta,
                           void* dq_acc, void* dq, void* dk, void* dv, int B, int T, int H, int KVH, const long long* qs,
                           const long long* ks, const long long* vs, const long long* os, const long long* dos, const long long* dqs,
-                          const long long* dks, const long long* dvs, float scale, int dtype, void* status, cudaStream_t st);
+                          const long long* dks, const long long* dvs, float scale, int dtype, int in_order, void* status, cudaStream_t st);
 
 #ifdef NNB_PROFILE
 extern "C" int nnb_flash_bwd_prof_read(unsigned long long* out) { return (int)cudaMemcpyFromSymbol(out, g_flash_prof, sizeof(g_flash_prof)); }
@@ -619,6 +619,8 @@ static int configure_bwd() {
 // All tensors are [B, T, heads, 64] views given by element strides (contiguous last dim), bf16 or fp16 (one dtype for all).
 // lse: fp32 [B, H, T] from the forward pass; delta: fp32 [B, H, T] scratch (written here);
 // dq_acc: fp32 [B, T, H, hd] contiguous scratch (cleared by the delta pre-pass; partial tiles are reduce-added into it).
+// in_order: dK and dV are summed in the order of the queries, one CTA a key tile, also where CTAs that share a tile and add up their parts
+// would be faster.
 // rope_cos / rope_sin: null, or fp32 [T, 32] tables: dQ and dK are then returned through the inverse rotation (head_dim 64).
 extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
                              void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int T, int H, int KVH, int hd,
@@ -627,7 +629,7 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
                              long long do_sb, long long do_st, long long do_sh, long long dq_sb, long long dq_st,
                              long long dq_sh, long long dk_sb, long long dk_st, long long dk_sh, long long dv_sb,
                              long long dv_st, long long dv_sh, float scale, int dtype, const void* rope_cos, const void* rope_sin,
-                             void* status, cudaStream_t st) {
+                             int in_order, void* status, cudaStream_t st) {
   NNB_REQUIRE(hd == HD || hd == 128, "flash_bwd: head_dim %d not supported (64, 128)", hd);
   NNB_REQUIRE(dtype == NNB_BF16 || dtype == NNB_F16, "flash_bwd: bf16 or fp16 only (dtype code %d)", dtype);
   const bool f16 = dtype == NNB_F16;
@@ -644,7 +646,7 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
     const long long dos[3] = {do_sb, do_st, do_sh}, dqs[3] = {dq_sb, dq_st, dq_sh}, dks[3] = {dk_sb, dk_st, dk_sh};
     const long long dvs[3] = {dv_sb, dv_st, dv_sh};
     return nnb_flash_bwd_t_impl(hd, q, k, v, o, d_o, lse, delta, dq_acc, dq, dk, dv, B, T, H, KVH, qs, ks, vs, os, dos, dqs, dks, dvs,
-                                scale, dtype, status, st);
+                                scale, dtype, in_order, status, st);
   }
   const CUtensorMapDataType dt = f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
@@ -688,7 +690,7 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
     if (int rc = configure_bwd<true>()) return rc;
     configured = true;
   }
-  p.split = nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
+  p.split = in_order ? 1 : nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);

@@ -541,7 +541,7 @@ template <int HD, bool F16>
 int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse, void* delta,
                  void* dq_acc, void* dq, void* dk, void* dv, int B, int T, int H, int KVH, const long long* qs, const long long* ks,
                  const long long* vs, const long long* os, const long long* dos, const long long* dqs, const long long* dks,
-                 const long long* dvs, float scale, void* status, cudaStream_t st) {
+                 const long long* dvs, float scale, int in_order, void* status, cudaStream_t st) {
   using C = Cfg<HD>;
   using T16 = typename sm100::Operand16<F16>::type;
   const CUtensorMapDataType dt = F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -580,7 +580,7 @@ int launch_bwd_t(const void* q, const void* k, const void* v, const void* o, con
     }
     configured = true;
   }
-  p.split = nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
+  p.split = in_order ? 1 : nnb_visits_split(T, BQ, (long long)KVH * B, p.group, nnb_num_sms());
   p.out[0] = dv;
   p.out[1] = dk;
   for (int i = 0; i < 3; ++i) {
@@ -607,9 +607,9 @@ extern "C" int nnb_flash_bwd_t_prof_read(unsigned long long* out) { return (int)
 int nnb_flash_bwd_t_impl(int hd, const void* q, const void* k, const void* v, const void* o, const void* d_o, const void* lse,
                          void* delta, void* dq_acc, void* dq, void* dk, void* dv, int B, int T, int H, int KVH, const long long* qs,
                          const long long* ks, const long long* vs, const long long* os, const long long* dos, const long long* dqs,
-                         const long long* dks, const long long* dvs, float scale, int dtype, void* status, cudaStream_t st) {
+                         const long long* dks, const long long* dvs, float scale, int dtype, int in_order, void* status, cudaStream_t st) {
 #define NNB_BWD_T(HD_, F16_) \
-  launch_bwd_t<HD_, F16_>(q, k, v, o, d_o, lse, delta, dq_acc, dq, dk, dv, B, T, H, KVH, qs, ks, vs, os, dos, dqs, dks, dvs, scale, status, st)
+  launch_bwd_t<HD_, F16_>(q, k, v, o, d_o, lse, delta, dq_acc, dq, dk, dv, B, T, H, KVH, qs, ks, vs, os, dos, dqs, dks, dvs, scale, in_order, status, st)
   const bool f16 = dtype == NNB_F16;
   if (hd == 64) return f16 ? NNB_BWD_T(64, true) : NNB_BWD_T(64, false);
   return f16 ? NNB_BWD_T(128, true) : NNB_BWD_T(128, false);

@@ -93,6 +93,9 @@ class Attention(nn.Module):
         self.rope_impl, self.attn_impl = r.rope_kernel, r.attn_kernel
         # one autograd node for projection + RoPE (GEMM epilogue) + attention when all three run on the sm100 kernels
         self.fused = cfg.fuse_epilogues and r.linear_impl == "sm100" and self.rope_impl == "sm100" and self.attn_impl == "sm100"
+        # Block-scaled products turn a last-bit difference into another 3-bit mantissa, and every product of a backward pass does so again:
+        # they get gradients whose sums do not depend on how a call is split over the GPU.
+        self.in_order = r.linear_impl == "mxfp8"
         self.tp = None  # parallel.tp.TPContext once the model has been sharded
 
     def split_qkv(self):
@@ -139,7 +142,7 @@ class Attention(nn.Module):
             # launch, attention reads Q/K/V heads from it through strides and each query head
             # reads its own KV head directly (no repeat_interleave, no transposes).
             qkv = ops.rope_qkv(qkv, cos, sin, H, KVH, hd, impl=self.rope_impl)
-            y = ops.attention_packed(qkv, H, KVH, hd, impl=self.attn_impl, backend=self.backend)
+            y = ops.attention_packed(qkv, H, KVH, hd, impl=self.attn_impl, backend=self.backend, in_order=self.in_order)
             return self.wo(y) if project else y
         q, k, v = qkv.split((self.q_dim, self.kv_dim, self.kv_dim), dim=-1)
         q = apply_rope(q.view(B, T, H, hd).transpose(1, 2), cos, sin)

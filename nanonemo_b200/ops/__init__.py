@@ -161,8 +161,9 @@ def apply_rope_qk(q, k, cos, sin, impl="torch"):
     return out[:, :H * hd].reshape(B, T, H, hd), out[:, H * hd:].reshape(B, T, KVH, hd)
 
 
-def attention_packed(qkv, n_heads, n_kv_heads, head_dim, impl="torch", backend=SDPBackend.MATH):
-    """Causal GQA attention on a packed (B, T, (H + 2 KVH) hd) projection -> (B, T, H hd)."""
+def attention_packed(qkv, n_heads, n_kv_heads, head_dim, impl="torch", backend=SDPBackend.MATH, in_order=False):
+    """Causal GQA attention on a packed (B, T, (H + 2 KVH) hd) projection -> (B, T, H hd). `in_order` (sm100): the backward pass sums dK and
+    dV in the order of the queries at every size, see ``attention.bwd_raw``."""
     B, T, _ = qkv.shape
     qd, kd = n_heads * head_dim, n_kv_heads * head_dim
     if impl == "torch":
@@ -175,10 +176,10 @@ def attention_packed(qkv, n_heads, n_kv_heads, head_dim, impl="torch", backend=S
     from nanonemo_b200.ops import direct, library
 
     if qkv.dtype not in _ATTN_DTYPES:  # the attention kernels take 16-bit operands: fp32 inputs go through bf16 and back
-        return attention_packed(qkv.to(torch.bfloat16), n_heads, n_kv_heads, head_dim, impl, backend).to(qkv.dtype)
+        return attention_packed(qkv.to(torch.bfloat16), n_heads, n_kv_heads, head_dim, impl, backend, in_order).to(qkv.dtype)
     if direct.ENABLED:
-        return direct.flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim)
-    return library.flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim)[0]
+        return direct.flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim, in_order)
+    return library.flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim, in_order)[0]
 
 
 def flash_attn(q, k, v, impl="sm100"):

@@ -99,7 +99,7 @@ _SIGNATURES = {
     "nnb_build_arch": "",
     "nnb_flash_bwd_registers": "i",
     "nnb_flash_bwd_split": "iiqii",
-    "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfipppp",
+    "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfippipp",
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
     "nnb_gemm_swiglu": "ppppiiiqqqqipp",

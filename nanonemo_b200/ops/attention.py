@@ -18,7 +18,8 @@ def fwd_raw(q, k, v, o, scale):
     return _lib.native().flash_fwd(q, k, v, o, scale)
 
 
-def bwd_raw(q, k, v, o, lse, do, dq, dk, dv, scale, rope_cos=None, rope_sin=None):
+def bwd_raw(q, k, v, o, lse, do, dq, dk, dv, scale, rope_cos=None, rope_sin=None, in_order=False):
     """With `rope_cos` / `rope_sin` (fp32 [T, hd / 2], head_dim 64 only) dQ and dK are returned through the inverse RoPE,
-    i.e. as gradients of the projection BEFORE the rotation that produced q and k."""
-    _lib.native().flash_bwd(q, k, v, o, lse, do, dq, dk, dv, scale, rope_cos, rope_sin)
+    i.e. as gradients of the projection BEFORE the rotation that produced q and k. `in_order`: dK and dV are one sum in the order of
+    the queries, whatever the size of the call (small calls otherwise add up the parts of two or four CTAs)."""
+    _lib.native().flash_bwd(q, k, v, o, lse, do, dq, dk, dv, scale, rope_cos, rope_sin, in_order)

@@ -73,7 +73,7 @@ def _split(t, B, T, H, KVH, hd):
 
 class _FlashPacked(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, qkv, H, KVH, hd):
+    def forward(ctx, qkv, H, KVH, hd, in_order):
         B, T, _ = qkv.shape
         qkv = qkv if qkv.is_contiguous() else qkv.contiguous()
         q, k, v = _split(qkv, B, T, H, KVH, hd)
@@ -81,19 +81,19 @@ class _FlashPacked(torch.autograd.Function):
         scale = 1.0 / math.sqrt(hd)
         lse = attention.fwd_raw(q, k, v, o, scale)
         ctx.save_for_backward(qkv, o, lse)
-        ctx.meta = (H, KVH, hd, scale)
+        ctx.meta = (H, KVH, hd, scale, in_order)
         return o.view(B, T, H * hd)
 
     @staticmethod
     def backward(ctx, do):
         qkv, o, lse = ctx.saved_tensors
-        H, KVH, hd, scale = ctx.meta
+        H, KVH, hd, scale, in_order = ctx.meta
         B, T, _ = qkv.shape
         do = do.reshape(B, T, H, hd)
         do = do if do.stride(-1) == 1 and do.dtype == qkv.dtype else do.to(qkv.dtype).contiguous()
         dqkv = torch.empty_like(qkv)
-        attention.bwd_raw(*_split(qkv, B, T, H, KVH, hd), o, lse, do, *_split(dqkv, B, T, H, KVH, hd), scale)
-        return dqkv, None, None, None
+        attention.bwd_raw(*_split(qkv, B, T, H, KVH, hd), o, lse, do, *_split(dqkv, B, T, H, KVH, hd), scale, in_order=in_order)
+        return dqkv, None, None, None, None
 
 
 def swiglu_packed(gu):
@@ -104,5 +104,5 @@ def rope_qkv(qkv, cos, sin, n_heads, n_kv_heads, head_dim):
     return _RopeQKV.apply(qkv, cos, sin, n_heads, n_kv_heads, head_dim)
 
 
-def flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim):
-    return _FlashPacked.apply(qkv, n_heads, n_kv_heads, head_dim)
+def flash_attn_packed(qkv, n_heads, n_kv_heads, head_dim, in_order=False):
+    return _FlashPacked.apply(qkv, n_heads, n_kv_heads, head_dim, in_order)

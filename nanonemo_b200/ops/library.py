@@ -12,7 +12,7 @@ here too under create_graph=True and for batched gradients. All routes call the 
     torch.ops.nanonemo_b200.add_rms_norm(x, delta, weight, eps)              -> (y, h, rstd)
     torch.ops.nanonemo_b200.swiglu(gu)                                       -> act
     torch.ops.nanonemo_b200.rope_qkv(qkv, cos, sin, H, KVH, hd, sign)        -> qkv_rot
-    torch.ops.nanonemo_b200.flash_attn_packed(qkv, H, KVH, hd)               -> (o, lse)
+    torch.ops.nanonemo_b200.flash_attn_packed(qkv, H, KVH, hd, in_order)     -> (o, lse)
     torch.ops.nanonemo_b200.matmul_nt(a, b, a_mn, b_mn, out_f32)             -> a @ b^T
     torch.ops.nanonemo_b200.linear_w(x2, weight)                             -> x2 @ weight^T (fp32 or 16-bit weight)
     torch.ops.nanonemo_b200.gemm_rope(x2, weight, cos, sin, T, cols, hd)     -> projection with RoPE in the epilogue
@@ -196,7 +196,8 @@ def _split(qkv, H, KVH, hd):
 
 
 @_operator
-def flash_attn_packed(qkv: Tensor, n_heads: int, n_kv_heads: int, head_dim: int) -> tuple[Tensor, Tensor]:
+def flash_attn_packed(qkv: Tensor, n_heads: int, n_kv_heads: int, head_dim: int, in_order: bool = False) -> tuple[Tensor, Tensor]:
+    """`in_order` is of the backward pass (``attention.bwd_raw``)."""
     qkv = qkv.contiguous()
     B, T, _ = qkv.shape
     q, k, v = _split(qkv, n_heads, n_kv_heads, head_dim)
@@ -206,37 +207,38 @@ def flash_attn_packed(qkv: Tensor, n_heads: int, n_kv_heads: int, head_dim: int)
 
 
 @_fake(flash_attn_packed)
-def _(qkv, n_heads, n_kv_heads, head_dim):
+def _(qkv, n_heads, n_kv_heads, head_dim, in_order=False):
     B, T, _ = qkv.shape
     return qkv.new_empty((B, T, n_heads * head_dim)), qkv.new_empty((B, n_heads, T), dtype=torch.float32)
 
 
 @_operator
-def flash_attn_packed_bwd(do: Tensor, qkv: Tensor, o: Tensor, lse: Tensor, n_heads: int, n_kv_heads: int, head_dim: int) -> Tensor:
+def flash_attn_packed_bwd(do: Tensor, qkv: Tensor, o: Tensor, lse: Tensor, n_heads: int, n_kv_heads: int, head_dim: int, in_order: bool = False) -> Tensor:
     qkv, do = qkv.contiguous(), do.contiguous()
     B, T, _ = qkv.shape
     q, k, v = _split(qkv, n_heads, n_kv_heads, head_dim)
     dqkv = torch.empty_like(qkv)
     dq, dk, dv = _split(dqkv, n_heads, n_kv_heads, head_dim)
-    attention.bwd_raw(q, k, v, o.view(B, T, n_heads, head_dim), lse, do.view(B, T, n_heads, head_dim), dq, dk, dv, 1.0 / math.sqrt(head_dim))
+    attention.bwd_raw(q, k, v, o.view(B, T, n_heads, head_dim), lse, do.view(B, T, n_heads, head_dim), dq, dk, dv, 1.0 / math.sqrt(head_dim),
+                      in_order=in_order)
     return dqkv
 
 
 @_fake(flash_attn_packed_bwd)
-def _(do, qkv, o, lse, n_heads, n_kv_heads, head_dim):
+def _(do, qkv, o, lse, n_heads, n_kv_heads, head_dim, in_order=False):
     return torch.empty_like(qkv, memory_format=torch.contiguous_format)
 
 
 def _fa_setup(ctx, inputs, output):
-    qkv, H, KVH, hd = inputs
+    qkv, H, KVH, hd, in_order = inputs
     o, lse = output
     ctx.save_for_backward(qkv, o, lse)
-    ctx.meta = (H, KVH, hd)
+    ctx.meta = (H, KVH, hd, in_order)
 
 
 def _fa_backward(ctx, do, _dlse):
     qkv, o, lse = ctx.saved_tensors
-    return _from_formula(flash_attn_packed_bwd, do, qkv, o, lse, *ctx.meta), None, None, None
+    return _from_formula(flash_attn_packed_bwd, do, qkv, o, lse, *ctx.meta), None, None, None, None
 
 
 _autograd(flash_attn_packed, _fa_backward, setup_context=_fa_setup)

@@ -195,3 +195,28 @@ def test_backward_whose_key_tiles_are_shared_by_two_ctas(B, T, H, KVH, hd):
 @pytest.mark.parametrize("B,T,hd", [(32, 255, 128), (32, 256, 128), (64, 255, 64), (64, 256, 64)])
 def test_backward_on_both_sides_of_the_size_from_which_its_pre_pass_is_launched_in_order(B, T, hd):
     test_backward_whose_key_tiles_are_shared_by_several_ctas(B, T, 16, 4, torch.float16, hd)
+
+
+@pytest.mark.parametrize("H,KVH,T,hd", [(12, 4, 333, 64), (6, 1, 1000, 64), (16, 4, 333, 128)])
+@pytest.mark.parametrize("direct_route", [False, True])
+def test_packed_attention_in_order_sums_a_sequence_the_same_way_in_calls_of_any_size(monkeypatch, H, KVH, T, hd, direct_route):
+    """dK and dV of one sequence alone, where key tiles would be shared, against the same sequence in a batch that fills the GPU."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.ops import _lib, direct
+
+    monkeypatch.setattr(direct, "ENABLED", direct_route)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = -(-2 * sms // (KVH * -(-T // 128)))
+    split = lambda b: _lib.lib().nnb_flash_bwd_split(T, 128 if hd == 64 else 64, ctypes.c_longlong(b * KVH), H // KVH, sms)  # noqa: E731
+    assert split(1) > 1 == split(B)
+    torch.manual_seed(T)
+    qkv, do = torch.randn(B, T, (H + 2 * KVH) * hd, device=DEV).bfloat16(), torch.randn(B, T, H * hd, device=DEV).bfloat16()
+
+    def grad(b, in_order):
+        x = qkv[:b].clone().requires_grad_()
+        (g,) = torch.autograd.grad(ops.attention_packed(x, H, KVH, hd, impl="sm100", in_order=in_order), x, do[:b])
+        return g[0, :, H * hd:]
+
+    full, alone, shared = grad(B, True), grad(1, True), grad(1, False)
+    assert torch.equal(alone, full)
+    assert (shared.float() - full.float()).norm() <= 2 ** -8 * full.float().norm()  # (two roundings to 16 bits of the same sums)
