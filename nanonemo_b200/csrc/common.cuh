@@ -46,7 +46,7 @@ static inline int nnb_num_sms() {
 // it, has finished and its writes are visible. A kernel lets its successor in with nnb_release_next() when its own work is nearly
 // handed out, not earlier: blocks that wait hold their SM's resources, which kernels of other streams may want.
 // An eager step of the 114M model in two micro-batches of 4096 tokens is 574 launches with 1.7 us of idle GPU before each: 12.0 ms
-// in plain launches, 11.1 in these (8192 tokens in fp8: 11.6 and 11.1).
+// in plain launches, 11.1 in these (8192 tokens in fp8: 11.6 and 11.1). Not every kernel gains: see nnb_launch_pre_pass.
 // `cluster`: CTAs of a cluster along x, 1 for a kernel without clusters (or with its own __cluster_dims__).
 template <typename... K, typename... A>
 static inline void nnb_launch_clusters(void (*kernel)(K...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
