@@ -98,6 +98,12 @@ Tensor status_tensor(int device) {
 }
 void* status_of(const Tensor& like) { return status_tensor(like.get_device()).data_ptr(); }
 
+// A kernel that is given pageable host memory faults, and the context is lost.
+void reachable(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->defined() && !t->is_cuda() && !(t->is_cpu() && t->is_pinned())) throw AssertionFailed("the GPU cannot reach an operand on " + t->device().str());
+}
+
 int code_of(at::ScalarType t) {  // -1: no operand format of the kernels
   return t == at::kFloat ? 0 : t == at::kBFloat16 ? 1 : t == at::kHalf ? 2 : -1;
 }
@@ -122,6 +128,8 @@ Tensor empty(at::IntArrayRef size, at::ScalarType dt, const Tensor& like) { retu
 Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, const optional<Tensor>& out_, optional<at::ScalarType> out_dtype, bool accumulate, int k_splits, int bn, int max_ctas) {
   a = rowmajor2d(std::move(a));
   b = rowmajor2d(std::move(b));
+  reachable({&a, &b});
+  if (out_ && out_->defined()) reachable({&a, &*out_});
   NNB_ASSERT(a.scalar_type() == b.scalar_type() && code16(a.scalar_type()) > 0,
              std::string("gemm needs matching bf16/fp16 inputs, got ") + c10::toString(a.scalar_type()) + "/" + c10::toString(b.scalar_type()));
   const int64_t K = a_mn ? a.size(0) : a.size(1), M = a_mn ? a.size(1) : a.size(0);
@@ -141,6 +149,7 @@ Tensor gemm_nt(const Tensor& a, const Tensor& b, bool b_mn = false) { return gem
 
 // x2 [M, K] @ w_gu [2 F, K]^T -> (gu, act), (undefined, act) without `keep`, or two undefined tensors where the CTA-pair kernel does not serve the shape
 std::pair<Tensor, Tensor> gemm_swiglu(const Tensor& x2, const Tensor& w, bool keep) {
+  reachable({&x2, &w});
   const int64_t M = x2.size(0), K = x2.size(1), F = w.size(0) / 2;
   if (M < 256 || F % 128 || w.stride(1) != 1 || x2.stride(1) != 1) return {};
   Tensor gu = keep ? empty({M, 2 * F}, x2.scalar_type(), x2) : Tensor(), act = empty({M, F}, x2.scalar_type(), x2);
@@ -155,6 +164,7 @@ std::pair<Tensor, Tensor> gemm_swiglu(const Tensor& x2, const Tensor& w, bool ke
 }
 
 Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
+  reachable({&dy, &w, &gu});
   const int64_t M = dy.size(0), K = dy.size(1), F = w.size(1);
   if (M < 256 || F < 128 || F % 64 || gu.dim() != 2 || gu.size(0) != M || gu.size(1) != 2 * F || gu.stride(1) != 1 || gu.stride(0) % 8 || w.stride(1) != 1 ||
       dy.stride(1) != 1 || gu.scalar_type() != dy.scalar_type() || w.scalar_type() != dy.scalar_type())
@@ -167,6 +177,7 @@ Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
 }
 
 Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
+  reachable({&x2, &w, &cos, &sin});
   const int64_t M = x2.size(0), K = x2.size(1), N = w.size(0);
   if (M < 256 || N < 128 || (hd != 64 && hd != 128) || N % hd || rope_cols % hd) return Tensor();
   const int code = code16(x2.scalar_type());
@@ -177,13 +188,16 @@ Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Ten
 }
 
 void rope_packed(const Tensor& x2, const Tensor& out2, const Tensor& cos, const Tensor& sin, int64_t T, int64_t n_rot, int64_t hd, int64_t n_copy, double sign) {
+  reachable({&x2, &out2, &cos, &sin});
   launched(nnb_rope_packed(x2.data_ptr(), out2.data_ptr(), cos.data_ptr(), sin.data_ptr(), x2.size(0), (int)T, (int)n_rot, (int)hd, (int)n_copy, x2.stride(0), out2.stride(0),
                            (float)sign, code_any(x2), stream()), "nnb_rope_packed");
 }
 void swiglu_fwd(const Tensor& g, const Tensor& u, const Tensor& out) {
+  reachable({&g, &u, &out});
   launched(nnb_swiglu_fwd(g.data_ptr(), u.data_ptr(), out.data_ptr(), out.size(0), (int)out.size(1), g.stride(0), u.stride(0), out.stride(0), code_any(out), stream()), "nnb_swiglu_fwd");
 }
 void swiglu_bwd(const Tensor& dy, const Tensor& g, const Tensor& u, const Tensor& dg, const Tensor& du) {
+  reachable({&dy, &g, &u, &dg, &du});
   launched(nnb_swiglu_bwd(dy.data_ptr(), g.data_ptr(), u.data_ptr(), dg.data_ptr(), du.data_ptr(), dy.size(0), (int)dy.size(1), dy.stride(0), g.stride(0), u.stride(0), dg.stride(0),
                           du.stride(0), code_any(dy), stream()), "nnb_swiglu_bwd");
 }
@@ -194,6 +208,7 @@ std::tuple<Tensor, Tensor, Tensor> rms_fwd(const Tensor& x, const optional<Tenso
   Tensor x2 = x.reshape({-1, N}).contiguous(), d2;
   if (delta && delta->defined()) d2 = delta->reshape({-1, N}).contiguous();
   const int64_t M = x2.size(0);
+  reachable({&x2, &d2, &weight});
   const Tensor w = as_dtype(weight, at::kFloat);
   Tensor y = empty({M, N}, y_dt, x), h = d2.defined() ? empty({M, N}, x2.scalar_type(), x) : x2, rstd = empty({M}, at::kFloat, x);
   const int y_code = code_any(y);
@@ -210,6 +225,8 @@ std::tuple<Tensor, Tensor, Tensor> rms_bwd(const Tensor& dy, const Tensor& h, co
   const int64_t M = h2.size(0);
   Tensor dr2;
   if (dres && dres->defined()) dr2 = as_dtype(dres->reshape({-1, N}).contiguous(), h2.scalar_type());
+  reachable({&h2, &dy2, &dr2, &rstd, &weight});
+  if (dw_out && dw_out->defined()) reachable({&h2, &*dw_out});
   const Tensor w = as_dtype(weight, at::kFloat);
   Tensor dx = at::empty_like(h2), ddelta;
   if (delta_dt && *delta_dt != h2.scalar_type()) ddelta = empty({M, N}, *delta_dt, h);
@@ -240,6 +257,7 @@ int attention_code(std::initializer_list<const Tensor*> ts) {
 // q, o: [B, T, H, hd] views; k, v: [B, T, KVH, hd] views
 Tensor flash_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, double scale) {
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), hd = q.size(3), KVH = k.size(2);
+  reachable({&q, &k, &v, &o});
   const int code = attention_code({&q, &k, &v, &o});
   Tensor lse = empty({B, H, T}, at::kFloat, q);
   launched(nnb_flash_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), (int)B, (int)T, (int)H, (int)KVH, (int)hd, NNB_STRIDES(q), NNB_STRIDES(k), NNB_STRIDES(v),
@@ -249,6 +267,8 @@ Tensor flash_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor
 void flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& dout, const Tensor& dq, const Tensor& dk, const Tensor& dv, double scale,
                const optional<Tensor>& cos, const optional<Tensor>& sin, bool in_order) {
   const int64_t B = q.size(0), T = q.size(1), H = q.size(2), hd = q.size(3), KVH = k.size(2);
+  reachable({&q, &k, &v, &o, &lse, &dout, &dq, &dk, &dv});
+  if (cos && sin) reachable({&q, &*cos, &*sin});
   const int code = attention_code({&q, &k, &v, &o, &dout, &dq, &dk, &dv});
   const Tensor delta = empty({B, H, T}, at::kFloat, q);     // rowsum(dO * O), computed by the launcher's pre-pass
   const Tensor dq_acc = empty({B, T, H, hd}, at::kFloat, q);  // cleared by the pre-pass
@@ -260,6 +280,7 @@ void flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& 
 
 // MXFP8: quantised copies (see nanonemo_b200/fp8) and the block-scaled product
 std::tuple<Tensor, Tensor, Tensor, Tensor> quantize_mx(const Tensor& x, bool rowwise, bool colwise) {
+  reachable({&x});
   NNB_ASSERT(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quantize_mx takes bf16 rows");
   const int64_t R = x.size(0), C = x.size(1), scales = (R / 128) * (C / 128) * 512;
   Tensor q, sf, qt, sft;
@@ -270,6 +291,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> quantize_mx(const Tensor& x, bool row
   return {q, sf, qt, sft};
 }
 Tensor gemm_mxfp8(const Tensor& aq, const Tensor& asf, const Tensor& bq, const Tensor& bsf, const optional<Tensor>& out_, at::ScalarType out_dtype, bool accumulate, int k_splits) {
+  reachable({&aq, &asf, &bq, &bsf});
+  if (out_ && out_->defined()) reachable({&aq, &*out_});
   const int64_t M = aq.size(0), K = aq.size(1), N = bq.size(0);
   NNB_ASSERT(bq.size(1) == K && aq.scalar_type() == at::kByte && bq.scalar_type() == at::kByte, "gemm_mxfp8: operands do not fit");
   const bool given = out_.has_value() && out_->defined();

@@ -172,6 +172,13 @@ def ptr(t: torch.Tensor | None) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def reachable(*tensors: torch.Tensor) -> None:
+    """A kernel that is given pageable host memory faults, and the context is lost."""
+    for t in tensors:
+        if not t.is_cuda and not (t.device.type == "cpu" and t.is_pinned()):
+            raise AssertionError(f"the GPU cannot reach an operand on {t.device}")
+
+
 i32 = i64 = operator.index  # an integer, as it is (anything else raises)
 f32 = float
 

@@ -19,6 +19,7 @@ def fwd_raw(idx, weight, out_dtype):
     flat = idx.reshape(-1)
     flat = flat if flat.dtype == torch.int64 else flat.long()
     flat = flat if flat.is_contiguous() else flat.contiguous()
+    _lib.reachable(flat, weight)
     V, D = weight.shape
     out = torch.empty((flat.numel(), D), dtype=out_dtype, device=weight.device)
     _lib.call("nnb_embedding_fwd", _lib.ptr(flat), _lib.ptr(weight), _lib.ptr(out), _lib.i64(flat.numel()), _lib.i32(D),
@@ -27,6 +28,7 @@ def fwd_raw(idx, weight, out_dtype):
 
 
 def bwd_raw(flat_idx, dout, dW):
+    _lib.reachable(flat_idx, dout, dW)
     V, D = dW.shape
     d2 = dout.reshape(-1, D)
     d2 = d2 if d2.is_contiguous() else d2.contiguous()

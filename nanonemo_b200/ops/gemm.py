@@ -89,6 +89,7 @@ def gemm_ce_stats(x2: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
     N = w.shape[0]
     if M < 256 or N < 128 or N % 64:
         return None
+    _lib.reachable(x2, w, out)
     stats = torch.empty((M, 2 * ((N + 255) // 256), 2), dtype=torch.float32, device=x2.device)
     ok = _fused_call("nnb_gemm_ce_stats", _lib.ptr(x2), _lib.ptr(w), _lib.ptr(out), _lib.ptr(stats), _lib.i32(M), _lib.i32(N),
                      _lib.i32(K), _lib.i64(x2.stride(0)), _lib.i64(w.stride(0)), _lib.i64(out.stride(0)), _lib.i32(_CODE[x2.dtype]),
@@ -103,6 +104,7 @@ def gemm_ce_loss(x2: torch.Tensor, w: torch.Tensor, targets: torch.Tensor):
     N = w.shape[0]
     if M < 256 or N < 128 or N % 64:
         return None
+    _lib.reachable(x2, w, targets)
     stats = torch.empty((M, 2 * ((N + 255) // 256), 2), dtype=torch.float32, device=x2.device)
     target_logit = torch.empty(M, dtype=torch.float32, device=x2.device)
     ok = _fused_call("nnb_gemm_ce_loss", _lib.ptr(x2), _lib.ptr(w), _lib.ptr(targets), _lib.ptr(stats), _lib.ptr(target_logit),

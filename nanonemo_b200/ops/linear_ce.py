@@ -21,6 +21,7 @@ DEFAULT_CHUNK_ROWS = 32768
 
 
 def ce_inplace(logits: torch.Tensor, targets: torch.Tensor, loss_rows: torch.Tensor, grad_scale: float):
+    _lib.reachable(logits, targets, loss_rows)
     R, V = logits.shape
     _lib.call("nnb_ce_inplace", _lib.ptr(logits), _lib.ptr(targets), _lib.ptr(loss_rows), _lib.i64(R), _lib.i32(V),
               _lib.i64(logits.stride(0)), _lib.f32(grad_scale), _lib.i32(_CODE[logits.dtype]), _lib.vp(_lib.stream_ptr()))
@@ -28,6 +29,7 @@ def ce_inplace(logits: torch.Tensor, targets: torch.Tensor, loss_rows: torch.Ten
 
 def ce_from_stats(logits: torch.Tensor, targets: torch.Tensor, tile_stats: torch.Tensor, loss_rows: torch.Tensor, grad_scale: float):
     """One-sweep form of `ce_inplace`: `tile_stats` [R, n_tiles, 2] came out of the head GEMM's epilogue (gemm_ce_stats)."""
+    _lib.reachable(logits, targets, tile_stats, loss_rows)
     R, V = logits.shape
     _lib.call("nnb_ce_grad_from_stats", _lib.ptr(logits), _lib.ptr(targets), _lib.ptr(tile_stats), _lib.i32(tile_stats.shape[1]),
               _lib.ptr(loss_rows), _lib.i64(R), _lib.i32(V), _lib.i64(logits.stride(0)), _lib.f32(grad_scale),
