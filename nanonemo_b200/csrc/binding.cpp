@@ -420,9 +420,11 @@ std::vector<int64_t> with_last(at::IntArrayRef sizes, int64_t last) {
 }
 
 // ------------------------------------------------------------------------------------------------ operators
+// x: any shape and dtype where the engine's weight is (nothing differentiates its gradients); otherwise the 16-bit rows, made before the
+// node, so that its saved tensor leads back to the caller's input under create_graph.
 struct LinearFn : torch::autograd::Function<LinearFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& w16, bool engine) {
-    const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), w16.scalar_type()));
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& w16, bool engine, const std::vector<int64_t>& y_sizes) {
+    const Tensor x2 = engine ? rowmajor2d(as_dtype(rows2d(x), w16.scalar_type())) : x;
     Tensor y = gemm_nt(x2, w16);
     ctx->save_for_backward({x2, weight});
     if (engine) ctx->saved_data["w16"] = w16;
@@ -430,7 +432,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     ctx->saved_data["x_dtype"] = (int64_t)x.scalar_type();
     ctx->saved_data["engine"] = engine;
     ctx->saved_data["trained"] = weight.requires_grad();
-    return fresh([&] { return y.view(with_last(x.sizes(), weight.size(0))); });
+    return fresh([&] { return y.view(y_sizes); });
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
@@ -441,9 +443,9 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     const bool need_dx = ctx->needs_input_grad(0), need_dw = engine ? ctx->saved_data["trained"].toBool() : ctx->needs_input_grad(1);
     Tensor dy2 = as_dtype(rows2d(grads[0]), x2.scalar_type()), dx, dw;
     if (!engine && through_dispatcher(grads[0])) {
-      dy2 = dy2.contiguous();
-      if (need_dx) dx = call_matmul_nt(dy2, as_dtype(weight, x2.scalar_type()), false, true, false);
-      if (need_dw) dw = as_dtype(call_matmul_nt(dy2, x2, true, true, true), weight.scalar_type());
+      dy2 = dy2.contiguous();  // (both, as the registered formula has it: what it refuses to differentiate further is refused here too)
+      dx = call_matmul_nt(dy2, as_dtype(weight, x2.scalar_type()), false, true, false);
+      dw = as_dtype(call_matmul_nt(dy2, x2, true, true, true), weight.scalar_type());
     } else {
       if (engine) engine_gradient(grads[0]);
       dy2 = rowmajor2d(dy2);
@@ -451,7 +453,7 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
       if (need_dw) dw = weight_gradient(dy2, x2, weight, engine);
     }
     if (dx.defined()) dx = as_dtype(dx.view(x_sizes), x_dtype);
-    return {dx, dw, Tensor(), Tensor()};
+    return {dx, dw, Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -463,7 +465,7 @@ py::object linear(py::handle x_, py::handle weight_) {
   {
     py::gil_scoped_release nogil;
     const Tensor w16 = w.in(weight, compute_dtype());
-    y = LinearFn::apply(x, weight, w16, w.engine);
+    y = LinearFn::apply(w.engine ? x : rowmajor2d(as_dtype(rows2d(x), w16.scalar_type())), weight, w16, w.engine, with_last(x.sizes(), weight.size(0)));
   }
   return py::cast(y);
 }

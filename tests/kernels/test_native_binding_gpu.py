@@ -240,6 +240,33 @@ def test_second_derivatives_batched_gradients_and_hooks_behave_as_before(python_
         torch.autograd.grad(out, w, torch.ones_like(out))
 
 
+@pytest.mark.parametrize("make", [lambda: _rand(66, 64), lambda: _rand(2, 33, 64, dtype=torch.bfloat16), lambda: _rand(2, 33, 64), lambda: _rand(66, 70, dtype=torch.bfloat16)[:, 3:67],
+                                  lambda: _rand(66, 64, dtype=torch.bfloat16)])
+def test_second_derivatives_of_a_linear_reach_its_input_or_are_refused_as_before(python_route, make):
+    """Also where the input is cast, reshaped or copied first: what the node saves has to lead back to it."""
+    from nanonemo_b200 import ops
+
+    x, w = make().detach().requires_grad_(), _rand(72, 64)
+    frozen = w.detach()
+
+    def penalty():  # of the weight's gradient, with respect to the input
+        (dw,) = torch.autograd.grad(ops.linear(x, w, impl="sm100").float().square().sum(), w, create_graph=True)
+        return torch.autograd.grad(dw.float().square().sum(), x)[0]
+
+    def hessian():
+        return torch.autograd.functional.hvp(lambda a: ops.linear(a, frozen, impl="sm100").float().sum(), x.detach(), torch.ones_like(x))[1]
+
+    for fn in (penalty, hessian):
+        got = []
+        for run in (lambda f: f(), python_route):
+            try:
+                got.append(run(fn))
+            except (RuntimeError, AssertionError) as e:
+                got.append(type(e))
+        a, b = got
+        assert torch.allclose(a.float(), b.float(), rtol=2e-2, atol=1e-3) if isinstance(b, torch.Tensor) else a is b
+
+
 def test_outputs_may_be_changed_in_place():
     for fn, x in _cases()[:2]:  # (attention keeps its output for the backward)
         fn(x).mul_(2).float().sum().backward()
