@@ -187,7 +187,10 @@ def linear_backward(dy2, x2, weight, w16, need_dx: bool, need_dw: bool):
 
 
 def linear_sm100(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    y = _lib.operator_call("linear", x, weight)
+    """The trainer's linear. A weight that the engine does not know, too (``linear_impl: mxfp8`` outside fp8): its node takes no part in
+    second derivatives, where the native one of such a weight is the registered operators', which refuse them."""
+    engine = getattr(weight, "_main_grad", None) is not None or getattr(weight, "_shadow", None) is not None
+    y = _lib.operator_call("linear", x, weight) if engine or no_backward(x, weight) else NotImplemented
     return y if y is not NotImplemented else _Linear.apply(x, weight)
 
 

@@ -267,6 +267,26 @@ def test_second_derivatives_of_a_linear_reach_its_input_or_are_refused_as_before
         assert torch.allclose(a.float(), b.float(), rtol=2e-2, atol=1e-3) if isinstance(b, torch.Tensor) else a is b
 
 
+def test_the_trainers_linear_takes_part_in_graphs_of_gradients_as_before(python_route):
+    """Weights with and without the engine's buffers, and calls without gradients."""
+    from nanonemo_b200.ops.gemm import linear_sm100
+
+    x = _rand(66, 64, dtype=torch.bfloat16)
+    for engine in (False, True):
+        w = _rand(72, 64)
+        if engine:
+            _engine(w)
+
+        def first():
+            (dx,) = torch.autograd.grad(linear_sm100(x, w).float().sum(), x, create_graph=True)  # noqa: B023
+            return dx.detach(), dx.requires_grad
+
+        (a, a_graph), (b, b_graph) = first(), python_route(first)
+        assert torch.equal(a, b) and a_graph == b_graph
+        with torch.no_grad():
+            assert torch.equal(linear_sm100(x, w), python_route(lambda: linear_sm100(x, w)))  # noqa: B023
+
+
 def test_outputs_may_be_changed_in_place():
     for fn, x in _cases()[:2]:  # (attention keeps its output for the backward)
         fn(x).mul_(2).float().sum().backward()
