@@ -1,10 +1,10 @@
 // Causal grouped-query FlashAttention forward on tcgen05 / TMEM / TMA for sm_100a.
 //
-// One CTA owns one 128-row query tile of one (batch, query head) and walks the key/value tiles (64 keys
-// each) up to the diagonal; two CTAs are resident per SM. 192 threads per CTA:
-//   warp 0        TMA producer: Q once, then K_j / V_j into a ring of stages (4-D tensor maps over
+// An item is one 128-row query tile of one (batch, query head); a CTA walks the key/value tiles (64 keys each) of one item after
+// the other up to the diagonal; two CTAs are resident per SM. 192 threads per CTA:
+//   warp 0        TMA producer: an item's Q, then K_j / V_j into a ring of stages (4-D tensor maps over
 //                 (head_dim, head, t, batch), so any (B,T,H,hd) / (B,H,T,hd) / packed-QKV strides work and
-//                 query head h reads KV head h / group directly — nothing is repeated or copied);
+//                 query head h reads KV head h / group directly — nothing is repeated or copied); takes the next item;
 //   warp 1        MMA issuer: S_j = Q K_j^T and O_j = P_j V_j with tcgen05.mma, accumulators in TMEM;
 //   warps 2..5    softmax, one thread per query row (= TMEM lane): tcgen05.ld the scores, online max and
 //                 sum with exp2, 16-bit P_j back into tensor memory over the scores it came from (the A operand of
@@ -15,7 +15,15 @@
 // The score tile (and the P tile in it) is DOUBLE BUFFERED and the MMA warp runs two tiles ahead: S_{j+2} is
 // issued as soon as the softmax threads have read S_j, and P_j V_j runs while they work on tile j+1, so
 // neither side waits for a hand-off in steady state.
-// Outputs: O (bf16) through a swizzled staging tile + TMA store, and L = m * scale + ln(l) per row (fp32)
+// Items follow one another without a seam: the grid has one block per item, heaviest first, and a block that is running takes over
+// blocks that have not started (cluster launch control: the hardware's own order and balance, no counter in memory). The producer asks
+// when it has requested its item's last keys, loads the next item's Q and first keys while the softmax works on the last ones, and the
+// MMA warp starts the next item's first scores beside the last products, at head_dim 64 into an O accumulator of its own. With a
+// launch per item a CTA spent 4.7 us on set-up, first loads, first and last products and its store, as long as six key tiles.
+// Forward alone, back to back (the card's power limit included), us, a CTA per item / items in sequence: 12/4 heads of 64, B200 T64
+// 30.8 / 17.9, B64 T300 49.4 / 39.3, B64 T512 81.1 / 67.6, B32 T1024 112.5 / 105.5, B8 T4096 322 / 323; 16/4 heads of 128, B64 T256
+// 58.8 / 49.4, B16 T1024 105 / 99, B8 T2048 166 / 160; a grid of one wave (B2 T333) 7.0 / 7.5.
+// Outputs: O (16 bits) through a swizzled staging tile + TMA store, and L = m * scale + ln(l) per row (fp32)
 // for the backward pass. Every mbarrier wait is bounded; on expiry the kernel records a status word
 // and leaves cleanly.
 //
@@ -48,15 +56,22 @@ struct FCfg {
   static constexpr int kQBytes = BQ * HD * 2;               // HD/64 swizzled K-blocks of 16 KB
   static constexpr int kKBytes = BN * HD * 2;
   static constexpr int kVBytes = BN * HD * 2;
-  static constexpr int kSmem = kQBytes + kStages * (kKBytes + kVBytes) + 1024 + 256;
+  // Q tiles, and O accumulators in tensor memory: two where they fit twice beside the rest, so that the next item starts early
+  static constexpr int kItems = HD == 64 ? 2 : 1;
+  static constexpr int kOBytes = BQ * 128;                  // staging of 64 columns of O
+  static constexpr int kBarBytes = 512;
+  // 113 KB a CTA is what two per SM leave: nothing to spare at head_dim 128 for aligning the base, which the kernel checks instead
+  static constexpr int kSmem = kItems * kQBytes + kStages * (kKBytes + kVBytes) + kOBytes + kBarBytes;
+  static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
   static constexpr int kColS = 0;                           // S buffers at columns 0 and 64; P_j takes the first 32 of S_j's
-  static constexpr int kColO = 128;                         // O accumulator from column 128
+  static constexpr int kColO = 128;                         // O accumulators from column 128
   static constexpr int kTmemCols = 256;
 };
 
 struct FParams {
   int B, H, KVH, T;
   int n_q_tiles;
+  int take;           // the grid has more blocks than run at once: blocks take over others
   float scale_log2;   // softmax scale * log2(e)
   float scale;        // softmax scale
   float* lse;         // [B, H, T]
@@ -70,42 +85,43 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FParams p) {
   using C = FCfg<HD>;
   constexpr int BN = C::BN;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;
-  uint8_t* sKV = sQ + C::kQBytes;                              // [stages][K | V]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + C::kStages * (C::kKBytes + C::kVBytes));
-  // barriers: q_full, k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_full[2], o_tile, o_all
-  const uint32_t bar_q = smem_u32(bars);
-  const uint32_t bar_k = bar_q + 8, bar_v = bar_k + 8 * C::kStages;
+  uint8_t* sKV = sQ + C::kItems * C::kQBytes;                  // [stages][K | V]
+  uint8_t* sO = sKV + C::kStages * (C::kKBytes + C::kVBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + C::kOBytes);
+  // k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_full[2], o_tile, o_all, q_full[2], q_empty[2], o_empty[2], next_full[2], next_empty[2]
+  const uint32_t bar_k = smem_u32(bars), bar_v = bar_k + 8 * C::kStages;
   const uint32_t bar_ke = bar_v + 8 * C::kStages, bar_ve = bar_ke + 8 * C::kStages;
-  const uint32_t bar_s = bar_ve + 8 * C::kStages, bar_p = bar_s + 16, bar_o = bar_p + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 4 * C::kStages + 6);
+  const uint32_t bar_s = bar_ve + 8 * C::kStages, bar_p = bar_s + 16, bar_o = bar_p + 16, bar_of = bar_o + 8;
+  const uint32_t bar_q = bar_of + 8, bar_qe = bar_q + 16, bar_oe = bar_qe + 16, bar_nf = bar_oe + 16, bar_ne = bar_nf + 16;
+  constexpr int kBars = 4 * C::kStages + 16;
+  static_assert(kBars % 2 == 0 && kBars * 8 + 32 + 12 <= C::kBarBytes, "the answers are 16-byte aligned behind the barriers");
+  const uint32_t answers = bar_k + 8 * kBars;  // [2] of 16 bytes: which block is taken over
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* never_set = abort_flag + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Longest-job-first over the WHOLE grid: the query tile is the slowest-varying block index, so every CTA of the latest
-  // (heaviest) query tile is scheduled before any of the next one and the kernel ends on the one-key-tile CTAs.
-  const int qt = p.n_q_tiles - 1 - blockIdx.z;
-  const int h = blockIdx.x, b = blockIdx.y;
-  const int kvh = h / (p.H / p.KVH);
+  if (smem_u32(smem) & 1023) {  // (swizzled tiles: see kSmem)
+    if (threadIdx.x == 0 && p.status != nullptr && atomicCAS(p.status, 0, 2) == 0) p.status[1] = 6;
+    return;
+  }
+  // Longest-job-first over the WHOLE grid: the query tile is the slowest-varying block index, so every
+  // (heaviest) latest query tile is begun before any of the next one and the kernel ends on the short ones.
   const int kv_total = (p.T + BN - 1) / BN;
-  const int n_kv = min(((qt + 1) * BQ + BN - 1) / BN, kv_total);  // KV tiles holding keys <= the tile's last row
+  auto query_tile = [&](int z) { return p.n_q_tiles - 1 - z; };
+  auto kv_tiles = [&](int qt) { return min(((qt + 1) * BQ + BN - 1) / BN, kv_total); };  // KV tiles holding keys <= the tile's last row
+  // Item i + 1 is the answer in slot i & 1, read by the MMA warp, the four softmax warps and the producer.
+  constexpr int kNextReaders = 5;  // (not the producer, who writes the slot again)
+  auto next_item = [&](int i, int& x, int& y, int& z) { return taken_block(answers + 16 * (i & 1), x, y, z); };
 
-  if (threadIdx.x == 0) {
-    mbar_init(bar_q, 1);
-    for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(bar_k + 8 * s, 1);
-      mbar_init(bar_v + 8 * s, 1);
-      mbar_init(bar_ke + 8 * s, 1);
-      mbar_init(bar_ve + 8 * s, 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_s + 8 * i, 1);
-      mbar_init(bar_p + 8 * i, kSoftmaxThreads);
-      mbar_init(bar_o + 8 * i, 1);
-    }
-    *abort_flag = 0;
+  if (warp == 0) {  // a barrier a lane
+    static_assert(kBars <= 32, "");
+    const uint32_t bar = bar_k + 8 * lane;
+    const bool softmax = (bar >= bar_p && bar < bar_o) || (bar >= bar_oe && bar < bar_nf);
+    if (lane < kBars) mbar_init(bar, softmax ? kSoftmaxThreads : (bar >= bar_ne ? kNextReaders : 1));
+    if (lane == 0) *abort_flag = *never_set = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
@@ -129,64 +145,123 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      mbar_expect_tx(bar_q, C::kQBytes);
+      int h = blockIdx.x, b = blockIdx.y, z = blockIdx.z;
+      uint32_t s = 0, ph = 0;  // ring position and phase of the next K and V tile, counted along over all items
+      bool ok = true;
+      for (int i = 0;; ++i) {
+        const int qt = query_tile(z), kvh = h / (p.H / p.KVH), n_kv = kv_tiles(qt);
+        const int qs = i % C::kItems;
+        ok = mbar_wait(bar_qe + 8 * qs, ((i / C::kItems) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        mbar_expect_tx(bar_q + 8 * qs, C::kQBytes);
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) tma_load_4d(smem_u32(sQ) + c * (BQ * 128), &tmQ, bar_q, c * 64, h, qt * BQ, b);
-      for (int j = 0; j < n_kv; ++j) {
-        const uint32_t s = j % C::kStages, ph = (j / C::kStages) & 1;
-        if (!mbar_wait(bar_ke + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
-        const uint32_t sk = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes), sv = sk + C::kKBytes;
-        mbar_expect_tx(bar_k + 8 * s, C::kKBytes);
+        for (int c = 0; c < HD / 64; ++c) tma_load_4d(smem_u32(sQ) + qs * C::kQBytes + c * (BQ * 128), &tmQ, bar_q + 8 * qs, c * 64, h, qt * BQ, b);
+        for (int j = 0; j < n_kv && ok; ++j) {
+          const uint32_t sk = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes), sv = sk + C::kKBytes;
+          ok = mbar_wait(bar_ke + 8 * s, ph ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar_k + 8 * s, C::kKBytes);
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) tma_load_4d(sk + c * (BN * 128), &tmK, bar_k + 8 * s, c * 64, kvh, j * BN, b);
-        if (!mbar_wait(bar_ve + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
-        mbar_expect_tx(bar_v + 8 * s, C::kVBytes);
+          for (int c = 0; c < HD / 64; ++c) tma_load_4d(sk + c * (BN * 128), &tmK, bar_k + 8 * s, c * 64, kvh, j * BN, b);
+          ok = mbar_wait(bar_ve + 8 * s, ph ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar_v + 8 * s, C::kVBytes);
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) tma_load_4d(sv + c * (BN * 128), &tmV, bar_v + 8 * s, c * 64, kvh, j * BN, b);
+          for (int c = 0; c < HD / 64; ++c) tma_load_4d(sv + c * (BN * 128), &tmV, bar_v + 8 * s, c * 64, kvh, j * BN, b);
+          if (++s == C::kStages) { s = 0; ph ^= 1; }
+        }
+        if (!ok || !p.take) break;
+        // not earlier: a block that is asked for at the beginning of a long item would go to the busiest CTA
+        ok = mbar_wait(bar_ne + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        take_block(answers + 16 * (i & 1), bar_nf + 8 * (i & 1));
+        // (the answer has to arrive before the shared memory is given up, whatever the others do)
+        ok = mbar_wait(bar_nf + 8 * (i & 1), (i >> 1) & 1, never_set);
+        if (!ok) *abort_flag = 1;
+        if (!ok || !next_item(i, h, b, z)) break;
       }
+      if (!ok) fail_role = 1;
       nnb_release_next();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (warp-uniform: see umma_f16_elect)
-    {
-      const bool el = elect_one();
-      bool ok = mbar_wait(bar_q, 0, abort_flag);
-      auto issue_s = [&](int j) -> bool {  // S_j = Q K_j^T into score buffer j & 1
-        const uint32_t s = j % C::kStages, ph = (j / C::kStages) & 1;
-        if (!mbar_wait(bar_k + 8 * s, ph, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t sk = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes);
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) {
-          const uint32_t off_q = (k / 4) * (BQ * 128) + (k % 4) * 32, off_k = (k / 4) * (BN * 128) + (k % 4) * 32;
-          umma_f16_elect(el, tmem_base + C::kColS + (j & 1) * BN, make_smem_desc(smem_u32(sQ) + off_q, 16, 1024),
-                   make_smem_desc(sk + off_k, 16, 1024), p.idesc_qk, k > 0 ? 1u : 0u);
-        }
-        umma_commit_elect(el, bar_s + 8 * (j & 1));
-        umma_commit_elect(el, bar_ke + 8 * s);
-        return true;
-      };
-      if (ok && n_kv > 0) ok = issue_s(0);
-      if (ok && n_kv > 1) ok = issue_s(1);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const uint32_t s = j % C::kStages, ph = (j / C::kStages) & 1;
-        const int pb = j & 1;
-        if (!mbar_wait(bar_v + 8 * s, ph, abort_flag)) { ok = false; break; }
-        if (!mbar_wait(bar_p + 8 * pb, (j >> 1) & 1, abort_flag)) { ok = false; break; }   // P_j written, S_j consumed, O rescaled if needed
-        tc_fence_after();
-        const uint32_t sv = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes) + C::kKBytes;
-        const uint32_t tp = tmem_base + C::kColS + pb * BN;
-#pragma unroll
-        for (int k = 0; k < BN / 16; ++k)  // P from tensor memory: 16 keys = 8 columns per step; V is MN-major: 16 key rows (2048 B)
-          umma_f16_ts_elect(el, tmem_base + C::kColO, tp + k * 8, make_smem_desc(sv + k * (16 * 128), BN * 128, 1024), p.idesc_pv,
-                            (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit_elect(el, bar_o);  // one completion per tile: O holds the sum over tiles 0..j
-        if (j == n_kv - 1) umma_commit_elect(el, bar_o + 8);  // one-shot "all products done" for the epilogue (no phase aliasing)
-        umma_commit_elect(el, bar_ve + 8 * s);  // V_j is free
-        if (j + 2 < n_kv) ok = issue_s(j + 2);  // score buffer j & 1 was released by bar_p above
+    // Two cursors over the CTA's key tiles, numbered on over all items: S (scores) runs up to two tiles ahead of PV (second products).
+    const bool el = elect_one();
+    bool ok = true, s_end = false;
+    uint32_t sg = 0, s_stage = 0, s_ph = 0;             // S: tile, its stage and phase
+    int s_item = 0, s_j = 0, s_n = kv_tiles(query_tile(blockIdx.z));
+    uint32_t first_tile = 0, last_tile = 0, o_of = 0, o_ph = 0;  // per score buffer (bit): what PV has to know of its tile
+    // S_j = Q K_j^T into score buffer sg & 1. Not blocking, it leaves the tile for later when the next item is not there yet.
+    auto issue_s = [&](bool block) -> bool {
+      if (s_j == s_n) {
+        if (!p.take) { s_end = true; return false; }
+        const uint32_t bar = bar_nf + 8 * (s_item & 1), ph = (s_item >> 1) & 1;
+        if (!block && !mbar_test_warp(bar, ph)) return false;
+        if (!mbar_wait(bar, ph, abort_flag)) { ok = false; return false; }
+        int x, y, z;
+        const bool more = next_item(s_item, x, y, z);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_ne + 8 * (s_item & 1));
+        if (!more) { s_end = true; return false; }
+        ++s_item;
+        s_j = 0;
+        s_n = kv_tiles(query_tile(z));
       }
-      if (!ok && lane == 0) fail_role = 2;
+      const uint32_t qs = s_item % C::kItems;
+      if (s_j == 0) {
+        const uint32_t ph = (s_item / C::kItems) & 1;
+        if (!block && !(mbar_test_warp(bar_q + 8 * qs, ph) && mbar_test_warp(bar_k + 8 * s_stage, s_ph))) return false;
+        if (!mbar_wait(bar_q + 8 * qs, ph, abort_flag)) { ok = false; return false; }
+      }
+      if (!mbar_wait(bar_k + 8 * s_stage, s_ph, abort_flag)) { ok = false; return false; }
+      tc_fence_after();
+      const uint32_t sk = smem_u32(sKV) + s_stage * (C::kKBytes + C::kVBytes), sq = smem_u32(sQ) + qs * C::kQBytes;
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k) {
+        const uint32_t off_q = (k / 4) * (BQ * 128) + (k % 4) * 32, off_k = (k / 4) * (BN * 128) + (k % 4) * 32;
+        umma_f16_elect(el, tmem_base + C::kColS + (sg & 1) * BN, make_smem_desc(sq + off_q, 16, 1024), make_smem_desc(sk + off_k, 16, 1024), p.idesc_qk,
+                       k > 0 ? 1u : 0u);
+      }
+      umma_commit_elect(el, bar_s + 8 * (sg & 1));
+      umma_commit_elect(el, bar_ke + 8 * s_stage);
+      if (s_j == s_n - 1) umma_commit_elect(el, bar_qe + 8 * qs);  // Q has been read
+      const uint32_t bit = 1u << (sg & 1);
+      auto note = [&](uint32_t& word, bool on) { word = on ? word | bit : word & ~bit; };
+      note(first_tile, s_j == 0);
+      note(last_tile, s_j == s_n - 1);
+      note(o_of, qs != 0);
+      note(o_ph, (s_item / C::kItems) & 1);
+      ++s_j;
+      ++sg;
+      if (++s_stage == C::kStages) { s_stage = 0; s_ph ^= 1; }
+      return true;
+    };
+    uint32_t s = 0, ph = 0;
+    for (uint32_t g = 0;; ++g) {  // PV: tile
+      while (ok && !s_end && sg < g + 2) {
+        if (!issue_s(sg == g)) break;  // (score buffer sg & 1 was released by the bar_p of tile sg - 2 below)
+      }
+      if (!ok || sg == g) break;
+      const uint32_t pb = g & 1;
+      if (!mbar_wait(bar_v + 8 * s, ph, abort_flag)) { ok = false; break; }
+      const bool first = (first_tile >> pb) & 1, last = (last_tile >> pb) & 1;
+      const uint32_t ob = (o_of >> pb) & 1;
+      if (first && !mbar_wait(bar_oe + 8 * ob, ((o_ph >> pb) & 1) ^ 1, abort_flag)) { ok = false; break; }  // the item before has taken its O
+      if (!mbar_wait(bar_p + 8 * pb, (g >> 1) & 1, abort_flag)) { ok = false; break; }   // P_j written, S_j consumed, O rescaled if needed
+      tc_fence_after();
+      const uint32_t sv = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes) + C::kKBytes;
+      const uint32_t tp = tmem_base + C::kColS + pb * BN;
+#pragma unroll
+      for (int k = 0; k < BN / 16; ++k)  // P from tensor memory: 16 keys = 8 columns per step; V is MN-major: 16 key rows (2048 B)
+        umma_f16_ts_elect(el, tmem_base + C::kColO + ob * HD, tp + k * 8, make_smem_desc(sv + k * (16 * 128), BN * 128, 1024), p.idesc_pv,
+                          (!first || k > 0) ? 1u : 0u);
+      umma_commit_elect(el, bar_o);              // one completion per tile: O holds the item's sum up to it
+      if (last) umma_commit_elect(el, bar_of);   // "all products of the item done" for the epilogue (no phase aliasing)
+      umma_commit_elect(el, bar_ve + 8 * s);     // V_j is free
+      if (++s == C::kStages) { s = 0; ph ^= 1; }
     }
+    if (!ok && lane == 0) fail_role = 2;
   } else {
 #include "flash_fwd_softmax.inc"
   }
@@ -207,7 +282,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 template <int HD, bool F16>
-int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const FParams& p,
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, FParams p,
                cudaStream_t st) {
   auto kern = flash_fwd_kernel<HD, F16>;
   static bool configured = false;
@@ -219,6 +294,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     configured = true;
   }
   dim3 grid(p.H, p.B, p.n_q_tiles);
+  p.take = (long long)p.H * p.B * p.n_q_tiles > 2 * nnb_num_sms();  // (asking costs a grid of one wave 0.8 of 7 us)
   nnb_launch(kern, grid, kThreads, FCfg<HD>::kSmem, st, tq, tk, tv, to, p);
   return 0;
 }

@@ -171,12 +171,10 @@ static __device__ unsigned long long g_flash_prof[8];
 #endif
 #define NNB_PROF_FLUSH_N(n_) do { if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == NNB_PROF_THREAD) { \
   for (int i_ = 0; i_ < 5; ++i_) g_flash_prof[i_] = prof_acc[i_]; g_flash_prof[5] = (n_); } } while (0)
-#define NNB_PROF_FLUSH NNB_PROF_FLUSH_N(n_kv)
 #else
 #define NNB_PROF_DECL
 #define NNB_PROF_T0
 #define NNB_PROF_ADD(i)
-#define NNB_PROF_FLUSH
 #define NNB_PROF_FLUSH_N(n_)
 #endif
 
@@ -211,6 +209,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
+}
+// Whether the phase has completed by now, the same answer for the whole warp.
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
 }
 // Bounded wait. Returns false (and raises *abort_flag, a shared-memory word every role polls) when
 // the phase did not complete within kSpinLimit polls or another role already gave up.
@@ -367,6 +372,24 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
+// ---- work of blocks that have not started yet (cluster launch control)
+// Ask for the next block of the grid that has not started; the 16-byte answer and its bytes arrive on `bar`. A block that is taken never
+// starts: the asker does its work. Not to be asked again once an answer was "none".
+__device__ __forceinline__ void take_block(uint32_t answer, uint32_t bar) {
+  mbar_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
+}
+// The answer: whether a block was taken, and which.
+__device__ __forceinline__ bool taken_block(uint32_t answer, int& x, int& y, int& z) {
+  uint32_t some;
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b128 r;\nld.shared.b128 r, [%4];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\nselp.u32 %3, 1, 0, p;\nmov.u32 %0, 0;\nmov.u32 %1, 0;\nmov.u32 %2, 0;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n}"
+      : "=r"(x), "=r"(y), "=r"(z), "=r"(some) : "r"(answer) : "memory");
+  return some != 0;
 }
 
 // ---- clusters

@@ -34,6 +34,26 @@ def test_forward_matches_reference(B, H, KVH, T, hd):
     torch.testing.assert_close(out.float(), _ref(q, k, v), rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,T", [(74, 64), (75, 65), (300, 1), (150, 17), (101, 129), (40, 300), (20, 1024)])
+def test_forward_of_a_grid_in_several_waves_is_that_of_its_sequences(B, T, hd):
+    """Blocks that are running take over blocks that have not started: each sequence comes out as in a call of its own (one wave), bit for bit."""
+    from nanonemo_b200.ops.attention import fwd_raw
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(B + T)
+    H, KVH = 4, 2
+    q, k, v = (torch.randn(B, T, h, hd, device=DEV).bfloat16() for h in (H, KVH, KVH))
+    o = torch.full_like(q, float("nan"))
+    lse = fwd_raw(q, k, v, o, hd**-0.5)
+    check_status()
+    for b in sorted({0, 1, B // 3, B // 2, B - 2, B - 1}):
+        alone = torch.full_like(o[b : b + 1], float("nan"))
+        lse_alone = fwd_raw(q[b : b + 1], k[b : b + 1], v[b : b + 1], alone, hd**-0.5)
+        assert torch.equal(o[b : b + 1], alone) and torch.equal(lse[b : b + 1], lse_alone)
+    assert torch.isfinite(o).all() and torch.isfinite(lse).all()
+
+
 def test_future_keys_do_not_leak():
     from nanonemo_b200 import ops
 
