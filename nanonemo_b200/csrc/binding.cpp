@@ -40,6 +40,9 @@ extern "C" {
 typedef struct CUstream_st* cudaStream_t;
 const char* nnb_last_error();
 int nnb_gemm_bf16(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, int, int, void*, cudaStream_t);
+int nnb_gemm_rows_rope(const void*, const void*, void*, const void*, const void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, void*, cudaStream_t);
+int nnb_gemm_rows_f32w(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
+int nnb_gemm_rows_f32w_swiglu(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
 int nnb_gemm_swiglu(const void*, const void*, void*, void*, int, int, int, long long, long long, long long, long long, int, void*, cudaStream_t);
 int nnb_gemm_swiglu_act(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
 int nnb_gemm_swiglu_bwd(const void*, const void*, const void*, void*, int, int, int, long long, long long, long long, long long, int, void*, cudaStream_t);
@@ -179,12 +182,43 @@ Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
 Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
   reachable({&x2, &w, &cos, &sin});
   const int64_t M = x2.size(0), K = x2.size(1), N = w.size(0);
-  if (M < 256 || N < 128 || (hd != 64 && hd != 128) || N % hd || rope_cols % hd) return Tensor();
+  if ((hd != 64 && hd != 128) || N % hd || rope_cols % hd) return Tensor();
   const int code = code16(x2.scalar_type());
   NNB_ASSERT(code > 0 && w.scalar_type() == x2.scalar_type(), "gemm_rope needs bf16 or fp16 operands of one dtype");
   Tensor out = empty({M, N}, x2.scalar_type(), x2);
   return served(nnb_gemm_rope(x2.data_ptr(), w.data_ptr(), out.data_ptr(), cos.data_ptr(), sin.data_ptr(), (int)M, (int)N, (int)K, x2.stride(0), w.stride(0), N, (int)t_len,
                               (int)rope_cols, (int)hd, code, status_of(x2), stream()), "nnb_gemm_rope") ? out : Tensor();
+}
+
+// Products of a few rows with a weight that has no 16-bit copy, straight from its fp32 values (the bits are those of the cast and the usual
+// product); undefined where that is not served.
+bool from_f32(const Tensor& x2, const Tensor& w) {
+  return w.scalar_type() == at::kFloat && w.dim() == 2 && w.stride(1) == 1 && x2.dim() == 2 && x2.stride(1) == 1 && x2.size(1) == w.size(1) && code16(x2.scalar_type()) > 0 &&
+         x2.size(0) > 0 && w.size(0) > 0 && w.size(1) > 0;
+}
+Tensor gemm_f32w(const Tensor& x2, const Tensor& w) {
+  if (!from_f32(x2, w)) return Tensor();
+  reachable({&x2, &w});
+  const int64_t M = x2.size(0), N = w.size(0);
+  Tensor y = empty({M, N}, x2.scalar_type(), x2);
+  return served(nnb_gemm_rows_f32w(x2.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)w.size(1), x2.stride(0), w.stride(0), N, code16(x2.scalar_type()), status_of(x2),
+                                   stream()), "nnb_gemm_rows_f32w") ? y : Tensor();
+}
+Tensor gemm_f32w_swiglu(const Tensor& x2, const Tensor& w) {
+  if (!from_f32(x2, w) || w.size(0) % 2) return Tensor();
+  reachable({&x2, &w});
+  const int64_t M = x2.size(0), F = w.size(0) / 2;
+  Tensor act = empty({M, F}, x2.scalar_type(), x2);
+  return served(nnb_gemm_rows_f32w_swiglu(x2.data_ptr(), w.data_ptr(), act.data_ptr(), (int)M, (int)F, (int)w.size(1), x2.stride(0), w.stride(0), F, code16(x2.scalar_type()),
+                                          status_of(x2), stream()), "nnb_gemm_rows_f32w_swiglu") ? act : Tensor();
+}
+Tensor gemm_f32w_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
+  if (!from_f32(x2, w) || (hd != 64 && hd != 128) || w.size(0) % hd || rope_cols % hd) return Tensor();
+  reachable({&x2, &w, &cos, &sin});
+  const int64_t M = x2.size(0), N = w.size(0);
+  Tensor y = empty({M, N}, x2.scalar_type(), x2);
+  return served(nnb_gemm_rows_rope(x2.data_ptr(), w.data_ptr(), y.data_ptr(), cos.data_ptr(), sin.data_ptr(), (int)M, (int)N, (int)w.size(1), x2.stride(0), w.stride(0), N, (int)t_len,
+                                   (int)rope_cols, (int)hd, code16(x2.scalar_type()), /*f32w=*/1, 16, status_of(x2), stream()), "nnb_gemm_rows_rope") ? y : Tensor();
 }
 
 void rope_packed(const Tensor& x2, const Tensor& out2, const Tensor& cos, const Tensor& sin, int64_t T, int64_t n_rot, int64_t hd, int64_t n_copy, double sign) {
@@ -347,8 +381,14 @@ struct Weight {
   Tensor shadow;
   bool engine;
   Weight(py::handle w) : shadow(tensor_or_undefined(attribute(w, "_shadow"))) { engine = shadow.defined() || !attribute(w, "_main_grad").is_none(); }
-  Tensor in(const Tensor& w, at::ScalarType dt) const { return shadow.defined() && shadow.scalar_type() == dt ? shadow : as_dtype(w.detach(), dt); }
+  bool has(at::ScalarType dt) const { return shadow.defined() && shadow.scalar_type() == dt; }
+  Tensor in(const Tensor& w, at::ScalarType dt) const { return has(dt) ? shadow : as_dtype(w.detach(), dt); }
 };
+// x2 w^T for a weight without a 16-bit copy
+Tensor weight_product(const Tensor& x2, const Tensor& weight) {
+  const Tensor w = weight.detach(), y = gemm_f32w(x2, w);
+  return y.defined() ? y : gemm_nt(x2, as_dtype(w, x2.scalar_type()));
+}
 
 // dW of an engine weight goes into the flat gradient buffer, and the strategy hears of it, in every backward pass through a weight that is
 // trained, also one that asks for other gradients only: as with the Python autograd functions, whose needs_input_grad is fixed in the
@@ -421,13 +461,13 @@ std::vector<int64_t> with_last(at::IntArrayRef sizes, int64_t last) {
 
 // ------------------------------------------------------------------------------------------------ operators
 // x: any shape and dtype where the engine's weight is (nothing differentiates its gradients); otherwise the 16-bit rows, made before the
-// node, so that its saved tensor leads back to the caller's input under create_graph.
+// node, so that its saved tensor leads back to the caller's input under create_graph. w16: none where the weight has no 16-bit copy.
 struct LinearFn : torch::autograd::Function<LinearFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& w16, bool engine, const std::vector<int64_t>& y_sizes) {
-    const Tensor x2 = engine ? rowmajor2d(as_dtype(rows2d(x), w16.scalar_type())) : x;
-    Tensor y = gemm_nt(x2, w16);
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const optional<Tensor>& w16, bool engine, const std::vector<int64_t>& y_sizes) {
+    const Tensor x2 = engine ? rowmajor2d(as_dtype(rows2d(x), w16->scalar_type())) : x;
+    Tensor y = w16 ? gemm_nt(x2, *w16) : weight_product(x2, weight);
     ctx->save_for_backward({x2, weight});
-    if (engine) ctx->saved_data["w16"] = w16;
+    if (engine) ctx->saved_data["w16"] = *w16;
     ctx->saved_data["x_sizes"] = x.sizes().vec();
     ctx->saved_data["x_dtype"] = (int64_t)x.scalar_type();
     ctx->saved_data["engine"] = engine;
@@ -464,8 +504,9 @@ py::object linear(py::handle x_, py::handle weight_) {
   Tensor y;
   {
     py::gil_scoped_release nogil;
-    const Tensor w16 = w.in(weight, compute_dtype());
-    y = LinearFn::apply(w.engine ? x : rowmajor2d(as_dtype(rows2d(x), w16.scalar_type())), weight, w16, w.engine, with_last(x.sizes(), weight.size(0)));
+    const at::ScalarType dt = compute_dtype();
+    const optional<Tensor> w16 = w.engine ? optional<Tensor>(w.in(weight, dt)) : std::nullopt;
+    y = LinearFn::apply(w.engine ? x : rowmajor2d(as_dtype(rows2d(x), dt)), weight, w16, w.engine, with_last(x.sizes(), weight.size(0)));
   }
   return py::cast(y);
 }
@@ -654,7 +695,22 @@ py::object qkv_rope_attention(py::handle x_, py::handle weight_, py::handle cos_
     auto table = [T](const Tensor& t) { return as_dtype(t.slice(0, 0, T), at::kFloat).contiguous(); };
     cos = table(cos);
     sin = table(sin);
-    y = QKVRopeAttentionFn::apply(x, weight, w.in(weight, compute_dtype()), cos, sin, H, KVH, hd);
+    const at::ScalarType dt = compute_dtype();
+    Tensor qkv, xc = x;
+    if (!w.engine) {
+      const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), dt));
+      qkv = gemm_f32w_rope(x2, weight.detach(), cos, sin, T, (H + KVH) * hd, hd);
+      xc = x2.view(x.sizes());
+    }
+    if (qkv.defined()) {  // (no gradient is wanted)
+      const int64_t B = x.size(0);
+      const Heads p(qkv, B, T, H, KVH, hd);
+      const Tensor o = empty({B, T, H, hd}, dt, x);
+      flash_fwd(p.q, p.k, p.v, o, 1.0 / std::sqrt((double)hd));
+      y = o.view({B, T, H * hd});
+    } else {
+      y = QKVRopeAttentionFn::apply(xc, weight, w.in(weight, dt), cos, sin, H, KVH, hd);
+    }
   }
   return py::cast(y);
 }
@@ -715,12 +771,13 @@ py::object mlp_swiglu(py::handle x_, py::handle gu_, py::handle down_) {
   {
     py::gil_scoped_release nogil;
     const at::ScalarType dt = compute_dtype();
-    const Tensor gu16 = gu.in(w_gu, dt), down16 = down.in(w_down, dt);  // (cast once, whichever launches follow)
     if (grad) {
-      y = MLPFn::apply(x, w_gu, w_down, gu16, down16);
+      y = MLPFn::apply(x, w_gu, w_down, gu.in(w_gu, dt), down.in(w_down, dt));
     } else {  // nobody will ask for the projection: where one launch serves, only the activation leaves it
       const Tensor x2 = rowmajor2d(as_dtype(rows2d(x), dt));
-      y = gemm_nt(gate_up(x2, gu16, false).second, down16).view(with_last(x.sizes(), w_down.size(0)));
+      Tensor act = gu.has(dt) ? Tensor() : gemm_f32w_swiglu(x2, w_gu.detach());
+      if (!act.defined()) act = gate_up(x2, gu.in(w_gu, dt), false).second;
+      y = (down.has(dt) ? gemm_nt(act, down.shadow) : weight_product(act, w_down)).view(with_last(x.sizes(), w_down.size(0)));
     }
   }
   return py::cast(y);

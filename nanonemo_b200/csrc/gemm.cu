@@ -658,6 +658,12 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   // (11264 x 2048 x 8192: 318 / 359; 2048 x 2048 x 8192: 57 / 64 / 90). It is not the best one for a 16-bit output whose 128-wide
   // tiles fit one wave, where a tile's latency is all that counts: 1024 x 768 x 768 17 / 17 / 15, 1024 x 768 x 2048 26 / 26 / 22,
   // 1024 x 2048 x 5632 44 / 46 / 38. The head's input gradient asks for the narrow tile there by its hint.
+  if (mode == 0 && bn_hint == 0 && !out_f32 && !a_mn && max_ctas <= 0) {
+    if (const int g = nnb_rows_tile(M, N, K, nnb_num_sms())) {
+      const int rc = nnb_gemm_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn, dtype, g, status, st);
+      if (rc <= 0) return rc;  // 1 = operands not aligned for it
+    }
+  }
   static const bool pair_enabled = [] { const char* e = getenv("NANONEMO_GEMM_PAIR"); return !(e && e[0] == '0'); }();
   if (mode == 0 && (bn_hint == 512 || (bn_hint == 0 && pair_enabled && M >= 256 && N >= 256))) {
     const NnbGemm2Args g{A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, dtype, out_f32, accumulate, k_splits, max_ctas, status};
@@ -824,6 +830,10 @@ extern "C" int nnb_gemm_swiglu_act(const void* X, const void* Wgu, void* ACT, in
 extern "C" int nnb_gemm_rope(const void* X, const void* W, void* QKV, const void* cos_t, const void* sin_t, int M, int N, int K,
                              long long lda, long long ldw, long long ldd, int t_len, int rope_cols, int head_dim, int dtype,
                              void* status, cudaStream_t st) {
+  if (const int tile = nnb_rows_tile(M, N, K, nnb_num_sms())) {
+    const int rc = nnb_gemm_rows_rope(X, W, QKV, cos_t, sin_t, M, N, K, lda, ldw, ldd, t_len, rope_cols, head_dim, dtype, 0, head_dim == 64 ? 32 : tile, status, st);
+    if (rc <= 0) return rc;
+  }
   NnbGemm2Args g{};
   if (int rc = fused_gemm_common(g, X, W, QKV, M, N, K, lda, ldw, ldd, dtype, status)) return rc;
   g.epilogue = EPI_ROPE; g.cos_t = cos_t; g.sin_t = sin_t; g.t_len = t_len; g.rope_cols = rope_cols; g.head_dim = head_dim;

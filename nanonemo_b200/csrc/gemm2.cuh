@@ -39,6 +39,22 @@ struct NnbGemm2Args {
 // Returns 0 on success, 1 when the shape is not served by the pair kernel (caller falls back), < 0 on error.
 int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st);
 
+// The kernel for few rows (gemm_rows.cu): columns of its tile / 2 (32 or 64) for a product with a 16-bit output that it serves faster than the
+// persistent kernels, 0 otherwise. Its tiles are narrow and short-lived: a set-up of 2.3 us against 4 to 5, and the SMs that a few wide tiles
+// would leave idle; with more tiles than SMs it is bound by the bytes an SM takes in. us in a row of products with 24 weights (pair kernel,
+// single-CTA kernel below 256 rows / 64-wide / 128-wide tiles): 201 x 768 x 768 6.5 / 4.5 / 6.2, 512 x 768 x 2048 13.9 / 8.0 / 10.9, 1024
+// x 768 x 4096 23.0 / 14.4 / 20.1, 512 x 2048 x 11264 54.9 / 39.3 / 56.7, 777 x 1280 x 768 8.1 / 4.9 / 6.4; more 64-wide tiles than SMs:
+// 1024 x 1280 x 768 8.2 / 6.7 / 6.6, 2048 x 768 x 2048 14.3 / 13.9 / 12.3, 512 x 4096 x 768 8.7 / 7.4 / 7.0, 2048 x 768 x 4096 23.2 / 26.1 /
+// 22.3, 1024 x 2048 x 5632 30.7 / 39.8 / 33.0; more 128-wide ones: 777 x 3072 x 2048 15.6 / 26.3 / 17.2, 4096 x 768 x 2048 15.3 / 27.1 / 19.0.
+inline int nnb_rows_tile(long long M, long long N, long long K, int sms) {
+  const long long m = (M + 127) / 128;
+  if (m * ((N + 63) / 64) <= sms) return 32;
+  if (m * ((N + 127) / 128) <= sms && K <= 4096) return 64;
+  return 0;
+}
+extern "C" int nnb_gemm_rows(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, void*, cudaStream_t);
+extern "C" int nnb_gemm_rows_rope(const void*, const void*, void*, const void*, const void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, void*, cudaStream_t);
+
 // K splits that even out the last wave of `tiles` tiles on `workers` persistent CTAs (or pairs), whatever traffic they add. This is how
 // long an accumulator's chain may get: with it as the limit a product is as exact as if it were cut into these splits.
 inline int nnb_even_k_splits(long long tiles, int workers, int kblocks) {

@@ -102,6 +102,10 @@ _SIGNATURES = {
     "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfippipp",
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
+    "nnb_gemm_rows": "pppiiiqqqiiipp",
+    "nnb_gemm_rows_rope": "pppppiiiqqqiiiiiipp",
+    "nnb_gemm_rows_f32w": "pppiiiqqqipp",
+    "nnb_gemm_rows_f32w_swiglu": "pppiiiqqqipp",
     "nnb_gemm_swiglu": "ppppiiiqqqqipp",
     "nnb_gemm_swiglu_act": "pppiiiqqqipp",
     "nnb_gemm_rope": "pppppiiiqqqiiiipp",

@@ -78,6 +78,14 @@ def _dx_tile(rows: int, width: int, device) -> int:
     return 128 if -(-rows // 128) * -(-width // 128) <= _sm_count(device) else 0
 
 
+def _dx_hint(rows: int, width: int, vocab: int, device) -> int:
+    """No hint while the dispatcher's 64-wide tiles (csrc/gemm_rows.cu) fit one wave, ``_dx_tile`` beyond and for a few thousand words (a short
+    K loop: a tile's width hardly matters). us, 64-wide / 128-wide / pair: K = 50304,
+    256 x 768 162 / 227 / 231, 1000 x 768 166 / 229 / 233, 1536 x 768 177 / 235 / 235, 2048 x 768 326 / 237 / 237; K = 32000, 512 x 2048 119 /
+    153 / 156, 768 x 2048 212 / 157 / 158."""
+    return 0 if vocab >= 4096 and -(-rows // 128) * -(-width // 64) <= _sm_count(device) else _dx_tile(rows, width, device)
+
+
 def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
     mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
@@ -97,7 +105,7 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
         else:
             gemm(xc, w16, out=lg)
             ce_inplace(lg, targets[r0:r1], loss_rows[r0:r1], 1.0 / N)
-        gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
+        gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_hint(r1 - r0, D, w16.shape[0], x16.device))
         gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=r0 > 0)
     return loss_rows.sum(), dx
 
@@ -207,7 +215,7 @@ class _VocabParallelLinearCE(torch.autograd.Function):
             lg, xc = logits[: r1 - r0], x16[r0:r1]
             gemm(xc, w16, out=lg)
             vocab_parallel_ce_inplace(lg, tg[r0:r1], loss_rows[r0:r1], 1.0 / N, v0, Vl * tp.world, tp.all_gather, tp.world)
-            gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_tile(r1 - r0, D, x16.device))
+            gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_hint(r1 - r0, D, w16.shape[0], x16.device))
             gemm(lg, xc, a_mn=True, b_mn=True, out=dW, accumulate=r0 > 0)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype
