@@ -302,6 +302,19 @@ int launch_rows(const CUtensorMap& ta, const CUtensorMap& tw, RParams p, int til
   return 0;
 }
 
+}  // namespace
+
+// Whether a product of M rows with an fp32 weight of N rows (2 N with `swiglu`) and K columns is taken straight from it, and not from its cast.
+// us, rows straight from fp32 / cast + product: 201 x 768 x 2048 9.5 / 7.9 + 4, 512 x 768 x 2048 10.2 / 8.0 + 4, and more tiles than SMs 201 x
+// 4096 x 768 8.2 / 5.0 + 4, 512 x 1280 x 768 8.0 / 4.7 + 3, 512 x 2048 x 2048 17.9 / 9.0 + 5. Weights below 2^17 elements are cast as ever: 2.3
+// us a call, and tests count their launches.
+extern "C" int nnb_gemm_rows_f32w_serves(int M, int N, int K, int swiglu) {
+  const long long sms = nnb_num_sms(), t = (long long)((M + BM - 1) / BM) * (swiglu ? (N + 15) / 16 : (N + 31) / 32);
+  return (t <= sms || (t <= 2 * sms && K <= 1024)) && (long long)(swiglu ? 2 * N : N) * K >= 1 << 17;
+}
+
+namespace {
+
 template <bool F32W, bool BMN, int EPI>
 int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long long lda, long long ldw, long long ldd, int dtype, RParams& p, int g, void* status, cudaStream_t st) {
   const int w_bytes = F32W ? 4 : 2;
@@ -326,11 +339,7 @@ int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long l
   }
 #define NNB_ROWS(GG) (dtype == NNB_BF16 ? launch_rows<GG, true, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st) : launch_rows<GG, false, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st))
   if constexpr (F32W) {
-    // Where a cast and the 16-bit product serve better. us, rows straight from fp32 / cast + product: 201 x 768 x 2048 9.5 / 7.9 + 4, 512 x 768 x 2048
-    // 10.2 / 8.0 + 4, and more tiles than SMs 201 x 4096 x 768 8.2 / 5.0 + 4, 512 x 1280 x 768 8.0 / 4.7 + 3, 512 x 2048 x 2048 17.9 / 9.0 + 5.
-    const long long t = (long long)tiles * m_blocks, sms = nnb_num_sms();
-    // (Weights below 2^17 elements are cast as ever: 2.3 us a call, and tests count their launches.)
-    if (!(t <= sms || (t <= 2 * sms && K <= 1024)) || (long long)(EPI == ROWS_SWIGLU ? 2 * N : N) * K < 1 << 17) return 1;
+    if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU)) return 1;
     NNB_REQUIRE(g == 16, "gemm_rows: no tile of %d", g);
     return NNB_ROWS(16);
   } else {

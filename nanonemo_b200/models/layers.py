@@ -199,7 +199,28 @@ class Block(nn.Module):
         self.norm_mlp = AddRMSNorm(cfg.d_model, cfg.norm_eps, impl)
         self.mlp = MLP(cfg)
 
+    def _one_call(self) -> bool:
+        """Whether the block is what it was built as, with every part on the sm100 kernels and nobody watching or replacing the parts."""
+        attn, mlp = self.attn, self.mlp
+        if type(attn) is not Attention or type(mlp) is not MLP or type(attn.wo) is not Linear or torch.nn.modules.module._has_any_global_hook():
+            return False
+        if not (attn.fused and mlp.fused and attn.tp is None and mlp.tp is None and attn.wo.impl == "sm100" and ops.fused_ok()):
+            return False
+        for m in (self.norm_attn, self.norm_mlp):
+            if type(m) is not AddRMSNorm or m.impl != "sm100":
+                return False
+        for m in (self.norm_attn, attn, attn.wo, self.norm_mlp, mlp):
+            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
+                return False
+        return True
+
     def forward(self, x, cos, sin, delta=None):
+        if not (torch.compiler.is_compiling() or torch.is_grad_enabled()) and x.is_cuda and self._one_call():
+            a, m = self.attn, self.mlp
+            out = ops.decoder_block(x, delta, self.norm_attn.weight, self.norm_attn.eps, a.wqkv.weight, a.wo.weight, self.norm_mlp.weight, self.norm_mlp.eps,
+                                    m.w_gu.weight, m.w_down.weight, cos, sin, a.n_heads, a.n_kv_heads, a.head_dim)
+            if out is not NotImplemented:
+                return out
         h, x = self.norm_attn(x, delta)
         h, x = self.norm_mlp(x, self.attn(h, cos, sin))
         return x, self.mlp(h)

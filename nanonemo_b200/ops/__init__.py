@@ -223,6 +223,11 @@ def fused_ok() -> bool:
     return compute_dtype() in _ATTN_DTYPES
 
 
+def decoder_block(*args):
+    """A whole pre-norm block without gradients as one native call (csrc/binding.cpp), or NotImplemented: see models/layers.py, Block."""
+    return _lib.operator_call("decoder_block", *args)
+
+
 def qkv_rope_attention(x, weight, cos, sin, n_heads, n_kv_heads, head_dim):
     """Packed QKV projection + RoPE (GEMM epilogue) + causal GQA attention (sm100 only)."""
     _need_cuda(x, "qkv_rope_attention")

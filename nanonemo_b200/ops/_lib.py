@@ -104,6 +104,7 @@ _SIGNATURES = {
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
     "nnb_gemm_rows": "pppiiiqqqiiipp",
     "nnb_gemm_rows_rope": "pppppiiiqqqiiiiiipp",
+    "nnb_gemm_rows_f32w_serves": "iiii",
     "nnb_gemm_rows_f32w": "pppiiiqqqipp",
     "nnb_gemm_rows_f32w_swiglu": "pppiiiqqqipp",
     "nnb_gemm_swiglu": "ppppiiiqqqqipp",

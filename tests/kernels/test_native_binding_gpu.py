@@ -444,3 +444,40 @@ def test_backward_nodes_find_the_registered_operators_in_a_new_process():
 
     r = subprocess.run([sys.executable, "-c", _FIRST_CALLS], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, None])
+@pytest.mark.parametrize("B,T,head_dim", [(1, 1, 64), (1, 201, 64), (2, 100, 128), (3, 300, 64), (1, 130, 128)])
+def test_a_block_without_gradients_is_its_operators_in_one_call(monkeypatch, B, T, head_dim, dtype):
+    """The same bits, few rows (one workspace) and many, with and without a pending delta; parts that are watched run one by one."""
+    from contextlib import nullcontext
+
+    from nanonemo_b200.models.config import ModelConfig
+    from nanonemo_b200.models.layers import Block, rope_cache
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(B * T)
+    cfg = ModelConfig.sm100(n_layers=1, d_model=768, n_heads=768 // head_dim, n_kv_heads=2, d_ff=2048, max_seq_len=512, head_dim_override=head_dim)
+    block = Block(cfg).to(DEV).eval()
+    cos, sin = rope_cache(head_dim, 512, device=DEV)
+    x, delta = torch.randn(B, T, 768, device=DEV), torch.randn(B, T, 768, device=DEV).to(dtype or torch.bfloat16)
+
+    def run(d):
+        with torch.no_grad(), torch.autocast("cuda", dtype=dtype) if dtype else nullcontext():
+            return block(x, cos, sin, d)
+
+    assert block._one_call() or dtype is None
+    for d in (None, delta):
+        got = run(d)
+        check_status()
+        with monkeypatch.context() as m:
+            m.setattr(Block, "_one_call", lambda self: False)
+            ref = run(d)
+        for a, b in zip(got, ref):
+            assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+    seen = []
+    handle = block.attn.wo.register_forward_hook(lambda *a: seen.append(1))
+    assert not block._one_call()
+    again = run(delta)
+    handle.remove()
+    assert seen == [1] and all(torch.equal(a, b) for a, b in zip(again, got))
