@@ -1,6 +1,6 @@
 // Causal grouped-query FlashAttention backward on tcgen05 / TMEM / TMA for sm_100a (head_dim 64).
 //
-// One CTA owns 128 keys of one (batch, KV head) and visits every (query head of the group, query tile)
+// An item is 128 keys of one (batch, KV head): a CTA visits every (query head of the group, query tile)
 // at or after its keys; dK and dV of the tile accumulate in TMEM over the whole GQA group, so they are
 // written once and need no atomics (as in the reference kernel, nanonemo/kernels/cuda/flash_attn.cu:
 // 176-340, which keeps them in registers). Per visit, five tensor-core products, on TRANSPOSED score tiles:
@@ -31,6 +31,12 @@
 // warps a scheduler do not hide. (A quarter or half of the exponentials as polynomials on the multiply-add pipe: no change.) Whole backward,
 // us, queries as rows / keys as rows: B32 H12/4 T1024 303 / 283, B128 T256 184 / 174, B64 H8/8 T200 84 / 80, B2 H12/4 T333 35 / 33, B8 H12/4 T4096
 // 697 / 702, where the card's power limit (1.63 GHz under this kernel) evens them out.
+// Items follow one another in a CTA without a seam, as in the forward kernel (flash_fwd.cu): a block that is running takes over blocks that have not
+// started, K and V of the next item have a tile of their own, its first scores are issued beside the last products, and the drain
+// warps, idle two thirds of a visit, store dV and dK while the compute warps are in the next item. A CTA per item spent 8.8 us on set-up, first
+// loads, the first visit's latencies, the epilogue and its store, as long as three visits and with an SM to itself. Whole backward in a
+// row (the card's power limit included), us, a CTA per item / items in sequence: B200 T64 85.9 / 74.9, B64 T300 131.5 / 119.5, B64
+// T512 222 / 203, B16 T1024 147 / 133, B32 T1024 315 / 293, B8 T4096 810 / 748.
 // All waits are bounded, except two: the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers), and, in a
 // cluster, the two barriers of all its threads at the end, which every role of every CTA reaches, after a wait that ran out too.
 #include <cstdlib>
@@ -56,12 +62,14 @@ static_assert(kRegsShares == kThreads / 128 * kRegsLaunch, "the shares have to b
 constexpr int kTile16 = 128 * 64 * 2;     // a [128 x 64] 16-bit tile = 16 KB
 constexpr int kStagesQ = 3;             // a stage is released when dK / dQ of its visit are done and refilled two visits ahead
 // shared memory map (bytes)
-constexpr int kOffK = 0, kOffV = kTile16, kOffQdO = 2 * kTile16;               // ring of (Q | dO)
+constexpr int kOffK = 0 /* V behind it */, kOffQdO = 2 * kTile16;               // ring of (Q | dO)
 constexpr int kOffdS = kOffQdO + kStagesQ * 2 * kTile16;                       // dS^T: [128 keys] x two groups of 64 queries
 constexpr int kOffStage = kOffdS + 2 * kTile16;                                // fp32 [128 x 64] = 32 KB
-constexpr int kOffBars = kOffStage + 2 * kTile16;
-constexpr int kOffLD = kOffBars + 256;                                         // float [2 parities][2 (-L log2e, -D scale)][128]
-constexpr int kSmem = kOffLD + 2 * 2 * BQ * 4 + 1024;
+constexpr int kOffKV1 = kOffStage + 2 * kTile16;                                // K and V of the next item (every other one)
+constexpr int kOffBars = kOffKV1 + 2 * kTile16;
+constexpr int kOffLD = kOffBars + 512;                                         // float [2 parities][2 (-L log2e, -D scale)][128]
+constexpr int kSmem = kOffLD + 2 * 2 * BQ * 4;                                 // (nothing to spare for aligning the base: the kernel checks it)
+static_assert(kSmem <= 227 * 1024, "one CTA per SM");
 // tensor memory columns
 constexpr int kColS = 0 /* two buffers: + 128 * (visit & 1) */, kColdP = 256, kColdV = 384, kColdK = 448, kTmemCols = 512;
 // A visit's S^T buffer also holds its P^T, the queries 0..63 in columns [0, 32) and 64..127 in [96, 128), and between them its dQ
@@ -82,6 +90,7 @@ struct BParams {
   const float* rope_sin;
   // A cluster of `split` CTAs shares one key tile: each takes a part of its visits, and they add up their dK and dV at the end.
   int split;
+  int take;                               // the grid has more blocks than SMs: blocks take over others (see flash_fwd.cu)
   void *dk, *dv;                          // split > 1: written directly, strides as the launcher's
   long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh;
 };
@@ -92,49 +101,62 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                  const __grid_constant__ CUtensorMap tmdQacc, const __grid_constant__ CUtensorMap tmdK,
                  const __grid_constant__ CUtensorMap tmdV, const BParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t s_base = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBars);
-  // barriers: kv_full, q_full[3], q_empty[3], s_full[2], dp_full, p_written, ds_written, dq_full, dq_read, ld_full[2], ld_empty[2], all_done
-  const uint32_t bar_kv = smem_u32(bars), bar_qf = bar_kv + 8, bar_qe = bar_qf + 8 * kStagesQ;
-  const uint32_t bar_s = bar_qe + 8 * kStagesQ, bar_dp = bar_s + 16, bar_p = bar_dp + 8, bar_ds = bar_p + 8;
-  const uint32_t bar_dq = bar_ds + 8, bar_dqr = bar_dq + 8, bar_lf = bar_dqr + 8, bar_le = bar_lf + 16, bar_fin = bar_le + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1 + 2 * kStagesQ + 12);
+  // barriers: kv_full[2], kv_empty[2], q_full[3], q_empty[3], s_full[2], dp_full, dq_full, all_done, next_full[2] | by compute: p_written, ds_written, ld_empty[2] |
+  // by drain: dq_read, acc_read | ld_full[2] | next_empty[2]
+  const uint32_t bar_kv = smem_u32(bars), bar_kve = bar_kv + 16, bar_qf = bar_kve + 16, bar_qe = bar_qf + 8 * kStagesQ;
+  const uint32_t bar_s = bar_qe + 8 * kStagesQ, bar_dp = bar_s + 16, bar_dq = bar_dp + 8, bar_fin = bar_dq + 8, bar_nf = bar_fin + 8;
+  const uint32_t bar_p = bar_nf + 16, bar_ds = bar_p + 8, bar_le = bar_ds + 8, bar_dqr = bar_le + 16, bar_acc = bar_dqr + 8, bar_lf = bar_acc + 8, bar_ne = bar_lf + 16;
+  constexpr int kBars = 4 + 2 * kStagesQ + 17;
+  constexpr int kNextReaders = 2 + kDrainThreads / 32 + kComputeThreads / 32;  // warps that read which item is next: MMA, L / D, drain, compute
+  const uint32_t answers = s_base + kOffBars + (kBars + 1) / 2 * 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBars + (kBars + 1) / 2 * 16 + 32);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* never_set = abort_flag + 1;
+  static_assert(kBars <= 32 && (kBars + 1) / 2 * 16 + 32 + 12 <= 512, "barriers");
   float* s_ld = reinterpret_cast<float*>(smem + kOffLD);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Longest-job-first over the whole grid: key tile 0 is visited by every query tile, the last one by a single tile, and the
-  // key tile is the slowest-varying block index, so the heavy CTAs all start first and the kernel ends on the short ones.
-  const int kt = blockIdx.z;          // key tile
+  const bool aligned = (s_base & 1023) == 0;  // (swizzled tiles; nothing runs otherwise)
+  // An item is a key tile of one (batch, KV head), or a part of its visits. Longest-job-first over the whole grid: key tile 0 is visited by every
+  // query tile, the last one by a single tile, and the key tile is the slowest-varying block index, so the heavy items all start first and the
+  // kernel ends on the short ones.
   const int split = SPLIT ? p.split : 1;
-  const int part = blockIdx.x % split, kvh = blockIdx.x / split, b = blockIdx.y;  // (part = rank in the cluster)
-  const int first_qt = (kt * BKV) / BQ;                     // first query tile that can see these keys
-  const int n_qt = p.n_q_tiles - first_qt;                  // query tiles per head of the group
-  // visits are numbered head by head; this CTA's are [visit0, visit0 + iters)
-  const int visit0 = n_qt * p.group * part / split, iters = n_qt * p.group * (part + 1) / split - visit0;
-  const int head0 = kvh * p.group + visit0 / n_qt, qt0 = first_qt + visit0 % n_qt;
+  const int part = blockIdx.x % split;  // (rank in the cluster)
+  struct Item { int kt, kvh, b, first_qt, n_qt, visit0, iters; };
+  auto item_at = [&](int x, int y, int z) {
+    Item i;
+    i.kt = z; i.kvh = x / split; i.b = y;
+    i.first_qt = (z * BKV) / BQ;                            // first query tile that can see these keys
+    i.n_qt = p.n_q_tiles - i.first_qt;                      // query tiles per head of the group
+    // visits are numbered head by head; this CTA's are [visit0, visit0 + iters)
+    i.visit0 = i.n_qt * p.group * part / split;
+    i.iters = i.n_qt * p.group * (part + 1) / split - i.visit0;
+    return i;
+  };
+  const Item item0 = item_at(blockIdx.x, blockIdx.y, blockIdx.z);
+  // The item after number k of this CTA: answer k, in slot k & 1. A warp reads it with next_item and lets the slot go. False: there is none.
+  auto next_item = [&](int k, Item& i) {
+    int x, y, z;
+    const bool more = taken_block(answers + 16 * (k & 1), x, y, z);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_ne + 8 * (k & 1));
+    if (more) i = item_at(x, y, z);
+    return more;
+  };
+  auto next_known = [&](int k, volatile int* flag) { return mbar_wait(bar_nf + 8 * (k & 1), (k >> 1) & 1, flag); };
 
-  if (threadIdx.x == 0) {
-    mbar_init(bar_kv, 1);
-    for (int s = 0; s < kStagesQ; ++s) {
-      mbar_init(bar_qf + 8 * s, 1);
-      mbar_init(bar_qe + 8 * s, 1);
+  if (warp == 0) {  // a barrier a lane
+    const uint32_t bar = bar_kv + 8 * lane;
+    const uint32_t count = bar < bar_p ? 1 : bar < bar_dqr ? kComputeThreads : bar < bar_lf ? kDrainThreads : bar < bar_ne ? 32 : kNextReaders;
+    if (lane < kBars) mbar_init(bar, count);
+    if (lane == 0) {
+      *abort_flag = aligned ? 0 : 1;
+      *never_set = 0;
     }
-    mbar_init(bar_s, 1);
-    mbar_init(bar_s + 8, 1);
-    mbar_init(bar_dp, 1);
-    mbar_init(bar_p, kComputeThreads);
-    mbar_init(bar_ds, kComputeThreads);
-    mbar_init(bar_dq, 1);
-    mbar_init(bar_dqr, kDrainThreads);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_lf + 8 * i, 32);
-      mbar_init(bar_le + 8 * i, kComputeThreads);
-    }
-    mbar_init(bar_fin, 1);
-    *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
   }
@@ -148,36 +170,73 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   const float *g_lse = p.lse, *g_delta = p.delta, *g_cos = p.rope_cos, *g_sin = p.rope_sin;
   nnb_after_previous(g_lse, g_delta, g_cos, g_sin);
-  int fail_role = 0;
+  int fail_role = aligned ? 0 : 6;
+  // dK of key position t leaves through the transpose of the forward rotation: lo' = lo c + hi s, hi' = hi c - lo s
+  auto unrotate = [&](uint32_t (&lo_)[32], uint32_t (&hi_)[32], int t) {
+    const float *cr = g_cos + (size_t)t * (HD / 2), *sr = g_sin + (size_t)t * (HD / 2);
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      const float4 c4 = __ldg(reinterpret_cast<const float4*>(cr + i)), s4 = __ldg(reinterpret_cast<const float4*>(sr + i));
+      const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float lo = __uint_as_float(lo_[i + e]), hi = __uint_as_float(hi_[i + e]);
+        lo_[i + e] = __float_as_uint(lo * cc[e] + hi * ss[e]);
+        hi_[i + e] = __float_as_uint(hi * cc[e] - lo * ss[e]);
+      }
+    }
+  };
 
   if (warp < kDrainWarp0) {
     regs_dec<kRegsIssue>();
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && lane == 0 && aligned) {
       // ---------------------------------------------------------------- TMA producer
-      mbar_expect_tx(bar_kv, 2 * kTile16);
-      tma_load_4d(s_base + kOffK, &tmK, bar_kv, 0, kvh, kt * BKV, b);
-      tma_load_4d(s_base + kOffV, &tmV, bar_kv, 0, kvh, kt * BKV, b);
-      for (int n = 0; n < iters; ++n) {
-        const int hq = kvh * p.group + (visit0 + n) / n_qt, qt = first_qt + (visit0 + n) % n_qt;
-        const uint32_t s = n % kStagesQ, ph = (n / kStagesQ) & 1;
-        if (!mbar_wait(bar_qe + 8 * s, ph ^ 1, abort_flag)) { fail_role = 1; break; }
-        const uint32_t dst = s_base + kOffQdO + s * 2 * kTile16;
-        mbar_expect_tx(bar_qf + 8 * s, 2 * kTile16);
-        tma_load_4d(dst, &tmQ, bar_qf + 8 * s, 0, hq, qt * BQ, b);
-        tma_load_4d(dst + kTile16, &tmdO, bar_qf + 8 * s, 0, hq, qt * BQ, b);
+      Item it = item0;
+      uint32_t s = 0, ph = 0;
+      bool ok = true;
+      for (int k = 0; ok; ++k) {
+        const uint32_t kv = s_base + ((k & 1) ? kOffKV1 : kOffK);
+        ok = mbar_wait(bar_kve + 8 * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        mbar_expect_tx(bar_kv + 8 * (k & 1), 2 * kTile16);
+        tma_load_4d(kv, &tmK, bar_kv + 8 * (k & 1), 0, it.kvh, it.kt * BKV, it.b);
+        tma_load_4d(kv + kTile16, &tmV, bar_kv + 8 * (k & 1), 0, it.kvh, it.kt * BKV, it.b);
+        for (int n = 0; n < it.iters; ++n) {
+          const int hq = it.kvh * p.group + (it.visit0 + n) / it.n_qt, qt = it.first_qt + (it.visit0 + n) % it.n_qt;
+          ok = mbar_wait(bar_qe + 8 * s, ph ^ 1, abort_flag);
+          if (!ok) break;
+          const uint32_t dst = s_base + kOffQdO + s * 2 * kTile16;
+          mbar_expect_tx(bar_qf + 8 * s, 2 * kTile16);
+          tma_load_4d(dst, &tmQ, bar_qf + 8 * s, 0, hq, qt * BQ, it.b);
+          tma_load_4d(dst + kTile16, &tmdO, bar_qf + 8 * s, 0, hq, qt * BQ, it.b);
+          if (++s == kStagesQ) { s = 0; ph ^= 1; }
+        }
+        if (SPLIT || !p.take || !ok) break;
+        // the next item: asked for when the last operands are on their way, not earlier (the longest CTA would take it)
+        ok = mbar_wait(bar_ne + 8 * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        take_block(answers + 16 * (k & 1), bar_nf + 8 * (k & 1));
+        ok = next_known(k, never_set);  // (has to arrive before the shared memory is given up, whatever the others do)
+        if (!ok) *abort_flag = 1;
+        int x, y, z;
+        if (!ok || !taken_block(answers + 16 * (k & 1), x, y, z)) break;
+        it = item_at(x, y, z);
       }
+      if (!ok) fail_role = 1;
       nnb_release_next();
     }
-    if (warp == 1) {
+    if (warp == 1 && aligned) {
       // ---------------------------------------------------------------- MMA issuer (warp-uniform: see umma_f16_elect)
+      // Its waits are votes: then the compiler knows the answers to be the warp's (with an answer a lane B8 T4096 took 787 us instead of 740,
+      // the products being issued later), and the warp leaves as one.
       const bool el = elect_one();
-      bool ok = mbar_wait(bar_kv, 0, abort_flag);
-      const uint32_t sK = s_base + kOffK, sV = s_base + kOffV, sdS = s_base + kOffdS;
+      const uint32_t sdS = s_base + kOffdS;
       // ring positions of visits n (cur) and n + 1 (nxt) and the phase of nxt, counted along instead of divided out
       uint32_t cur = 0, nxt = 0, nxt_ph = 0;
       auto stage_at = [&](uint32_t s) { return s_base + kOffQdO + s * 2 * kTile16; };
+      auto k_of = [&](int k) { return s_base + ((k & 1) ? kOffKV1 : kOffK); };  // K of item k, V behind it
       // S^T(n) = K Q^T into score buffer n & 1 (K-major operands, 4 k-steps of 16 over head_dim)
-      auto issue_s = [&](int n, uint32_t s) {
+      auto issue_s = [&](uint32_t n, uint32_t s, uint32_t sK) {
         const uint32_t sQ = stage_at(s);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
@@ -185,34 +244,56 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         umma_commit_elect(el, bar_s + 8 * (n & 1));
       };
       // dP^T(n) = V dO^T
-      auto issue_dp = [&](uint32_t s) {
+      auto issue_dp = [&](uint32_t s, uint32_t sV) {
         const uint32_t sdO = stage_at(s) + kTile16;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
           umma_f16_elect(el, tmem_base + kColdP, make_smem_desc(sV + k * 32, 16, 1024), make_smem_desc(sdO + k * 32, 16, 1024), p.idesc_s, k > 0);
         umma_commit_elect(el, bar_dp);
       };
-      if (ok && iters > 0) {
-        ok = mbar_wait(bar_qf, 0, abort_flag);
-        if (ok) {
-          tc_fence_after();
-          issue_s(0, 0);
-          issue_dp(0);
-        }
+      Item it = item0;
+      bool ok = it.iters == 0 || (mbar_wait_warp(bar_kv, 0, abort_flag) && mbar_wait_warp(bar_qf, 0, abort_flag));
+      if (ok && it.iters > 0) {
+        tc_fence_after();
+        issue_s(0, 0, k_of(0));
+        issue_dp(0, k_of(0) + kTile16);
       }
-      for (int n = 0; n < iters && ok; ++n) {
-        const uint32_t sQ = stage_at(cur), sdO = sQ + kTile16;
+      int item = 0, v = 0;  // number of the item, visit within it; n counts visits on over all items
+      for (uint32_t n = 0; ok && it.iters > 0; ++n) {
+        const uint32_t sQ = stage_at(cur), sdO = sQ + kTile16, sK = k_of(item);
+        const bool first = v == 0, last = v == it.iters - 1;
         if (++nxt == kStagesQ) { nxt = 0; nxt_ph ^= 1; }
         // S^T(n + 1) goes into the other score buffer: its scores were read before bar_p(n - 1), its P^T(n - 1) is read by dV(n - 1),
         // which is ahead in order, and its dQ(n - 1) must have been drained. (Waited for in every visit, so that bar_dq is never two
         // phases ahead of the drain.)
-        if (n >= 1 && !mbar_wait(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }
-        if (n + 1 < iters) {
-          if (!mbar_wait(bar_qf + 8 * nxt, nxt_ph, abort_flag)) { ok = false; break; }
+        if (n >= 1 && !mbar_wait_warp(bar_dqr, (n - 1) & 1, abort_flag)) { ok = false; break; }
+        Item next = it;
+        bool known = !last, more = !last, s_next = false;
+        const uint32_t sK_next = last ? k_of(item + 1) : sK;
+        auto operands = [&](bool wait) {  // of visit n + 1, when it begins an item
+          const uint32_t b = bar_kv + 8 * ((item + 1) & 1), ph = ((item + 1) >> 1) & 1;
+          if (!wait) return mbar_test_warp(b, ph) && mbar_test_warp(bar_qf + 8 * nxt, nxt_ph);
+          return mbar_wait_warp(b, ph, abort_flag) && mbar_wait_warp(bar_qf + 8 * nxt, nxt_ph, abort_flag);
+        };
+        if (!last) {
+          if (!mbar_wait_warp(bar_qf + 8 * nxt, nxt_ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          issue_s(n + 1, nxt);
+          issue_s(n + 1, nxt, sK);
+          s_next = true;
+        } else if (SPLIT || !p.take) {
+          known = true;
+        } else if (mbar_test_warp(bar_nf + 8 * (item & 1), (item >> 1) & 1)) {  // the next item, if it is there already: else after this visit's products
+          known = true;
+          more = __all_sync(0xffffffffu, next_known(item, abort_flag)) && next_item(item, next);
+          if (more && operands(false)) {
+            operands(true);
+            tc_fence_after();
+            issue_s(n + 1, nxt, sK_next);
+            s_next = true;
+          }
         }
-        if (!mbar_wait(bar_p, n & 1, abort_flag)) { ok = false; break; }     // P^T(n) is in tensor memory, S^T(n) has been read
+        if (!mbar_wait_warp(bar_p, n & 1, abort_flag)) { ok = false; break; }     // P^T(n) is in tensor memory, S^T(n) has been read
+        if (first && item > 0 && !mbar_wait_warp(bar_acc, (item - 1) & 1, abort_flag)) { ok = false; break; }  // the dK and dV of the item before have been read
         tc_fence_after();
         // dV += P^T dO: A = P^T in tensor memory (16 queries = 8 columns per k-step), B = [query][hd] tile read MN-major (16 query rows =
         // 2048 bytes per step)
@@ -220,8 +301,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k)
           umma_f16_ts_elect(el, tmem_base + kColdV, buf + col_of_queries(k), make_smem_desc(sdO + k * 2048, kTile16, 1024), p.idesc_dkv,
-                            (n > 0 || k > 0) ? 1u : 0u);
-        if (!mbar_wait(bar_ds, n & 1, abort_flag)) { ok = false; break; }    // dS^T(n) is written, dP^T(n) has been read
+                            (!first || k > 0) ? 1u : 0u);
+        if (!mbar_wait_warp(bar_ds, n & 1, abort_flag)) { ok = false; break; }    // dS^T(n) is written, dP^T(n) has been read
         tc_fence_after();
         // dQ(n) = dS K into the middle of the score buffer of this visit: A = [key][query] tile read MN-major (M = queries: two groups of 64,
         // 16 KB apart), B = K tile read MN-major; 8 k-steps of 16 key rows
@@ -234,39 +315,69 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < BQ / 16; ++k)
           umma_f16_ts_elect(el, tmem_base + kColdK, tdS + col_of_queries(k), make_smem_desc(sQ + k * 2048, kTile16, 1024), p.idesc_dkv,
-                            (n > 0 || k > 0) ? 1u : 0u);
+                            (!first || k > 0) ? 1u : 0u);
         umma_commit_elect(el, bar_qe + 8 * cur);
-        if (n + 1 < iters) issue_dp(nxt);   // over dS^T(n), which dK(n), ahead in order, reads; Q / dO of visit n + 1 were awaited above
-        else umma_commit_elect(el, bar_fin);            // one-shot: every product has been accumulated
+        if (last) {
+          umma_commit_elect(el, bar_fin);                      // every product of the item has been accumulated
+          umma_commit_elect(el, bar_kve + 8 * (item & 1));     // its K and V have been read
+          if (!known) {
+            if (!__all_sync(0xffffffffu, next_known(item, abort_flag))) { ok = false; break; }
+            more = next_item(item, next);
+          }
+          if (!more) break;
+          if (!s_next) {
+            if (!operands(true)) { ok = false; break; }
+            tc_fence_after();
+            issue_s(n + 1, nxt, sK_next);
+          }
+        }
+        issue_dp(nxt, sK_next + kTile16);   // over dS^T(n), which dK(n), ahead in order, reads; Q / dO of visit n + 1 were awaited above
         cur = nxt;
+        ++v;
+        if (last) {
+          it = next;
+          ++item;
+          v = 0;
+        }
       }
       if (!ok && lane == 0) fail_role = 2;
     }
-    if (warp == 2) {
+    if (warp == 2 && aligned) {
       // ---------------------------------------------------------------- L and D of a visit's 128 queries, up to two visits ahead:
       // -L log2(e) and -D scale, the addends of the packed multiply-adds
       constexpr float kLog2e = 1.4426950408889634f;
-      const float* gL = g_lse + ((size_t)b * p.H + head0) * p.T;
-      const float* gD = g_delta + ((size_t)b * p.H + head0) * p.T;
-      int qt = qt0;
-      for (int n = 0; n < iters; ++n) {
-        float l[4], d[4];
+      Item it = item0;
+      uint32_t n = 0;
+      bool ok = true;
+      for (int k = 0; ok; ++k) {
+        const float* gL = g_lse + ((size_t)it.b * p.H + it.kvh * p.group + it.visit0 / it.n_qt) * p.T;
+        const float* gD = g_delta + ((size_t)it.b * p.H + it.kvh * p.group + it.visit0 / it.n_qt) * p.T;
+        int qt = it.first_qt + it.visit0 % it.n_qt;
+        for (int v = 0; v < it.iters; ++v, ++n) {
+          float l[4], d[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int qi = qt * BQ + i * 32 + lane;
-          l[i] = qi < p.T ? -gL[qi] * kLog2e : 0.f;
-          d[i] = qi < p.T ? -gD[qi] * p.scale : 0.f;
-        }
-        if (++qt == p.n_q_tiles) { qt = first_qt; gL += p.T; gD += p.T; }
-        if (n >= 2 && !mbar_wait(bar_le + 8 * (n & 1), ((n >> 1) - 1) & 1, abort_flag)) { fail_role = 5; break; }
-        float* dst = s_ld + (n & 1) * 2 * BQ + lane;
+          for (int i = 0; i < 4; ++i) {
+            const int qi = qt * BQ + i * 32 + lane;
+            l[i] = qi < p.T ? -gL[qi] * kLog2e : 0.f;
+            d[i] = qi < p.T ? -gD[qi] * p.scale : 0.f;
+          }
+          if (++qt == p.n_q_tiles) { qt = it.first_qt; gL += p.T; gD += p.T; }
+          if (n >= 2) ok = mbar_wait(bar_le + 8 * (n & 1), ((n >> 1) - 1) & 1, abort_flag);
+          if (!ok) break;
+          float* dst = s_ld + (n & 1) * 2 * BQ + lane;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          dst[i * 32] = l[i];
-          dst[BQ + i * 32] = d[i];
+          for (int i = 0; i < 4; ++i) {
+            dst[i * 32] = l[i];
+            dst[BQ + i * 32] = d[i];
+          }
+          mbar_arrive(bar_lf + 8 * (n & 1));
         }
-        mbar_arrive(bar_lf + 8 * (n & 1));
+        if (SPLIT || !p.take) break;
+        ok = ok && next_known(k, abort_flag);
+        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }  // (the lanes leave together)
+        if (!next_item(k, it)) break;
       }
+      if (!ok) fail_role = 5;
     }
     if constexpr (SPLIT) {  // every thread of the cluster meets twice: see the compute warps
       cluster_sync();
@@ -274,37 +385,83 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp < kComputeWarp0) {
     regs_dec<kRegsDrain>();
-    // ------------------------------------------------------------------ drain warps: the dQ partial tile of every visit
+    // ------------------------------------------------------------------ drain warps: the dQ partial tile of every visit, dV and dK of every item
     // TMEM (score buffer m & 1) -> swizzled fp32 staging (two [128 x 32] boxes) -> TMA reduce-add into the fp32 accumulator
     const int row = (warp & 3) * 32 + lane, sw = row & 7;
     const bool leader = warp == kDrainWarp0 && lane == 0;
-    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColdQ;
+    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     uint8_t* my_stage = smem + kOffStage + row * 128;
-    int hq = head0, qt = qt0;
-    for (int m = 0; m < iters; ++m) {
-      const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
-      tc_fence_after();
-      if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
-      if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }  // all leave together
-      uint32_t r0[32], r1[32];
-      tmem_ld_32x32b_x32(t_row + (m & 1) * BQ, r0);
-      tmem_ld_32x32b_x32(t_row + (m & 1) * BQ + 32, r1);
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(bar_dqr);
+    Item it = item0;
+    uint32_t m = 0;
+    for (int k = 0;; ++k) {
+      int hq = it.kvh * p.group + it.visit0 / it.n_qt, qt = it.first_qt + it.visit0 % it.n_qt;
+      bool left = false;
+      for (int v = 0; v < it.iters; ++v, ++m) {
+        const bool ok = mbar_wait(bar_dq, m & 1, abort_flag);
+        tc_fence_after();
+        if (leader) tma_wait_group_read<0>();      // the previous reduce has finished reading the staging tile
+        if (named_barrier_or(1, kDrainThreads, !ok)) { left = true; break; }  // all leave together
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(t_row + kColdQ + (m & 1) * BQ, r0);
+        tmem_ld_32x32b_x32(t_row + kColdQ + (m & 1) * BQ + 32, r1);
+        tmem_ld_wait();
+        tc_fence_before();
+        mbar_arrive(bar_dqr);
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        *reinterpret_cast<uint4*>(my_stage + ((jj ^ sw) << 4)) = make_uint4(r0[4 * jj], r0[4 * jj + 1], r0[4 * jj + 2], r0[4 * jj + 3]);
-        *reinterpret_cast<uint4*>(my_stage + kTile16 + ((jj ^ sw) << 4)) = make_uint4(r1[4 * jj], r1[4 * jj + 1], r1[4 * jj + 2], r1[4 * jj + 3]);
+        for (int jj = 0; jj < 8; ++jj) {
+          *reinterpret_cast<uint4*>(my_stage + ((jj ^ sw) << 4)) = make_uint4(r0[4 * jj], r0[4 * jj + 1], r0[4 * jj + 2], r0[4 * jj + 3]);
+          *reinterpret_cast<uint4*>(my_stage + kTile16 + ((jj ^ sw) << 4)) = make_uint4(r1[4 * jj], r1[4 * jj + 1], r1[4 * jj + 2], r1[4 * jj + 3]);
+        }
+        fence_proxy_async_smem();
+        named_barrier_sync(1, kDrainThreads);
+        if (leader) {
+          tma_reduce_add_4d(&tmdQacc, s_base + kOffStage, 0, hq, qt * BQ, it.b);
+          tma_reduce_add_4d(&tmdQacc, s_base + kOffStage + kTile16, 32, hq, qt * BQ, it.b);
+          tma_commit_group();
+        }
+        if (++qt == p.n_q_tiles) { qt = it.first_qt; ++hq; }
+      }
+      if (left) { fail_role = 4; break; }
+      if constexpr (SPLIT) break;
+      // The item's dV and dK: TMEM -> 16-bit tiles in the staging tile's place -> TMA store, while the other roles are in the next item
+      bool ok = mbar_wait(bar_fin, k & 1, abort_flag);
+      if (p.take) ok = ok && next_known(k, abort_flag);
+      tc_fence_after();
+      if (leader) tma_wait_group_read<0>();
+      if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }
+      Item next = it;
+      const bool more = p.take && next_item(k, next);
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(t_row + (which == 0 ? kColdV : kColdK), r0);
+        tmem_ld_32x32b_x32(t_row + (which == 0 ? kColdV : kColdK) + 32, r1);
+        tmem_ld_wait();
+        if (which == 1) {
+          tc_fence_before();
+          mbar_arrive(bar_acc);
+          if (p.rope_cos != nullptr && it.kt * BKV + row < p.T) unrotate(r0, r1, it.kt * BKV + row);
+        }
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = (jj & 3) * 8 + 2 * e;
+            w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
+          }
+          *reinterpret_cast<uint4*>(my_stage + which * kTile16 + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
       }
       fence_proxy_async_smem();
       named_barrier_sync(1, kDrainThreads);
       if (leader) {
-        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage, 0, hq, qt * BQ, b);
-        tma_reduce_add_4d(&tmdQacc, s_base + kOffStage + kTile16, 32, hq, qt * BQ, b);
+        tma_store_4d(&tmdV, s_base + kOffStage, 0, it.kvh, it.kt * BKV, it.b);
+        tma_store_4d(&tmdK, s_base + kOffStage + kTile16, 0, it.kvh, it.kt * BKV, it.b);
         tma_commit_group();
       }
-      if (++qt == p.n_q_tiles) { qt = first_qt; ++hq; }
+      if (!more) break;
+      it = next;
     }
     if (leader) tma_wait_group<0>();
     if constexpr (SPLIT) {
@@ -316,168 +473,141 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ------------------------------------------------------------------ compute warps (two threads per key row)
     const int half = (warp - kComputeWarp0) >> 2;  // 0: queries 0..63 / dV; 1: queries 64..127 / dK
     const int q = warp & 3, row = q * 32 + lane, sw = row & 7;
-    const bool leader = half == 0 && row == 0;
     const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
     uint8_t* my_ds = smem + kOffdS + half * kTile16 + row * 128;
-    const int key = kt * BKV + row;
     // A thread works on 32 of its 64 queries and then on the others, in steps of 16. Each 32 leave their P^T (and dS^T) in 16 columns that
     // this thread has read already: for the upper half that takes its last 32 queries first.
     const int first = half * 32;
     auto query = [&](int c) { return (c < 2 ? first : 32 - first) + (c & 1) * 16; };  // first query of step c
     bool ok = true;
     NNB_PROF_DECL;
-    int qt = qt0;
+    Item it = item0;
+    uint32_t n = 0;
     const uint64_t scale2 = pack_f32x2(p.scale, p.scale), scale_log2_2 = pack_f32x2(p.scale_log2, p.scale_log2);
-    for (int n = 0; n < iters && ok; ++n) {
-      NNB_PROF_T0;
-      const int q0 = qt * BQ + half * 64;
-      if (++qt == p.n_q_tiles) qt = first_qt;
-      // Only tiles on the diagonal, past the end of the sequence, or with padded key rows need the
-      // per-element mask; every other tile takes the branch-free version.
-      const bool need_mask = q0 < kt * BKV + BKV - 1 || q0 + 64 > p.T || kt * BKV + BKV > p.T;
-      const uint32_t t_buf = t_lane + kColS + (n & 1) * BQ, t_s = t_buf + half * 64, t_dp = t_lane + kColdP + half * 64;
-      const float* sL = s_ld + (n & 1) * 2 * BQ + half * 64;
-      float prob[64];  // P^T of this thread's 64 queries, kept in fp32 from phase A to phase B
-      // ---- phase A: P^T = exp2(S^T scale log2e - L log2e)
-      if (!mbar_wait(bar_lf + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
-      if (!mbar_wait(bar_s + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      NNB_PROF_ADD(0);
-      auto phase_a = [&](auto masked) {
-        constexpr bool kMask = decltype(masked)::value;
-        uint32_t rs[2][16], pk[16];  // 16 columns at a time, the next load in flight while these are worked on
-        tmem_ld_32x32b_x16(t_s + query(0), rs[0]);
+    for (int k = 0;; ++k) {
+      const int key = it.kt * BKV + row;
+      int qt = it.first_qt + it.visit0 % it.n_qt;
+      for (int v = 0; v < it.iters && ok; ++v, ++n) {
+        NNB_PROF_T0;
+        const int q0 = qt * BQ + half * 64;
+        if (++qt == p.n_q_tiles) qt = it.first_qt;
+        // Only tiles on the diagonal, past the end of the sequence, or with padded key rows need the
+        // per-element mask; every other tile takes the branch-free version.
+        const bool need_mask = q0 < it.kt * BKV + BKV - 1 || q0 + 64 > p.T || it.kt * BKV + BKV > p.T;
+        const uint32_t t_buf = t_lane + kColS + (n & 1) * BQ, t_s = t_buf + half * 64, t_dp = t_lane + kColdP + half * 64;
+        const float* sL = s_ld + (n & 1) * 2 * BQ + half * 64;
+        float prob[64];  // P^T of this thread's 64 queries, kept in fp32 from phase A to phase B
+        // ---- phase A: P^T = exp2(S^T scale log2e - L log2e)
+        if (!mbar_wait(bar_lf + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(bar_s + 8 * (n & 1), (n >> 1) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        NNB_PROF_ADD(0);
+        auto phase_a = [&](auto masked) {
+          constexpr bool kMask = decltype(masked)::value;
+          uint32_t rs[2][16], pk[16];  // 16 columns at a time, the next load in flight while these are worked on
+          tmem_ld_32x32b_x16(t_s + query(0), rs[0]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const ulonglong2* l4 = reinterpret_cast<const ulonglong2*>(sL + query(c));
+            const ulonglong2 l[4] = {l4[0], l4[1], l4[2], l4[3]};  // (arrive while the scores are waited for)
+            tmem_ld_wait(rs[c & 1]);
+            if (c < 3) tmem_ld_32x32b_x16(t_s + query(c + 1), rs[(c + 1) & 1]);
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              const uint64_t s2 = pack_f32x2(__uint_as_float(rs[c & 1][i]), __uint_as_float(rs[c & 1][i + 1]));
+              const float2 e = unpack_f32x2(fma_f32x2(s2, scale_log2_2, (i & 2) ? l[i / 4].y : l[i / 4].x));
+              float p0 = exp2f(e.x), p1 = exp2f(e.y);
+              if (kMask) {
+                const int qi = q0 + query(c) + i;
+                p0 = (key <= qi && qi < p.T && key < p.T) ? p0 : 0.f;
+                p1 = (key <= qi + 1 && qi + 1 < p.T && key < p.T) ? p1 : 0.f;
+              }
+              prob[c * 16 + i] = p0;
+              prob[c * 16 + i + 1] = p1;
+              pk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(p0, p1);
+            }
+            if (c & 1) tmem_st_32x32b_x16(t_buf + half * 96 + query(c - 1) / 2, pk);
+          }
+        };
+        if (need_mask) phase_a(std::true_type{});
+        else phase_a(std::false_type{});
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(bar_p);
+        NNB_PROF_ADD(1);
+        // ---- phase B: dS^T = P^T (dP^T scale - D scale)
+        // (dP^T(n) was issued after dK(n - 1) and dQ(n - 1): once it is complete they have read dS^T)
+        if (!mbar_wait(bar_dp, n & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        NNB_PROF_ADD(2);
+        uint32_t rp[2][16], dk[16];
+        tmem_ld_32x32b_x16(t_dp + query(0), rp[0]);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const ulonglong2* l4 = reinterpret_cast<const ulonglong2*>(sL + query(c));
-          const ulonglong2 l[4] = {l4[0], l4[1], l4[2], l4[3]};  // (arrive while the scores are waited for)
-          tmem_ld_wait(rs[c & 1]);
-          if (c < 3) tmem_ld_32x32b_x16(t_s + query(c + 1), rs[(c + 1) & 1]);
+          const ulonglong2* d4 = reinterpret_cast<const ulonglong2*>(sL + BQ + query(c));
+          const ulonglong2 d[4] = {d4[0], d4[1], d4[2], d4[3]};
+          tmem_ld_wait(rp[c & 1]);
+          if (c < 3) tmem_ld_32x32b_x16(t_dp + query(c + 1), rp[(c + 1) & 1]);
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
-            const uint64_t s2 = pack_f32x2(__uint_as_float(rs[c & 1][i]), __uint_as_float(rs[c & 1][i + 1]));
-            const float2 e = unpack_f32x2(fma_f32x2(s2, scale_log2_2, (i & 2) ? l[i / 4].y : l[i / 4].x));
-            float p0 = exp2f(e.x), p1 = exp2f(e.y);
-            if (kMask) {
-              const int qi = q0 + query(c) + i;
-              p0 = (key <= qi && qi < p.T && key < p.T) ? p0 : 0.f;
-              p1 = (key <= qi + 1 && qi + 1 < p.T && key < p.T) ? p1 : 0.f;
-            }
-            prob[c * 16 + i] = p0;
-            prob[c * 16 + i + 1] = p1;
-            pk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(p0, p1);
+            const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c & 1][i]), __uint_as_float(rp[c & 1][i + 1])), scale2, (i & 2) ? d[i / 4].y : d[i / 4].x);
+            const float2 g = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i], prob[c * 16 + i + 1]), t));
+            dk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(g.x, g.y);
           }
-          if (c & 1) tmem_st_32x32b_x16(t_buf + half * 96 + query(c - 1) / 2, pk);
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj)
+            *reinterpret_cast<uint4*>(my_ds + (((query(c) / 8 + jj) ^ sw) << 4)) =
+                make_uint4(dk[(c & 1) * 8 + 4 * jj], dk[(c & 1) * 8 + 4 * jj + 1], dk[(c & 1) * 8 + 4 * jj + 2], dk[(c & 1) * 8 + 4 * jj + 3]);
+          if (c & 1) tmem_st_32x32b_x16(t_lane + kColdP + half * 96 + query(c - 1) / 2, dk);
         }
-      };
-      if (need_mask) phase_a(std::true_type{});
-      else phase_a(std::false_type{});
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(bar_p);
-      NNB_PROF_ADD(1);
-      // ---- phase B: dS^T = P^T (dP^T scale - D scale)
-      // (dP^T(n) was issued after dK(n - 1) and dQ(n - 1): once it is complete they have read dS^T)
-      if (!mbar_wait(bar_dp, n & 1, abort_flag)) { ok = false; break; }
+        mbar_arrive(bar_le + 8 * (n & 1));
+        fence_proxy_async_smem();
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(bar_ds);
+        NNB_PROF_ADD(3);
+      }
+      if (SPLIT || !p.take) break;
+      ok = ok && next_known(k, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }  // (the lanes leave together)
+      if (!next_item(k, it)) break;
+    }
+    NNB_PROF_FLUSH_N(n);
+    if (!ok) fail_role = 3;
+    if constexpr (SPLIT) {
+      // dV (half 0) and dK (half 1) of this CTA's visits: TMEM -> fp32 tiles in the ring, which every CTA of the cluster then reads for the rows it
+      // adds up and stores
+      const int iters = it.iters;
+      if (ok && iters > 0 && !mbar_wait(bar_fin, 0, abort_flag)) ok = false;
       tc_fence_after();
-      NNB_PROF_ADD(2);
-      uint32_t rp[2][16], dk[16];
-      tmem_ld_32x32b_x16(t_dp + query(0), rp[0]);
+      if (named_barrier_or(2, kComputeThreads, !ok)) {  // all leave together
+        ok = false;
+        fail_role = 3;
+      }
+      if (ok) {
+        uint32_t r0[32], r1[32];
+        if (iters > 0) {
+          tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
+          tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const ulonglong2* d4 = reinterpret_cast<const ulonglong2*>(sL + BQ + query(c));
-        const ulonglong2 d[4] = {d4[0], d4[1], d4[2], d4[3]};
-        tmem_ld_wait(rp[c & 1]);
-        if (c < 3) tmem_ld_32x32b_x16(t_dp + query(c + 1), rp[(c + 1) & 1]);
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const uint64_t t = fma_f32x2(pack_f32x2(__uint_as_float(rp[c & 1][i]), __uint_as_float(rp[c & 1][i + 1])), scale2, (i & 2) ? d[i / 4].y : d[i / 4].x);
-          const float2 g = unpack_f32x2(mul_f32x2(pack_f32x2(prob[c * 16 + i], prob[c * 16 + i + 1]), t));
-          dk[(c & 1) * 8 + (i >> 1)] = pack2_16<F16>(g.x, g.y);
+          for (int i = 0; i < 32; ++i) r0[i] = r1[i] = 0u;
         }
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj)
-          *reinterpret_cast<uint4*>(my_ds + (((query(c) / 8 + jj) ^ sw) << 4)) =
-              make_uint4(dk[(c & 1) * 8 + 4 * jj], dk[(c & 1) * 8 + 4 * jj + 1], dk[(c & 1) * 8 + 4 * jj + 2], dk[(c & 1) * 8 + 4 * jj + 3]);
-        if (c & 1) tmem_st_32x32b_x16(t_lane + kColdP + half * 96 + query(c - 1) / 2, dk);
-      }
-      mbar_arrive(bar_le + 8 * (n & 1));
-      fence_proxy_async_smem();
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(bar_ds);
-      NNB_PROF_ADD(3);
-    }
-    if (ok && iters > 0 && !mbar_wait(bar_fin, 0, abort_flag)) ok = false;
-    tc_fence_after();
-    if (named_barrier_or(2, kComputeThreads, !ok)) {  // all leave together
-      ok = false;
-      fail_role = 3;
-    }
-    NNB_PROF_FLUSH_N(iters);
-    // dV (half 0) and dK (half 1) of this key tile: TMEM -> bf16 staging (reuse the dS^T tiles) -> TMA store; in a cluster
-    // TMEM -> fp32 tiles in the ring, which every CTA of the cluster then reads for the rows it adds up and stores
-    if (ok && (iters > 0 || SPLIT)) {
-      uint32_t r0[32], r1[32];
-      if (iters > 0) {
-        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
-        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) r0[i] = r1[i] = 0u;
-      }
-      if (half == 1 && p.rope_cos != nullptr && kt * BKV + row < p.T) {
-        // dK of key position t leaves through the transpose of the forward rotation: lo' = lo c + hi s, hi' = hi c - lo s
-        const float* cr = g_cos + (size_t)(kt * BKV + row) * (HD / 2);
-        const float* sr = g_sin + (size_t)(kt * BKV + row) * (HD / 2);
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const float4 c4 = __ldg(reinterpret_cast<const float4*>(cr + i)), s4 = __ldg(reinterpret_cast<const float4*>(sr + i));
-          const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float lo = __uint_as_float(r0[i + e]), hi = __uint_as_float(r1[i + e]);
-            r0[i + e] = __float_as_uint(lo * cc[e] + hi * ss[e]);
-            r1[i + e] = __float_as_uint(hi * cc[e] - lo * ss[e]);
-          }
-        }
-      }
-      if constexpr (SPLIT) {
+        if (half == 1 && p.rope_cos != nullptr && it.kt * BKV + row < p.T) unrotate(r0, r1, it.kt * BKV + row);
         uint8_t* mine = smem + kOffQdO + half * 2 * kTile16 + row * 256;  // [128 x 64] fp32, 16-byte units swizzled by the row
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           *reinterpret_cast<uint4*>(mine + ((u ^ sw) << 4)) = make_uint4(r0[4 * u], r0[4 * u + 1], r0[4 * u + 2], r0[4 * u + 3]);
           *reinterpret_cast<uint4*>(mine + 128 + ((u ^ sw) << 4)) = make_uint4(r1[4 * u], r1[4 * u + 1], r1[4 * u + 2], r1[4 * u + 3]);
         }
-      } else {
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = (jj & 3) * 8 + 2 * e;
-            w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
-          }
-          *reinterpret_cast<uint4*>(my_ds + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        fence_proxy_async_smem();
-        named_barrier_sync(2, kComputeThreads);
       }
-      if (leader && !SPLIT) {
-        tma_store_4d(&tmdV, s_base + kOffdS, 0, kvh, kt * BKV, b);
-        tma_store_4d(&tmdK, s_base + kOffdS + kTile16, 0, kvh, kt * BKV, b);
-        tma_commit_group();
-      }
-    }
-    if (leader) tma_wait_group<0>();
-    if constexpr (SPLIT) {
       cluster_sync();  // every CTA's tiles are written
       // 2 tensors x 128 rows x 16 units of four values, 256 units at a time, dealt out to the CTAs; added in the order of the parts
       if (ok) {
         const uint32_t tiles = s_base + kOffQdO;
         for (int u = part * kComputeThreads + (int)threadIdx.x - kComputeWarp0 * 32; u < 2 * BKV * 16; u += kComputeThreads * split) {
-          const int which = u >> 11, r = (u >> 4) & (BKV - 1), c = u & 15, t = kt * BKV + r;
+          const int which = u >> 11, r = (u >> 4) & (BKV - 1), c = u & 15, t = it.kt * BKV + r;
           const uint32_t at = tiles + which * 2 * kTile16 + r * 256 + (c >> 3) * 128 + (((c & 7) ^ (r & 7)) << 4);
           float4 v = load_cluster(at, 0);
           for (int k = 1; k < split; ++k) {
@@ -485,8 +615,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
           }
           if (t < p.T) {
-            uint16_t* out = which == 0 ? static_cast<uint16_t*>(p.dv) + b * p.dv_sb + t * p.dv_st + kvh * p.dv_sh
-                                       : static_cast<uint16_t*>(p.dk) + b * p.dk_sb + t * p.dk_st + kvh * p.dk_sh;
+            uint16_t* out = which == 0 ? static_cast<uint16_t*>(p.dv) + it.b * p.dv_sb + t * p.dv_st + it.kvh * p.dv_sh
+                                       : static_cast<uint16_t*>(p.dk) + it.b * p.dk_sb + t * p.dk_st + it.kvh * p.dk_sh;
             *reinterpret_cast<uint2*>(out + c * 4) = make_uint2(pack2_16<F16>(v.x, v.y), pack2_16<F16>(v.z, v.w));
           }
         }
@@ -694,6 +824,7 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
+  p.take = p.split == 1 && (long long)KVH * B * grid.z > nnb_num_sms();
   if (p.split > 1)
     nnb_launch_clusters(f16 ? flash_bwd_kernel<true, true> : flash_bwd_kernel<false, true>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   // (full grids in plain stream order: an early start measured the same, B32 H12/4 T1024 285-287 us in either form, B128 T256 178-180 / 180)

@@ -196,13 +196,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (s_j == s_n) {
         if (!p.take) { s_end = true; return false; }
         const uint32_t bar = bar_nf + 8 * (s_item & 1), ph = (s_item >> 1) & 1;
-        if (!block && !mbar_test_warp(bar, ph)) return false;
+        if (!block && !mbar_test_warp(bar, ph, __activemask())) return false;
         if (!mbar_wait(bar, ph, abort_flag)) { ok = false; return false; }
         int x, y, z;
         const bool more = next_item(s_item, x, y, z);
         fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_ne + 8 * (s_item & 1));
+        if (el) mbar_arrive(bar_ne + 8 * (s_item & 1));  // (what the elected lane reads is what is done)
         if (!more) { s_end = true; return false; }
         ++s_item;
         s_j = 0;
@@ -211,7 +210,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t qs = s_item % C::kItems;
       if (s_j == 0) {
         const uint32_t ph = (s_item / C::kItems) & 1;
-        if (!block && !(mbar_test_warp(bar_q + 8 * qs, ph) && mbar_test_warp(bar_k + 8 * s_stage, s_ph))) return false;
+        if (!block && !(mbar_test_warp(bar_q + 8 * qs, ph, __activemask()) && mbar_test_warp(bar_k + 8 * s_stage, s_ph, __activemask()))) return false;
         if (!mbar_wait(bar_q + 8 * qs, ph, abort_flag)) { ok = false; return false; }
       }
       if (!mbar_wait(bar_k + 8 * s_stage, s_ph, abort_flag)) { ok = false; return false; }

@@ -210,12 +210,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Whether the phase has completed by now, the same answer for the whole warp.
-__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
+// Whether the phase has completed by now, the same answer for the lanes of `mask` (__activemask() where lanes may have left alone, after a
+// wait that ran out).
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity, uint32_t mask = 0xffffffffu) {
   uint32_t ok;
   asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return __all_sync(0xffffffffu, ok != 0);
+  return __all_sync(mask, ok != 0);
 }
 // Bounded wait. Returns false (and raises *abort_flag, a shared-memory word every role polls) when
 // the phase did not complete within kSpinLimit polls or another role already gave up.
@@ -226,6 +227,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
   *abort_flag = 1;
   return false;
+}
+
+// The same with one answer for the whole warp, which the compiler then knows to be one (its lanes leave together).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 // ---- TMA (tensor maps live in kernel parameters: __grid_constant__ const CUtensorMap)

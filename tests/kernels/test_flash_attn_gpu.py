@@ -54,6 +54,31 @@ def test_forward_of_a_grid_in_several_waves_is_that_of_its_sequences(B, T, hd):
     assert torch.isfinite(o).all() and torch.isfinite(lse).all()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,T", [(75, 64), (74, 65), (160, 1), (90, 17), (50, 129), (27, 300), (10, 1024)])
+def test_backward_of_a_grid_in_several_waves_is_that_of_its_sequences(B, T, hd):
+    """dK and dV of a sequence, summed in the order of its queries, are the same bits in a large call and alone; dQ is reduce-added in the order of
+    arrival, fp32 sums rounded once to 16 bits: at most two neighbouring values apart."""
+    from nanonemo_b200.ops.attention import bwd_raw, fwd_raw
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(B + T)
+    H, KVH = 4, 2
+    q, k, v, do = (torch.randn(B, T, h, hd, device=DEV).bfloat16() for h in (H, KVH, KVH, H))
+    o = torch.empty_like(q)
+    lse = fwd_raw(q, k, v, o, hd**-0.5)
+    got = [torch.full_like(t, float("nan")) for t in (q, k, v)]
+    bwd_raw(q, k, v, o, lse, do, *got, hd**-0.5, in_order=True)
+    check_status()
+    for b in sorted({0, 1, B // 3, B // 2, B - 2, B - 1}):
+        at = slice(b, b + 1)
+        alone = [torch.full_like(t[at], float("nan")) for t in (q, k, v)]
+        bwd_raw(q[at], k[at], v[at], o[at], lse[at].contiguous(), do[at], *alone, hd**-0.5, in_order=True)
+        assert torch.equal(got[1][at], alone[1]) and torch.equal(got[2][at], alone[2])
+        torch.testing.assert_close(got[0][at].float(), alone[0].float(), rtol=2**-7, atol=1e-5)
+    assert all(torch.isfinite(t).all() for t in got)
+
+
 def test_future_keys_do_not_leak():
     from nanonemo_b200 import ops
 
