@@ -42,7 +42,7 @@ const char* nnb_last_error();
 int nnb_gemm_bf16(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, int, int, void*, cudaStream_t);
 int nnb_gemm_rows_rope(const void*, const void*, void*, const void*, const void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, void*, cudaStream_t);
 int nnb_gemm_rows_f32w_serves(int, int, int, int);
-int nnb_gemm_rows_f32w(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
+int nnb_gemm_rows_f32w(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, void*, cudaStream_t);
 int nnb_gemm_rows_f32w_swiglu(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
 int nnb_gemm_swiglu(const void*, const void*, void*, void*, int, int, int, long long, long long, long long, long long, int, void*, cudaStream_t);
 int nnb_gemm_swiglu_act(const void*, const void*, void*, int, int, int, long long, long long, long long, int, void*, cudaStream_t);
@@ -202,8 +202,19 @@ Tensor gemm_f32w(const Tensor& x2, const Tensor& w) {
   reachable({&x2, &w});
   const int64_t M = x2.size(0), N = w.size(0);
   Tensor y = empty({M, N}, x2.scalar_type(), x2);
-  return served(nnb_gemm_rows_f32w(x2.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)w.size(1), x2.stride(0), w.stride(0), N, code16(x2.scalar_type()), status_of(x2),
+  return served(nnb_gemm_rows_f32w(x2.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)w.size(1), x2.stride(0), w.stride(0), N, 0, code16(x2.scalar_type()), status_of(x2),
                                    stream()), "nnb_gemm_rows_f32w") ? y : Tensor();
+}
+// dy2 w, the input gradient of such a product
+Tensor gemm_f32w_dgrad(const Tensor& dy2, const Tensor& w) {
+  if (w.scalar_type() != at::kFloat || w.dim() != 2 || w.stride(1) != 1 || dy2.dim() != 2 || dy2.stride(1) != 1 || dy2.size(1) != w.size(0) || code16(dy2.scalar_type()) < 0 || dy2.numel() == 0 ||
+      w.numel() == 0)
+    return Tensor();
+  reachable({&dy2, &w});
+  const int64_t M = dy2.size(0), N = w.size(1);
+  Tensor dx = empty({M, N}, dy2.scalar_type(), dy2);
+  return served(nnb_gemm_rows_f32w(dy2.data_ptr(), w.data_ptr(), dx.data_ptr(), (int)M, (int)N, (int)w.size(0), dy2.stride(0), w.stride(0), N, 1, code16(dy2.scalar_type()), status_of(dy2),
+                                   stream()), "nnb_gemm_rows_f32w") ? dx : Tensor();
 }
 Tensor gemm_f32w_swiglu(const Tensor& x2, const Tensor& w) {
   if (!from_f32(x2, w) || w.size(0) % 2) return Tensor();
@@ -490,7 +501,8 @@ struct LinearFn : torch::autograd::Function<LinearFn> {
     } else {
       if (engine) engine_gradient(grads[0]);
       dy2 = rowmajor2d(dy2);
-      if (need_dx) dx = gemm_nt(dy2, engine ? ctx->saved_data["w16"].toTensor() : as_dtype(weight, x2.scalar_type()), true);
+      if (need_dx && !engine) dx = gemm_f32w_dgrad(dy2, weight.detach());
+      if (need_dx && !dx.defined()) dx = gemm_nt(dy2, engine ? ctx->saved_data["w16"].toTensor() : as_dtype(weight, x2.scalar_type()), true);
       if (need_dw) dw = weight_gradient(dy2, x2, weight, engine);
     }
     if (dx.defined()) dx = as_dtype(dx.view(x_sizes), x_dtype);
@@ -831,10 +843,10 @@ bool block_of_few_rows(const Tensor& x, const Tensor& delta, const Tensor& norm1
            "nnb_gemm_rows_rope");
   launched(nnb_flash_fwd(v, v + 2 * A, v + 2 * (A + s.KVH * s.hd), o, base + at_lse, (int)s.B, (int)s.T, (int)s.H, (int)s.KVH, (int)s.hd, s.T * row, row, heads, s.T * row, row, heads, s.T * row,
                          row, heads, s.T * A, A, heads, (float)(1.0 / std::sqrt((double)s.hd)), code, status, st), "nnb_flash_fwd");
-  launched(nnb_gemm_rows_f32w(o, wo.data_ptr(), p, m, d, a, a, a, d, code, status, st), "nnb_gemm_rows_f32w");
+  launched(nnb_gemm_rows_f32w(o, wo.data_ptr(), p, m, d, a, a, a, d, 0, code, status, st), "nnb_gemm_rows_f32w");
   launched(nnb_add_rmsnorm_fwd(h, p, norm2.data_ptr(), n, h_out.data_ptr(), rstd, m, d, (float)eps2, 0, code, code, st), "nnb_add_rmsnorm_fwd");
   launched(nnb_gemm_rows_f32w_swiglu(n, w_gu.data_ptr(), act, m, f, d, d, d, f, code, status, st), "nnb_gemm_rows_f32w_swiglu");
-  launched(nnb_gemm_rows_f32w(act, w_down.data_ptr(), y_out.data_ptr(), m, d, f, f, f, d, code, status, st), "nnb_gemm_rows_f32w");
+  launched(nnb_gemm_rows_f32w(act, w_down.data_ptr(), y_out.data_ptr(), m, d, f, f, f, d, 0, code, status, st), "nnb_gemm_rows_f32w");
   return true;
 }
 

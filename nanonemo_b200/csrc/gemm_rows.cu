@@ -12,8 +12,8 @@
 //     of the same features meet in one thread of the epilogue, whose arithmetic on the rounded values is that of the stand-alone kernels;
 //   * a block that waits for the previous kernel (programmatic launch) meanwhile asks for its weight tiles in L2.
 // Roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 convert the weight, then run the epilogue. All waits are bounded.
-// In a row with 24 weights (as a model has them), us, before / now: 201 rows of 768, cast + product of 768 x 768 9.7 / 5.3, + RoPE of 1280 x 768
-// 10.3 + 4.3 / 6.3, + SwiGLU of 4096 x 768 11.0 + 2.2 / 8.7, 768 x 2048 15.7 / 9.4; 16-bit weights: see nnb_rows_tile.
+// In a row with 24 weights (as a model has them), us, before / now: 201 rows of 768, cast + product of 768 x 768 9.7 / 5.1, + RoPE of 1280 x 768
+// 10.3 + 4.3 / 6.3, + SwiGLU of 4096 x 768 11.0 + 2.2 / 8.7, 768 x 2048 15.7 / 9.2; 16-bit weights: see nnb_rows_tile.
 // Replaces the cuBLAS calls behind nn.Linear in the reference's evaluation (nanonemo/model/layers.py:80-83, 128-130).
 #include "common.cuh"
 #include "gemm2.cuh"
@@ -33,7 +33,7 @@ enum RowsEpilogue : int { ROWS_NONE = 0, ROWS_ROPE = 1, ROWS_SWIGLU = 2 };
 // are more tiles than SMs.
 template <int G, bool F32W>
 struct RCfg {
-  static constexpr int BN = 2 * G, SUB = G == 64 ? 1 : 2, BK = SUB * kBlock;
+  static constexpr int BN = 2 * G, SUB = G == 64 || (F32W && G == 32) ? 1 : 2 /* (two stages of 80 KB in fp32: 29 us for 777 x 768 x 4096, five of 40 27) */, BK = SUB * kBlock;
   static constexpr int kBytesA = BM * BK * 2, kBytesW = BN * BK * 2, kBytesF = F32W ? BN * BK * 4 : 0;
   static constexpr int kStageBytes = kBytesA + kBytesF + kBytesW;
   static constexpr int kMaxStages = 225 * 1024 / kStageBytes < 8 ? 225 * 1024 / kStageBytes : 8;
@@ -65,12 +65,12 @@ __device__ __forceinline__ float round16(float x) {
   else return __half2float(__float2half_rn(x));
 }
 
-// BMN: W is stored [K, N] (an input gradient's weight), 16-bit only.
+// BMN: W is stored [K, N] (an input gradient's weight). In fp32 its boxes, [64 K rows][32 columns], are as many and as large as those of 64 weight rows.
 template <int G, bool BF16, bool F32W, bool BMN, int EPI>
 __global__ void __launch_bounds__(kThreads) gemm_rows_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW, const RParams p) {
   using C = RCfg<G, F32W>;
   constexpr int BN = C::BN, BK = C::BK;
-  static_assert(!BMN || (!F32W && G >= 32 && EPI == ROWS_NONE), "");
+  static_assert(!BMN || (G >= 32 && EPI == ROWS_NONE && (!F32W || G == 32)), "");
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t stages = p.stages;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + stages * C::kStageBytes);
@@ -115,8 +115,9 @@ __global__ void __launch_bounds__(kThreads) gemm_rows_kernel(const __grid_consta
       for (int x = 0; x < BK; x += F32W ? 32 : 64) {
         if (kb * BK + x >= p.K) break;
         if (BMN) {
+          if (x % kBlock) continue;
           tma_prefetch_l2_2d(&tmW, r0, kb * BK + x);
-          if (G > 32 && r1 < p.N) tma_prefetch_l2_2d(&tmW, r1, kb * BK + x);
+          if ((G > 32 || F32W) && r1 < p.N) tma_prefetch_l2_2d(&tmW, r1, kb * BK + x);
         } else {
           tma_prefetch_l2_2d(&tmW, kb * BK + x, r0);
           if (EPI != ROWS_NONE || r1 < p.N) tma_prefetch_l2_2d(&tmW, kb * BK + x, r1);
@@ -152,7 +153,9 @@ __global__ void __launch_bounds__(kThreads) gemm_rows_kernel(const __grid_consta
         for (int x = 0; x < BK / 64; ++x) tma_load_2d(sa + x * BM * 128, &tmA, full, kb * BK + x * 64, m0);
 #pragma unroll
         for (int x = 0; x < BK / kWCols; ++x) {
-          if (BMN) {  // [64 K rows][64 columns] boxes, one after the other along the tile's columns
+          if (BMN && F32W) {  // [64 K rows][32 columns] boxes: r0 and r1 are 32 columns apart
+            tma_load_2d(sw + x * BN * 128, &tmW, full, x % 2 ? r1 : r0, kb * BK + x / 2 * kBlock);
+          } else if (BMN) {  // [64 K rows][64 columns] boxes, one after the other along the tile's columns
             tma_load_2d(sw + x * BN * 128, &tmW, full, r0, kb * BK + x * kBlock);
             if (G > 32) tma_load_2d(sw + x * BN * 128 + kBlock * 128, &tmW, full, r1, kb * BK + x * kBlock);
           } else {
@@ -193,19 +196,23 @@ __global__ void __launch_bounds__(kThreads) gemm_rows_kernel(const __grid_consta
         if (!ok) { fail_role = 4; break; }
         const uint8_t* src = smem + s * C::kStageBytes + C::kBytesA;
         uint8_t* dst = smem + s * C::kStageBytes + C::kBytesA + C::kBytesF;
+        constexpr int kUnits = BN * BK / 8 / kWorkThreads;  // all loads before the first store: which the compiler, for all it knows, may overwrite what is to be loaded
+        float4 v[kUnits][2];
 #pragma unroll
-        for (int u = t; u < BN * BK / 8; u += kWorkThreads) {
-          const int r = (u >> 3) % BN, c = u & 7, x = u / (8 * BN), sw = r & 7;  // 16-byte unit c of the 16-bit row of block x = units 2 (c % 4), + 1 of its half c / 4
+        for (int i = 0; i < kUnits; ++i) {
+          const int u = t + i * kWorkThreads, r = (u >> 3) % BN, c = u & 7, x = u / (8 * BN);  // 16-byte unit c of the 16-bit row of block x = units 2 (c % 4), + 1 of its half c / 4
           const uint8_t* row = src + (2 * x + (c >> 2)) * BN * 128 + r * 128;
           const int odd = c >> 2;  // (the lanes of the second half take their units in the other order: eight different bank groups)
-          float4 a = *reinterpret_cast<const float4*>(row + (((2 * (c & 3) + odd) ^ sw) << 4));
-          float4 b = *reinterpret_cast<const float4*>(row + (((2 * (c & 3) + 1 - odd) ^ sw) << 4));
-          if (odd) {
-            const float4 o = a;
-            a = b;
-            b = o;
-          }
-          *reinterpret_cast<uint4*>(dst + x * BN * 128 + r * 128 + ((c ^ sw) << 4)) = make_uint4(pack_rn<BF16>(a.x, a.y), pack_rn<BF16>(a.z, a.w), pack_rn<BF16>(b.x, b.y), pack_rn<BF16>(b.z, b.w));
+          v[i][0] = *reinterpret_cast<const float4*>(row + (((2 * (c & 3) + odd) ^ (r & 7)) << 4));
+          v[i][1] = *reinterpret_cast<const float4*>(row + (((2 * (c & 3) + 1 - odd) ^ (r & 7)) << 4));
+        }
+#pragma unroll
+        for (int i = 0; i < kUnits; ++i) {
+          const int u = t + i * kWorkThreads, r = (u >> 3) % BN, c = u & 7, x = u / (8 * BN);
+          const bool odd = c >> 2;
+          const float4 a = odd ? v[i][1] : v[i][0], b = odd ? v[i][0] : v[i][1];
+          *reinterpret_cast<uint4*>(dst + x * BN * 128 + r * 128 + ((c ^ (r & 7)) << 4)) =
+              make_uint4(pack_rn<BF16>(a.x, a.y), pack_rn<BF16>(a.z, a.w), pack_rn<BF16>(b.x, b.y), pack_rn<BF16>(b.z, b.w));
         }
         fence_proxy_async_smem();
         mbar_arrive(bar_conv + 8 * s);
@@ -333,15 +340,22 @@ int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long l
   CUtensorMap ta, tw;
   if (!nnb_make_tmap_2d(&ta, in_dt, 2, A, M, K, lda * 2, BM, kBlock, "gemm_rows A")) return -4;
   if (BMN) {
-    if (!nnb_make_tmap_2d(&tw, in_dt, 2, W, K, N, ldw * 2, kBlock, kBlock, "gemm_rows W^T")) return -4;
+    if (!nnb_make_tmap_2d(&tw, F32W ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : in_dt, w_bytes, W, K, N, ldw * w_bytes, kBlock, F32W ? 32 : kBlock, "gemm_rows W^T")) return -4;
   } else if (!nnb_make_tmap_2d(&tw, F32W ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : in_dt, w_bytes, W, EPI == ROWS_SWIGLU ? 2 * N : N, K, ldw * w_bytes, g, F32W ? 32 : kBlock, "gemm_rows W")) {
     return -4;
   }
 #define NNB_ROWS(GG) (dtype == NNB_BF16 ? launch_rows<GG, true, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st) : launch_rows<GG, false, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st))
   if constexpr (F32W) {
-    if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU)) return 1;
-    NNB_REQUIRE(g == 16, "gemm_rows: no tile of %d", g);
-    return NNB_ROWS(16);
+    NNB_REQUIRE(g == (BMN ? 32 : 16), "gemm_rows: no tile of %d", g);
+    if constexpr (BMN) {
+      // us in a row, from fp32 / cast + 64-wide tiles: 201 x 768 x 768 6.3 / 6.9, 201 x 2048 x 768 6.7 / 8.4, 777 x 768 x 768 6.7 / 7.0, 777 x 768 x 1280
+      // 9.5 / 9.1, 777 x 768 x 4096 26.7 / 20.1 (a stage waits for its 32 KB of weights to be rounded).
+      if ((long long)tiles * m_blocks > nnb_num_sms() || K > 1024 || (long long)N * K < 1 << 17) return 1;
+      return NNB_ROWS(32);
+    } else {
+      if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU)) return 1;
+      return NNB_ROWS(16);
+    }
   } else {
     NNB_REQUIRE(g == 32 || g == 64, "gemm_rows: no tile of %d", g);
     return g == 32 ? NNB_ROWS(32) : NNB_ROWS(64);
@@ -382,10 +396,12 @@ extern "C" int nnb_gemm_rows_rope(const void* A, const void* W, void* D, const v
               : rows_impl<false, false, ROWS_ROPE>(A, W, D, M, N, K, lda, ldw, ldd, dtype, p, g, status, st);
 }
 
-// D[M, N] = A[M, K] W[N, K]^T with W in fp32, rounded to the dtype of A on the way.
-extern "C" int nnb_gemm_rows_f32w(const void* A, const void* W, void* D, int M, int N, int K, long long lda, long long ldw, long long ldd, int dtype, void* status, cudaStream_t st) {
+// D[M, N] = A[M, K] W[N, K]^T (w_mn: W is stored [K, N]) with W in fp32, rounded to the dtype of A on the way.
+extern "C" int nnb_gemm_rows_f32w(const void* A, const void* W, void* D, int M, int N, int K, long long lda, long long ldw, long long ldd, int w_mn, int dtype, void* status,
+                                  cudaStream_t st) {
   if (!operands_ok(M, N, K, dtype)) return -1;
   RParams p{};
+  if (w_mn) return rows_impl<true, true, ROWS_NONE>(A, W, D, M, N, K, lda, ldw, ldd, dtype, p, 32, status, st);
   return rows_impl<true, false, ROWS_NONE>(A, W, D, M, N, K, lda, ldw, ldd, dtype, p, 16, status, st);
 }
 

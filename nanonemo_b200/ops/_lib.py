@@ -105,7 +105,7 @@ _SIGNATURES = {
     "nnb_gemm_rows": "pppiiiqqqiiipp",
     "nnb_gemm_rows_rope": "pppppiiiqqqiiiiiipp",
     "nnb_gemm_rows_f32w_serves": "iiii",
-    "nnb_gemm_rows_f32w": "pppiiiqqqipp",
+    "nnb_gemm_rows_f32w": "pppiiiqqqiipp",
     "nnb_gemm_rows_f32w_swiglu": "pppiiiqqqipp",
     "nnb_gemm_swiglu": "ppppiiiqqqqipp",
     "nnb_gemm_swiglu_act": "pppiiiqqqipp",
