@@ -11,9 +11,10 @@
 //   * the columns of a tile are two groups of weight rows that may lie apart, so that rotate-half partners (RoPE) or gate and up (SwiGLU)
 //     of the same features meet in one thread of the epilogue, whose arithmetic on the rounded values is that of the stand-alone kernels;
 //   * a block that waits for the previous kernel (programmatic launch) meanwhile asks for its weight tiles in L2.
-// Roles (192 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 convert the weight, then run the epilogue. All waits are bounded.
+// Roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2..9 convert the weight, then run the epilogue (with four of them 201 x 768 x
+// 768 from 16 bits took 4.5 us, now 4.2). All waits are bounded.
 // In a row with 24 weights (as a model has them), us, before / now: 201 rows of 768, cast + product of 768 x 768 9.7 / 5.1, + RoPE of 1280 x 768
-// 10.3 + 4.3 / 6.3, + SwiGLU of 4096 x 768 11.0 + 2.2 / 8.7, 768 x 2048 15.7 / 9.2; 16-bit weights: see nnb_rows_tile.
+// 10.3 + 4.3 / 6.3, + SwiGLU of 4096 x 768 11.0 + 2.2 / 7.3, 768 x 2048 15.7 / 9.2; 16-bit weights: see nnb_rows_tile.
 // Replaces the cuBLAS calls behind nn.Linear in the reference's evaluation (nanonemo/model/layers.py:80-83, 128-130).
 #include "common.cuh"
 #include "gemm2.cuh"
@@ -25,7 +26,7 @@ using namespace sm100;
 
 constexpr int BM = 128;
 constexpr int kBlock = 64;  // K columns of a swizzled operand block
-constexpr int kThreads = 192, kWorkThreads = 128;
+constexpr int kThreads = 320, kWorkThreads = 256;
 enum RowsEpilogue : int { ROWS_NONE = 0, ROWS_ROPE = 1, ROWS_SWIGLU = 2 };
 
 // G: weight rows per group; a tile has 2 G columns. SUB: 64-column blocks of K in a stage (a pass of the MMA warp over its barriers takes as
@@ -228,6 +229,8 @@ __global__ void __launch_bounds__(kThreads) gemm_rows_kernel(const __grid_consta
       float* mine = reinterpret_cast<float*>(smem) + (q * 32 + lane) * C::kRowFloats;
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) {
+        if (BN > 32 && (c & 1) != (t >> 7)) continue;  // (two warps a lane quadrant)
+        if (BN == 32 && t >= 128) break;
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + c * 32, r);
         tmem_ld_wait();
@@ -346,7 +349,7 @@ int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long l
   }
 #define NNB_ROWS(GG) (dtype == NNB_BF16 ? launch_rows<GG, true, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st) : launch_rows<GG, false, F32W, BMN, EPI>(ta, tw, p, tiles, m_blocks, st))
   if constexpr (F32W) {
-    NNB_REQUIRE(g == (BMN ? 32 : 16), "gemm_rows: no tile of %d", g);
+    NNB_REQUIRE(g == (BMN ? 32 : 16) || (EPI == ROWS_SWIGLU && g == 32), "gemm_rows: no tile of %d", g);
     if constexpr (BMN) {
       // us in a row, from fp32 / cast + 64-wide tiles: 201 x 768 x 768 6.3 / 6.9, 201 x 2048 x 768 6.7 / 8.4, 777 x 768 x 768 6.7 / 7.0, 777 x 768 x 1280
       // 9.5 / 9.1, 777 x 768 x 4096 26.7 / 20.1 (a stage waits for its 32 KB of weights to be rounded).
@@ -354,6 +357,9 @@ int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long l
       return NNB_ROWS(32);
     } else {
       if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU)) return 1;
+      if constexpr (EPI == ROWS_SWIGLU) {
+        if (g == 32) return NNB_ROWS(32);
+      }
       return NNB_ROWS(16);
     }
   } else {
@@ -410,5 +416,6 @@ extern "C" int nnb_gemm_rows_f32w_swiglu(const void* A, const void* W, void* act
                                          cudaStream_t st) {
   if (!operands_ok(M, F, K, dtype)) return -1;
   RParams p{};
-  return rows_impl<true, false, ROWS_SWIGLU>(A, W, act, M, F, K, lda, ldw, ldact, dtype, p, 16, status, st);
+  const int g = F % 32 == 0 && (long long)((M + BM - 1) / BM) * (F / 16) > nnb_num_sms() ? 32 : 16;
+  return rows_impl<true, false, ROWS_SWIGLU>(A, W, act, M, F, K, lda, ldw, ldact, dtype, p, g, status, st);
 }
