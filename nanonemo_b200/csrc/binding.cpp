@@ -50,6 +50,8 @@ int nnb_gemm_swiglu_bwd(const void*, const void*, const void*, void*, int, int, 
 int nnb_gemm_rope(const void*, const void*, void*, const void*, const void*, int, int, int, long long, long long, long long, int, int, int, int, void*, cudaStream_t);
 int nnb_gemm_mxfp8(const void*, const void*, const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, int, void*, cudaStream_t);
 int nnb_mxfp8_quantize_sw(const void*, long long, void*, long long, void*, void*, long long, void*, int, int, cudaStream_t);
+int nnb_mxfp8_swiglu(const void*, long long, void*, long long, void*, void*, long long, void*, int, int, cudaStream_t);
+int nnb_mxfp8_swiglu_bwd(const void*, long long, const void*, long long, void*, long long, void*, void*, long long, void*, int, int, cudaStream_t);
 int nnb_add_rmsnorm_fwd(const void*, const void*, const void*, void*, void*, void*, int, int, float, int, int, int, cudaStream_t);
 int nnb_rmsnorm_bwd_blocks();
 int nnb_add_rmsnorm_bwd(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, int, int, int, int, int, int, cudaStream_t);
@@ -325,16 +327,41 @@ void flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& 
 }
 
 // MXFP8: quantised copies (see nanonemo_b200/fp8) and the block-scaled product
-std::tuple<Tensor, Tensor, Tensor, Tensor> quantize_mx(const Tensor& x, bool rowwise, bool colwise) {
+struct Quantized {
+  Tensor q, sf, qt, sft;
+  Quantized(int64_t R, int64_t C, bool rowwise, bool colwise, const Tensor& like) {
+    const int64_t scales = (R / 128) * (C / 128) * 512;
+    if (rowwise) { q = empty({R, C}, at::kByte, like); sf = empty({scales}, at::kByte, like); }
+    if (colwise) { qt = empty({C, R}, at::kByte, like); sft = empty({scales}, at::kByte, like); }
+  }
+  static void* at_(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+};
+Quantized quantize_mx(const Tensor& x, bool rowwise, bool colwise) {
   reachable({&x});
   NNB_ASSERT(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quantize_mx takes bf16 rows");
-  const int64_t R = x.size(0), C = x.size(1), scales = (R / 128) * (C / 128) * 512;
-  Tensor q, sf, qt, sft;
-  if (rowwise) { q = empty({R, C}, at::kByte, x); sf = empty({scales}, at::kByte, x); }
-  if (colwise) { qt = empty({C, R}, at::kByte, x); sft = empty({scales}, at::kByte, x); }
-  auto at_ = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
-  launched(nnb_mxfp8_quantize_sw(x.data_ptr(), x.stride(0), at_(q), C, at_(sf), at_(qt), R, at_(sft), (int)R, (int)C, stream()), "nnb_mxfp8_quantize_sw");
-  return {q, sf, qt, sft};
+  const int64_t R = x.size(0), C = x.size(1);
+  Quantized o(R, C, rowwise, colwise, x);
+  launched(nnb_mxfp8_quantize_sw(x.data_ptr(), x.stride(0), o.at_(o.q), C, o.at_(o.sf), o.at_(o.qt), R, o.at_(o.sft), (int)R, (int)C, stream()), "nnb_mxfp8_quantize_sw");
+  return o;
+}
+// of the activation silu(gate) * up of a packed projection, and of the projection's gradient for a gradient of the activation
+Quantized swiglu_mx(const Tensor& gu, bool rowwise, bool colwise) {
+  reachable({&gu});
+  NNB_ASSERT(gu.dim() == 2 && gu.scalar_type() == at::kBFloat16 && gu.stride(1) == 1 && gu.size(1) % 2 == 0, "swiglu_mx takes bf16 rows");
+  const int64_t R = gu.size(0), F = gu.size(1) / 2;
+  Quantized o(R, F, rowwise, colwise, gu);
+  launched(nnb_mxfp8_swiglu(gu.data_ptr(), gu.stride(0), o.at_(o.q), F, o.at_(o.sf), o.at_(o.qt), R, o.at_(o.sft), (int)R, (int)F, stream()), "nnb_mxfp8_swiglu");
+  return o;
+}
+Quantized swiglu_bwd_mx(const Tensor& dact, const Tensor& gu, bool rowwise, bool colwise) {
+  reachable({&dact, &gu});
+  NNB_ASSERT(gu.dim() == 2 && gu.scalar_type() == at::kBFloat16 && gu.stride(1) == 1 && dact.dim() == 2 && dact.scalar_type() == at::kBFloat16 && dact.stride(1) == 1 &&
+             dact.size(0) == gu.size(0) && 2 * dact.size(1) == gu.size(1), "swiglu_bwd_mx takes bf16 rows that fit");
+  const int64_t R = gu.size(0), F = dact.size(1);
+  Quantized o(R, 2 * F, rowwise, colwise, gu);
+  launched(nnb_mxfp8_swiglu_bwd(dact.data_ptr(), dact.stride(0), gu.data_ptr(), gu.stride(0), o.at_(o.q), 2 * F, o.at_(o.sf), o.at_(o.qt), R, o.at_(o.sft), (int)R, (int)F, stream()),
+           "nnb_mxfp8_swiglu_bwd");
+  return o;
 }
 Tensor gemm_mxfp8(const Tensor& aq, const Tensor& asf, const Tensor& bq, const Tensor& bsf, const optional<Tensor>& out_, at::ScalarType out_dtype, bool accumulate, int k_splits) {
   reachable({&aq, &asf, &bq, &bsf});
@@ -936,10 +963,10 @@ PYBIND11_MODULE(_native, m) {
   }, nogil);
   m.def("flash_fwd", &flash_fwd, nogil);
   m.def("flash_bwd", &flash_bwd, nogil);
-  m.def("quantize_mx", [opt](const Tensor& x, bool r, bool c) {
-    auto [q, s, qt, st] = quantize_mx(x, r, c);
-    return std::make_tuple(opt(q), opt(s), opt(qt), opt(st));
-  }, nogil);
+  auto four = [opt](const Quantized& o) { return std::make_tuple(opt(o.q), opt(o.sf), opt(o.qt), opt(o.sft)); };
+  m.def("quantize_mx", [four](const Tensor& x, bool r, bool c) { return four(quantize_mx(x, r, c)); }, nogil);
+  m.def("swiglu_mx", [four](const Tensor& gu, bool r, bool c) { return four(swiglu_mx(gu, r, c)); }, nogil);
+  m.def("swiglu_bwd_mx", [four](const Tensor& dact, const Tensor& gu, bool r, bool c) { return four(swiglu_bwd_mx(dact, gu, r, c)); }, nogil);
   m.def("gemm_mxfp8", &gemm_mxfp8, nogil);
   m.def("linear", &linear);
   m.def("add_rms_norm", &add_rms_norm);

@@ -161,6 +161,67 @@ class _LinearMXFP8(torch.autograd.Function):
         return dx, dw
 
 
+def _wgrad(weight, dqt, dst, xqt, xst):
+    """dW of an engine weight into the flat gradient buffer, and the strategy told of it."""
+    gemm_mxfp8(dqt, dst, xqt, xst, out=weight._main_grad, accumulate=True)
+    cb = getattr(weight, "_grad_ready_cb", None)
+    if cb is not None:
+        cb(weight, True)
+
+
+class _MLPMXFP8(torch.autograd.Function):
+    """down(silu(gate(x)) * up(x)) on engine weights: the products of two ``_LinearMXFP8``, with the activation and its backward inside the quantisers
+    that follow them (the activation and the gradient of the projection exist in 8 bits only)."""
+
+    @staticmethod
+    def forward(ctx, x, w_gu, w_down):
+        x2 = x.reshape(-1, x.shape[-1])
+        x2 = x2 if x2.dtype == torch.bfloat16 else x2.to(torch.bfloat16)
+        x2 = x2 if x2.stride(-1) == 1 else x2.contiguous()
+        ctx.x_dtype, ctx.k_in = x.dtype, x2.shape[-1]
+        need_x, need_gu, need_down = ctx.flags = ctx.needs_input_grad[:3]
+        xq, xs, xtq, xts = quantize_mx(x2, True, need_gu)
+        gq, gs, gtq, gts = quantized_weight(w_gu, shadow_of(w_gu, torch.bfloat16))
+        gu = gemm_mxfp8(xq, xs, gq, gs)
+        aq, a_s, atq, ats = _lib.native().swiglu_mx(gu, True, need_down)
+        wq, ws, wtq, wts = quantized_weight(w_down, shadow_of(w_down, torch.bfloat16))
+        y = gemm_mxfp8(aq, a_s, wq, ws)
+        below = need_x or need_gu  # something before the activation takes a gradient
+        ctx.save_for_backward(w_gu, w_down, gu if below else None, xtq, xts, *((gtq, gts) if need_x else (None, None)), atq, ats, *((wtq, wts) if below else (None, None)))
+        return y.view(*x.shape[:-1], w_down.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        w_gu, w_down, gu, xtq, xts, gtq, gts, atq, ats, wtq, wts = ctx.saved_tensors
+        need_x, need_gu, need_down = ctx.flags
+        dq, ds, dtq, dts = quantize_mx(dy.reshape(-1, dy.shape[-1]).to(torch.bfloat16).contiguous(), gu is not None, need_down)
+        dact = gemm_mxfp8(dq, ds, wtq, wts) if gu is not None else None
+        if need_down:
+            _wgrad(w_down, dtq, dts, atq, ats)
+        dx = None
+        if gu is not None:
+            dq, ds, dtq, dts = _lib.native().swiglu_bwd_mx(dact, gu, need_x, need_gu)
+            if need_x:
+                dx = gemm_mxfp8(dq, ds, gtq, gts).view(*dy.shape[:-1], ctx.k_in).to(ctx.x_dtype)
+            if need_gu:
+                _wgrad(w_gu, dtq, dts, xtq, xts)
+        return dx, None, None
+
+
+def mlp_mxfp8(x: torch.Tensor, w_gu: torch.Tensor, w_down: torch.Tensor):
+    """The SwiGLU feed-forward with block-scaled products and the activation inside the quantisers, or NotImplemented: outside ``fp8_context``, for
+    shapes that are not multiples of 128, and for weights that are not the engine's (whose gradients nobody differentiates)."""
+    if not _ENABLED or torch.compiler.is_compiling() or not x.is_cuda or x.dim() < 2 or x.numel() == 0:
+        return NotImplemented
+    for w in (w_gu, w_down):
+        main = getattr(w, "_main_grad", None)
+        if main is None or main.dtype != torch.float32:
+            return NotImplemented
+    if not _tensor_core_ok(x.numel() // x.shape[-1], x.shape[-1], w_down.shape[0], w_down.shape[1]) or w_gu.shape != (2 * w_down.shape[1], x.shape[-1]):
+        return NotImplemented
+    return _MLPMXFP8.apply(x, w_gu, w_down)
+
+
 _ENABLED = False
 
 

@@ -17,7 +17,7 @@ import torch.nn.functional as F
 from torch import nn
 from torch.nn.attention import SDPBackend, sdpa_kernel
 
-from nanonemo_b200 import ops
+from nanonemo_b200 import fp8, ops
 from nanonemo_b200.models.config import ModelConfig
 
 
@@ -152,6 +152,13 @@ class Attention(nn.Module):
         return self.wo(y) if project else y
 
 
+def _unwatched(*modules) -> bool:
+    """Whether nobody watches or replaces the forward pass of these modules, so that an operator may take their place."""
+    if torch.nn.modules.module._has_any_global_hook():
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__ for m in modules)
+
+
 def silu_mul(g: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
     return F.silu(g) * u
 
@@ -167,6 +174,7 @@ class MLP(nn.Module):
         self.w_down = make_linear(cfg, cfg.d_ff, cfg.d_model)
         self.act_impl = r.swiglu_kernel
         self.fused = cfg.fuse_epilogues and r.linear_impl == "sm100" and self.act_impl == "sm100"
+        self.fused_mx = cfg.fuse_epilogues and r.linear_impl == "mxfp8" and self.act_impl == "sm100"
         self.tp = None
 
     def split_gu(self):
@@ -184,6 +192,10 @@ class MLP(nn.Module):
             return self.tp.scatter_tokens(self.w_down(ops.swiglu_packed(self.w_gu(full), impl=self.act_impl)))
         if self.fused and x.is_cuda and ops.fused_ok():
             return ops.mlp_swiglu(x, self.w_gu.weight, self.w_down.weight)
+        if self.fused_mx and type(self.w_gu) is type(self.w_down) is Linear and _unwatched(self.w_gu, self.w_down):
+            y = fp8.mlp_mxfp8(x, self.w_gu.weight, self.w_down.weight)
+            if y is not NotImplemented:
+                return y
         return self.w_down(ops.swiglu_packed(self.w_gu(x), impl=self.act_impl))
 
 
@@ -202,17 +214,14 @@ class Block(nn.Module):
     def _one_call(self) -> bool:
         """Whether the block is what it was built as, with every part on the sm100 kernels and nobody watching or replacing the parts."""
         attn, mlp = self.attn, self.mlp
-        if type(attn) is not Attention or type(mlp) is not MLP or type(attn.wo) is not Linear or torch.nn.modules.module._has_any_global_hook():
+        if type(attn) is not Attention or type(mlp) is not MLP or type(attn.wo) is not Linear:
             return False
         if not (attn.fused and mlp.fused and attn.tp is None and mlp.tp is None and attn.wo.impl == "sm100" and ops.fused_ok()):
             return False
         for m in (self.norm_attn, self.norm_mlp):
             if type(m) is not AddRMSNorm or m.impl != "sm100":
                 return False
-        for m in (self.norm_attn, attn, attn.wo, self.norm_mlp, mlp):
-            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__:
-                return False
-        return True
+        return _unwatched(self.norm_attn, attn, attn.wo, self.norm_mlp, mlp)
 
     def forward(self, x, cos, sin, delta=None):
         if not (torch.compiler.is_compiling() or torch.is_grad_enabled()) and x.is_cuda and self._one_call():

@@ -120,6 +120,8 @@ _SIGNATURES = {
     "nnb_gather_b_gemm_bf16": "pppppppiiiiqqqiiiqqipp",
     "nnb_gemm_mxfp8": "pppppiiiqqqiiiipp",
     "nnb_mxfp8_quantize_sw": "pqpqppqpiip",
+    "nnb_mxfp8_swiglu": "pqpqppqpiip",
+    "nnb_mxfp8_swiglu_bwd": "pqpqpqppqpiip",
     "nnb_mxfp8_fake_quant": "ppqiqqp",
     "nnb_mxfp8_quantize": "pppqiqqp",
 }

@@ -190,3 +190,56 @@ def test_gradients_of_an_fp8_step_are_those_of_the_bf16_engine_to_the_operands_r
         moments.append(strategy.store.exp_avg.clone())
     off = (moments[1] - moments[0]).norm() / moments[0].norm()
     assert 0 < off <= 6e-2 * 16 ** 0.5
+
+
+@pytest.mark.parametrize("M,F", [(128, 128), (384, 640), (256, 2048)])
+def test_activation_in_the_quantiser_gives_the_bytes_of_activation_and_quantiser(M, F):
+    from nanonemo_b200 import fp8
+    from nanonemo_b200.ops import _lib, swiglu_act
+
+    torch.manual_seed(0)
+    wide = torch.randn(M, 2 * F + 8, device="cuda").bfloat16() * torch.logspace(-3, 2, M, device="cuda").bfloat16()[:, None]
+    wide[0, :32], wide[1, 5], wide[2, F + 7] = 0.0, 3e38, float("inf")
+    gu, dact = wide[:, : 2 * F], torch.randn(M, F, device="cuda").bfloat16()  # (rows further apart than they are long)
+    act, dgu = torch.empty(M, F, device="cuda", dtype=torch.bfloat16), torch.empty(M, 2 * F, device="cuda", dtype=torch.bfloat16)
+    swiglu_act.fwd_raw(gu[:, :F], gu[:, F:], act)
+    swiglu_act.bwd_raw(dact, gu[:, :F], gu[:, F:], dgu[:, :F], dgu[:, F:])
+    for row, col in ((True, True), (True, False), (False, True)):
+        for got, want in ((_lib.native().swiglu_mx(gu, row, col), fp8.quantize_mx(act, row, col)), (_lib.native().swiglu_bwd_mx(dact, gu, row, col), fp8.quantize_mx(dgu, row, col))):
+            for a, b in zip(got, want):
+                assert (a is None and b is None) or torch.equal(a, b)
+
+
+@pytest.mark.parametrize("trained", ["xgd", "x", "g", "d", "xd", ""])  # the input, the gate and up projection, the down projection
+def test_block_scaled_mlp_in_one_node_is_that_of_its_linears(trained):
+    from nanonemo_b200 import fp8
+    from nanonemo_b200.models.config import ModelConfig
+    from nanonemo_b200.models.layers import MLP
+
+    torch.manual_seed(0)
+    mlp = MLP(ModelConfig.sm100(n_layers=1, vocab_size=512, linear_impl="mxfp8")).to("cuda")
+    told = []
+    for w, name in ((mlp.w_gu.weight, "g"), (mlp.w_down.weight, "d")):
+        w.requires_grad_(name in trained)
+        w._shadow, w._main_grad = w.detach().bfloat16(), torch.zeros_like(w)
+        w._grad_ready_cb = lambda p, direct, name=name: told.append(name)
+    x0, dy = torch.randn(2, 128, mlp.w_gu.in_features, device="cuda").bfloat16(), torch.randn(2, 128, mlp.w_gu.in_features, device="cuda").bfloat16()
+
+    def run():
+        x = x0.clone().requires_grad_("x" in trained)
+        for w in (mlp.w_gu.weight, mlp.w_down.weight):
+            w._main_grad.zero_()
+        told.clear()
+        with fp8.fp8_context()():
+            y = mlp(x)
+        if trained:
+            y.backward(dy)
+        return [y.detach(), x.grad, mlp.w_gu.weight._main_grad.clone(), mlp.w_down.weight._main_grad.clone()], list(told), type(y.grad_fn).__name__
+
+    one, told_one, node = run()
+    hook = mlp.w_down.register_forward_hook(lambda *a: None)  # somebody watches the linears
+    two, told_two, node_two = run()
+    hook.remove()
+    assert told_one == told_two and (not trained or ("MLP" in node and "MLP" not in node_two))
+    for a, b in zip(one, two):
+        assert (a is None and b is None) or torch.equal(a, b)
