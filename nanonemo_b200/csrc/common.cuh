@@ -138,6 +138,22 @@ struct Chunk8<__half> {
   }
 };
 
+// A chunk in global memory, at 32-byte aligned addresses where WIDE: eight fp32 values are then one access of a whole sector a lane instead of
+// two of half a sector.
+template <typename T, bool WIDE>
+struct GlobalChunk8 : Chunk8<T> {};
+template <>
+struct GlobalChunk8<float, true> {
+  static __device__ __forceinline__ void load(const float* p, float (&v)[8]) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+  }
+};
+
 template <typename T> __device__ __forceinline__ T from_f32(float x);
 template <> __device__ __forceinline__ float from_f32<float>(float x) { return x; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }

@@ -5,6 +5,8 @@
 // for the norms) and reads each input exactly once; the roofline for all of them is the HBM3e copy
 // bandwidth. Contracts follow the reference operators (nanonemo/kernels/cuda/rmsnorm.cu:64-167,
 // nanonemo/kernels/triton/{rope,swiglu}.py) with bf16 added (the reference kernels reject it).
+#include <initializer_list>
+
 #include "common.cuh"
 
 // ============================================================================ add + RMSNorm
@@ -22,8 +24,9 @@ __device__ __forceinline__ float row_sum(float v, float (*s_part)[2][2], int pai
 // y = rmsnorm(h) * w,  h = round_to_TX(x + delta);  rstd saved for backward. WPR warps per row (two for rows wider than 1024, so
 // that a lane never holds more than four chunks); lane l of them owns 8-element chunks l, l + 32 WPR, ...; MAXC chunks per lane.
 // HBM-bound. M = 32768, N = 2048, fp32 residual, bf16 delta and y, cold L2: 129 us with two warps a row, 158 with one
-// (floor 123); 8192 rows 41 and 49 us.
-template <typename TX, typename TD, typename TY, int MAXC, int WPR>
+// (floor 123); 8192 rows 41 and 49 us. Whole sectors a lane (WIDE) count where the rows come out of L2: 4096 x 768 7.7 -> 6.3 us, 8192 x 768
+// 13.2 -> 11.5, 32768 x 768 46.5 (the floor) both ways.
+template <typename TX, typename TD, typename TY, int MAXC, int WPR, bool WIDE>
 __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restrict__ x, const TD* __restrict__ delta,
                                                               const float* __restrict__ w, TY* __restrict__ y,
                                                               TX* __restrict__ h, float* __restrict__ rstd, int M,
@@ -42,13 +45,13 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restri
   for (int c = 0; c < MAXC; ++c) {
     const int ch = lane + kLanes * c;
     if (ch < nchunks) {
-      Chunk8<TX>::load(x + base + ch * 8, v[c]);
+      GlobalChunk8<TX, WIDE>::load(x + base + ch * 8, v[c]);
       if (delta != nullptr) {
         float d[8];
         Chunk8<TD>::load(delta + base + ch * 8, d);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[c][i] = to_f32(from_f32<TX>(v[c][i] + d[i]));
-        Chunk8<TX>::store(h + base + ch * 8, v[c]);
+        GlobalChunk8<TX, WIDE>::store(h + base + ch * 8, v[c]);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) ss += v[c][i] * v[c][i];
@@ -77,8 +80,9 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fwd_kernel(const TX* __restri
 // use, so a warp has its whole ~8 KB in flight at once instead of paying the memory latency twice per row, and blocks are
 // 128 threads with at most 128 registers so that four of them (16 warps) share an SM. Rows wider than 1024 take two warps: with one, a
 // row's loads did not fit the registers, the residual gradient was fetched late and only half the warps fitted. With the reduction
-// of dw, cold L2, fp32 residual, bf16 dy and ddelta: M = 32768, N = 2048 278 -> 198 us (floor 164), 8192 rows 99 -> 73 us.
-template <typename TX, typename TD, typename TY, int MAXC, int WPR>
+// of dw, cold L2, fp32 residual, bf16 dy and ddelta: M = 32768, N = 2048 278 -> 198 us (floor 164), 8192 rows 99 -> 73 us. With
+// whole sectors a lane (WIDE) 4096 x 768 14.3 -> 13.7 us, 32768 x 768 70.8 -> 69.6, 8192 x 2048 58.5 -> 56.8.
+template <typename TX, typename TD, typename TY, int MAXC, int WPR, bool WIDE>
 __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __restrict__ dy, const TX* __restrict__ h,
                                                                  const float* __restrict__ rstd,
                                                                  const float* __restrict__ w, const TX* __restrict__ dres,
@@ -104,9 +108,9 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
     for (int c = 0; c < MAXC; ++c) {
       const int ch = lane + kLanes * c;
       if (ch < nchunks) {
-        Chunk8<TX>::load(h + base + ch * 8, n_[c]);
+        GlobalChunk8<TX, WIDE>::load(h + base + ch * 8, n_[c]);
         Chunk8<TY>::load(dy + base + ch * 8, dn[c]);
-        if (dres != nullptr) Chunk8<TX>::load(dres + base + ch * 8, res[c]);
+        if (dres != nullptr) GlobalChunk8<TX, WIDE>::load(dres + base + ch * 8, res[c]);
       }
     }
     const float r = rstd[row];
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(128, 4) add_rmsnorm_bwd_kernel(const TY* __res
         float o[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = r * (dn[c][i] - n_[c][i] * dot) + (dres != nullptr ? res[c][i] : 0.f);
-        Chunk8<TX>::store(dx + base + ch * 8, o);
+        GlobalChunk8<TX, WIDE>::store(dx + base + ch * 8, o);
         if (ddelta != nullptr) Chunk8<TD>::store(ddelta + base + ch * 8, o);
       }
     }
@@ -195,13 +199,27 @@ __global__ void __launch_bounds__(1024) dw_reduce_kernel(const float* __restrict
   X(NNB_F32, NNB_F16, NNB_F16, float, __half, __half)       \
   X(NNB_F16, NNB_F16, NNB_F16, __half, __half, __half)
 
+// fp32 rows whose 8-element chunks start at multiples of 32 bytes (the length of a row is a multiple of eight)
+static bool wide_rows(std::initializer_list<const void*> rows) {
+  for (const void* p : rows)
+    if (reinterpret_cast<uintptr_t>(p) % 32) return false;
+  return true;
+}
+
 template <typename TX, typename TD, typename TY>
 static void rmsnorm_fwd_t(const void* x, const void* delta, const float* w, void* y, void* h, float* rstd, int M, int N,
                           float eps, cudaStream_t st) {
-#define NNB_RMS_FWD(MAXC, WPR) \
-  nnb_launch(add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC, WPR>, (M * WPR + 7) / 8, 256, 0, st, (const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
-  if (N <= 1024) NNB_RMS_FWD(4, 1);
-  else NNB_RMS_FWD(4, 2);
+#define NNB_RMS_FWD(MAXC, WPR, WIDE) \
+  nnb_launch(add_rmsnorm_fwd_kernel<TX, TD, TY, MAXC, WPR, WIDE>, (M * WPR + 7) / 8, 256, 0, st, (const TX*)x, (const TD*)delta, w, (TY*)y, (TX*)h, rstd, M, N, eps)
+  if constexpr (sizeof(TX) == 4) {
+    if (wide_rows({x, delta != nullptr ? h : x})) {
+      if (N <= 1024) NNB_RMS_FWD(4, 1, true);
+      else NNB_RMS_FWD(4, 2, true);
+      return;
+    }
+  }
+  if (N <= 1024) NNB_RMS_FWD(4, 1, false);
+  else NNB_RMS_FWD(4, 2, false);
 #undef NNB_RMS_FWD
 }
 
@@ -232,16 +250,24 @@ extern "C" int nnb_rmsnorm_bwd_blocks() { return 4 * nnb_num_sms(); }  // four 1
 template <typename TX, typename TD, typename TY>
 static int rmsnorm_bwd_t(const void* dy, const void* h, const float* rstd, const float* w, const void* dres, void* dx,
                          void* ddelta, float* partial, int blocks, int M, int N, cudaStream_t st) {
-#define NNB_RMS_BWD(MAXC, WPR)                                                                                    \
+#define NNB_RMS_BWD(MAXC, WPR, WIDE)                                                                              \
   {                                                                                                               \
     const size_t smem = (size_t)N * (1 + 4 / WPR) * sizeof(float); /* the weight, and an accumulator per row in flight */ \
-    auto k = add_rmsnorm_bwd_kernel<TX, TD, TY, MAXC, WPR>;                                                       \
+    auto k = add_rmsnorm_bwd_kernel<TX, TD, TY, MAXC, WPR, WIDE>;                                                 \
     if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -3; \
     nnb_launch(k, blocks, 128, smem, st, (const TY*)dy, (const TX*)h, rstd, w, (const TX*)dres, (TX*)dx, (TD*)ddelta, partial, M, N); \
   }
-  if (N <= 768) NNB_RMS_BWD(3, 1)   // one row fits 3 chunks per lane: fewer registers, more resident warps
-  else if (N <= 1024) NNB_RMS_BWD(4, 1)
-  else NNB_RMS_BWD(4, 2)
+  if constexpr (sizeof(TX) == 4) {
+    if (wide_rows({h, dx, dres})) {
+      if (N <= 768) NNB_RMS_BWD(3, 1, true)   // one row fits 3 chunks per lane: fewer registers, more resident warps
+      else if (N <= 1024) NNB_RMS_BWD(4, 1, true)
+      else NNB_RMS_BWD(4, 2, true)
+      return 0;
+    }
+  }
+  if (N <= 768) NNB_RMS_BWD(3, 1, false)
+  else if (N <= 1024) NNB_RMS_BWD(4, 1, false)
+  else NNB_RMS_BWD(4, 2, false)
 #undef NNB_RMS_BWD
   return 0;
 }

@@ -46,6 +46,29 @@ def test_add_rms_norm_fwd_bwd(M, N, xd, cd, has_delta):
     torch.testing.assert_close(w.grad, wr.grad, rtol=gtol, atol=gtol * max(1.0, M ** 0.5))
 
 
+@pytest.mark.parametrize("M,N", [(3, 8), (9, 768), (5, 1000), (4, 2048)])
+def test_add_rms_norm_of_rows_between_sectors_is_that_of_aligned_rows(M, N):
+    from nanonemo_b200.ops import _lib
+
+    torch.manual_seed(0)
+
+    def at(offset, t):  # the values of t, `offset` fp32 values behind a sector's start
+        room = torch.empty(t.numel() + 8, device=DEV)
+        assert room.data_ptr() % 32 == 0
+        return room[offset : offset + t.numel()].view(t.shape).copy_(t)
+
+    x, dres, w, r = torch.randn(M, N, device=DEV), torch.randn(M, N, device=DEV), torch.randn(N, device=DEV), torch.rand(M, device=DEV)
+    d = torch.randn(M, N, device=DEV).bfloat16()
+    out = []
+    for offset in (0, 4):
+        dw = torch.zeros(N, device=DEV)
+        fwd = _lib.native().rms_fwd(at(offset, x), d, w, 1e-5, torch.bfloat16)
+        bwd = _lib.native().rms_bwd(d, at(offset, x), r, w, at(offset, dres), torch.bfloat16, dw, True)
+        out.append([*fwd, *(t for t in bwd if t is not None), dw])
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("B,T,H,KVH,hd", [(2, 16, 4, 2, 32), (1, 33, 12, 4, 64), (3, 8, 16, 4, 128), (2, 5, 2, 2, 16)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
 def test_rope_qkv(B, T, H, KVH, hd, dtype):
