@@ -197,10 +197,11 @@ Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Ten
 // product); undefined where that is not served.
 bool from_f32(const Tensor& x2, const Tensor& w) {
   return w.scalar_type() == at::kFloat && w.dim() == 2 && w.stride(1) == 1 && x2.dim() == 2 && x2.stride(1) == 1 && x2.size(1) == w.size(1) && code16(x2.scalar_type()) > 0 &&
-         x2.size(0) > 0 && w.size(0) > 0 && w.size(1) > 0;
+         x2.numel() > 0 && w.numel() > 0;
 }
+bool f32w_serves(int64_t M, int64_t N, int64_t K, int kind) { return nnb_gemm_rows_f32w_serves((int)M, (int)N, (int)K, kind) != 0; }
 Tensor gemm_f32w(const Tensor& x2, const Tensor& w) {
-  if (!from_f32(x2, w)) return Tensor();
+  if (!from_f32(x2, w) || !f32w_serves(x2.size(0), w.size(0), w.size(1), 0)) return Tensor();
   reachable({&x2, &w});
   const int64_t M = x2.size(0), N = w.size(0);
   Tensor y = empty({M, N}, x2.scalar_type(), x2);
@@ -210,7 +211,7 @@ Tensor gemm_f32w(const Tensor& x2, const Tensor& w) {
 // dy2 w, the input gradient of such a product
 Tensor gemm_f32w_dgrad(const Tensor& dy2, const Tensor& w) {
   if (w.scalar_type() != at::kFloat || w.dim() != 2 || w.stride(1) != 1 || dy2.dim() != 2 || dy2.stride(1) != 1 || dy2.size(1) != w.size(0) || code16(dy2.scalar_type()) < 0 || dy2.numel() == 0 ||
-      w.numel() == 0)
+      w.numel() == 0 || !f32w_serves(dy2.size(0), w.size(1), w.size(0), 2))
     return Tensor();
   reachable({&dy2, &w});
   const int64_t M = dy2.size(0), N = w.size(1);
@@ -219,7 +220,7 @@ Tensor gemm_f32w_dgrad(const Tensor& dy2, const Tensor& w) {
                                    stream()), "nnb_gemm_rows_f32w") ? dx : Tensor();
 }
 Tensor gemm_f32w_swiglu(const Tensor& x2, const Tensor& w) {
-  if (!from_f32(x2, w) || w.size(0) % 2) return Tensor();
+  if (!from_f32(x2, w) || w.size(0) % 2 || !f32w_serves(x2.size(0), w.size(0) / 2, w.size(1), 1)) return Tensor();
   reachable({&x2, &w});
   const int64_t M = x2.size(0), F = w.size(0) / 2;
   Tensor act = empty({M, F}, x2.scalar_type(), x2);
@@ -227,7 +228,7 @@ Tensor gemm_f32w_swiglu(const Tensor& x2, const Tensor& w) {
                                           status_of(x2), stream()), "nnb_gemm_rows_f32w_swiglu") ? act : Tensor();
 }
 Tensor gemm_f32w_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
-  if (!from_f32(x2, w) || (hd != 64 && hd != 128) || w.size(0) % hd || rope_cols % hd) return Tensor();
+  if (!from_f32(x2, w) || (hd != 64 && hd != 128) || w.size(0) % hd || rope_cols % hd || !f32w_serves(x2.size(0), w.size(0), w.size(1), 0)) return Tensor();
   reachable({&x2, &w, &cos, &sin});
   const int64_t M = x2.size(0), N = w.size(0);
   Tensor y = empty({M, N}, x2.scalar_type(), x2);
@@ -842,14 +843,14 @@ bool block_of_few_rows(const Tensor& x, const Tensor& delta, const Tensor& norm1
   auto fits = [](const Tensor& t, at::ScalarType type, at::IntArrayRef sizes) {
     return t.scalar_type() == type && t.sizes() == sizes && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
   };
-  auto serves = [&](int64_t n, int64_t k, bool swiglu) { return nnb_gemm_rows_f32w_serves((int)M, (int)n, (int)k, swiglu) != 0; };
+  auto serves = [&](int64_t n, int64_t k, int kind) { return f32w_serves(M, n, k, kind); };
   auto table = [&](const Tensor& t) {
     return t.dim() == 2 && t.scalar_type() == at::kFloat && t.is_contiguous() && t.size(0) >= s.T && t.size(1) == s.hd / 2 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
   };
   if (code < 0 || M < 1 || M > 4096 || s.D % 8 || s.D > 2048 || s.F % 16 || (s.hd != 64 && s.hd != 128) || s.KVH < 1 || s.H % s.KVH || !fits(x, at::kFloat, {s.B, s.T, s.D}) ||
       (delta.defined() && !fits(delta, dt, {s.B, s.T, s.D})) || !fits(norm1, at::kFloat, {s.D}) || !fits(norm2, at::kFloat, {s.D}) || !fits(wqkv, at::kFloat, {Q, s.D}) ||
-      !fits(wo, at::kFloat, {s.D, A}) || !fits(w_gu, at::kFloat, {2 * s.F, s.D}) || !fits(w_down, at::kFloat, {s.D, s.F}) || !table(cos) || !table(sin) || !serves(Q, s.D, false) ||
-      !serves(s.D, A, false) || !serves(s.F, s.D, true) || !serves(s.D, s.F, false))
+      !fits(wo, at::kFloat, {s.D, A}) || !fits(w_gu, at::kFloat, {2 * s.F, s.D}) || !fits(w_down, at::kFloat, {s.D, s.F}) || !table(cos) || !table(sin) || !serves(Q, s.D, 0) ||
+      !serves(s.D, A, 0) || !serves(s.F, s.D, 1) || !serves(s.D, s.F, 0))
     return false;
   int64_t bytes = 0;
   auto room = [&](int64_t n) { const int64_t at = bytes; bytes += (n + 255) / 256 * 256; return at; };

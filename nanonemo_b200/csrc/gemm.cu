@@ -657,7 +657,7 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   // 472 / 507 / 780, 4096 x 768 x 50304 255 / 292 / 416, 16384 x 768 x 4096 87 / 99 / 134, 2048^3 23 / 24 / 30; weight gradients likewise
   // (11264 x 2048 x 8192: 318 / 359; 2048 x 2048 x 8192: 57 / 64 / 90). It is not the best one for a 16-bit output whose 128-wide
   // tiles fit one wave, where a tile's latency is all that counts: 1024 x 768 x 768 17 / 17 / 15, 1024 x 768 x 2048 26 / 26 / 22,
-  // 1024 x 2048 x 5632 44 / 46 / 38. The head's input gradient asks for the narrow tile there by its hint.
+  // 1024 x 2048 x 5632 44 / 46 / 38; most of these now go to gemm_rows.cu (nnb_rows_tile).
   if (mode == 0 && bn_hint == 0 && !out_f32 && !a_mn && max_ctas <= 0) {
     if (const int g = nnb_rows_tile(M, N, K, nnb_num_sms())) {
       const int rc = nnb_gemm_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn, dtype, g, status, st);

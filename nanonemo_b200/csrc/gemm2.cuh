@@ -42,7 +42,8 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st);
 
 // The kernel for few rows (gemm_rows.cu): columns of its tile / 2 (32 or 64) for a product with a 16-bit output that it serves faster than the
 // persistent kernels, 0 otherwise. Its tiles are narrow and short-lived: a set-up of 2.3 us against 4 to 5, and the SMs that a few wide tiles
-// would leave idle; with more tiles than SMs it is bound by the bytes an SM takes in. us in a row of products with 24 weights (pair kernel,
+// would leave idle; with more tiles than SMs it is bound by the bytes an SM takes in. us in a row of products with 24 weights, taken with four
+// epilogue warps (the eight it has are 0.3 us faster; pair kernel,
 // single-CTA kernel below 256 rows / 64-wide / 128-wide tiles): 201 x 768 x 768 6.5 / 4.5 / 6.2, 512 x 768 x 2048 13.9 / 8.0 / 10.9, 1024
 // x 768 x 4096 23.0 / 14.4 / 20.1, 512 x 2048 x 11264 54.9 / 39.3 / 56.7, 777 x 1280 x 768 8.1 / 4.9 / 6.4; more 64-wide tiles than SMs:
 // 1024 x 1280 x 768 8.2 / 6.7 / 6.6, 2048 x 768 x 2048 14.3 / 13.9 / 12.3, 512 x 4096 x 768 8.7 / 7.4 / 7.0, 2048 x 768 x 4096 23.2 / 26.1 /

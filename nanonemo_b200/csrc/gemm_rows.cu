@@ -6,7 +6,7 @@
 // a weight that exists in fp32 only (a model that no training engine keeps a 16-bit copy of) cost a launch and three passes over it
 // for the cast. Hence:
 //   * tiles of 128 rows x 32, 64 or 128 columns, each one K loop (the sums, and so the bits, are those of gemm.cu);
-//   * W arrives as it is, fp32 by TMA into a ring, and four warps round it into the swizzled 16-bit operand tile (round to nearest even, the
+//   * W arrives as it is, fp32 by TMA into a ring, and eight warps round it into the swizzled 16-bit operand tile (round to nearest even, the
 //     bits that the cast would give);
 //   * the columns of a tile are two groups of weight rows that may lie apart, so that rotate-half partners (RoPE) or gate and up (SwiGLU)
 //     of the same features meet in one thread of the epilogue, whose arithmetic on the rounded values is that of the stand-alone kernels;
@@ -314,13 +314,16 @@ int launch_rows(const CUtensorMap& ta, const CUtensorMap& tw, RParams p, int til
 
 }  // namespace
 
-// Whether a product of M rows with an fp32 weight of N rows (2 N with `swiglu`) and K columns is taken straight from it, and not from its cast.
+// Whether a product of M rows with an fp32 weight of N rows (kind 0; kind 1, SwiGLU: 2 N) and K columns is taken straight from it, and not from its cast.
 // us, rows straight from fp32 / cast + product: 201 x 768 x 2048 9.5 / 7.9 + 4, 512 x 768 x 2048 10.2 / 8.0 + 4, and more tiles than SMs 201 x
 // 4096 x 768 8.2 / 5.0 + 4, 512 x 1280 x 768 8.0 / 4.7 + 3, 512 x 2048 x 2048 17.9 / 9.0 + 5. Weights below 2^17 elements are cast as ever: 2.3
 // us a call, and tests count their launches.
-extern "C" int nnb_gemm_rows_f32w_serves(int M, int N, int K, int swiglu) {
-  const long long sms = nnb_num_sms(), t = (long long)((M + BM - 1) / BM) * (swiglu ? (N + 15) / 16 : (N + 31) / 32);
-  return (t <= sms || (t <= 2 * sms && K <= 1024)) && (long long)(swiglu ? 2 * N : N) * K >= 1 << 17;
+// Input gradients (kind 2: the weight has K rows and N columns), us in a row, from fp32 / cast + 64-wide tiles: 201 x 768 x 768 6.3 / 6.9, 201 x 2048
+// x 768 6.7 / 8.4, 777 x 768 x 768 6.7 / 7.0, 777 x 768 x 1280 9.5 / 9.1, 777 x 768 x 4096 26.7 / 20.1 (a stage waits for its 32 KB of weights to be
+// rounded).
+extern "C" int nnb_gemm_rows_f32w_serves(int M, int N, int K, int kind) {
+  const long long sms = nnb_num_sms(), cols = kind == 2 ? 64 : kind == 1 ? 16 : 32, t = (long long)((M + BM - 1) / BM) * ((N + cols - 1) / cols);
+  return (kind == 2 ? t <= sms && K <= 1024 : t <= sms || (t <= 2 * sms && K <= 1024)) && (long long)(kind == 1 ? 2 * N : N) * K >= 1 << 17;
 }
 
 namespace {
@@ -351,12 +354,10 @@ int rows_impl(const void* A, const void* W, void* D, int M, int N, int K, long l
   if constexpr (F32W) {
     NNB_REQUIRE(g == (BMN ? 32 : 16) || (EPI == ROWS_SWIGLU && g == 32), "gemm_rows: no tile of %d", g);
     if constexpr (BMN) {
-      // us in a row, from fp32 / cast + 64-wide tiles: 201 x 768 x 768 6.3 / 6.9, 201 x 2048 x 768 6.7 / 8.4, 777 x 768 x 768 6.7 / 7.0, 777 x 768 x 1280
-      // 9.5 / 9.1, 777 x 768 x 4096 26.7 / 20.1 (a stage waits for its 32 KB of weights to be rounded).
-      if ((long long)tiles * m_blocks > nnb_num_sms() || K > 1024 || (long long)N * K < 1 << 17) return 1;
+      if (!nnb_gemm_rows_f32w_serves(M, N, K, 2)) return 1;
       return NNB_ROWS(32);
     } else {
-      if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU)) return 1;
+      if (!nnb_gemm_rows_f32w_serves(M, N, K, EPI == ROWS_SWIGLU ? 1 : 0)) return 1;
       if constexpr (EPI == ROWS_SWIGLU) {
         if (g == 32) return NNB_ROWS(32);
       }
