@@ -82,7 +82,6 @@ struct Params2 {
   int M, N, K;
   int m_pairs, n_blocks, k_splits, kblocks_total, kblocks_per_split;
   int chain;    // EPI_CHAINED: k-blocks per accumulator
-  int split_rows;  // see NnbGemm2Args
   int group_m;  // tile order: groups of group_m 256-row blocks are swept n-block by n-block
   int a_mn, b_mn, out_f32, reduce_add, out_bf16;
   uint32_t idesc;
@@ -720,7 +719,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           named_barrier_sync(epi_bar, kGroup);
           if (et == 0) {
             if (p.reduce_add) tma_reduce_add_2d(&tmD, smem_u32(buf), n_blk * BN + col0, d_row);
-            else tma_store_2d(&tmD, smem_u32(buf), n_blk * BN + col0, d_row + (item - tile * p.k_splits) * p.split_rows);
+            else tma_store_2d(&tmD, smem_u32(buf), n_blk * BN + col0, d_row);
             tma_commit_group();
           }
           if (pending_stores < 2) ++pending_stores;
@@ -795,7 +794,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   const int resident = max_resident_pairs<EPI, BF16>();
   if (resident < 0) return resident;
   const int pairs = min(sms / 2, resident);  // persistent pairs must all be resident at once
-  if (pairs < 1 || (a.M < 2 * BM && a.split_rows == 0) || a.N < BN / 2) return 1;
+  if (pairs < 1 || a.M < 2 * BM || a.N < BN / 2) return 1;
   Params2 p{};
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.m_pairs = (a.M + 2 * BM - 1) / (2 * BM);
@@ -841,8 +840,7 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   p.a_mn = a.a_mn ? 1 : 0;
   p.b_mn = a.b_mn ? 1 : 0;
   p.out_f32 = a.out_f32 ? 1 : 0;
-  p.split_rows = a.split_rows;
-  p.reduce_add = a.split_rows == 0 && (a.accumulate || p.k_splits > 1) ? 1 : 0;
+  p.reduce_add = (a.accumulate || p.k_splits > 1) ? 1 : 0;
   p.out_bf16 = a.dtype == NNB_BF16 ? 1 : 0;
   p.idesc = sm100::make_idesc_f16(a.dtype == NNB_BF16 ? 1 : 0, p.a_mn, p.b_mn, 2 * BM, BN);
   p.status = static_cast<int*>(a.status);
@@ -858,11 +856,11 @@ int launch2(const NnbGemm2Args& a, cudaStream_t st) {
   const int d_cols = EPI == EPI_SWIGLU_BWD ? 2 * a.N : a.N;
   if (EPI == EPI_CE_LOSS) tmD = tmA;  // nothing is stored
   else if (EPI == EPI_SWIGLU_ACT) { if (!nnb_make_tmap_2d(&tmD, in_dt, 2, a.E, a.M, a.N / 2, a.lde * 2, BM, 64, "gemm2 act")) return -4; }
-  else if (!nnb_make_tmap_2d(&tmD, d_dt, d_bytes, a.D, a.split_rows > 0 ? (uint64_t)p.k_splits * a.split_rows : a.M, d_cols, a.ldd * d_bytes, BM, d_box, "gemm2 D")) return -4;
+  else if (!nnb_make_tmap_2d(&tmD, d_dt, d_bytes, a.D, a.M, d_cols, a.ldd * d_bytes, BM, d_box, "gemm2 D")) return -4;
   tmE = tmD;
   if (EPI == EPI_SWIGLU_BWD && !nnb_make_tmap_2d(&tmE, in_dt, 2, a.E, a.M, 2 * a.N, a.lde * 2, BM, 64, "gemm2 gate|up")) return -4;
   if (EPI == EPI_SWIGLU && !nnb_make_tmap_2d(&tmE, in_dt, 2, a.E, a.M, a.N / 2, a.lde * 2, BM, 64, "gemm2 act")) return -4;
-  if (a.out_f32 && !a.accumulate && p.k_splits > 1 && a.split_rows == 0) {
+  if (a.out_f32 && !a.accumulate && p.k_splits > 1) {
     if (a.ldd == a.N) cudaMemsetAsync(a.D, 0, (size_t)a.M * a.N * 4, st);
     else cudaMemset2DAsync(a.D, a.ldd * 4, 0, (size_t)a.N * 4, a.M, st);
   }
@@ -897,64 +895,4 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st) {
     default: nnb_set_error("gemm2: unknown epilogue %d", a.epilogue); return -1;
   }
 #undef NNB_LAUNCH2
-}
-
-// ---- 16-bit products of few rows and a very long K (the head's input gradient: K is the vocabulary), cut along K
-// D[m, n] = sum of the splits' fp32 values in their order, rounded once. Bound by memory: reads splits x 4 bytes, writes 2, in 16-byte accesses.
-template <typename T>
-__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ parts, T* __restrict__ out, int M, int N, long long ldd, int splits, long long part_stride) {
-  nnb_after_previous(parts, out);
-  nnb_release_next();
-  const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * 8;
-  if (i >= (long long)M * N) return;
-  float v[8];
-  Chunk8<float>::load(parts + i, v);
-  for (int s = 1; s < splits; ++s) {
-    float w[8];
-    Chunk8<float>::load(parts + s * part_stride + i, w);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] += w[e];
-  }
-  const long long m = i / N;
-  Chunk8<T>::store(out + m * ldd + (i - m * N), v);
-}
-
-// Splits of K for a product whose tiles leave pairs idle, 1 where cutting it does not pay. A pair takes 0.32 us for a k-block of a tile, and
-// each split's fp32 values are written and read (M N 8 bytes at 5 TB/s) before the sum, 6 us after the product.
-// Head's input gradient, us, one K loop (64-wide tiles up to 1500 rows of 768) / cut: 50304 words x 768, 256 rows 162 / 43 (24 parts), 1000 166 / 70
-// (6), 2048 239 / 109 (3), 4096 251 / 207 (3), 6000 289 / 291 (not cut), 8192 528 / 429; 32000 x 2048, 512 rows 119 / 63, 1536 165 / 135, 2048
-// 172 / 170 (not cut). Error off 64 bits: 2-norm 1.660e-3 of the result both ways (its rounding to 16 bits), but a scale of -3.2e-5 with one sum
-// (the tensor core truncates as it adds, over 786 k-blocks) and +1e-6 with parts (4096 x 768). The gradient norm of a step moves up by that:
-// off 64 bits by -0.8e-4 ... 8.4e-4 from one input to the next, before -1.4e-4 ... 7.8e-4.
-extern "C" int nnb_gemm_split_plan(int M, int N, int K) {
-  const int kb = (K + BK - 1) / BK, pairs = nnb_num_sms() / 2;
-  if (M < 1 || N % 8 || N < BN / 2) return 1;
-  const long long tiles = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-  auto takes = [&](int s) { return (double)((tiles * s + pairs - 1) / pairs) * ((kb + s - 1) / s) * 0.32 + (s > 1 ? 6.0 + s * (double)M * N * 8 / 5e6 : 0.0); };
-  int best = 1;
-  for (int s = 2; s <= 32 && kb / s >= 8; ++s)
-    if ((s - 1) * ((kb + s - 1) / s) < kb && takes(s) < takes(best)) best = s;
-  // one K loop takes less where 64-wide tiles serve (gemm_rows.cu): two thirds
-  const double one = takes(1) * (nnb_rows_tile(M, N, K, nnb_num_sms()) == 32 ? 0.67 : 1.0);
-  return takes(best) < 0.9 * one ? best : 1;
-}
-
-// D[M, N] = A[M, K] B (B stored [K, N] where b_mn, else [N, K]), 16-bit, by `splits` parts of K. parts: fp32 scratch, splits x Mp x N with Mp = M rounded up
-// to 256. The sum has a fixed order: it does not depend on scheduling.
-extern "C" int nnb_gemm_split(const void* A, const void* B, void* D, void* parts, int M, int N, int K, long long lda, long long ldb, long long ldd, int b_mn, int dtype, int splits,
-                              void* status, cudaStream_t st) {
-  const int kb = (K + BK - 1) / BK;
-  NNB_REQUIRE(M > 0 && N >= BN / 2 && N % 8 == 0 && ldd % 8 == 0 && nnb_aligned16(D) && nnb_aligned16(parts) && splits > 1 && (splits - 1) * ((kb + splits - 1) / splits) < kb &&
-                  (dtype == NNB_BF16 || dtype == NNB_F16), "gemm_split: bad problem %dx%dx%d in %d", M, N, K, splits);
-  NnbGemm2Args g{A, B, parts, M, N, K, lda, ldb, N, 0, b_mn, dtype, 1, 0, splits, 0, status};
-  g.split_rows = (M + 255) / 256 * 256;
-  const int rc = dtype == NNB_BF16 ? launch2<EPI_NONE, true>(g, st) : launch2<EPI_NONE, false>(g, st);
-  NNB_REQUIRE(rc <= 0, "gemm_split: no room for a pair of CTAs");
-  if (rc != 0) return rc;
-  const long long values = (long long)M * N;
-  NNB_DISPATCH_16(dtype, T, {
-    nnb_launch(split_sum_kernel<T>, (unsigned)((values / 8 + 255) / 256), 256, 0, st, (const float*)parts, (T*)D, M, N, ldd, splits, (long long)g.split_rows * N);
-  });
-  NNB_LAUNCH_OK("split_sum");
-  return 0;
 }

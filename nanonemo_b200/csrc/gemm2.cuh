@@ -34,7 +34,6 @@ struct NnbGemm2Args {
   const void* targets = nullptr;
   void* target_logit = nullptr;
   int chain = 0;  // EPI_CHAINED: k-blocks per accumulator
-  int split_rows = 0;  // > 0 (fp32 output, a multiple of 256): split s of K is stored on its own, at rows [s split_rows, s split_rows + M) of D
 };
 
 // Returns 0 on success, 1 when the shape is not served by the pair kernel (caller falls back), < 0 on error.

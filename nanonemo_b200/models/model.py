@@ -27,7 +27,6 @@ class NanoNemo(nn.Module):
         self.lm_head = Linear(cfg.d_model, cfg.vocab_size, "sm100" if cfg.uses_sm100("linear_impl") else "torch")
         self.lm_head.weight = self.tok_emb.weight  # tied input/output embedding
         self.loss_impl, self.embed_impl = r.loss_kernel, r.embed_kernel
-        self.in_order = r.linear_impl == "mxfp8"  # block-scaled products multiply a last bit: see models/layers.py, Attention
         self.tp, self.vocab_start = None, 0  # set by parallel.tp.shard_model_
 
         cos, sin = rope_cache(cfg.head_dim, cfg.max_seq_len, cfg.rope_base)
@@ -83,7 +82,7 @@ class NanoNemo(nn.Module):
             x, delta = block(x, self.rope_cos, self.rope_sin, delta)
         h = self.norm_out(x, delta)[0]
         if targets is not None and self.loss_impl == "sm100":
-            loss = ops.linear_cross_entropy(h.reshape(-1, h.size(-1)), self.lm_head.weight, targets.reshape(-1), in_order=self.in_order)
+            loss = ops.linear_cross_entropy(h.reshape(-1, h.size(-1)), self.lm_head.weight, targets.reshape(-1))
             return None, loss
         logits = self.lm_head(h)
         loss = None

@@ -294,15 +294,14 @@ def embedding(idx, weight, impl="torch"):
     return library.embedding(idx, weight, True)
 
 
-def linear_cross_entropy(x, weight, targets, impl="sm100", chunk_rows=None, in_order=False):
-    """Mean next-token cross entropy of ``x @ weight.T`` without materialising the full logits. `in_order`: the gradient of x is one sum over the
-    vocabulary, whatever the number of rows."""
+def linear_cross_entropy(x, weight, targets, impl="sm100", chunk_rows=None):
+    """Mean next-token cross entropy of ``x @ weight.T`` without materialising the full logits."""
     if impl == "torch" or not x.is_cuda:
         return linear_cross_entropy_torch(x, weight, targets)
     if in_flat_store(weight) or getattr(weight, "_shadow", None) is not None:
         from nanonemo_b200.ops.linear_ce import linear_cross_entropy as f
 
-        return f(x, weight, targets, chunk_rows, in_order)
+        return f(x, weight, targets, chunk_rows)
     from nanonemo_b200.ops import library
 
-    return library.linear_cross_entropy(x, weight, targets, chunk_rows, in_order)
+    return library.linear_cross_entropy(x, weight, targets, chunk_rows)

@@ -102,8 +102,6 @@ _SIGNATURES = {
     "nnb_flash_bwd": "pppppppppppiiiiiqqqqqqqqqqqqqqqqqqqqqqqqfippipp",
     "nnb_flash_fwd": "pppppiiiiiqqqqqqqqqqqqfipp",
     "nnb_gemm_bf16": "pppiiiqqqiiiiiiiipp",
-    "nnb_gemm_split_plan": "iii",
-    "nnb_gemm_split": "ppppiiiqqqiiipp",
     "nnb_gemm_rows": "pppiiiqqqiiipp",
     "nnb_gemm_rows_rope": "pppppiiiqqqiiiiiipp",
     "nnb_gemm_rows_f32w_serves": "iiii",

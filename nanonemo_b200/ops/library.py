@@ -466,19 +466,18 @@ _autograd(embedding, _emb_backward, setup_context=_emb_setup)
 
 # ----------------------------------------------------------------------------- fused linear + cross-entropy
 @_operator
-def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int, in_order: bool = False) -> tuple[Tensor, Tensor, Tensor]:
+def linear_ce(x2: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int) -> tuple[Tensor, Tensor, Tensor]:
     """Mean cross-entropy of x2 @ weight^T against targets, and the gradients of that mean with respect to x2 (16-bit)
     and weight (fp32), all produced in the same pass (the logits exist one row chunk at a time, in 16 bits)."""
     w16 = _w16(weight, x2.dtype)
     tg = (targets if targets.dtype == torch.int64 else targets.long()).contiguous()
     dW = torch.empty(weight.shape, dtype=torch.float32, device=x2.device)
-    order = {"in_order": True} if in_order else {}
-    loss_sum, dx = ce_mod.linear_ce_fwd(x2, w16.contiguous(), tg, chunk_rows, dW, **order)
+    loss_sum, dx = ce_mod.linear_ce_fwd(x2, w16.contiguous(), tg, chunk_rows, dW)
     return loss_sum / x2.shape[0], dx, dW
 
 
 @_fake(linear_ce)
-def _(x2, weight, targets, chunk_rows, in_order=False):
+def _(x2, weight, targets, chunk_rows):
     return x2.new_empty((), dtype=torch.float32), torch.empty_like(x2), weight.new_empty(weight.shape, dtype=torch.float32)
 
 
@@ -514,9 +513,9 @@ def _lce_setup(ctx, inputs, output):
 def _lce_backward(ctx, dloss, _ddx, _ddw):
     dx, dW = ctx.saved_tensors
     if dloss is None:
-        return None, None, None, None, None
+        return None, None, None, None
     times = scaled if unpack_dual(dloss).tangent is None else ce_mod.times_upstream  # (`scaled` has no forward-mode formula)
-    return times(dx, dloss), times(dW, dloss).to(ctx.w_dtype), None, None, None
+    return times(dx, dloss), times(dW, dloss).to(ctx.w_dtype), None, None
 
 
 _autograd(linear_ce, _lce_backward, setup_context=_lce_setup)
@@ -534,7 +533,7 @@ def _(x2, weight, targets, chunk_rows):
     return x2.new_empty((), dtype=torch.float32)
 
 
-def linear_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int | None = None, in_order: bool = False) -> Tensor:
+def linear_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, chunk_rows: int | None = None) -> Tensor:
     """x: [N, D]; weight: [V, D] (fp32 master or 16-bit); targets: [N] -> scalar mean loss (fp32)."""
     dt = gemm_mod.compute_dtype()
     x2 = x if x.dtype == dt else x.to(dt)
@@ -542,7 +541,7 @@ def linear_cross_entropy(x: Tensor, weight: Tensor, targets: Tensor, chunk_rows:
         if not torch.compiler.is_compiling() and not gemm_mod.no_backward(x, weight):
             raise NotImplementedError("linear_cross_entropy has no forward-mode derivative")  # as with gradients
         return linear_ce_loss(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
-    loss, _, _ = linear_ce(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS, in_order)
+    loss, _, _ = linear_ce(x2.contiguous(), weight, targets, chunk_rows or ce_mod.DEFAULT_CHUNK_ROWS)
     return loss
 
 

@@ -15,7 +15,7 @@ from functools import lru_cache
 import torch
 
 from nanonemo_b200.ops import _lib
-from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_loss, gemm_ce_stats, no_backward, shadow_of, status_tensor
+from nanonemo_b200.ops.gemm import _CODE, compute_dtype, gemm, gemm_ce_loss, gemm_ce_stats, no_backward, shadow_of
 
 DEFAULT_CHUNK_ROWS = 32768
 
@@ -86,30 +86,9 @@ def _dx_hint(rows: int, width: int, vocab: int, device) -> int:
     return 0 if vocab >= 4096 and -(-rows // 128) * -(-width // 64) <= _sm_count(device) else _dx_tile(rows, width, device)
 
 
-@lru_cache(maxsize=None)
-def _dx_splits(rows: int, width: int, vocab: int) -> int:
-    """Parts of the vocabulary that the input gradient is summed in (see nnb_gemm_split_plan); 1: one sum over all of it."""
-    return _lib.lib().nnb_gemm_split_plan(rows, width, vocab) if vocab >= 4096 else 1
-
-
-def _input_gradient(lg: torch.Tensor, w16: torch.Tensor, out: torch.Tensor, in_order: bool):
-    R, V = lg.shape
-    D = out.shape[1]
-    splits = 1 if in_order else _dx_splits(R, D, V)
-    if splits == 1 or not (lg.stride(1) == 1 and w16.is_contiguous() and lg.stride(0) % 8 == 0):
-        gemm(lg, w16, b_mn=True, out=out, bn=_dx_hint(R, D, V, lg.device))
-        return
-    _lib.reachable(lg, w16, out)
-    parts = torch.empty((splits, -(-R // 256) * 256, D), dtype=torch.float32, device=lg.device)
-    _lib.call("nnb_gemm_split", _lib.ptr(lg), _lib.ptr(w16), _lib.ptr(out), _lib.ptr(parts), _lib.i32(R), _lib.i32(D), _lib.i32(V), _lib.i64(lg.stride(0)),
-              _lib.i64(w16.stride(0)), _lib.i64(out.stride(0)), _lib.i32(1), _lib.i32(_CODE[lg.dtype]), _lib.i32(splits), _lib.ptr(status_tensor(lg.device)),
-              _lib.vp(_lib.stream_ptr()))
-
-
-def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out, in_order=False):
+def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out):
     """Returns (sum of row losses [fp32 scalar], dx [N, D] 16-bit for the MEAN loss); writes the
-    mean-loss weight gradient to dW_out (fp32 [V, D], any content). `in_order`: dx is one sum over the vocabulary whatever the number of rows
-    (few rows otherwise add up the sums of parts of it, in a fixed order: closer to the exact sum, but other last bits)."""
+    mean-loss weight gradient to dW_out (fp32 [V, D], any content)."""
     N, D = x16.shape
     V = w16.shape[0]
     chunk_rows = min(chunk_rows, N)
@@ -126,7 +105,7 @@ def linear_ce_fwd(x16, w16, targets, chunk_rows, dW_out, in_order=False):
         else:
             gemm(xc, w16, out=lg)
             ce_inplace(lg, targets[r0:r1], loss_rows[r0:r1], 1.0 / N)
-        _input_gradient(lg, w16, dx[r0:r1], in_order)
+        gemm(lg, w16, b_mn=True, out=dx[r0:r1], bn=_dx_hint(r1 - r0, D, w16.shape[0], x16.device))
         gemm(lg, xc, a_mn=True, b_mn=True, out=dW_out, accumulate=r0 > 0)
     return loss_rows.sum(), dx
 
@@ -152,7 +131,7 @@ def linear_ce_loss(x16, w16, targets, chunk_rows):
 
 class _LinearCE(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, weight, targets, chunk_rows, in_order):
+    def forward(ctx, x, weight, targets, chunk_rows):
         dt = compute_dtype()
         w16 = shadow_of(weight, dt)
         x16 = x if x.dtype == dt else x.to(dt)
@@ -160,8 +139,7 @@ class _LinearCE(torch.autograd.Function):
         tg = targets if targets.dtype == torch.int64 else targets.long()
         tg = tg if tg.is_contiguous() else tg.contiguous()
         dW = torch.empty(weight.shape, dtype=torch.float32, device=x.device)
-        order = {"in_order": True} if in_order else {}
-        loss_sum, dx = linear_ce_fwd(x16, w16, tg, chunk_rows or DEFAULT_CHUNK_ROWS, dW, **order)
+        loss_sum, dx = linear_ce_fwd(x16, w16, tg, chunk_rows or DEFAULT_CHUNK_ROWS, dW)
         ctx.save_for_backward(dx, dW, weight)
         ctx.x_dtype = x.dtype
         return loss_sum / x.shape[0]
@@ -177,16 +155,16 @@ class _LinearCE(torch.autograd.Function):
                 times_upstream(dW, dloss, out=main)  # readiness of the tied weight is reported by the embedding backward
             else:
                 gw = times_upstream(dW, dloss).to(weight.dtype)
-        return gx, gw, None, None, None
+        return gx, gw, None, None
 
 
-def linear_cross_entropy(x, weight, targets, chunk_rows=None, in_order=False):
+def linear_cross_entropy(x, weight, targets, chunk_rows=None):
     """x: [N, D]; weight: [V, D] (fp32 master or 16-bit); targets: [N] int64 -> scalar mean loss (fp32)."""
     if no_backward(x, weight):
         dt = compute_dtype()
         loss = linear_ce_loss(x.to(dt).contiguous(), shadow_of(weight, dt), targets.long().contiguous(), chunk_rows or DEFAULT_CHUNK_ROWS)
         return loss / x.shape[0]
-    return _LinearCE.apply(x, weight, targets, chunk_rows, in_order)
+    return _LinearCE.apply(x, weight, targets, chunk_rows)
 
 
 # ----------------------------------------------------------------------------- vocabulary-parallel variant
