@@ -18,8 +18,10 @@
 // Items follow one another without a seam: the grid has one block per item, heaviest first, and a block that is running takes over
 // blocks that have not started (cluster launch control: the hardware's own order and balance, no counter in memory). The producer asks
 // when it has requested its item's last keys, loads the next item's Q and first keys while the softmax works on the last ones, and the
-// MMA warp starts the next item's first scores beside the last products, at head_dim 64 into an O accumulator of its own. With a
-// launch per item a CTA spent 4.7 us on set-up, first loads, first and last products and its store, as long as six key tiles.
+// MMA warp starts the next item's first scores right behind the last product, while the softmax stores, at head_dim 64 into an O accumulator of its own. With a
+// launch per item a CTA spent 4.7 us on set-up, first loads, first and last products and its store, as long as six key tiles. (First scores ahead of
+// the last products, where a test found the next item there already: B32 T1024 99.2 us, now 94.4, B8 T4096 307 and 299, B64 T512 64.1 and 60.6, head_dim
+// 128 B64 T256 41.3 and 40.5; and each lane of the MMA warp made that test for itself.)
 // Forward alone, back to back (the card's power limit included), us, a CTA per item / items in sequence: 12/4 heads of 64, B200 T64
 // 30.8 / 17.9, B64 T300 49.4 / 39.3, B64 T512 81.1 / 67.6, B32 T1024 112.5 / 105.5, B8 T4096 322 / 323; 16/4 heads of 128, B64 T256
 // 58.8 / 49.4, B16 T1024 105 / 99, B8 T2048 166 / 160; a grid of one wave (B2 T333) 7.0 / 7.5.
@@ -113,7 +115,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   auto query_tile = [&](int z) { return p.n_q_tiles - 1 - z; };
   auto kv_tiles = [&](int qt) { return min(((qt + 1) * BQ + BN - 1) / BN, kv_total); };  // KV tiles holding keys <= the tile's last row
   // Item i + 1 is the answer in slot i & 1, read by the MMA warp, the four softmax warps and the producer.
-  constexpr int kNextReaders = 5;  // (not the producer, who writes the slot again)
+  constexpr int kNextReaders = 32 + 4;  // lanes of the MMA warp, each for itself, and softmax warps (not the producer, who writes the slot again)
   auto next_item = [&](int i, int& x, int& y, int& z) { return taken_block(answers + 16 * (i & 1), x, y, z); };
 
   if (warp == 0) {  // a barrier a lane
@@ -185,23 +187,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (warp-uniform: see umma_f16_elect)
-    // Two cursors over the CTA's key tiles, numbered on over all items: S (scores) runs up to two tiles ahead of PV (second products).
+    // Two cursors over the CTA's key tiles, numbered on over all items: S (scores) runs up to two tiles ahead of PV (second products). Every lane keeps
+    // both, and nothing that a lane does next depends on when it asks: the order of the products is that of the tiles.
     const bool el = elect_one();
     bool ok = true, s_end = false;
     uint32_t sg = 0, s_stage = 0, s_ph = 0;             // S: tile, its stage and phase
     int s_item = 0, s_j = 0, s_n = kv_tiles(query_tile(blockIdx.z));
     uint32_t first_tile = 0, last_tile = 0, o_of = 0, o_ph = 0;  // per score buffer (bit): what PV has to know of its tile
-    // S_j = Q K_j^T into score buffer sg & 1. Not blocking, it leaves the tile for later when the next item is not there yet.
-    auto issue_s = [&](bool block) -> bool {
+    // S_j = Q K_j^T into score buffer sg & 1.
+    auto issue_s = [&]() -> bool {
       if (s_j == s_n) {
         if (!p.take) { s_end = true; return false; }
         const uint32_t bar = bar_nf + 8 * (s_item & 1), ph = (s_item >> 1) & 1;
-        if (!block && !mbar_test_warp(bar, ph, __activemask())) return false;
         if (!mbar_wait(bar, ph, abort_flag)) { ok = false; return false; }
         int x, y, z;
         const bool more = next_item(s_item, x, y, z);
         fence_proxy_async_smem();
-        if (el) mbar_arrive(bar_ne + 8 * (s_item & 1));  // (what the elected lane reads is what is done)
+        mbar_arrive(bar_ne + 8 * (s_item & 1));  // (each lane for itself)
         if (!more) { s_end = true; return false; }
         ++s_item;
         s_j = 0;
@@ -210,7 +212,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t qs = s_item % C::kItems;
       if (s_j == 0) {
         const uint32_t ph = (s_item / C::kItems) & 1;
-        if (!block && !(mbar_test_warp(bar_q + 8 * qs, ph, __activemask()) && mbar_test_warp(bar_k + 8 * s_stage, s_ph, __activemask()))) return false;
         if (!mbar_wait(bar_q + 8 * qs, ph, abort_flag)) { ok = false; return false; }
       }
       if (!mbar_wait(bar_k + 8 * s_stage, s_ph, abort_flag)) { ok = false; return false; }
@@ -238,8 +239,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     };
     uint32_t s = 0, ph = 0;
     for (uint32_t g = 0;; ++g) {  // PV: tile
-      while (ok && !s_end && sg < g + 2) {
-        if (!issue_s(sg == g)) break;  // (score buffer sg & 1 was released by the bar_p of tile sg - 2 below)
+      // (score buffer sg & 1 was released by the bar_p of tile sg - 2 below; the next item's first scores follow this item's last second product)
+      while (ok && !s_end && sg < g + 2 && (s_j < s_n || sg == g)) {
+        if (!issue_s()) break;
       }
       if (!ok || sg == g) break;
       const uint32_t pb = g & 1;

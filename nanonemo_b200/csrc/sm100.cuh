@@ -210,13 +210,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Whether the phase has completed by now, the same answer for the lanes of `mask` (__activemask() where lanes may have left alone, after a
-// wait that ran out).
-__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity, uint32_t mask = 0xffffffffu) {
+// Whether the phase has completed by now, one answer for the whole warp. (Not over __activemask(): lanes that leave a wait apart would vote apart,
+// get different answers and go different ways.)
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return __all_sync(mask, ok != 0);
+  return __all_sync(0xffffffffu, ok != 0);
 }
 // Bounded wait. Returns false (and raises *abort_flag, a shared-memory word every role polls) when
 // the phase did not complete within kSpinLimit polls or another role already gave up.
