@@ -22,9 +22,8 @@
 // launch per item a CTA spent 4.7 us on set-up, first loads, first and last products and its store, as long as six key tiles. (First scores ahead of
 // the last products, where a test found the next item there already: B32 T1024 99.2 us, now 94.4, B8 T4096 307 and 299, B64 T512 64.1 and 60.6, head_dim
 // 128 B64 T256 41.3 and 40.5; and each lane of the MMA warp made that test for itself.)
-// Forward alone, back to back (the card's power limit included), us, a CTA per item / items in sequence: 12/4 heads of 64, B200 T64
-// 30.8 / 17.9, B64 T300 49.4 / 39.3, B64 T512 81.1 / 67.6, B32 T1024 112.5 / 105.5, B8 T4096 322 / 323; 16/4 heads of 128, B64 T256
-// 58.8 / 49.4, B16 T1024 105 / 99, B8 T2048 166 / 160; a grid of one wave (B2 T333) 7.0 / 7.5.
+// Forward alone, in a row, us, a CTA per item / items in sequence: 12/4 heads of 64, B200 T64 30.5 / 17.8, B64 T300 49.1 / 36.2, B64 T512 81.3 / 60.8,
+// B32 T1024 112.7 / 94.2, B8 T4096 305 / 296; 16/4 heads of 128, B64 T256 56.0 / 40.9, B16 T1024 90 / 82.5, B8 T2048 142 / 137 to 143 (power).
 // Outputs: O (16 bits) through a swizzled staging tile + TMA store, and L = m * scale + ln(l) per row (fp32)
 // for the backward pass. Every mbarrier wait is bounded; on expiry the kernel records a status word
 // and leaves cleanly.
@@ -48,7 +47,8 @@ constexpr int BQ = 128;  // query rows per tile (= TMEM lanes)
 constexpr int kThreads = 192;
 constexpr int kSoftmaxThreads = 128;
 
-template <int HD>
+// TAKE: a CTA goes on to blocks that have not started (nnb_flash_fwd has the rule).
+template <int HD, bool TAKE>
 struct FCfg {
   static constexpr int BN = 64;                             // keys per KV tile
   // K and V have rings of their own: K_j is free once S_j has been computed, V_j only after P_j V_j. Two CTAs per SM at both head
@@ -59,11 +59,13 @@ struct FCfg {
   static constexpr int kKBytes = BN * HD * 2;
   static constexpr int kVBytes = BN * HD * 2;
   // Q tiles, and O accumulators in tensor memory: two where they fit twice beside the rest, so that the next item starts early
-  static constexpr int kItems = HD == 64 ? 2 : 1;
-  static constexpr int kOBytes = BQ * 128;                  // staging of 64 columns of O
+  static constexpr int kItems = TAKE && HD == 64 ? 2 : 1;
+  static constexpr int kOBytes = TAKE ? BQ * 128 : 0;       // staging of 64 columns of O; a CTA with one item stages all of O where its Q was
   static constexpr int kBarBytes = 512;
-  // 113 KB a CTA is what two per SM leave: nothing to spare at head_dim 128 for aligning the base, which the kernel checks instead
-  static constexpr int kSmem = kItems * kQBytes + kStages * (kKBytes + kVBytes) + kOBytes + kBarBytes;
+  // 113 KB a CTA is what two per SM leave: nothing to spare for aligning the base at head_dim 128 with the staging tile. There the kernel checks it,
+  // which costs a CTA 0.1 us.
+  static constexpr int kSpare = TAKE && HD == 128 ? 0 : 1024;
+  static constexpr int kSmem = kItems * kQBytes + kStages * (kKBytes + kVBytes) + kOBytes + kBarBytes + kSpare;
   static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
   static constexpr int kColS = 0;                           // S buffers at columns 0 and 64; P_j takes the first 32 of S_j's
   static constexpr int kColO = 128;                         // O accumulators from column 128
@@ -73,7 +75,6 @@ struct FCfg {
 struct FParams {
   int B, H, KVH, T;
   int n_q_tiles;
-  int take;           // the grid has more blocks than run at once: blocks take over others
   float scale_log2;   // softmax scale * log2(e)
   float scale;        // softmax scale
   float* lse;         // [B, H, T]
@@ -81,17 +82,17 @@ struct FParams {
   int* status;
 };
 
-template <int HD, bool F16>
+template <int HD, bool F16, bool TAKE>
 __global__ void __launch_bounds__(kThreads, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FParams p) {
-  using C = FCfg<HD>;
+  using C = FCfg<HD, TAKE>;
   constexpr int BN = C::BN;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sQ = smem;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* sQ = C::kSpare == 0 ? smem_raw : reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sKV = sQ + C::kItems * C::kQBytes;                  // [stages][K | V]
-  uint8_t* sO = sKV + C::kStages * (C::kKBytes + C::kVBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + C::kOBytes);
+  uint8_t* sO = TAKE ? sKV + C::kStages * (C::kKBytes + C::kVBytes) : sQ;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + C::kStages * (C::kKBytes + C::kVBytes) + C::kOBytes);
   // k_full[S], v_full[S], k_empty[S], v_empty[S], s_full[2], p_full[2], o_tile, o_all, q_full[2], q_empty[2], o_empty[2], next_full[2], next_empty[2]
   const uint32_t bar_k = smem_u32(bars), bar_v = bar_k + 8 * C::kStages;
   const uint32_t bar_ke = bar_v + 8 * C::kStages, bar_ve = bar_ke + 8 * C::kStages;
@@ -105,7 +106,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* never_set = abort_flag + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (smem_u32(smem) & 1023) {  // (swizzled tiles: see kSmem)
+  if (C::kSpare == 0 && (smem_u32(sQ) & 1023)) {  // (swizzled tiles)
     if (threadIdx.x == 0 && p.status != nullptr && atomicCAS(p.status, 0, 2) == 0) p.status[1] = 6;
     return;
   }
@@ -153,7 +154,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int i = 0;; ++i) {
         const int qt = query_tile(z), kvh = h / (p.H / p.KVH), n_kv = kv_tiles(qt);
         const int qs = i % C::kItems;
-        ok = mbar_wait(bar_qe + 8 * qs, ((i / C::kItems) & 1) ^ 1, abort_flag);
+        if (TAKE) ok = mbar_wait(bar_qe + 8 * qs, ((i / C::kItems) & 1) ^ 1, abort_flag);
         if (!ok) break;
         mbar_expect_tx(bar_q + 8 * qs, C::kQBytes);
 #pragma unroll
@@ -172,7 +173,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int c = 0; c < HD / 64; ++c) tma_load_4d(sv + c * (BN * 128), &tmV, bar_v + 8 * s, c * 64, kvh, j * BN, b);
           if (++s == C::kStages) { s = 0; ph ^= 1; }
         }
-        if (!ok || !p.take) break;
+        if (!TAKE || !ok) break;
         // not earlier: a block that is asked for at the beginning of a long item would go to the busiest CTA
         ok = mbar_wait(bar_ne + 8 * (i & 1), ((i >> 1) & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -197,7 +198,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // S_j = Q K_j^T into score buffer sg & 1.
     auto issue_s = [&]() -> bool {
       if (s_j == s_n) {
-        if (!p.take) { s_end = true; return false; }
+        if (!TAKE) { s_end = true; return false; }
         const uint32_t bar = bar_nf + 8 * (s_item & 1), ph = (s_item >> 1) & 1;
         if (!mbar_wait(bar, ph, abort_flag)) { ok = false; return false; }
         int x, y, z;
@@ -246,9 +247,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (!ok || sg == g) break;
       const uint32_t pb = g & 1;
       if (!mbar_wait(bar_v + 8 * s, ph, abort_flag)) { ok = false; break; }
-      const bool first = (first_tile >> pb) & 1, last = (last_tile >> pb) & 1;
-      const uint32_t ob = (o_of >> pb) & 1;
-      if (first && !mbar_wait(bar_oe + 8 * ob, ((o_ph >> pb) & 1) ^ 1, abort_flag)) { ok = false; break; }  // the item before has taken its O
+      const bool first = TAKE ? (first_tile >> pb) & 1 : g == 0, last = TAKE ? (last_tile >> pb) & 1 : (int)g == s_n - 1;
+      const uint32_t ob = TAKE ? (o_of >> pb) & 1 : 0;
+      if (TAKE && first && !mbar_wait(bar_oe + 8 * ob, ((o_ph >> pb) & 1) ^ 1, abort_flag)) { ok = false; break; }  // the item before has taken its O
       if (!mbar_wait(bar_p + 8 * pb, (g >> 1) & 1, abort_flag)) { ok = false; break; }   // P_j written, S_j consumed, O rescaled if needed
       tc_fence_after();
       const uint32_t sv = smem_u32(sKV) + s * (C::kKBytes + C::kVBytes) + C::kKBytes;
@@ -282,21 +283,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-template <int HD, bool F16>
-int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, FParams p,
-               cudaStream_t st) {
-  auto kern = flash_fwd_kernel<HD, F16>;
+template <int HD, bool F16, bool TAKE>
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const FParams& p, cudaStream_t st) {
+  auto kern = flash_fwd_kernel<HD, F16, TAKE>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FCfg<HD>::kSmem) != cudaSuccess) {
-      nnb_set_error("flash_fwd: cannot reserve %d bytes of shared memory", FCfg<HD>::kSmem);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FCfg<HD, TAKE>::kSmem) != cudaSuccess) {
+      nnb_set_error("flash_fwd: cannot reserve %d bytes of shared memory", FCfg<HD, TAKE>::kSmem);
       return -3;
     }
     configured = true;
   }
-  dim3 grid(p.H, p.B, p.n_q_tiles);
-  p.take = (long long)p.H * p.B * p.n_q_tiles > 2 * nnb_num_sms();  // (asking costs a grid of one wave 0.8 of 7 us)
-  nnb_launch(kern, grid, kThreads, FCfg<HD>::kSmem, st, tq, tk, tv, to, p);
+  nnb_launch(kern, dim3(p.H, p.B, p.n_q_tiles), kThreads, FCfg<HD, TAKE>::kSmem, st, tq, tk, tv, to, p);
   return 0;
 }
 
@@ -328,8 +326,13 @@ extern "C" int nnb_flash_fwd(const void* q, const void* k, const void* v, void* 
   p.idesc_qk = sm100::make_idesc_f16(f16 ? 0 : 1, 0, 0, BQ, BN);
   p.idesc_pv = sm100::make_idesc_f16(f16 ? 0 : 1, 0, 1, BQ, hd);
   p.status = static_cast<int*>(status);
-  const int rc = hd == 64 ? (f16 ? launch_fwd<64, true>(tq, tk, tv, to, p, st) : launch_fwd<64, false>(tq, tk, tv, to, p, st))
-                          : (f16 ? launch_fwd<128, true>(tq, tk, tv, to, p, st) : launch_fwd<128, false>(tq, tk, tv, to, p, st));
+  // A grid that runs at once has nothing to take over, and an instance without what that takes. us, in a row, that instance / the other one, with
+  // a switch at run time: 12/4 heads of 64, B2 T333 6.7 / 7.3, B1 T201 5.4 / 5.85, B1 T1024 13.2 / 14.5, 16/4 heads of 128, B1 T200 6.2 / 6.6, B1 T1000
+  // 14.5 / 15.8. Asking costs 0.8 more.
+  const bool take = (long long)H * B * p.n_q_tiles > 2 * nnb_num_sms();
+#define NNB_FWD(HD, F16) (take ? launch_fwd<HD, F16, true>(tq, tk, tv, to, p, st) : launch_fwd<HD, F16, false>(tq, tk, tv, to, p, st))
+  const int rc = hd == 64 ? (f16 ? NNB_FWD(64, true) : NNB_FWD(64, false)) : (f16 ? NNB_FWD(128, true) : NNB_FWD(128, false));
+#undef NNB_FWD
   if (rc != 0) return rc;
   NNB_LAUNCH_OK("flash_fwd");
   return 0;
