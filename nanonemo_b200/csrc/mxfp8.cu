@@ -101,7 +101,7 @@ __device__ __forceinline__ void quant_block(const float (&v)[N], float amax, uin
 // (two lanes share a scale), and store them as one 128-byte line. Columns: a thread takes 32 rows of two neighbouring columns out of
 // shared memory (four-byte accesses, no bank conflicts) and writes each as one 32-byte store; the four lanes that have the same columns
 // fill a 128-byte line. When a warp wrote 64 different lines in halves of sectors, and two blocks were on an SM instead of three, bf16 8192 x 4096
-// took 38.6 us, now 29.1; 8192 x 11264 99 and 72 (the bytes alone 21 and 57); 1024 x 4096 in a row with itself 5.1 and 6.0.
+// took 32.6 us, now 29.1 (the bytes alone 21); 2048 x 4096 9.1 and 8.5, 1024 x 4096 6.5 and 5.95, 1024 x 2048 3.1 and 2.95.
 //
 // SRC: what the tile's values are. MX_PLAIN: x. MX_SWIGLU: silu(gate) * up of the projection gu = gate | up [R, 2 C]. MX_SWIGLU_BWD: the gradient
 // d(gate) | d(up) [R, C] of that projection (gu [R, C]) where x [R, C / 2] is the activation's; a tile is 64 columns of either half, which share the
