@@ -185,7 +185,7 @@ Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
 Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
   reachable({&x2, &w, &cos, &sin});
   const int64_t M = x2.size(0), K = x2.size(1), N = w.size(0);
-  if ((hd != 64 && hd != 128) || N % hd || rope_cols % hd) return Tensor();
+  if ((hd != 64 && hd != 128) || N % hd || rope_cols % hd || w.stride(1) != 1 || x2.stride(1) != 1) return Tensor();
   const int code = code16(x2.scalar_type());
   NNB_ASSERT(code > 0 && w.scalar_type() == x2.scalar_type(), "gemm_rope needs bf16 or fp16 operands of one dtype");
   Tensor out = empty({M, N}, x2.scalar_type(), x2);

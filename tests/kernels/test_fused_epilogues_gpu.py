@@ -291,6 +291,24 @@ def test_gemm_rope_epilogue_with_an_odd_number_of_rotated_heads(B, T, H, KVH, hd
     assert ((out.float() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-6 * pair).all()  # one rounding to bf16, fp32 arithmetic
 
 
+@pytest.mark.parametrize("rows", [100, 300, 10240])  # (both kernels with this epilogue)
+@pytest.mark.parametrize("hd", [64, 128])
+def test_rope_projections_of_strided_weights(rows, hd):
+    """16-bit weights whose columns lie apart: the epilogues take rows only, so another route has to serve; the result is that of the weight's copy."""
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+    from nanonemo_b200.ops.gemm import check_status, gemm_rope
+
+    torch.manual_seed(rows)
+    cos, sin = (t.contiguous() for t in rope_cache(hd, rows, device=DEV))
+    x, wide = torch.randn(1, rows, 192, device=DEV).bfloat16(), torch.randn(4 * hd, 384, device=DEV).bfloat16() * 0.05
+    with torch.no_grad():
+        for w in (wide[:, ::2], wide[:, :192], wide.t().contiguous()[:192].t()):
+            assert torch.equal(ops.qkv_rope_attention(x, w, cos, sin, 2, 1, hd), ops.qkv_rope_attention(x, w.contiguous(), cos, sin, 2, 1, hd))
+        assert gemm_rope(x[0], wide[:, ::2], cos, sin, rows, 3 * hd, hd) is None
+    check_status()
+
+
 def test_mlp_node_matches_unfused_composition():
     """The one-node feed-forward (SwiGLU backward inside the down projection's dgrad) against linear -> swiglu -> linear built
     from the separate operators, and against fp32 PyTorch: output, input gradient and both weight gradients."""
