@@ -131,6 +131,9 @@ Tensor dense_rows(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous
 Tensor empty(at::IntArrayRef size, at::ScalarType dt, const Tensor& like) { return at::empty(size, like.options().dtype(dt).requires_grad(false).memory_format(std::nullopt)); }
 
 // ------------------------------------------------------------------------------------------------ raw functions
+// (A kernel takes one of the two for both operands: it would read past the end of the shorter one.)
+void inner_dimensions(int64_t a, int64_t b) { NNB_ASSERT(a == b, "inner dimensions differ: " + std::to_string(a) + " vs " + std::to_string(b)); }
+
 Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, const optional<Tensor>& out_, optional<at::ScalarType> out_dtype, bool accumulate, int k_splits, int bn, int max_ctas) {
   a = rowmajor2d(std::move(a));
   b = rowmajor2d(std::move(b));
@@ -140,7 +143,7 @@ Tensor gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, const optional<Tensor>& ou
              std::string("gemm needs matching bf16/fp16 inputs, got ") + c10::toString(a.scalar_type()) + "/" + c10::toString(b.scalar_type()));
   const int64_t K = a_mn ? a.size(0) : a.size(1), M = a_mn ? a.size(1) : a.size(0);
   const int64_t Kb = b_mn ? b.size(0) : b.size(1), N = b_mn ? b.size(1) : b.size(0);
-  NNB_ASSERT(K == Kb, "inner dimensions differ: " + std::to_string(K) + " vs " + std::to_string(Kb));
+  inner_dimensions(K, Kb);
   const bool given = out_.has_value() && out_->defined();
   const at::ScalarType dt = out_dtype ? *out_dtype : given ? out_->scalar_type() : a.scalar_type();
   NNB_ASSERT(dt == a.scalar_type() || dt == at::kFloat, "gemm: the output is of the operands' dtype or fp32");
@@ -158,6 +161,7 @@ std::pair<Tensor, Tensor> gemm_swiglu(const Tensor& x2, const Tensor& w, bool ke
   reachable({&x2, &w});
   const int64_t M = x2.size(0), K = x2.size(1), F = w.size(0) / 2;
   if (M < 256 || F % 128 || w.stride(1) != 1 || x2.stride(1) != 1) return {};
+  inner_dimensions(K, w.size(1));
   Tensor gu = keep ? empty({M, 2 * F}, x2.scalar_type(), x2) : Tensor(), act = empty({M, F}, x2.scalar_type(), x2);
   const int code = code16(x2.scalar_type());
   NNB_ASSERT(code > 0 && w.scalar_type() == x2.scalar_type(), "gemm_swiglu needs bf16 or fp16 operands of one dtype");
@@ -175,6 +179,7 @@ Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
   if (M < 256 || F < 128 || F % 64 || gu.dim() != 2 || gu.size(0) != M || gu.size(1) != 2 * F || gu.stride(1) != 1 || gu.stride(0) % 8 || w.stride(1) != 1 ||
       dy.stride(1) != 1 || gu.scalar_type() != dy.scalar_type() || w.scalar_type() != dy.scalar_type())
     return Tensor();
+  inner_dimensions(K, w.size(0));
   const int code = code16(dy.scalar_type());
   NNB_ASSERT(code > 0, "gemm_swiglu_bwd needs bf16 or fp16 operands");
   Tensor dgu = empty({M, 2 * F}, gu.scalar_type(), gu);
@@ -185,6 +190,7 @@ Tensor gemm_swiglu_bwd(const Tensor& dy, const Tensor& w, const Tensor& gu) {
 Tensor gemm_rope(const Tensor& x2, const Tensor& w, const Tensor& cos, const Tensor& sin, int64_t t_len, int64_t rope_cols, int64_t hd) {
   reachable({&x2, &w, &cos, &sin});
   const int64_t M = x2.size(0), K = x2.size(1), N = w.size(0);
+  inner_dimensions(K, w.size(1));
   if ((hd != 64 && hd != 128) || N % hd || rope_cols % hd || w.stride(1) != 1 || x2.stride(1) != 1) return Tensor();
   const int code = code16(x2.scalar_type());
   NNB_ASSERT(code > 0 && w.scalar_type() == x2.scalar_type(), "gemm_rope needs bf16 or fp16 operands of one dtype");

@@ -309,6 +309,25 @@ def test_rope_projections_of_strided_weights(rows, hd):
     check_status()
 
 
+@pytest.mark.parametrize("rows", [100, 300, 10240])
+def test_fused_products_refuse_operands_that_do_not_fit(rows):
+    from nanonemo_b200 import ops
+    from nanonemo_b200.models.layers import rope_cache
+    from nanonemo_b200.ops.gemm import check_status, gemm_rope, gemm_swiglu, gemm_swiglu_bwd
+
+    cos, sin = (t.contiguous() for t in rope_cache(64, rows, device=DEV))
+    x, w = torch.randn(1, rows, 256, device=DEV).bfloat16(), torch.randn(256, 192, device=DEV).bfloat16()
+    with torch.no_grad():
+        calls = [lambda: ops.qkv_rope_attention(x, w, cos, sin, 2, 1, 64), lambda: ops.qkv_rope_attention(x, w.float(), cos, sin, 2, 1, 64),
+                 lambda: gemm_rope(x[0], w, cos, sin, rows, 192, 64), lambda: ops.mlp_swiglu(x, w, w)]
+        if rows >= 256:  # (these two serve from here on)
+            calls += [lambda: gemm_swiglu(x[0], w), lambda: gemm_swiglu_bwd(x[0], w[:192], torch.randn(rows, 384, device=DEV).bfloat16())]
+        for call in calls:
+            with pytest.raises(AssertionError, match="inner dimensions"):
+                call()
+    check_status()
+
+
 def test_mlp_node_matches_unfused_composition():
     """The one-node feed-forward (SwiGLU backward inside the down projection's dgrad) against linear -> swiglu -> linear built
     from the separate operators, and against fp32 PyTorch: output, input gradient and both weight gradients."""
