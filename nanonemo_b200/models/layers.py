@@ -192,7 +192,7 @@ class MLP(nn.Module):
             return self.tp.scatter_tokens(self.w_down(ops.swiglu_packed(self.w_gu(full), impl=self.act_impl)))
         if self.fused and x.is_cuda and ops.fused_ok():
             return ops.mlp_swiglu(x, self.w_gu.weight, self.w_down.weight)
-        if self.fused_mx and type(self.w_gu) is type(self.w_down) is Linear and _unwatched(self.w_gu, self.w_down):
+        if self.fused_mx and type(self.w_gu) is type(self.w_down) is Linear and self.w_gu.impl == self.w_down.impl == "mxfp8" and _unwatched(self.w_gu, self.w_down):
             y = fp8.mlp_mxfp8(x, self.w_gu.weight, self.w_down.weight)
             if y is not NotImplemented:
                 return y

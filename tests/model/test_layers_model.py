@@ -117,6 +117,31 @@ def test_mlp_identities():
     assert mlp(x).abs().max() == 0
 
 
+@pytest.mark.parametrize("watched", [None, "w_gu", "w_down"])
+def test_fp8_mlp_node_takes_the_place_of_fp8_linears_only(monkeypatch, watched):
+    """A linear layer that was given another implementation, or that somebody watches, runs on its own."""
+    from nanonemo_b200 import fp8
+
+    mlp = MLP(ModelConfig.sm100(n_layers=1, d_model=16, n_heads=2, n_kv_heads=1, d_ff=32, vocab_size=32, max_seq_len=8, head_dim_override=64, linear_impl="mxfp8"))
+    mlp.act_impl = "torch"
+    x, seen, node = torch.randn(2, 3, 16), [], []
+    monkeypatch.setattr(fp8, "mlp_mxfp8", lambda x, gu, down: node.append(1) or NotImplemented)
+    monkeypatch.setattr(ops, "linear", lambda x, w, impl: seen.append(impl) or F.linear(x, w))
+    mlp(x)
+    assert (node, seen) == ([1], ["mxfp8", "mxfp8"])
+    for name in ("w_gu", "w_down"):
+        node.clear(), seen.clear()
+        layer = getattr(mlp, name)
+        handle = layer.register_forward_hook(lambda *a: None) if watched == name else None
+        if watched is None:
+            layer.impl = "sm100"
+        mlp(x)
+        assert (len(node), seen) == (0 if watched in (None, name) else 1, ["sm100" if getattr(mlp, n).impl == "sm100" else "mxfp8" for n in ("w_gu", "w_down")])
+        layer.impl = "mxfp8"
+        if handle is not None:
+            handle.remove()
+
+
 def test_block_residual_stream_convention():
     torch.manual_seed(4)
     cfg = ModelConfig(**SMALL)
