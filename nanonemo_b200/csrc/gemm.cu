@@ -659,7 +659,7 @@ int gemm_impl(const void* A, const void* B, void* D, int M, int N, int K, long l
   // tiles fit one wave, where a tile's latency is all that counts: 1024 x 768 x 768 17 / 17 / 15, 1024 x 768 x 2048 26 / 26 / 22,
   // 1024 x 2048 x 5632 44 / 46 / 38; most of these now go to gemm_rows.cu (nnb_rows_tile).
   if (mode == 0 && bn_hint == 0 && !out_f32 && !a_mn && max_ctas <= 0) {
-    if (const int g = nnb_rows_tile(M, N, K, nnb_num_sms())) {
+    if (const int g = nnb_rows_tile(M, N, K, nnb_rows_on_lines(A, B, lda, ldb), nnb_num_sms())) {
       const int rc = nnb_gemm_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn, dtype, g, status, st);
       if (rc <= 0) return rc;  // 1 = operands not aligned for it
     }
@@ -830,7 +830,7 @@ extern "C" int nnb_gemm_swiglu_act(const void* X, const void* Wgu, void* ACT, in
 extern "C" int nnb_gemm_rope(const void* X, const void* W, void* QKV, const void* cos_t, const void* sin_t, int M, int N, int K,
                              long long lda, long long ldw, long long ldd, int t_len, int rope_cols, int head_dim, int dtype,
                              void* status, cudaStream_t st) {
-  if (const int tile = nnb_rows_tile(M, N, K, nnb_num_sms())) {
+  if (const int tile = nnb_rows_tile(M, N, K, nnb_rows_on_lines(X, W, lda, ldw), nnb_num_sms())) {
     const int rc = nnb_gemm_rows_rope(X, W, QKV, cos_t, sin_t, M, N, K, lda, ldw, ldd, t_len, rope_cols, head_dim, dtype, 0, head_dim == 64 ? 32 : tile, status, st);
     if (rc <= 0) return rc;
   }

@@ -1,5 +1,7 @@
 // Host entry of the CTA-pair GEMM (gemm2.cu); called by the dispatcher in gemm.cu.
 #pragma once
+#include <stdint.h>
+
 #include <cuda_runtime.h>
 
 // Work fused into the epilogue while a tile leaves tensor memory (see gemm2.cu).
@@ -41,17 +43,30 @@ int nnb_gemm2_launch(const NnbGemm2Args& a, cudaStream_t st);
 
 // The kernel for few rows (gemm_rows.cu): columns of its tile / 2 (32 or 64) for a product with a 16-bit output that it serves faster than the
 // persistent kernels, 0 otherwise. Its tiles are narrow and short-lived: a set-up of 2.3 us against 4 to 5, and the SMs that a few wide tiles
-// would leave idle; with more tiles than SMs it is bound by the bytes an SM takes in. us in a row of products with 24 weights, taken with four
-// epilogue warps (the eight it has are 0.3 us faster; pair kernel,
-// single-CTA kernel below 256 rows / 64-wide / 128-wide tiles): 201 x 768 x 768 6.5 / 4.5 / 6.2, 512 x 768 x 2048 13.9 / 8.0 / 10.9, 1024
-// x 768 x 4096 23.0 / 14.4 / 20.1, 512 x 2048 x 11264 54.9 / 39.3 / 56.7, 777 x 1280 x 768 8.1 / 4.9 / 6.4; more 64-wide tiles than SMs:
-// 1024 x 1280 x 768 8.2 / 6.7 / 6.6, 2048 x 768 x 2048 14.3 / 13.9 / 12.3, 512 x 4096 x 768 8.7 / 7.4 / 7.0, 2048 x 768 x 4096 23.2 / 26.1 /
-// 22.3, 1024 x 2048 x 5632 30.7 / 39.8 / 33.0; more 128-wide ones: 777 x 3072 x 2048 15.6 / 26.3 / 17.2, 4096 x 768 x 2048 15.3 / 27.1 / 19.0.
-inline int nnb_rows_tile(long long M, long long N, long long K, int sms) {
-  const long long m = (M + 127) / 128;
-  if (m * ((N + 63) / 64) <= sms) return 32;
-  if (m * ((N + 127) / 128) <= sms && K <= 4096) return 64;
-  return 0;
+// would leave idle; with more tiles than SMs it is bound by the bytes an SM takes in. us in a row of products with 24 weights, pair kernel (single-CTA
+// kernel below 256 rows) / 64-wide / 128-wide tiles: 201 x 768 x 768 6.4 / 4.25 / 5.65, 512 x 768 x 2048 13.9 / 7.8 / 10.5, 1024 x 768 x 4096 23.0 / 14.3 / 20.1,
+// 512 x 2048 x 11264 54.5 / 37.7 / 56.7, 777 x 1280 x 768 8.2 / 4.8 / 5.9; more 64-wide tiles than SMs: 1024 x 1280 x 768 8.1 / 6.8 / 6.2, 2048 x 768 x 2048
+// 14.4 / 13.7 / 11.9, 512 x 4096 x 768 8.75 / 7.6 / 6.6, 2048 x 768 x 4096 23.4 / 25.9 / 22.0, UNSERVED. Weights stored [K, N] (input gradients) within 0.3 us of these.
+// Three limits to that. `lines`: rows of both operands start at multiples of 128 bytes; others cost every row of a box two lines, which tiles with a long K
+// loop do not make good: 555 x 2896 x 2424 19.3 / 28.9 / 21.6 (512 x 2944 x 2432 16.3 / 16.2 / 13.7), 63 x 680 x 8920 46.8 / 49.9 / -; 2304 x 560 x 896 8.8 / 7.6 / 7.2.
+// Very wide weights, where 128-wide tiles lose: 16384 x 2048 with 32 to 100 rows 14.9 / - / 14.2, 7488 x 3008 17.1 / - / 17.7, 11264 x 4096 22.0 / - / 22.5, 18944 x 4096 29.7 / - / 32.6.
+// Fewest rows: an A of less than 128 KB is the same few lines of L2 for every CTA, and the more of them read it the longer that takes. 32 CTAs and more,
+// 1 to 12 rows: 2048 x 4096 19.9 / 18.2 / 20.1, 2048 x 5632 25.3 / 26.9 / 26.5, 3072 x 5632 25.8 / 29.6 / 27.2; 64 and more, where 128-wide tiles are half as many:
+// 4096 x 1024 7.8 / 6.4 / 6.1, 6144 x 1024 7.9 / 9.5 / 6.2, 9472 x 768 7.5 / 7.7 / 6.1, 4096 x 4096 20.1 / 24.8 / 20.4, 4096 x 5632 25.9 / 33.6 / 30.6,
+// 8192 x 2048 (stored [K, N]) 13.3 / 17.6 / 14.6; not on lines, 1904 x 3152 16.0 / 17.1 / 18.0, 1536 x 3152 15.9 / 12.0 / 17.9, 5048 x 792 7.5 / 8.9 / -. The same with 16 or 32 rows, A of
+// 128 KB or more: 4096 x 4096 20.2 / 14.7 / 20.4, 3072 x 5632 25.8 / 18.8 / 27.3.
+inline int nnb_rows_tile(long long M, long long N, long long K, bool lines, int sms) {
+  const long long m = (M + 127) / 128, weights = N * K;
+  const bool narrow = m * ((N + 63) / 64) <= sms && (lines || K <= 4096), wide = m * ((N + 127) / 128) <= sms && K <= (lines ? 4096 : 1024);
+  if (M * K < 1 << 16 && N >= 1600 && (weights > 1 << 22 || (N >= 4096 && !lines))) {
+    if (N < 4096) return narrow && lines && weights <= 1 << 23 ? 32 : 0;
+    return wide && K <= 1536 && weights < 1 << 24 ? 64 : 0;
+  }
+  return narrow ? 32 : wide && weights <= (K <= 2560 ? 1 << 25 : 1 << 24) ? 64 : 0;
+}
+// Row strides in elements of 16 bits
+inline bool nnb_rows_on_lines(const void* a, const void* w, long long lda, long long ldw) {
+  return lda % 64 == 0 && ldw % 64 == 0 && reinterpret_cast<uintptr_t>(a) % 128 == 0 && reinterpret_cast<uintptr_t>(w) % 128 == 0;
 }
 extern "C" int nnb_gemm_rows(const void*, const void*, void*, int, int, int, long long, long long, long long, int, int, int, void*, cudaStream_t);
 extern "C" int nnb_gemm_rows_rope(const void*, const void*, void*, const void*, const void*, int, int, int, long long, long long, long long, int, int, int, int, int, int, void*, cudaStream_t);

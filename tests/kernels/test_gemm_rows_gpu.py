@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 # rows and sizes at the edges of tiles (128 rows, 32 / 64 / 128 columns, 64 or 128 of K a stage) and of the rule that picks them
 SIZES = [(1, 8, 8), (17, 40, 72), (127, 264, 136), (128, 768, 2048), (129, 4096, 768), (201, 1280, 768), (255, 1000, 520), (300, 104, 64), (896, 1280, 768), (897, 1280, 768),
-         (2048, 768, 1024), (2100, 1104, 200)]
+         (2048, 768, 1024), (2100, 1104, 200),
+         # an A of less than 128 KB and one of as much, in front of weights of 2^23 and 2^24 elements and a few more; wide weights
+         (3, 2048, 4096), (3, 2048, 4104), (15, 4096, 4096), (16, 4096, 4096), (9, 4104, 2040), (31, 8192, 2048), (1, 9480, 1024), (64, 16384, 2048), (64, 16392, 2048)]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
