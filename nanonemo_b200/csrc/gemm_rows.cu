@@ -315,19 +315,18 @@ int launch_rows(const CUtensorMap& ta, const CUtensorMap& tw, RParams p, int til
 }  // namespace
 
 // Whether a product of M rows with an fp32 weight of N rows (kind 0; kind 1, SwiGLU: 2 N) and K columns is taken straight from it, and not from its cast.
-// GPU time, us in a row, straight from fp32 / cast + product: 201 x 768 x 2048 9.2 / 11.6, 512 x 768 x 2048 10.2 / 11.7; more tiles than
+// GPU time, us in a row, straight from fp32 / cast + product: 256 x 128 weights 2.7 / 4.5, 201 x 768 x 2048 9.2 / 11.6, 512 x 768 x 2048 10.2 / 11.7; more tiles than
 // SMs 201 x 4096 x 768 8.4 / 9.3, 512 x 2048 x 768 8.3 / 8.4, 512 x 1280 x 768 8.1 / 7.7, 777 x 768 x 1024 9.7 / 8.0, 512 x 2048 x 2048 17.4 / 13.9 (not served). Up to K = 1024 the second
 // wave is taken all the same: a cast costs the host of an eager call 5.5 us (10.0 / 15.5 us a forward call, whichever of these sizes) and few rows of a block
 // their one workspace (binding.cpp): scoring 512 tokens 964 us, 1002 with a line at one wave, 800 tokens 1021 and 1125. SwiGLU gains at every size that it
-// serves (201 x 2048 x 768 7.4 / 11.6). Fewest rows (nnb_rows_tile says why): 13 x 8304 x 856 17.9 / 14.8, 2 x 3040 x 4016 33.1 / 28.7; 1 x 4096 x 768 7.2 / 9.6. Weights below 2^17 elements are cast
-// as ever.
+// serves (201 x 2048 x 768 7.4 / 11.6). Fewest rows (nnb_rows_tile says why): 13 x 8304 x 856 17.9 / 14.8, 2 x 3040 x 4016 33.1 / 28.7; 1 x 4096 x 768 7.2 / 9.6.
 // Input gradients (kind 2: the weight has K rows and N columns), us in a row, from fp32 / cast + 64-wide tiles: 201 x 768 x 768 6.3 / 6.9, 201 x 2048
 // x 768 6.7 / 8.4, 777 x 768 x 768 6.7 / 7.0, 777 x 768 x 1280 9.5 / 9.1, 777 x 768 x 4096 26.7 / 20.1 (a stage waits for its 32 KB of weights to be
 // rounded).
 extern "C" int nnb_gemm_rows_f32w_serves(int M, int N, int K, int kind) {
   const long long sms = nnb_num_sms(), cols = kind == 2 ? 64 : kind == 1 ? 16 : 32, t = (long long)((M + BM - 1) / BM) * ((N + cols - 1) / cols);
   if (kind == 0 && (long long)M * K < 1 << 16 && ((long long)N * K > 1 << 22 || t > sms)) return 0;
-  return (kind == 2 ? t <= sms && K <= 1024 : t <= sms || (t <= 2 * sms && K <= 1024)) && (long long)(kind == 1 ? 2 * N : N) * K >= 1 << 17;
+  return kind == 2 ? t <= sms && K <= 1024 : t <= sms || (t <= 2 * sms && K <= 1024);
 }
 
 namespace {

@@ -66,15 +66,15 @@ def test_rope_and_swiglu_from_fp32_weights_are_the_unfused_operators(rows, T, hd
         assert torch.equal(z.view(-1, 768), gemm(act, down.to(dtype), bn=128))
 
 
-@pytest.mark.parametrize("n_out", [776, 1032])  # (the input gradient's K: up to 1024 straight from fp32)
+@pytest.mark.parametrize("n_out,n_in", [(776, 520), (1032, 520), (8, 8), (40, 72), (136, 64), (4104, 1032)])  # (the input gradient's K: up to 1024 straight from fp32)
 @pytest.mark.parametrize("rows", [1, 33, 201, 512, 4100])
-def test_linear_from_its_fp32_weight_and_its_gradients(rows, n_out):
+def test_linear_from_its_fp32_weight_and_its_gradients(rows, n_out, n_in):
     """With and without gradients, few rows and many: the product of the cast weight; gradients as from the cast weight, too."""
     from nanonemo_b200 import ops
     from nanonemo_b200.ops.gemm import gemm
 
     torch.manual_seed(rows)
-    x, w = torch.randn(rows, 520, device=DEV).bfloat16().requires_grad_(), (torch.randn(n_out, 520, device=DEV) * 0.05).requires_grad_()
+    x, w = torch.randn(rows, n_in, device=DEV).bfloat16().requires_grad_(), (torch.randn(n_out, n_in, device=DEV) * 0.05).requires_grad_()
     y = ops.linear(x, w, impl="sm100")
     w16 = w.detach().bfloat16()
     assert torch.equal(y, gemm(x.detach(), w16, bn=128))

@@ -362,16 +362,19 @@ def test_launches_are_counted_once():
     assert math.isfinite(y.float().sum().item())
 
 
+@pytest.mark.parametrize("direct", [True, False])
 @pytest.mark.parametrize("rows", [33, 201, 300])
-def test_calls_without_gradients_cast_no_more_than_the_registered_operators(python_route, rows):
-    """Each fp32 weight once, and the input: also where the fused kernel does not serve the rows and others take over."""
+def test_calls_without_gradients_cast_no_more_than_the_registered_operators(python_route, rows, direct):
+    """The input, and no fp32 weight that the kernels take as it is; others (here: not at a multiple of 16 bytes) once each, also where the fused kernel does
+    not serve the rows and others take over."""
     from torch.profiler import ProfilerActivity, profile
 
     from nanonemo_b200 import ops
     from nanonemo_b200.models.layers import rope_cache
 
     cos, sin = rope_cache(64, 512, device=DEV)
-    x, wq, gu, down = _rand(1, rows, 128, grad=False), _rand(256, 128), _rand(512, 128), _rand(128, 256)
+    weight = lambda *s: _rand(*s) if direct else _rand(s[0] * s[1] + 1)[1:].view(s)  # noqa: E731
+    x, wq, gu, down = _rand(1, rows, 128, grad=False), weight(256, 128), weight(512, 128), weight(128, 256)
 
     def casts(fn):
         with torch.no_grad():
@@ -381,7 +384,7 @@ def test_calls_without_gradients_cast_no_more_than_the_registered_operators(pyth
         return sum(e.count for e in p.key_averages() if e.key == "aten::_to_copy")
 
     for fn, weights in ((lambda: ops.mlp_swiglu(x, gu, down), 2), (lambda: ops.qkv_rope_attention(x, wq, cos, sin, 2, 1, 64), 1), (lambda: ops.linear(x, wq, impl="sm100"), 1)):
-        assert casts(fn) == weights + 1 <= python_route(lambda: casts(fn))  # noqa: B023
+        assert casts(fn) == 1 + (0 if direct else weights) <= python_route(lambda: casts(fn))  # noqa: B023
 
 
 def test_the_fused_swiglu_backward_can_be_switched_off_on_the_models_path(monkeypatch):
