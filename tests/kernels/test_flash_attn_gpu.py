@@ -79,6 +79,51 @@ def test_backward_of_a_grid_in_several_waves_is_that_of_its_sequences(B, T, hd):
     assert all(torch.isfinite(t).all() for t in got)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T", [(75, 65), (150, 1), (38, 129), (25, 300), (10, 1000)])
+def test_packed_backward_with_inverse_rope_of_a_grid_in_several_waves(B, T, dtype):
+    """What a training step calls: gradients of the packed projection before its rotation. Key tiles follow one another in a CTA, each with rotations of its
+    own: dK and dV of a sequence are the bits of a call of its own, and the rotated gradients of the same call without tables."""
+    from nanonemo_b200.models.layers import rope_cache
+    from nanonemo_b200.ops import rope
+    from nanonemo_b200.ops.attention import bwd_raw, fwd_raw
+    from nanonemo_b200.ops.gemm import check_status
+
+    torch.manual_seed(B + T)
+    H, KVH, hd = 4, 2, 64
+    heads, cols = (H, KVH, KVH), (H + 2 * KVH) * hd
+    cos, sin = (t.contiguous() for t in rope_cache(hd, T, device=DEV))
+    qkv, do = torch.randn(B, T, cols, device=DEV).to(dtype), torch.randn(B, T, H, hd, device=DEV).to(dtype)
+
+    def split(t):
+        return t.view(t.shape[0], T, -1, hd).split(heads, dim=2)
+
+    def backward(b0, b1, **tables):
+        at = slice(b0, b1)
+        o, g = torch.empty_like(do[at]), torch.full_like(qkv[at], float("nan"))
+        lse = fwd_raw(*split(qkv[at]), o, hd**-0.5)
+        bwd_raw(*split(qkv[at]), o, lse, do[at], *split(g), hd**-0.5, in_order=True, **tables)
+        check_status()
+        return g
+
+    tables = dict(rope_cos=cos, rope_sin=sin)
+    got, plain = backward(0, B, **tables), backward(0, B)
+    kv = H * hd
+    for b in sorted({0, 1, B // 3, B // 2, B - 2, B - 1}):
+        alone = backward(b, b + 1, **tables)
+        assert torch.equal(got[b : b + 1, :, kv:], alone[:, :, kv:])
+        torch.testing.assert_close(got[b : b + 1, :, :kv].float(), alone[:, :, :kv].float(), rtol=2**-7, atol=1e-5)  # (dQ: added in the order of arrival)
+    assert torch.equal(got[:, :, kv + KVH * hd :], plain[:, :, kv + KVH * hd :])  # dV is not rotated
+    ref = torch.empty_like(plain)
+    rope.rope_packed_raw(plain.view(B * T, cols), ref.view(B * T, cols), cos, sin, T, H + KVH, hd, KVH * hd, -1.0)
+    # rounded once, against once before and once after the rotation: half a unit of either partner, and half a unit of each result (dQ: its sums differ, too)
+    unit = 2**-8 if dtype == torch.bfloat16 else 2**-11
+    pair = plain.float().view(B * T, -1, 2, hd // 2).abs().sum(2, keepdim=True).expand(-1, -1, 2, -1).reshape(B, T, cols)
+    off = (got.float() - ref.float()).abs()
+    assert (off[:, :, kv:] <= (unit * (pair + ref.float().abs()) + 1e-6)[:, :, kv:]).all()
+    assert (off[:, :, :kv] <= (2 * unit * (pair + ref.float().abs()) + 1e-5)[:, :, :kv]).all()
+
+
 def test_future_keys_do_not_leak():
     from nanonemo_b200 import ops
 

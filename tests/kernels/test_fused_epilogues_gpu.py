@@ -86,7 +86,8 @@ def test_gemm_swiglu_declines_shapes_it_does_not_serve():
 
 
 @pytest.mark.parametrize("B,T,H,KVH,hd,K", [(2, 128, 4, 2, 64, 256), (3, 100, 12, 4, 64, 768), (2, 256, 16, 4, 128, 512),
-                                             (1, 384, 2, 1, 128, 64), (4, 64, 5, 5, 64, 136)])
+                                             (1, 384, 2, 1, 128, 64), (4, 64, 5, 5, 64, 136),
+                                             (9, 512, 12, 4, 64, 768), (5, 1000, 16, 4, 128, 512)])  # (these two: more tiles than gemm_rows.cu takes)
 def test_gemm_rope_epilogue(B, T, H, KVH, hd, K):
     from nanonemo_b200 import ops
     from nanonemo_b200.models.layers import rope_cache
@@ -271,7 +272,8 @@ def test_swiglu_epilogues_over_many_tiles_and_ragged_edges(M, F_, K):
         assert ((got.float() - ref).abs() <= bound).all()
 
 
-@pytest.mark.parametrize("B,T,H,KVH,hd", [(3, 333, 4, 1, 64), (70, 128, 2, 1, 64), (5, 257, 2, 1, 128)])
+@pytest.mark.parametrize("B,T,H,KVH,hd", [(3, 333, 4, 1, 64), (70, 128, 2, 1, 64), (5, 257, 2, 1, 128),
+                                          (26, 333, 4, 1, 64), (83, 128, 2, 1, 64), (40, 257, 2, 1, 128)])  # (the last three: the CTA-pair kernel)
 def test_gemm_rope_epilogue_with_an_odd_number_of_rotated_heads(B, T, H, KVH, hd):
     """The last rotated head shares its 128 columns with one that passes through; rows end inside a tile, tokens wrap inside one."""
     from nanonemo_b200 import ops

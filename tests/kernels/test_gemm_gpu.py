@@ -20,7 +20,8 @@ def _check(out, ref, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (128, 128, 128), (256, 512, 768), (384, 1280, 768), (130, 264, 72),
-                                   (1000, 768, 2048), (64, 64, 64), (4096, 768, 768), (2560, 20096, 64)])
+                                   (1000, 768, 2048), (64, 64, 64), (4096, 768, 768), (2560, 20096, 64),
+                                   (200, 20008, 72), (2600, 2064, 200), (3001, 1280, 776)])  # (the last five: more tiles than gemm_rows.cu takes)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_fprop_layout(M, N, K, dtype):
     from nanonemo_b200.ops.gemm import check_status, gemm
@@ -33,7 +34,7 @@ def test_fprop_layout(M, N, K, dtype):
     _check(out, _ref(a, b, False, False), K)
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 768, 1280), (384, 2048, 768), (200, 136, 264)])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 768, 1280), (384, 2048, 768), (200, 136, 264), (200, 20008, 72), (2600, 2064, 200), (3001, 1280, 776)])
 def test_dgrad_layout(M, N, K):
     from nanonemo_b200.ops.gemm import check_status, gemm
 

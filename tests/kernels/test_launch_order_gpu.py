@@ -67,7 +67,7 @@ def _same(got, ref):
         assert torch.equal(a, b) if a.dtype != torch.float32 else torch.allclose(a, b, rtol=1e-5, atol=1e-5)
 
 
-@pytest.mark.parametrize("rows", [64, 200, 512])
+@pytest.mark.parametrize("rows", [64, 200, 512, 9600])  # (the last one: the projection by the CTA-pair kernel)
 def test_dependent_kernels_see_what_their_predecessors_wrote(rows):
     ref = _chain(rows, torch.cuda.synchronize)()
     run = _chain(rows, lambda: None)

@@ -455,8 +455,12 @@ def test_a_block_without_gradients_is_its_operators_in_one_call(monkeypatch, B, 
     """The same bits, few rows (one workspace) and many, with and without a pending delta; parts that are watched run one by one."""
     from contextlib import nullcontext
 
+    from torch.profiler import ProfilerActivity, profile
+
+    from nanonemo_b200 import ops
     from nanonemo_b200.models.config import ModelConfig
     from nanonemo_b200.models.layers import Block, rope_cache
+    from nanonemo_b200.ops import _lib
     from nanonemo_b200.ops.gemm import check_status
 
     torch.manual_seed(B * T)
@@ -469,10 +473,17 @@ def test_a_block_without_gradients_is_its_operators_in_one_call(monkeypatch, B, 
         with torch.no_grad(), torch.autocast("cuda", dtype=dtype) if dtype else nullcontext():
             return block(x, cos, sin, d)
 
-    assert block._one_call() or dtype is None
+    answers, in_one = [], ops.decoder_block
+    monkeypatch.setattr(ops, "decoder_block", lambda *a: answers.append(in_one(*a)) or answers[-1])
     for d in (None, delta):
-        got = run(d)
+        before = _lib.LAUNCHES
+        with profile(activities=[ProfilerActivity.CPU]) as p:
+            got = run(d)
         check_status()
+        assert _lib.LAUNCHES - before == 7 and len(answers) == 1 and answers.pop() is not NotImplemented
+        # few rows with an output in the compute type (without autocast and a delta it is that of x, fp32): one workspace and the two results
+        allocated = sum(e.count for e in p.key_averages() if e.key.startswith("aten::empty"))
+        assert (allocated == 3) == (B * T <= 201 and (dtype is not None or d is not None)), allocated
         with monkeypatch.context() as m:
             m.setattr(Block, "_one_call", lambda self: False)
             ref = run(d)
