@@ -2,7 +2,7 @@
 a few hundred MB, so an `ncu --set full` capture ends by itself in about a minute.
 
     python benchmarks/kernels/ncu_target.py {gemm,gemm_single,gemm_mxfp8,gemm_swiglu,gemm_swiglu_bwd,gemm_rope,gemm_swiglu_act,
-                                             gemm_wgrad,flash,flash128,rmsnorm,rmsnorm_wide,swiglu,rope,ce,ce_loss,adamw,embedding,quantize}[,more targets] [iters]
+                                             gemm_wgrad,flash,flash128,rmsnorm,rmsnorm_wide,swiglu,rope,ce,ce_loss,adamw,embedding,quantize,swiglu_mx,rows}[,more targets] [iters]
 """
 
 import sys
@@ -73,6 +73,30 @@ def build(kind: str):
 
         x = torch.randn(M, 2048, device=dev, dtype=bf)
         fn = lambda: fp8.quantize_mx(x, True, True)  # one read -> row-wise e4m3 copy + transposed copy + both scale sets
+    elif kind == "swiglu_mx":
+        from nanonemo_b200.ops import _lib
+
+        gu, dact = torch.randn(M, 4096, device=dev, dtype=bf), torch.randn(M, 2048, device=dev, dtype=bf)
+        n = _lib.native()
+        fn = lambda: (n.swiglu_mx(gu, True, True), n.swiglu_bwd_mx(dact, gu, True, True))  # SwiGLU and its backward inside the quantiser
+    elif kind == "rows":
+        # scoring a text of 201 tokens: products of a block straight from its fp32 weights, 24 blocks of them (more than L2)
+        from nanonemo_b200.models.layers import rope_cache
+        from nanonemo_b200.ops.gemm import gemm
+
+        cos, sin = rope_cache(64, 1024, device=dev)
+        x, x16, weights = torch.randn(1, 201, 768, device=dev), torch.randn(201, 768, device=dev, dtype=bf), []
+        for _ in range(24):
+            weights.append([torch.randn(*s, device=dev) * 0.05 for s in ((1280, 768), (768, 768), (4096, 768), (768, 2048))])
+        turn = iter(range(10**9))
+
+        @torch.no_grad()
+        def fn():
+            wqkv, wo, gu, down = weights[next(turn) % 24]
+            ops.qkv_rope_attention(x, wqkv, cos, sin, 12, 4, 64)
+            ops.linear(x, wo, impl="sm100")
+            ops.mlp_swiglu(x, gu, down)
+            gemm(x16, wo.to(bf))  # 16-bit weight, 64-wide tiles
     elif kind == "flash128":
         qkv = torch.randn(4, 2048, 24 * 128, device=dev, dtype=bf, requires_grad=True)
         fn = lambda: ops.attention_packed(qkv, 16, 4, 128, impl="sm100").sum().backward()
