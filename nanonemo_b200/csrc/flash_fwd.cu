@@ -115,6 +115,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int kv_total = (p.T + BN - 1) / BN;
   auto query_tile = [&](int z) { return p.n_q_tiles - 1 - z; };
   auto kv_tiles = [&](int qt) { return min(((qt + 1) * BQ + BN - 1) / BN, kv_total); };  // KV tiles holding keys <= the tile's last row
+  const int group = p.H / p.KVH, first_kvh = blockIdx.x / group;  // (divisions: not on the way to the first load)
   // Item i + 1 is the answer in slot i & 1, read by the MMA warp, the four softmax warps and the producer.
   constexpr int kNextReaders = 32 + 4;  // lanes of the MMA warp, each for itself, and softmax warps (not the producer, who writes the slot again)
   auto next_item = [&](int i, int& x, int& y, int& z) { return taken_block(answers + 16 * (i & 1), x, y, z); };
@@ -148,11 +149,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int h = blockIdx.x, b = blockIdx.y, z = blockIdx.z;
+      int h = blockIdx.x, b = blockIdx.y, z = blockIdx.z, kvh = first_kvh;
       uint32_t s = 0, ph = 0;  // ring position and phase of the next K and V tile, counted along over all items
       bool ok = true;
       for (int i = 0;; ++i) {
-        const int qt = query_tile(z), kvh = h / (p.H / p.KVH), n_kv = kv_tiles(qt);
+        const int qt = query_tile(z), n_kv = kv_tiles(qt);
         const int qs = i % C::kItems;
         if (TAKE) ok = mbar_wait(bar_qe + 8 * qs, ((i / C::kItems) & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -182,6 +183,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         ok = mbar_wait(bar_nf + 8 * (i & 1), (i >> 1) & 1, never_set);
         if (!ok) *abort_flag = 1;
         if (!ok || !next_item(i, h, b, z)) break;
+        kvh = h / group;
       }
       if (!ok) fail_role = 1;
       nnb_release_next();
