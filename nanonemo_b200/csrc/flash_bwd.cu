@@ -37,6 +37,9 @@
 // loads, the first visit's latencies, the epilogue and its store, as long as three visits and with an SM to itself. Whole backward in a
 // row (the card's power limit included), us, a CTA per item / items in sequence: B200 T64 85.9 / 74.9, B64 T300 131.5 / 119.5, B64
 // T512 222 / 203, B16 T1024 147 / 133, B32 T1024 315 / 293, B8 T4096 810 / 748.
+// A grid of one wave has an instance of its own, whose compute warps, free when the visits are over, store dV and dK side by side: one after the
+// other in the four drain warps they took longer than a CTA per item had. 8/8 heads, us, a CTA per item / drain warps / compute warps: B1 T64 9.4 / 9.8 / 9.3,
+// B2 T100 9.7 / 10.1 / 9.6, B16 T128 13.1 / 13.3 / 12.8, B4 T512 18.2 / 17.8 / 17.1.
 // All waits are bounded, except two: the register hand-over, which the launcher checks before it can start (nnb_flash_bwd_registers), and, in a
 // cluster, the two barriers of all its threads at the end, which every role of every CTA reaches, after a wait that ran out too.
 #include <cstdlib>
@@ -90,12 +93,12 @@ struct BParams {
   const float* rope_sin;
   // A cluster of `split` CTAs shares one key tile: each takes a part of its visits, and they add up their dK and dV at the end.
   int split;
-  int take;                               // the grid has more blocks than SMs: blocks take over others (see flash_fwd.cu)
   void *dk, *dv;                          // split > 1: written directly, strides as the launcher's
   long long dk_sb, dk_st, dk_sh, dv_sb, dv_st, dv_sh;
 };
 
-template <bool F16, bool SPLIT = false>
+// SPLIT: a cluster shares a key tile (BParams). TAKE: the grid has more blocks than SMs, and blocks take over others (see flash_fwd.cu); never both.
+template <bool F16, bool SPLIT = false, bool TAKE = false>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -187,6 +190,20 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   };
 
+  // a row of 64 fp32 values, rounded, into a 16-bit tile
+  auto stage16 = [&](uint8_t* row_at, int sw, const uint32_t (&r0)[32], const uint32_t (&r1)[32]) {
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) {
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = (jj & 3) * 8 + 2 * e;
+        w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
+      }
+      *reinterpret_cast<uint4*>(row_at + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  };
+
   if (warp < kDrainWarp0) {
     regs_dec<kRegsIssue>();
     if (warp == 0 && lane == 0 && aligned) {
@@ -211,7 +228,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tma_load_4d(dst + kTile16, &tmdO, bar_qf + 8 * s, 0, hq, qt * BQ, it.b);
           if (++s == kStagesQ) { s = 0; ph ^= 1; }
         }
-        if (SPLIT || !p.take || !ok) break;
+        if (!TAKE || !ok) break;
         // the next item: asked for when the last operands are on their way, not earlier (the longest CTA would take it)
         ok = mbar_wait(bar_ne + 8 * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -280,7 +297,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tc_fence_after();
           issue_s(n + 1, nxt, sK);
           s_next = true;
-        } else if (SPLIT || !p.take) {
+        } else if (!TAKE) {
           known = true;
         } else if (mbar_test_warp(bar_nf + 8 * (item & 1), (item >> 1) & 1)) {  // the next item, if it is there already: else after this visit's products
           known = true;
@@ -372,7 +389,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
           mbar_arrive(bar_lf + 8 * (n & 1));
         }
-        if (SPLIT || !p.take) break;
+        if (!TAKE) break;
         ok = ok && next_known(k, abort_flag);
         if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }  // (the lanes leave together)
         if (!next_item(k, it)) break;
@@ -422,15 +439,14 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (++qt == p.n_q_tiles) { qt = it.first_qt; ++hq; }
       }
       if (left) { fail_role = 4; break; }
-      if constexpr (SPLIT) break;
+      if (!TAKE) break;
       // The item's dV and dK: TMEM -> 16-bit tiles in the staging tile's place -> TMA store, while the other roles are in the next item
-      bool ok = mbar_wait(bar_fin, k & 1, abort_flag);
-      if (p.take) ok = ok && next_known(k, abort_flag);
+      const bool ok = mbar_wait(bar_fin, k & 1, abort_flag) && next_known(k, abort_flag);
       tc_fence_after();
       if (leader) tma_wait_group_read<0>();
       if (named_barrier_or(1, kDrainThreads, !ok)) { fail_role = 4; break; }
       Item next = it;
-      const bool more = p.take && next_item(k, next);
+      const bool more = next_item(k, next);
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
         uint32_t r0[32], r1[32];
@@ -442,16 +458,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           mbar_arrive(bar_acc);
           if (p.rope_cos != nullptr && it.kt * BKV + row < p.T) unrotate(r0, r1, it.kt * BKV + row);
         }
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = (jj & 3) * 8 + 2 * e;
-            w[e] = pack2_16<F16>(__uint_as_float(jj < 4 ? r0[i] : r1[i]), __uint_as_float(jj < 4 ? r0[i + 1] : r1[i + 1]));
-          }
-          *reinterpret_cast<uint4*>(my_stage + which * kTile16 + ((jj ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
+        stage16(my_stage + which * kTile16, sw, r0, r1);
       }
       fence_proxy_async_smem();
       named_barrier_sync(1, kDrainThreads);
@@ -567,13 +574,35 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive(bar_ds);
         NNB_PROF_ADD(3);
       }
-      if (SPLIT || !p.take) break;
+      if (!TAKE) break;
       ok = ok && next_known(k, abort_flag);
       if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }  // (the lanes leave together)
       if (!next_item(k, it)) break;
     }
     NNB_PROF_FLUSH_N(n);
     if (!ok) fail_role = 3;
+    if constexpr (!SPLIT && !TAKE) {  // Nothing follows the CTA's one item: these warps are free, and do dV (half 0) and dK (half 1) at the same time
+      ok = ok && mbar_wait(bar_fin, 0, abort_flag);
+      tc_fence_after();
+      if (named_barrier_or(2, kComputeThreads, !ok)) {  // all leave together
+        fail_role = 3;
+      } else {
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK), r0);
+        tmem_ld_32x32b_x32(t_lane + (half == 0 ? kColdV : kColdK) + 32, r1);
+        tmem_ld_wait();
+        if (half == 1 && p.rope_cos != nullptr && it.kt * BKV + row < p.T) unrotate(r0, r1, it.kt * BKV + row);
+        stage16(my_ds, sw, r0, r1);  // (every product that read dS^T is complete)
+        fence_proxy_async_smem();
+        named_barrier_sync(2, kComputeThreads);
+        if (half == 0 && row == 0) {
+          tma_store_4d(&tmdV, s_base + kOffdS, 0, it.kvh, it.kt * BKV, it.b);
+          tma_store_4d(&tmdK, s_base + kOffdS + kTile16, 0, it.kvh, it.kt * BKV, it.b);
+          tma_commit_group();
+          tma_wait_group<0>();
+        }
+      }
+    }
     if constexpr (SPLIT) {
       // dV (half 0) and dK (half 1) of this CTA's visits: TMEM -> fp32 tiles in the ring, which every CTA of the cluster then reads for the rows it
       // adds up and stores
@@ -734,7 +763,7 @@ extern "C" int nnb_flash_bwd_split(int T, int query_rows, long long kv_heads, in
 
 template <bool F16>
 static int configure_bwd() {
-  for (auto kernel : {flash_bwd_kernel<F16>, flash_bwd_kernel<F16, true>}) {
+  for (auto kernel : {flash_bwd_kernel<F16>, flash_bwd_kernel<F16, true>, flash_bwd_kernel<F16, false, true>}) {
     cudaFuncAttributes a;
     if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) {
@@ -824,10 +853,12 @@ extern "C" int nnb_flash_bwd(const void* q, const void* k, const void* v, const 
   p.dk = dk; p.dk_sb = dk_sb; p.dk_st = dk_st; p.dk_sh = dk_sh;
   p.dv = dv; p.dv_sb = dv_sb; p.dv_st = dv_st; p.dv_sh = dv_sh;
   dim3 grid(KVH * p.split, B, (T + BKV - 1) / BKV);
-  p.take = p.split == 1 && (long long)KVH * B * grid.z > nnb_num_sms();
+  // A grid that runs at once has nothing to take over: its instance leaves dV and dK to the compute warps, which have nothing to do by then.
+  const bool take = (long long)KVH * B * grid.z > nnb_num_sms();
   if (p.split > 1)
     nnb_launch_clusters(f16 ? flash_bwd_kernel<true, true> : flash_bwd_kernel<false, true>, p.split, grid, kThreads, kSmem, st, tq, tk, tv, tdo, tdq, tdk, tdv, p);
   // (full grids in plain stream order: an early start measured the same, B32 H12/4 T1024 285-287 us in either form, B128 T256 178-180 / 180)
+  else if (take) (f16 ? flash_bwd_kernel<true, false, true> : flash_bwd_kernel<false, false, true>)<<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
   else if (f16) flash_bwd_kernel<true><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
   else flash_bwd_kernel<false><<<grid, kThreads, kSmem, st>>>(tq, tk, tv, tdo, tdq, tdk, tdv, p);
   NNB_LAUNCH_OK("flash_bwd");
